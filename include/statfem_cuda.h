@@ -454,9 +454,11 @@ int32_t sfc_system_set_mpnn(sfc_system_t *sys, sfc_mpnn_t *net);
  * (0: 8; the largest size the device can co-schedule is used).
  * One sfc_batch_run assembles all instances (coefficients from
  * sfc_batch_set_coefficients, one value per element of the union mesh) and
- * runs one persistent kernel, captured once in a CUDA graph, that solves the
- * ns adjoint systems of every instance (FP32 block PCG, FP64 residual
- * refinement to the relative residual tol), forms mean and C_s at the
+ * replays a captured CUDA graph that solves the ns adjoint systems of every
+ * instance to the relative residual tol (FP64 block elimination along the
+ * grid lines where the mesh couples neighbouring lines only and max_iter is
+ * at least 32 per line; FP32 block PCG with FP64 residual refinement
+ * otherwise, or where the elimination misses tol), forms mean and C_s at the
  * sensors (C_s with the Kronecker-factored forcing covariance) and evaluates
  * the log-likelihood and the posterior mean / covariance at the sensors in
  * FP64.  Per-instance status: SFC_OK, SFC_ERR_NOT_CONVERGED or
@@ -490,7 +492,8 @@ int32_t sfc_batch_run(sfc_batch_t *batch);
 int32_t sfc_batch_autotune(sfc_batch_t *batch, int32_t remeasure, int32_t *cluster);
 /* Host copies of the last run's results (any pointer may be NULL):
  * loglik (n), mean_s (n x 32), cov_s (n x 32 x 32), post_mean (n x 32),
- * post_cov (n x 32 x 32), status (n), iterations (n, inner iterations). */
+ * post_cov (n x 32 x 32), status (n), iterations (n, inner PCG
+ * iterations; 0 where the elimination met tol). */
 int32_t sfc_batch_results(sfc_batch_t *batch, double *loglik, double *mean_s, double *cov_s,
                           double *post_mean, double *post_cov, int32_t *status, int32_t *iterations);
 

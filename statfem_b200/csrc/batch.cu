@@ -25,7 +25,10 @@
 // reductions go through distributed shared memory and cluster barriers, the
 // only waits in the kernel (hardware barriers among co-scheduled CTAs).
 //
-// Solve: FP32 block Jacobi-PCG inner iterations; at the start of each cycle
+// Solve: the direct elimination of btd.cu where the pattern allows it (a grid
+// line couples to its two neighbours only), whose solution is checked here
+// against the true residual and iterated on if it misses tol; else, and then:
+// FP32 block Jacobi-PCG inner iterations; at the start of each cycle
 // the FP64 residual b - S x64 replaces the recurrence residual (reliable
 // update: the search direction is kept unless the recurrence drifted);
 // converged columns are frozen; the instance stops when every column meets
@@ -50,6 +53,7 @@
 #include <numeric>
 #include <vector>
 
+#include "btd.cuh"
 #include "common.cuh"
 
 namespace cg = cooperative_groups;
@@ -89,6 +93,7 @@ struct BatchArgs {
     // controls
     double tol, itol;
     int max_iter, max_cycles;
+    int warm;  // x64 holds the direct solution (btd.cu)
     // outputs
     double *loglik, *mean_s, *cov_s, *pmean, *pcov;
     int *status, *iters;
@@ -213,7 +218,12 @@ __device__ void warp_trsm(const double *L, double *X, int n, int m)
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(BT, 4) k_batch(BatchArgs a)
+// OCC: CTAs per SM.  Four (64 registers) where the iterations dominate, which
+// wait on their operands' loads; two (128 registers) behind the direct solve,
+// where the statistics' register tiles bound it (40 instances of sides 32 to
+// 150: 3.5 -> 2.1 ms).
+template <int OCC>
+__global__ void __launch_bounds__(BT, OCC) k_batch(BatchArgs a)
 {
     cg::cluster_group cl = cg::this_cluster();
     const unsigned CS = cl.num_blocks(), rank = cl.block_rank();
@@ -253,8 +263,9 @@ __global__ void __launch_bounds__(BT, 4) k_batch(BatchArgs a)
         float4 *X4 = reinterpret_cast<float4 *>(a.x32), *R4 = reinterpret_cast<float4 *>(a.r32);
         float4 *P4 = reinterpret_cast<float4 *>(a.p32), *Q4 = reinterpret_cast<float4 *>(a.q32);
         // right-hand sides b = P^T, dense in W (W is free until the statistics)
+        bool warm = a.warm != 0;
         for (int64_t i = my0 + warp; i < my1; i += BW) {
-            a.x64[i * BK + lane] = 0.0;
+            if (!warm) a.x64[i * BK + lane] = 0.0;
             a.W[i * BK + lane] = 0.0;
         }
         cluster_barrier(cl);
@@ -276,7 +287,7 @@ __global__ void __launch_bounds__(BT, 4) k_batch(BatchArgs a)
                 const double2 b01 = b2[0], b23 = b2[1];
                 double r[4] = {b01.x, b01.y, b23.x, b23.y};
                 const double bv[4] = {b01.x, b01.y, b23.x, b23.y};
-                if (cycle > 0)
+                if (cycle > 0 || warm)
                     for (int32_t k = a.rp[i]; k < a.rp[i + 1]; ++k) {
                         const double av = a.a64[k];
                         const double2 *x2 = reinterpret_cast<const double2 *>(a.x64 + (int64_t)a.col[k] * BK + 4 * fl);
@@ -296,13 +307,23 @@ __global__ void __launch_bounds__(BT, 4) k_batch(BatchArgs a)
             }
             cluster_sum_q(cl, s, slot, prr, pbb);
             double rr0[4], bb[4];
-            bool done[4], bad = false;
+            bool done[4], bad = false, lost = false;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 rr0[q] = s.sres[4 * fl + q];
                 bb[q] = s.sres[32 + 4 * fl + q];
                 bad = bad || !(rr0[q] == rr0[q]) || !(bb[q] == bb[q]);
                 done[q] = bb[q] == 0.0 || rr0[q] <= a.tol * a.tol * bb[q];
+                lost = lost || !(rr0[q] <= bb[q]);
+            }
+            if (warm && cycle == 0 && __any_sync(0xffffffffu, lost)) {
+                // a matrix the direct elimination cannot take (not positive
+                // definite, not finite): from zero, as without it
+                warm = false;
+                for (int64_t i = my0 + warp; i < my1; i += BW) a.x64[i * BK + lane] = 0.0;
+                cluster_barrier(cl);
+                cycle = -1;
+                continue;
             }
             if (__any_sync(0xffffffffu, bad)) {
                 status = SFC_ERR_NOT_SPD;
@@ -493,24 +514,42 @@ __global__ void __launch_bounds__(BT, 4) k_batch(BatchArgs a)
         }
         cluster_sum2(cl, s, slot, pu, 0.0);  // also publishes W to the cluster
         if (threadIdx.x < 32) s.sub[threadIdx.x] = s.sres[threadIdx.x];
-        // x pass: T[a][b] = sum_b' k1d[|b - b'|] W[a][b']
-        for (int64_t i = my0 + warp; i < my1; i += BW) {
-            const int ra = (int)((i - r0) / m), b = (int)((i - r0) % m);
-            const double *wl = a.W + (r0 + (int64_t)ra * m) * BK + lane;
-            double acc = 0.0;
-            for (int b2 = 0; b2 < m; ++b2) acc += s.k1d[abs(b - b2)] * wl[(int64_t)b2 * BK];
-            a.T[i * BK + lane] = acc;
-        }
+        // T = (I (x) Kx) W, then Z = (Ky (x) I) T, Z into x64 (R^T is no longer
+        // needed).  A warp takes eight outputs along the axis: eight loads of
+        // the operand and 15 of the factor feed 64 multiply-adds per lane
+        // (one output per warp took two loads per multiply-add: this
+        // kernel 4.9 ms for 40 instances of sides 32 to 150, 2.1 ms so with
+        // the registers it needs).
+        auto axis = [&](const double *in, double *out, int64_t step, int64_t line_step) {
+            const int nblk = (m + 7) / 8;
+            for (int u = (int)rank * BW + warp; u < m * nblk; u += (int)CS * BW) {
+                const int o0 = (u % nblk) * 8;
+                const int64_t base = (r0 + (u / nblk) * line_step) * BK + lane;
+                const double *src = in + base;
+                double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                for (int i0 = 0; i0 < m; i0 += 8) {
+                    double w[8], kr[15];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) w[i] = i0 + i < m ? src[(i0 + i) * step * BK] : 0.0;
+#pragma unroll
+                    for (int t = 0; t < 15; ++t) {
+                        const int d = abs(o0 - i0 + t - 7);
+                        kr[t] = d < m ? s.k1d[d] : 0.0;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) acc[j] += kr[j - i + 7] * w[i];
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (o0 + j < m) out[base + (o0 + j) * step * BK] = acc[j];
+            }
+        };
+        axis(a.W, a.T, 1, m);
         cluster_barrier(cl);
-        // y pass: Z[a][b] = sum_a' k1d[|a - a'|] T[a'][b], into x64 (R^T is no longer needed)
-        for (int64_t i = my0 + warp; i < my1; i += BW) {
-            const int ra = (int)((i - r0) / m), b = (int)((i - r0) % m);
-            const double *tl = a.T + (r0 + b) * BK + lane;
-            double acc = 0.0;
-            for (int a2 = 0; a2 < m; ++a2) acc += s.k1d[abs(ra - a2)] * tl[(int64_t)a2 * m * BK];
-            a.x64[i * BK + lane] = acc;
-        }
-        __syncthreads();
+        axis(a.T, a.x64, m, 1);
+        cluster_barrier(cl);
         // C_s partial = W^T Z over this CTA's rows, 32-row tiles
         {
             double acc[4] = {0.0, 0.0, 0.0, 0.0};
@@ -664,6 +703,7 @@ struct sfc_batch {
     sfc::DBuf<float> x32, r32, p32, q32;
     sfc::DBuf<uint32_t> bc_idx;
     bool have_y = false, have_hp = false;
+    sfc::BtdPlan btd;  // direct solve of the instances' grids
     // launch
     int cluster = 0, grid = 0;
     size_t smem = 0;
@@ -692,6 +732,12 @@ void batch_release_graph(sfc_batch *b)
     b->graph = nullptr;
 }
 
+// The direct solve (btd.cu) is used where the pattern allows it.  A cap on the
+// iterations asks for an early stop of the iterative solve: Jacobi-PCG takes
+// at most about 10 iterations per grid line to 1e-12 (measured 900 at side
+// 150), so a cap above 32 per line never stops it and below it is kept.
+bool batch_direct(const sfc_batch *b) { return b->btd.usable && b->max_iter >= 32 * (b->smax + 1); }
+
 size_t batch_smem(int smax)
 {
     const int k1d = ((smax + 1) + 1) & ~1;
@@ -700,11 +746,19 @@ size_t batch_smem(int smax)
 
 // cluster size and persistent grid: the largest cluster size (of those
 // tried, in preference order) that the device can co-schedule
+using BatchKernel = void (*)(BatchArgs);
+
+BatchKernel batch_kernel(const sfc_batch *b)
+{
+    return batch_direct(b) ? k_batch<2> : k_batch<4>;
+}
+
 void batch_configure(sfc_batch *b, int want_cluster)
 {
+    const BatchKernel kernel = batch_kernel(b);
     const size_t smem = batch_smem(b->smax);
-    SFC_CK(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SFC_CK(cudaFuncSetAttribute(k_batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     const int tries[] = {want_cluster, 8, 4, 2, 1};
     for (int cs : tries) {
         if (cs < 1 || cs > 16) continue;
@@ -720,7 +774,7 @@ void batch_configure(sfc_batch *b, int want_cluster)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int nclusters = 0;
-        cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, k_batch, &cfg);
+        cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, kernel, &cfg);
         if (e != cudaSuccess) {
             cudaGetLastError();
             continue;
@@ -749,7 +803,19 @@ void batch_launch(sfc_batch *b, cudaStream_t st)
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    SFC_CK(cudaLaunchKernelEx(&cfg, k_batch, b->args));
+    SFC_CK(cudaLaunchKernelEx(&cfg, batch_kernel(b), b->args));
+}
+
+// dense right-hand sides W = P^T of the instances (W zeroed before)
+__global__ void k_batch_rhs(BatchArgs a)
+{
+    const int inst = blockIdx.x, c = threadIdx.x;
+    if (c >= a.ns[inst]) return;
+    const int64_t r0 = a.row0[inst], r1 = a.row0[inst + 1];
+    for (int k = 0; k < 3; ++k) {
+        const int64_t d = a.sdof[((int64_t)inst * BK + c) * 3 + k];
+        if (d >= r0 && d < r1) a.W[d * BK + c] += a.sw[((int64_t)inst * BK + c) * 3 + k];
+    }
 }
 
 __global__ void k_zero_at(double *v, const uint32_t *idx, int64_t n)
@@ -812,6 +878,7 @@ void batch_build_args(sfc_batch *b)
     a.itol = b->itol;
     a.max_iter = b->max_iter;
     a.max_cycles = b->max_cycles;
+    a.warm = batch_direct(b);
     a.loglik = b->loglik.p;
     a.mean_s = b->mean_s.p;
     a.cov_s = b->cov_s.p;
@@ -832,6 +899,16 @@ void batch_capture(sfc_batch *b)
     if (e == cudaSuccess) {
         cudaMemsetAsync(b->queue.p, 0, sizeof(int), st);
         try {
+            if (b->args.warm) {
+                SFC_CK(cudaMemsetAsync(b->W.p, 0, b->sys->N * BK * sizeof(double), st));
+                k_batch_rhs<<<b->n, BK, 0, st>>>(b->args);
+                SFC_CK(cudaGetLastError());
+                BtdArgs d = btd_args(b->btd, b->args.rp, b->args.col, b->args.a64);
+                d.B = b->W.p;
+                d.U = b->x64.p;
+                d.ld = d.ncols = BK;
+                btd_launch_batch(b->ctx, b->btd, d, st);
+            }
             batch_launch(b, st);
         } catch (const Error &) {
             cudaGraph_t g;
@@ -860,7 +937,7 @@ void batch_run(sfc_batch *b)
     if (!b->gexec) batch_capture(b);
     ProfScope ps(ctx, "phase:batch_solve_likelihood", 0.0);
     SFC_CK(cudaGraphLaunch(b->gexec, ctx->stream));
-    count_launch(ctx);
+    count_launch(ctx, b->args.warm ? 4 : 1);
     ++ctx->graph_replays;
 }
 
@@ -968,6 +1045,9 @@ int32_t sfc_batch_create(sfc_ctx_t *ctx, const sfc_mesh_t *mesh, int32_t num_ins
         b->status.alloc(n);
         b->iters.alloc(n);
         b->hp.alloc((size_t)n * 6);
+        std::vector<int32_t> line(n);
+        for (int i = 0; i < n; ++i) line[i] = grid_side[i] + 1;
+        btd_plan(ctx, b->btd, mesh->row_ptr.p, mesh->col.p, N, n, dof_offset, line.data(), ord.data(), false);
         batch_configure(b, cluster_size > 0 ? cluster_size : 8);
     });
     if (rc != SFC_OK) {
@@ -1002,7 +1082,7 @@ int32_t sfc_batch_set_solver(sfc_batch_t *b, double tol, double inner_tol, int32
     b->itol = inner_tol;
     b->max_iter = max_iter;
     batch_release_graph(b);
-    return SFC_OK;
+    return bguard(b->ctx, [&] { batch_configure(b, b->cluster); });  // the cap may change the solve
 }
 
 int32_t sfc_batch_set_coefficients(sfc_batch_t *b, const double *elem_coeff)
