@@ -99,7 +99,10 @@ typedef struct sfc_solver_options {
                                        one-level preconditioner otherwise)    */
 
 typedef struct sfc_solve_stats {
-    int32_t iterations;       /* max over right-hand sides, inner iterations   */
+    int32_t iterations;       /* max over right-hand sides, inner iterations
+                                 (0: solved by block elimination, the solves
+                                 inside the statX objects on small-bandwidth
+                                 meshes)                                      */
     int32_t refinements;      /* FP64 refinement cycles (mixed solver)         */
     int32_t num_rhs;
     int32_t converged;        /* 1 when every RHS met tol                      */

@@ -30,6 +30,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "btd.cuh"
@@ -707,6 +708,56 @@ __global__ void k_btd_entries(BtdArgs a, int *bad)
     }
 }
 
+// largest distance of an entry from the diagonal
+__global__ void k_bandwidth(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int64_t N, int *bw)
+{
+    int w = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
+        for (int32_t k = rp[i]; k < rp[i + 1]; ++k) w = max(w, abs(col[k] - (int)i));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w = max(w, __shfl_xor_sync(0xffffffffu, w, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(bw, w);
+}
+
+// per column: |b - S x|^2, |b|^2, |x|^2 (out[3][ncols]) and the largest
+// absolute row sum of S (out[3 ncols], the bits of a non-negative double).
+// A block takes 32 columns (a lane each) and a share of the rows.
+__global__ void __launch_bounds__(256) k_btd_check(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
+                                                   const double *__restrict__ a, const double *__restrict__ B,
+                                                   const double *__restrict__ X, int64_t N, int ld, int ncols,
+                                                   double *out)
+{
+    __shared__ double sh[3][8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 32 + lane;
+    const bool ok = c < ncols;
+    double rr = 0.0, bb = 0.0, xx = 0.0, big = 0.0;
+    for (int64_t i = blockIdx.x * 8 + warp; i < N; i += (int64_t)gridDim.x * 8) {
+        const double b = ok ? B[i * ld + c] : 0.0, x = ok ? X[i * ld + c] : 0.0;
+        double r = b, sum = 0.0;
+        for (int32_t k = rp[i]; k < rp[i + 1]; ++k) {
+            const double v = a[k];
+            sum += fabs(v);
+            if (ok) r -= v * X[(int64_t)col[k] * ld + c];
+        }
+        rr += r * r;
+        bb += b * b;
+        xx += x * x;
+        big = fmax(big, sum);
+    }
+    sh[0][warp][lane] = rr;
+    sh[1][warp][lane] = bb;
+    sh[2][warp][lane] = xx;
+    __syncthreads();
+    if (warp < 3 && ok) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += sh[warp][w][lane];
+        atomicAdd(out + (int64_t)warp * ncols + c, t);
+    }
+    if (blockIdx.y == 0 && lane == 0)
+        atomicMax(reinterpret_cast<unsigned long long *>(out + 3 * (int64_t)ncols),
+                  (unsigned long long)__double_as_longlong(big));
+}
+
 template <class K>
 cudaLaunchConfig_t btd_config(K kernel, const BtdPlan &p, int clusters, cudaStream_t st, cudaLaunchAttribute *attr)
 {
@@ -851,6 +902,73 @@ void btd_launch_solve(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a)
     cudaLaunchConfig_t cfg = btd_config(k_btd_solve, p, (a.ncols + kBtdCols - 1) / kBtdCols, ctx->stream, &attr);
     SFC_CK(cudaLaunchKernelEx(&cfg, k_btd_solve, a));
     count_launch(ctx);
+}
+
+namespace {
+
+// The lines of a small-bandwidth system: 32 dofs where the bandwidth allows
+// it (one panel per line; the whole system as one line up to 64 dofs), else
+// the grid line of a triangulated grid (bandwidth - 1: the last node of a
+// line has no neighbour two lines on), else the bandwidth.
+void plan_system(sfc_system *s)
+{
+    BtdPlan &p = s->btd;
+    sfc_ctx *ctx = s->ctx;
+    p.tried = true;
+    p.usable = false;
+    if (s->N > (1 << 20) || s->has_bsr) return;
+    p.word.reserve(2);
+    SFC_CK(cudaMemsetAsync(p.word.p, 0, 2 * sizeof(int), ctx->stream));
+    k_bandwidth<<<grid_for(s->N, 256), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->N, p.word.p);
+    count_launch(ctx);
+    int bw = 0;
+    download(ctx, &bw, p.word.p, 1);
+    const int64_t row0[2] = {0, s->N};
+    const int32_t order = 0;
+    for (const int m : {s->N <= 64 ? (int)s->N : 32, bw - 1, bw}) {
+        if (m < 1 || m > kLineMax || (int64_t)m > s->N || m < bw - 1) continue;
+        const int32_t line = m;
+        if (btd_plan(ctx, p, s->row_ptr.p, s->col.p, s->N, 1, row0, &line, &order, true)) return;
+    }
+}
+
+}  // namespace
+
+bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int ld, double tol, double *max_rel)
+{
+    sfc_ctx *ctx = s->ctx;
+    BtdPlan &p = s->btd;
+    if (!p.tried) plan_system(s);
+    if (!p.usable) return false;
+    BtdArgs a = btd_args(p, s->row_ptr.p, s->col.p, s->a_op.p);
+    a.B = B;
+    a.U = X;
+    a.ld = ld;
+    a.ncols = nrhs;
+    if (p.factored != s->op_serial) {
+        btd_launch_factor(ctx, p, a);
+        p.factored = s->op_serial;
+    }
+    btd_launch_solve(ctx, p, a);
+    const size_t nn = 3 * (size_t)nrhs + 1;
+    p.norms.reserve(nn);
+    SFC_CK(cudaMemsetAsync(p.norms.p, 0, nn * sizeof(double), ctx->stream));
+    const dim3 grid((unsigned)std::min<int64_t>((s->N + 31) / 32, 2 * ctx->sm_count), (unsigned)((nrhs + 31) / 32));
+    k_btd_check<<<grid, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op.p, B, X, s->N, ld, nrhs, p.norms.p);
+    count_launch(ctx);
+    std::vector<double> h(nn);
+    download(ctx, h.data(), p.norms.p, nn);
+    double worst = 0.0;
+    for (int c = 0; c < nrhs; ++c) {
+        const double r = std::sqrt(h[c]), b = std::sqrt(h[nrhs + c]), x = std::sqrt(h[2 * (size_t)nrhs + c]);
+        // tol, or a residual at the rounding of its own terms, which the
+        // recurrence residual of FP64 PCG does not see
+        const double floor = 8.0 * 2.2e-16 * (h[3 * (size_t)nrhs] * x + b);
+        if (!(r <= tol * b || r <= floor)) return false;
+        if (b > 0) worst = std::max(worst, r / b);
+    }
+    *max_rel = worst;
+    return true;
 }
 
 }  // namespace sfc

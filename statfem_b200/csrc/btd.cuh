@@ -34,20 +34,6 @@ struct BtdArgs {
     int lmax;    // longest line
 };
 
-struct BtdPlan {
-    bool usable = false;
-    int n = 0, lmax = 0, chain = 0, slots = 0;
-    size_t smem = 0;
-    int64_t N = 0;
-    DBuf<int64_t> row0;
-    DBuf<int32_t> line, order;
-    DBuf<int16_t> cols;
-    DBuf<double> vals;
-    DBuf<double> X, Y;
-    DBuf<int> word;
-    uint64_t factored = 0;  // operator serial of the inverse blocks in X (single systems)
-};
-
 // Looks whether the system's pattern has the form above and sizes the
 // workspace; false when the direct solve does not apply.
 bool btd_plan(sfc_ctx *ctx, BtdPlan &p, const int32_t *rp, const int32_t *col, int64_t N, int n_inst,
@@ -58,5 +44,8 @@ void btd_launch_batch(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a, cudaStre
 // one system: the inverse blocks, then any number of columns
 void btd_launch_factor(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a);
 void btd_launch_solve(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a);
+// S X = B of a system whose operator is built; false (X undefined) where the
+// elimination does not apply or a column misses tol
+bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int ld, double tol, double *max_rel);
 
 }  // namespace sfc

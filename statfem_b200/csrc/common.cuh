@@ -273,6 +273,23 @@ struct EventPair {
     }
 };
 
+// Direct block-tridiagonal solve (btd.cu): the pattern's lines, the cluster
+// shape and the workspace.
+struct BtdPlan {
+    bool tried = false, usable = false;  // for the pattern at hand
+    int n = 0, lmax = 0, chain = 0, slots = 0;
+    size_t smem = 0;
+    int64_t N = 0;
+    DBuf<int64_t> row0;
+    DBuf<int32_t> line, order;
+    DBuf<int16_t> cols;
+    DBuf<double> vals;
+    DBuf<double> X, Y;
+    DBuf<int> word;
+    DBuf<double> norms;      // residual check
+    uint64_t factored = 0;  // operator serial of the inverse blocks in X (single systems)
+};
+
 struct CoarseSpace {
     bool built = false;                 // aggregates for (mesh, size)
     const sfc_mesh *mesh = nullptr;
@@ -470,6 +487,7 @@ struct sfc_system {
     // per launch configuration (block widths 32, 64, 128)
     sfc::GraphExec blk_graph[3];
     sfc::EventPair solve_ev;  // device time of the last solve call
+    sfc::BtdPlan btd;         // direct solve of small-bandwidth systems
 };
 
 // ---------------------------------------------------------------------------
@@ -550,10 +568,12 @@ void ensure_pattern_from_mesh(sfc_system *s, const sfc_mesh *m);
 void element_matrices_unit(const sfc_mesh *m, double *ke0);
 void gather_weighted(const sfc_mesh *m, const double *ke0, const double *w_dev, int kc, double *out);
 // solvers.cu
-void solve_forward(sfc_system *s);
+// `direct`: the statX objects' own solves may take the block elimination
+void solve_forward(sfc_system *s, bool direct = false);
+void solve_adjoint(sfc_system *s, const double *B_dev, double *X_dev, int nrhs, int ld);
 void solve_block(sfc_system *s, const double *B_dev, double *X_dev, int nrhs, int ld);
 void transpose_fixup(sfc_system *s, const double *B_dev, double *X_dev, int nrhs, int ld);
-void solve_multi(sfc_system *s, const double *B_dev, double *X_dev, int nrhs, int ld);
+void solve_multi(sfc_system *s, const double *B_dev, double *X_dev, int nrhs, int ld, bool direct = false);
 double device_dot(sfc_ctx *ctx, const double *a, const double *b, int64_t n);
 void spmv_op64(sfc_system *s, const double *x, double *y);
 // y = S x and *xy += x . y, skipped entirely when *done != 0 (done may be NULL)

@@ -152,7 +152,7 @@ void perturbation_update(sfc_perturbation *pt, const sfc_hparams_t *hp, double m
     const int64_t N = s->N, ns = fg->ns, E = m->num_elems;
     // R^T = A^-T P^T, mean = R F (ForwardGaussRHS update) and u = A^-1 F
     forward_gauss_update(fg, hp);
-    solve_forward(s);
+    solve_forward(s, true);
     build_operator(s);
     if (!pt->ke0.p) {
         pt->ke0.alloc(E * m->L * m->L);
@@ -198,7 +198,7 @@ void perturbation_update(sfc_perturbation *pt, const sfc_hparams_t *hp, double m
         atb_accumulate(ctx, V.p, V.p, kc, ns, ns, pt->cov.p);
         // Y = A^-T B^T (one block adjoint solve), then Y^T C_f Y per k
         Y.reserve(N * w);
-        solve_block(s, Bt.p, Y.p, (int)w, (int)w);
+        solve_adjoint(s, Bt.p, Y.p, (int)w, (int)w);
         transpose_fixup(s, Bt.p, Y.p, (int)w, (int)w);
         W.reserve(N * w);
         T.reserve(2 * N * w);

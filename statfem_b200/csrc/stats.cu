@@ -636,7 +636,7 @@ void forward_gauss_update(sfc_forward_gauss *fg, const sfc_hparams_t *hp)
     flush_staged(s);
     {
         ProfScope ps(ctx, "phase:adjoint_solve", 0.0);
-        solve_block(s, B.p, fg->R.p, (int)ns, (int)ns);
+        solve_adjoint(s, B.p, fg->R.p, (int)ns, (int)ns);
         transpose_fixup(s, B.p, fg->R.p, (int)ns, (int)ns);
     }
     ProfScope ps_cov(ctx, "phase:mean_and_covariance", 0.0);
@@ -997,7 +997,7 @@ void koh_woodbury_mean(sfc_koh *k, const sfc_hparams_t *hp, double *mean)
     host_chol_solve(Ls, n, t);
     for (int a = 0; a < n; ++a) w[a] = rho * kys[a] - t[a];
     // ubar = A^-1 F (forward solve, the system's own method)
-    solve_forward(s);
+    solve_forward(s, true);
     // G = A^-1 (C_f R^T) + (sigma_f reg)^2 P^T
     DBuf<double> W, T, G, wd, out;
     W.alloc(N * ns);
@@ -1008,7 +1008,7 @@ void koh_woodbury_mean(sfc_koh *k, const sfc_hparams_t *hp, double *mean)
     kernel_times(ctx, fg->cf, hp->forcing_sigma, hp->forcing_length, W.p, T.p, ns, T.p + N * ns);
     k_scale_rows<<<grid_for(N * ns, 256), 256, 0, ctx->stream>>>(T.p, fg->cf->phibar.p, N, ns, W.p);
     count_launch(ctx);
-    solve_multi(s, W.p, G.p, (int)ns, (int)ns);
+    solve_multi(s, W.p, G.p, (int)ns, (int)ns, true);
     const double add = hp->forcing_sigma * fg->reg;
     k_add_scaled<<<grid_for(N * ns, 256), 256, 0, ctx->stream>>>(G.p, fg->B.p, add * add, N * ns);
     count_launch(ctx);
@@ -1059,7 +1059,7 @@ void koh_woodbury(sfc_koh *k, const sfc_hparams_t *hp, double *mean, double *cov
     for (int64_t i = 0; i < N; ++i) hI[(size_t)i * N + i] = 1.0;
     upload(ctx, I, hI.data(), hI.size());
     RI.alloc(N * N);
-    solve_block(s, I.p, RI.p, (int)N, (int)N);
+    solve_adjoint(s, I.p, RI.p, (int)N, (int)N);
     transpose_fixup(s, I.p, RI.p, (int)N, (int)N);
     ubar.alloc(N);
     k_colsum_dot<<<(unsigned)std::min<int64_t>(N, 1024), 256, 0, ctx->stream>>>(RI.p, s->F.p, N, N, ubar.p);
