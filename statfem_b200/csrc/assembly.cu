@@ -785,7 +785,7 @@ void ensure_pattern_from_mesh(sfc_system *s, const sfc_mesh *m)
     s->a_op32.alloc(s->nnz);
     SFC_CK(cudaMemsetAsync(s->a_ref.p, 0, s->nnz * 8, ctx->stream));
     s->has_pattern = true;
-    s->btd.tried = false;
+    s->btd.tried = s->dia_tried = false;
     s->pattern_mesh = m;
     s->coarse.built = false;  // aggregates belong to the installed mesh
     s->op_valid = false;
@@ -1165,7 +1165,7 @@ void flush_staged(sfc_system *s)
     s->st_cols.clear();
     s->st_vals.clear();
     s->has_pattern = true;
-    s->btd.tried = false;
+    s->btd.tried = s->dia_tried = false;
     s->pattern_mesh = nullptr;
     s->op_valid = false;
 }

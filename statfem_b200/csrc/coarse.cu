@@ -76,7 +76,8 @@ __device__ __forceinline__ int mask_bits(const float4 m) { return (int)m.w; }
 // per node: offset from its aggregate's centroid in units of the box edge
 // (x, y, z) and the constrained components as bits in w
 __global__ void k_coarse_modes(const float4 *__restrict__ offset, const unsigned char *__restrict__ mask,
-                               int64_t nodes, int dof, float4 *__restrict__ mode)
+                               const int32_t *__restrict__ node_agg, int64_t nodes, int dof,
+                               float4 *__restrict__ mode, int32_t *__restrict__ agg_free)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nodes; i += (int64_t)gridDim.x * blockDim.x) {
         float4 m = offset[i];
@@ -84,6 +85,7 @@ __global__ void k_coarse_modes(const float4 *__restrict__ offset, const unsigned
                                   : (mask[3 * i] ? 1 : 0) | (mask[3 * i + 1] ? 2 : 0) | (mask[3 * i + 2] ? 4 : 0);
         m.w = (float)bits;
         mode[i] = m;
+        if (dof == 1) agg_free[i] = bits ? -1 : node_agg[i];
     }
 }
 
@@ -518,110 +520,6 @@ __global__ void __cluster_dims__(1, 1, kGemmSplit) __launch_bounds__(128)
     if (tid < kGemmCols) atomicAdd(rz + col0 + tid, sred[0][tid] + sred[1][tid] + sred[2][tid] + sred[3][tid]);
 }
 
-// single FP64 vector: c[6a + m] = (P^T r)[6a + m]
-__global__ void __launch_bounds__(256) k_coarse_restrict64(const double *__restrict__ r,
-                                                           const int32_t *__restrict__ agg_ptr,
-                                                           const int32_t *__restrict__ agg_nodes,
-                                                           const float4 *__restrict__ mode, double *__restrict__ c,
-                                                           const int *done)
-{
-    __shared__ double red[6][8];
-    if (done && *done) return;
-    const int a = blockIdx.x;
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int32_t t = agg_ptr[a] + threadIdx.x; t < agg_ptr[a + 1]; t += blockDim.x) {
-        const int32_t i = agg_nodes[t];
-        const float4 m = mode[i];
-        const int bits = (int)m.w;
-        const double r0 = (bits & 1) ? 0.0 : r[3 * (int64_t)i], r1 = (bits & 2) ? 0.0 : r[3 * (int64_t)i + 1],
-                     r2 = (bits & 4) ? 0.0 : r[3 * (int64_t)i + 2];
-        acc[0] += r0;
-        acc[1] += r1;
-        acc[2] += r2;
-        acc[3] += (double)m.y * r2 - (double)m.z * r1;
-        acc[4] += (double)m.z * r0 - (double)m.x * r2;
-        acc[5] += (double)m.x * r1 - (double)m.y * r0;
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-        double v = acc[m];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[m][w] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double s = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += red[threadIdx.x][q];
-        c[6 * a + threadIdx.x] = s;
-    }
-}
-
-// scalar meshes, one FP64 vector: c[a] = sum of r over the free nodes of a
-__global__ void __launch_bounds__(256) k_coarse_restrict64_1(const double *__restrict__ r,
-                                                             const int32_t *__restrict__ agg_ptr,
-                                                             const int32_t *__restrict__ agg_nodes,
-                                                             const float4 *__restrict__ mode, double *__restrict__ c,
-                                                             const int *done)
-{
-    __shared__ double red[8];
-    if (done && *done) return;
-    const int a = blockIdx.x;
-    double acc = 0.0;
-    for (int32_t t = agg_ptr[a] + threadIdx.x; t < agg_ptr[a + 1]; t += blockDim.x) {
-        const int32_t i = agg_nodes[t];
-        if (!((int)mode[i].w & 1)) acc += r[i];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double sum = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) sum += red[q];
-        c[a] = sum;
-    }
-}
-
-// e = A c (FP64, warp per row); rz += c.e
-__global__ void __launch_bounds__(256) k_coarse_apply64(const double *__restrict__ A, const double *__restrict__ c,
-                                                        double *__restrict__ e, int64_t nc, double *rz, const int *done)
-{
-    __shared__ double sh[8];
-    if (done && *done) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t row = (int64_t)blockIdx.x * 8 + w;
-    double part = 0.0;
-    if (row < nc) {
-        // four independent partial sums keep four loads of the row in flight
-        const double *Ar = A + row * nc;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        int64_t k = lane;
-        for (; k + 96 < nc; k += 128) {
-            s0 += Ar[k] * c[k];
-            s1 += Ar[k + 32] * c[k + 32];
-            s2 += Ar[k + 64] * c[k + 64];
-            s3 += Ar[k + 96] * c[k + 96];
-        }
-        for (; k < nc; k += 32) s0 += Ar[k] * c[k];
-        double s = (s0 + s1) + (s2 + s3);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            e[row] = s;
-            part = s * c[row];
-        }
-    }
-    if (lane == 0) sh[w] = part;
-    __syncthreads();
-    if (threadIdx.x == 0 && rz) {
-        double t = 0.0;
-        for (int q = 0; q < 8; ++q) t += sh[q];
-        atomicAdd(rz, t);
-    }
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -805,6 +703,7 @@ static bool coarse_aggregate(sfc_system *s, int size)
     upload(ctx, cs.nbr, nbr.data(), nbr.size());
     upload(ctx, cs.offset, off.data(), nodes);
     cs.mode.alloc(nodes);
+    if (dof == 1) cs.agg_free.alloc(nodes);
     cs.mesh = m;
     cs.size = size;
     cs.built = true;
@@ -825,7 +724,8 @@ bool coarse_prepare(sfc_system *s)
     sfc_ctx *ctx = s->ctx;
     ProfScope ps(ctx, "phase:coarse_setup", 0.0);
     const int64_t nodes = cs.nodes, nc = cs.nc;
-    k_coarse_modes<<<grid_for(nodes, 256), 256, 0, ctx->stream>>>(cs.offset.p, s->mask.p, nodes, cs.dof, cs.mode.p);
+    k_coarse_modes<<<grid_for(nodes, 256), 256, 0, ctx->stream>>>(cs.offset.p, s->mask.p, cs.node_agg.p, nodes,
+                                                                    cs.dof, cs.mode.p, cs.agg_free.p);
     cs.a64.alloc(nc * nc);
     cs.lda = (nc + 63) / 64 * 64;
     cs.a32.alloc(cs.lda * cs.lda);
@@ -914,29 +814,6 @@ void coarse_block_gemm(sfc_system *s, double *rz, const int *stop)
 template void coarse_block_gemm<1>(sfc_system *, double *, const int *);
 template void coarse_block_gemm<2>(sfc_system *, double *, const int *);
 template void coarse_block_gemm<4>(sfc_system *, double *, const int *);
-
-void coarse_vec_apply(sfc_system *s, const double *r, double *rz, const int *done)
-{
-    CoarseSpace &cs = s->coarse;
-    sfc_ctx *ctx = s->ctx;
-    cs.c64.reserve(cs.nc);
-    cs.e64.reserve(cs.nc);
-    {
-        ProfScope ps(ctx, "coarse_restrict64", (double)cs.dof * cs.nodes * 8 + 20.0 * cs.nodes + 8.0 * cs.nc);
-        if (cs.dof == 3)
-            k_coarse_restrict64<<<(unsigned)cs.nagg, 256, 0, ctx->stream>>>(r, cs.agg_ptr.p, cs.agg_nodes.p,
-                                                                            cs.mode.p, cs.c64.p, done);
-        else
-            k_coarse_restrict64_1<<<(unsigned)cs.nagg, 256, 0, ctx->stream>>>(r, cs.agg_ptr.p, cs.agg_nodes.p,
-                                                                              cs.mode.p, cs.c64.p, done);
-    }
-    {
-        ProfScope ps(ctx, "coarse_apply64", 8.0 * cs.nc * cs.nc + 16.0 * cs.nc);
-        k_coarse_apply64<<<(unsigned)((cs.nc + 7) / 8), 256, 0, ctx->stream>>>(cs.a64.p, cs.c64.p, cs.e64.p, cs.nc,
-                                                                                rz, done);
-    }
-    count_launch(ctx, 2);
-}
 
 }  // namespace sfc
 

@@ -301,6 +301,7 @@ struct CoarseSpace {
     int nb[3] = {1, 1, 1};              // boxes per axis
     int dropped = 0;                    // dependent coarse dofs left out of the inverse
     DBuf<int32_t> node_agg;             // nodes
+    DBuf<int32_t> agg_free;             // scalar meshes: node_agg, -1 on constrained nodes (per operator)
     DBuf<int32_t> agg_ptr, agg_nodes;   // aggregate -> its nodes
     DBuf<int32_t> agg_slot;             // colour class (box index mod 3 per axis)
     DBuf<int32_t> nbr;                  // [nagg][27]: neighbour aggregate per colour class
@@ -488,6 +489,13 @@ struct sfc_system {
     sfc::GraphExec blk_graph[3];
     sfc::EventPair solve_ev;  // device time of the last solve call
     sfc::BtdPlan btd;         // direct solve of small-bandwidth systems
+    // diagonal copy of the operator (pcg.cu): [offset][row], or
+    // [offset][3 x 3][node] on 3-dof meshes, from the main diagonal up
+    sfc::DBuf<double> dia;
+    int dia_nd = 0, dia_off[32] = {};
+    bool dia_tried = false;      // for the pattern at hand
+    uint64_t dia_serial = 0;     // operator the values belong to
+    bool dia_ok = false;         // which is symmetric
 };
 
 // ---------------------------------------------------------------------------
@@ -583,7 +591,12 @@ struct PcgStats {
     int iters;
     bool converged;
 };
-PcgStats pcg64_public(sfc_system *s, const double *b, double *x, double tol, int max_iter, int check);
+// pcg.cu: FP64 PCG on S x = b (point Jacobi; `two`: the two-level
+// preconditioner, whose coarse space the caller has prepared)
+PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_iter, bool two);
+// y = S x through the diagonal copy of the operator; false where there is none
+bool dia_spmv64(sfc_system *s, const double *x, double *y, double *dot, const int *done);
+void dia_ensure(sfc_system *s);  // makes the copy for the products that follow
 // mpnn.cu
 void solve_forward_fcg(sfc_system *s);
 // solvers.cu: FP64 SpMV with a given number of lanes per row (4, 8, 16, 32)
@@ -600,7 +613,6 @@ template <int V>
 void coarse_block_apply(sfc_system *s, const float *r, double *rz, const int *stop);
 template <int V>
 void coarse_block_gemm(sfc_system *s, double *rz, const int *stop);  // e = A_c^+ c of cs.c32
-void coarse_vec_apply(sfc_system *s, const double *r, double *rz, const int *done);
 // stats.cu
 void forward_gauss_update(sfc_forward_gauss *fg, const sfc_hparams_t *hp);
 void projected_covar(sfc_ctx *ctx, sfc_covar_forcing *cf, double sigma, double length, const double *X, int64_t ns,

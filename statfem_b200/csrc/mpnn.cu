@@ -1507,9 +1507,9 @@ void make_pairs(sfc_mpnn *m, sfc_system *s, int max_pairs, double floor, bool no
     xk.alloc(N);
     t.alloc(N);
     lifted_rhs(s, b.p);
-    const PcgStats ref = pcg64_public(s, b.p, xs.p, 1e-12, 200000, 32);
+    const PcgStats ref = pcg64(s, b.p, xs.p, 1e-12, 200000, false);
     SFC_REQUIRE(ref.converged, "Jacobi-PCG did not converge while generating training pairs");
-    const PcgStats fl = pcg64_public(s, b.p, xk.p, floor, 200000, 1);
+    const PcgStats fl = pcg64(s, b.p, xk.p, floor, 200000, false);
     const int kmax = std::max(1, fl.iters);
     std::vector<int> ks{0};
     for (int j = 1; j < max_pairs; ++j) {
@@ -1524,7 +1524,7 @@ void make_pairs(sfc_mpnn *m, sfc_system *s, int max_pairs, double floor, bool no
         if (ks[j] == 0)
             SFC_CK(cudaMemsetAsync(xk.p, 0, N * 8, ctx->stream));
         else
-            pcg64_public(s, b.p, xk.p, 1e-300, ks[j], 1 << 30);
+            pcg64(s, b.p, xk.p, 1e-300, ks[j], false);
         spmv_op64(s, xk.p, t.p);
         k_resid_pair<<<grid_for(N, 256), 256, 0, ctx->stream>>>(b.p, t.p, xs.p, xk.p, N, m->pr.p + j * N,
                                                                m->pe.p + j * N);
@@ -1733,7 +1733,7 @@ void solve_forward_fcg(sfc_system *s)
             rel = true_residual();
             if (rel > tol) {
                 fallback = 1;
-                const PcgStats pr = pcg64_public(s, r, z, tol / rel, max_iter, 32);
+                const PcgStats pr = pcg64(s, r, z, tol / rel, max_iter, false);
                 k_axpy<<<g, 256, 0, ctx->stream>>>(s->X.p, z, 1.0, N);
                 count_launch(ctx);
                 iters += pr.iters;

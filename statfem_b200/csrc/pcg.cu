@@ -1,0 +1,827 @@
+// FP64 PCG for one right-hand side as one persistent cooperative kernel, and
+// the diagonal (DIA) copy of the operator that its product reads.
+//
+// The iteration of the plain method (point Jacobi) and of the two-level
+// preconditioner (coarse.cu) on S x = b, with the scalars of every iteration
+// in their own slots, as separate launches cost five launches and 26 us an
+// iteration on small meshes, whatever their work.  Here the phases of an
+// iteration (product with p.q; x, r update with the dots and the coarse
+// restriction; coarse product; p update) follow one another behind grid
+// barriers of a cooperative launch (co-resident blocks by construction; every
+// wait has a limit, after which the kernel reports a timeout).
+//
+// On meshes numbered along a lattice every row couples to the same offsets,
+// so the values are also kept by diagonals, [offset][row] ([offset][3 x 3]
+// [node] on 3-dof meshes): a warp reads 32 consecutive rows of a diagonal in
+// one piece and no column indices.  Only the diagonals above and on the main
+// one are kept (the operator is symmetric, which is checked): the entry below
+// is read from the row above it, and the copy is a third of the CSR's bytes,
+// so that it stays in L2 between iterations up to about a million rows (80^3
+// Poisson: 60 MB against 172; all 27 diagonals, 115 MB, took 27 us a product,
+// the CSR 79).
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cmath>
+#include <vector>
+
+#include "common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace sfc {
+namespace {
+
+constexpr int kDiaMax = 32;    // diagonals of the pattern
+// Nonzeros up to which one cluster of 16 blocks runs the solve.  An iteration
+// takes it 10.3 us at 29 thousand (64 x 64 square; the grid 11.7) and 19.5 at
+// 230 thousand (181 x 181; the grid 13).
+constexpr double kClusterWork = 1e5;
+
+enum Format { CSR = 0, DIA = 1, BSR = 2, BDIA = 3 };
+
+struct PcgArgs {
+    int64_t N, nodes;          // dofs; nodes of a 3-dof mesh
+    const int32_t *rp, *col;   // CSR rows, or node-block rows
+    const double *a;           // CSR values, diagonals or node blocks
+    int lanes;                 // lanes per CSR row
+    int nd;                    // diagonals kept: the main one, then those above it
+    int off[kDiaMax / 2 + 1];
+    const double *b, *dinv;
+    const float *bdinv;        // nodal block inverses
+    double *x, *r, *p, *q;
+    // coarse space
+    const int32_t *agg;        // aggregate of a node; scalar meshes: -1 where constrained
+    const float4 *mode;
+    const double *ac;          // nc x nc inverse
+    int64_t nc;
+    double *c, *e;             // [2][nc], [nc]
+    double *sums;              // [4][max_iter + 2]: zeroed slots of the sums
+    unsigned *bar;
+    double tol;
+    int max_iter;
+    int *out;                  // iterations, converged, error
+};
+
+__device__ __forceinline__ double warp_total(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+struct CommShared {
+    double warps[2][32], rows[32];
+    double part[2][2];
+    int ok;
+};
+
+// Sums over all blocks, each of them also a barrier.  CL: the blocks are one
+// cluster (hardware barrier, shares read through distributed shared memory).
+// Else a cooperative grid: an atomic per block into the sum's own slot and a
+// counter (2.3 us a sum; reading every block's share instead took 2.9, and
+// polling the shares themselves, without a counter, 4.3: the polls queue up
+// behind one another on a few lines of L2).  The counter's wait is bounded
+// (2^22 polls, seconds): a block that gives up reports it, and so does every
+// other in its turn.
+template <bool CL>
+struct Comm {
+    const PcgArgs &g;
+    CommShared &sh;
+    unsigned target = 0;
+    int turn = 0;
+
+    __device__ bool barrier()
+    {
+        if constexpr (CL) {
+            cg::this_cluster().sync();  // releases and acquires global memory too
+            return true;
+        } else {
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                target += gridDim.x;
+                __threadfence();
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.bar) : "memory");
+                unsigned v = 0;
+                int n = 0;
+                do {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.bar) : "memory");
+                } while ((int)(v - target) < 0 && ++n < (1 << 22));
+                sh.ok = (int)(v - target) >= 0;
+                if (!sh.ok) atomicExch(g.out + 2, 2);
+                __threadfence();
+            }
+            __syncthreads();
+            return sh.ok != 0;
+        }
+    }
+
+    // a (and b, M = 2) <- the sum over all threads
+    template <int M>
+    __device__ bool sum(double &a, double &b, int slot0, int slot1)
+    {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        a = warp_total(a);
+        if (M == 2) b = warp_total(b);
+        if (lane == 0) {
+            sh.warps[0][warp] = a;
+            if (M == 2) sh.warps[1][warp] = b;
+        }
+        __syncthreads();
+        if (warp < M) {
+            const double t = warp_total(lane < nw ? sh.warps[warp][lane] : 0.0);
+            if (lane == 0) {
+                if (CL) sh.part[turn][warp] = t;
+                else atomicAdd(g.sums + (warp ? slot1 : slot0), t);
+            }
+        }
+        if (!barrier()) return false;
+        if constexpr (CL) {
+            cg::cluster_group cl = cg::this_cluster();
+            const bool in = lane < (int)cl.num_blocks();
+            const double *part = cl.map_shared_rank(&sh.part[turn][0], in ? lane : 0);
+            a = warp_total(in ? part[0] : 0.0);
+            if (M == 2) b = warp_total(in ? part[1] : 0.0);
+            turn ^= 1;
+        } else {
+            a = g.sums[slot0];
+            if (M == 2) b = g.sums[slot1];
+        }
+        return true;
+    }
+};
+
+// row i of S x
+__device__ __forceinline__ double dia_row(const double *a, const int *off, int nd, int64_t N, int64_t i, const double *x)
+{
+    double s = a[i] * x[i];
+    constexpr int U = 4;
+    for (int d0 = 1; d0 < nd; d0 += U) {
+        double v[2 * U], xv[2 * U];
+#pragma unroll
+        for (int d = 0; d < U; ++d) {
+            const bool in = d0 + d < nd;
+            const int64_t o = in ? off[d0 + d] : 0, up = i + o, dn = i - o;
+            const double *ad = a + (int64_t)(in ? d0 + d : 0) * N;
+            const bool u = in && up < N, l = in && dn >= 0;
+            v[2 * d] = u ? ad[i] : 0.0;
+            xv[2 * d] = u ? x[up] : 0.0;
+            v[2 * d + 1] = l ? ad[dn] : 0.0;
+            xv[2 * d + 1] = l ? x[dn] : 0.0;
+        }
+#pragma unroll
+        for (int d = 0; d < 2 * U; ++d) s += v[d] * xv[d];
+    }
+    return s;
+}
+
+// the three rows of node i, a thread per node: the operand's three values
+// serve three rows (a thread per row read them three times and was bound by
+// its L1 wavefronts: 63 us for 48^3 elasticity)
+__device__ __forceinline__ void bdia_node(const double *a, const int *off, int nd, int64_t nodes, int64_t i,
+                                          const double *x, double (&s)[3])
+{
+    s[0] = s[1] = s[2] = 0.0;
+    // block d of node at, times x of node j; below: the block's transpose
+    auto block = [&](int d, int64_t at, int64_t j, bool below) {
+        double v[9], xv[3];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[k] = a[((int64_t)d * 9 + k) * nodes + at];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) xv[k] = x[3 * j + k];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+            s[r] += below ? v[r] * xv[0] + v[3 + r] * xv[1] + v[6 + r] * xv[2]
+                          : v[3 * r] * xv[0] + v[3 * r + 1] * xv[1] + v[3 * r + 2] * xv[2];
+    };
+    block(0, i, i, false);
+#pragma unroll 1
+    for (int d = 1; d < nd; ++d) {
+        const int64_t up = i + off[d], dn = i - off[d];
+        if (up < nodes) block(d, i, up, false);
+        if (dn >= 0) block(d, dn, dn, true);
+    }
+}
+
+// q = S p over the grid's share of the rows; returns this thread's part of p.q
+template <int F>
+__device__ double product(const PcgArgs &g, const double *p, double *q)
+{
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    double dot = 0.0;
+    if constexpr (F == DIA) {
+        for (int64_t i = t0; i < g.N; i += nt) {
+            const double s = dia_row(g.a, g.off, g.nd, g.N, i, p);
+            q[i] = s;
+            dot += p[i] * s;
+        }
+    } else if constexpr (F == BDIA) {
+        for (int64_t i = t0; i < g.nodes; i += nt) {
+            double s[3];
+            bdia_node(g.a, g.off, g.nd, g.nodes, i, p, s);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                q[3 * i + k] = s[k];
+                dot += p[3 * i + k] * s[k];
+            }
+        }
+    } else if constexpr (F == BSR) {
+        for (int64_t i = t0 >> 5; i < g.nodes; i += nt >> 5) {
+            double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+            for (int32_t b = g.rp[i] + lane; b < g.rp[i + 1]; b += 32) {
+                const int64_t j = g.col[b];
+                const double *v = g.a + 9 * (int64_t)b;
+                const double x0 = p[3 * j], x1 = p[3 * j + 1], x2 = p[3 * j + 2];
+                s0 += v[0] * x0 + v[1] * x1 + v[2] * x2;
+                s1 += v[3] * x0 + v[4] * x1 + v[5] * x2;
+                s2 += v[6] * x0 + v[7] * x1 + v[8] * x2;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+                s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+            }
+            if (lane < 3) {
+                const double s = lane == 0 ? s0 : lane == 1 ? s1 : s2;
+                q[3 * i + lane] = s;
+                dot += p[3 * i + lane] * s;
+            }
+        }
+    } else {
+        const int G = g.lanes, per = 32 / G;
+        for (int64_t base = (t0 >> 5) * per; base < g.N; base += (nt >> 5) * per) {
+            const int64_t i = base + lane / G;
+            double s = 0.0;
+            if (i < g.N)
+                for (int32_t k = g.rp[i] + lane % G; k < g.rp[i + 1]; k += G) s += g.a[k] * p[g.col[k]];
+            for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
+            if (i < g.N && lane % G == 0) {
+                q[i] = s;
+                dot += p[i] * s;
+            }
+        }
+    }
+    return dot;
+}
+
+// Adds the M values of the warp's lanes to c[M agg ..]: lanes of consecutive
+// nodes of one aggregate (a run of the lattice's line) are summed first.
+template <int M>
+__device__ void restrict_add(double *c, int agg, double (&v)[M])
+{
+    const int lane = threadIdx.x & 31;
+    const int left = __shfl_up_sync(0xffffffffu, agg, 1);
+    const bool head = lane == 0 || left != agg;
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const unsigned after = lane == 31 ? 0u : heads >> (lane + 1);
+    const int run = after ? __ffs(after) : 32 - lane;  // lanes to the end of the run
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const double w = __shfl_down_sync(0xffffffffu, v[m], o);
+            if (o < run) v[m] += w;
+        }
+    if (head && agg >= 0)
+#pragma unroll
+        for (int m = 0; m < M; ++m) atomicAdd(c + (int64_t)M * agg + m, v[m]);
+}
+
+__device__ __forceinline__ void block_jacobi(const float *D, const double (&r)[3], double (&z)[3])
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        z[i] = (double)D[3 * i] * r[0] + (double)D[3 * i + 1] * r[1] + (double)D[3 * i + 2] * r[2];
+}
+
+// PRE: 0 point Jacobi, 1 two-level with one constant per aggregate, 2
+// two-level with nodal blocks and six rigid-body modes.  r -= alpha q (INIT:
+// r = b) with r.z (the Jacobi share) and r.r, and the restriction of r into c.
+// x += alpha p waits for the p update, which reads p anyway.
+template <int PRE, bool INIT>
+__device__ void update(const PcgArgs &g, double alpha, double *c, double &rz, double &rr)
+{
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    rz = rr = 0.0;
+    if constexpr (PRE == 0) {
+        for (int64_t i = t0; i < g.N; i += nt) {
+            const double ri = INIT ? g.b[i] : g.r[i] - alpha * g.q[i];
+            g.r[i] = ri;
+            rz += ri * (g.dinv[i] * ri);
+            rr += ri * ri;
+        }
+    } else if constexpr (PRE == 1) {
+        // whole warps take every trip: the restriction shuffles
+        for (int64_t base = t0 - (threadIdx.x & 31); base < g.N; base += nt) {
+            const int64_t i = base + (threadIdx.x & 31);
+            double v[1] = {0.0};
+            int a = -1;
+            if (i < g.N) {
+                const double ri = INIT ? g.b[i] : g.r[i] - alpha * g.q[i];
+                g.r[i] = ri;
+                rz += ri * (g.dinv[i] * ri);
+                rr += ri * ri;
+                a = g.agg[i];
+                v[0] = a >= 0 ? ri : 0.0;
+            }
+            restrict_add<1>(c, a, v);
+        }
+    } else {
+        for (int64_t base = t0 - (threadIdx.x & 31); base < g.nodes; base += nt) {
+            const int64_t n = base + (threadIdx.x & 31);
+            double v[6] = {0, 0, 0, 0, 0, 0};
+            int a = -1;
+            if (n < g.nodes) {
+                double rv[3], zv[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int64_t k = 3 * n + i;
+                    rv[i] = INIT ? g.b[k] : g.r[k] - alpha * g.q[k];
+                    g.r[k] = rv[i];
+                }
+                block_jacobi(g.bdinv + 9 * n, rv, zv);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    rz += rv[i] * zv[i];
+                    rr += rv[i] * rv[i];
+                }
+                const float4 m = g.mode[n];
+                const int bits = (int)m.w;
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    if ((bits >> i) & 1) rv[i] = 0.0;
+                a = g.agg[n];
+                v[0] = rv[0];
+                v[1] = rv[1];
+                v[2] = rv[2];
+                v[3] = (double)m.y * rv[2] - (double)m.z * rv[1];
+                v[4] = (double)m.z * rv[0] - (double)m.x * rv[2];
+                v[5] = (double)m.x * rv[1] - (double)m.y * rv[0];
+            }
+            restrict_add<6>(c, a, v);
+        }
+    }
+}
+
+// e = Ac c, one, two or four warps per row, as many as the grid's warps allow
+// in one pass; returns this thread's part of c.e
+__device__ double coarse_product(const PcgArgs &g, const double *c, double *shr)
+{
+    const int nw = blockDim.x >> 5;
+    const int64_t warps = (int64_t)gridDim.x * nw;
+    const int W = 4 * g.nc <= warps ? 4 : 2 * g.nc <= warps ? 2 : 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % W, per = nw / W;
+    double dot = 0.0;
+    for (int64_t row0 = (int64_t)blockIdx.x * per; row0 < g.nc; row0 += (int64_t)gridDim.x * per) {
+        const int64_t row = row0 + warp / W;
+        const bool in = row < g.nc && warp / W < per;
+        double s[4] = {0, 0, 0, 0};
+        if (in) {
+            const double *A = g.ac + row * g.nc;
+            int64_t k = sub * 32 + lane;
+            for (; k + 7 * 32 * W < g.nc; k += 8 * 32 * W)
+#pragma unroll
+                for (int u = 0; u < 8; ++u) s[u & 3] += A[k + 32 * W * u] * c[k + 32 * W * u];
+            for (; k + 3 * 32 * W < g.nc; k += 4 * 32 * W)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[u] += A[k + 32 * W * u] * c[k + 32 * W * u];
+            for (; k < g.nc; k += 32 * W) s[0] += A[k] * c[k];
+        }
+        double t = warp_total((s[0] + s[1]) + (s[2] + s[3]));
+        if (W > 1) {
+            if (lane == 0) shr[warp] = t;
+            __syncthreads();
+            t = 0.0;
+            if (sub == 0)
+                for (int w = 0; w < W; ++w) t += shr[min(warp + w, 31)];
+            __syncthreads();
+        }
+        if (in && sub == 0 && lane == 0) {
+            g.e[row] = t;
+            dot += t * c[row];
+        }
+    }
+    return dot;
+}
+
+// x += alpha p, p = z + beta p (INIT: x = 0, p = z)
+template <int PRE, bool INIT>
+__device__ void direction(const PcgArgs &g, double alpha, double beta)
+{
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    if constexpr (PRE == 2) {
+        for (int64_t n = t0; n < g.nodes; n += nt) {
+            double rv[3], zv[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) rv[i] = g.r[3 * n + i];
+            block_jacobi(g.bdinv + 9 * n, rv, zv);
+            const float4 m = g.mode[n];
+            const int bits = (int)m.w;
+            const double *ea = g.e + 6 * (int64_t)g.agg[n];
+            const double dx = m.x, dy = m.y, dz = m.z;
+            const double cc[3] = {ea[0] + ea[4] * dz - ea[5] * dy, ea[1] + ea[5] * dx - ea[3] * dz,
+                                  ea[2] + ea[3] * dy - ea[4] * dx};
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double z = zv[i] + (((bits >> i) & 1) ? 0.0 : cc[i]);
+                const int64_t k = 3 * n + i;
+                const double p = INIT ? 0.0 : g.p[k];
+                g.x[k] = INIT ? 0.0 : g.x[k] + alpha * p;
+                g.p[k] = INIT ? z : z + beta * p;
+            }
+        }
+    } else {
+        for (int64_t i = t0; i < g.N; i += nt) {
+            double z = g.dinv[i] * g.r[i];
+            if constexpr (PRE == 1) {
+                const int a = g.agg[i];
+                if (a >= 0) z += g.e[a];
+            }
+            const double p = INIT ? 0.0 : g.p[i];
+            g.x[i] = INIT ? 0.0 : g.x[i] + alpha * p;
+            g.p[i] = INIT ? z : z + beta * p;
+        }
+    }
+}
+
+template <int F, int PRE, bool CL>
+__global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_constant__ PcgArgs g)
+{
+    __shared__ CommShared sh;
+    Comm<CL> comm{g, sh};
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    double rz, rr, none = 0.0;
+    const int len = g.max_iter + 2;  // slots of one sum
+    update<PRE, true>(g, 0.0, g.c, rz, rr);
+    if (!comm.template sum<2>(rz, rr, len, 2 * len)) return;
+    if (rr == 0.0) {
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x) g.x[i] = 0.0;
+        if (first) g.out[1] = 1;
+    } else {
+        if constexpr (PRE > 0) {
+            double ce = coarse_product(g, g.c, sh.rows);
+            if (!comm.template sum<1>(ce, none, 3 * len, 0)) return;
+            rz += ce;
+        }
+        direction<PRE, true>(g, 0.0, 0.0);
+        if (!comm.barrier()) return;
+        const double thr = g.tol * g.tol * rr;
+        int it = 0;
+        for (; it < g.max_iter; ++it) {
+            double pq = product<F>(g, g.p, g.q);
+            if (!comm.template sum<1>(pq, none, it, 0)) return;
+            if (!(pq > 0.0)) {
+                if (first) g.out[2] = 1;
+                break;
+            }
+            // c of this iteration; the other one is cleared for the next
+            double *c = g.c + ((it + 1) & 1) * g.nc;
+            const double alpha = rz / pq;
+            double rzn;
+            update<PRE, false>(g, alpha, c, rzn, rr);
+            if (!comm.template sum<2>(rzn, rr, len + it + 1, 2 * len + it + 1)) return;
+            if (rr <= thr) {
+                for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x)
+                    g.x[i] += alpha * g.p[i];
+                if (first) {
+                    g.out[0] = it + 1;
+                    g.out[1] = 1;
+                }
+                break;
+            }
+            if constexpr (PRE > 0) {
+                double ce = coarse_product(g, c, sh.rows);
+                double *other = g.c + (it & 1) * g.nc;
+                for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < g.nc; k += (int64_t)gridDim.x * blockDim.x)
+                    other[k] = 0.0;
+                if (!comm.template sum<1>(ce, none, 3 * len + it + 1, 0)) return;
+                rzn += ce;
+            }
+            direction<PRE, false>(g, alpha, rzn / rz);
+            rz = rzn;
+            if (!comm.barrier()) return;
+        }
+        if (first && it == g.max_iter) g.out[0] = it;
+    }
+    if constexpr (CL) cg::this_cluster().sync();  // shared memory stays until the others have read it
+}
+
+// y = S x by diagonals; dot += x.y; skipped when *done
+template <bool BLOCK>
+__global__ void __launch_bounds__(256) k_dia_spmv64(const __grid_constant__ PcgArgs g, const double *x, double *y,
+                                                    double *dot, const int *done)
+{
+    __shared__ double sh[8];
+    if (done && *done) return;
+    double d = 0.0;
+    const int64_t rows = BLOCK ? g.nodes : g.N;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
+        if constexpr (BLOCK) {
+            double s[3];
+            bdia_node(g.a, g.off, g.nd, g.nodes, i, x, s);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                y[3 * i + k] = s[k];
+                d += x[3 * i + k] * s[k];
+            }
+        } else {
+            const double s = dia_row(g.a, g.off, g.nd, g.N, i, x);
+            y[i] = s;
+            d += x[i] * s;
+        }
+    }
+    if (dot) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = d;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double v = 0.0;
+            for (int w = 0; w < 8; ++w) v += sh[w];
+            atomicAdd(dot, v);
+        }
+    }
+}
+
+// the longest row (length << 32 | row)
+__global__ void k_longest_row(const int32_t *__restrict__ rp, int64_t rows, unsigned long long *best)
+{
+    unsigned long long b = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x)
+        b = max(b, ((unsigned long long)(rp[i + 1] - rp[i]) << 32) | (unsigned long long)i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(best, b);
+}
+
+struct Offsets {
+    int nd;
+    int off[kDiaMax];  // ascending, symmetric about the main diagonal at nd / 2
+};
+
+// Every entry lies on one of the diagonals (else *bad)
+__global__ void k_dia_check(const __grid_constant__ Offsets o, const int32_t *__restrict__ rp,
+                            const int32_t *__restrict__ col, int64_t rows, int *bad)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
+        int32_t k = rp[i];
+        const int32_t e = rp[i + 1];
+        for (int d = 0; d < o.nd && k < e; ++d) k += col[k] - (int)i == o.off[d];
+        if (k < e) atomicExch(bad, 1);  // the columns are sorted
+    }
+}
+
+// BELOW = false: the diagonals on and above the main one (W values per
+// entry).  BELOW = true: compares the entries below with them, *bad where
+// they differ by more than rounding of the main diagonal.
+template <int W, bool BELOW>
+__global__ void k_dia_fill(const __grid_constant__ Offsets o, const int32_t *__restrict__ rp,
+                           const int32_t *__restrict__ col, const double *__restrict__ a, int64_t rows,
+                           double *__restrict__ dia, int *bad)
+{
+    const int h = o.nd / 2;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
+        int32_t k = rp[i];
+        const int32_t e = rp[i + 1];
+        for (int d = 0; d < (BELOW ? h : o.nd); ++d) {
+            const bool hit = k < e && col[k] - (int)i == o.off[d];
+            if (BELOW && hit) {
+                const int64_t at = i + o.off[d];
+                const double tol = 1e-12 * (fabs(dia[i]) + fabs(dia[at]));
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+                    const int t = W == 9 ? (w % 3) * 3 + w / 3 : 0;  // transposed block
+                    const double up = dia[((int64_t)(h - d) * W + t) * rows + at];
+                    if (!(fabs(a[(int64_t)k * W + w] - up) <= tol)) atomicExch(bad, 1);
+                }
+            }
+            if (!BELOW && d >= h)
+#pragma unroll
+                for (int w = 0; w < W; ++w)
+                    dia[((int64_t)(d - h) * W + w) * rows + i] = hit ? a[(int64_t)k * W + w] : 0.0;
+            k += hit;
+        }
+    }
+}
+
+// The pattern's diagonals (scalar rows or node rows): those of its longest
+// row, if every entry lies on one and the padding stays below a quarter.
+void dia_pattern(sfc_system *s)
+{
+    sfc_ctx *ctx = s->ctx;
+    s->dia_tried = true;
+    s->dia_nd = 0;
+    const bool block = s->has_bsr;
+    const int32_t *rp = block ? s->bptr.p : s->row_ptr.p, *col = block ? s->bcol.p : s->col.p;
+    const int64_t rows = block ? s->nodes : s->N, entries = block ? s->nblocks : s->nnz;
+    unsigned long long *best = reinterpret_cast<unsigned long long *>(ctx->dsmall.p + 8);
+    SFC_CK(cudaMemsetAsync(best, 0, sizeof(*best), ctx->stream));
+    k_longest_row<<<grid_for(rows, 256), 256, 0, ctx->stream>>>(rp, rows, best);
+    count_launch(ctx);
+    unsigned long long h = 0;
+    download(ctx, &h, best, 1);
+    const int len = (int)(h >> 32);
+    const int64_t row = (int64_t)(h & 0xffffffffu);
+    if (len < 1 || len > kDiaMax || (double)len * rows > 1.25 * entries + 1024.0 * len) return;
+    int32_t start = 0;
+    download(ctx, &start, rp + row, 1);
+    int32_t c[kDiaMax];
+    download(ctx, c, col + start, len);
+    Offsets o{};
+    o.nd = len;
+    for (int d = 0; d < len; ++d) o.off[d] = c[d] - (int)row;
+    DevInt bad = status_word(ctx, 4);
+    SFC_CK(cudaMemsetAsync(bad.p, 0, sizeof(int), ctx->stream));
+    if (len % 2 == 0 || o.off[len / 2] != 0) return;
+    for (int d = 0; d < len; ++d)
+        if (o.off[d] != -o.off[len - 1 - d]) return;
+    k_dia_check<<<grid_for(rows, 256), 256, 0, ctx->stream>>>(o, rp, col, rows, bad.p);
+    count_launch(ctx);
+    int hb = 1;
+    download(ctx, &hb, bad.p, 1);
+    if (hb) return;
+    s->dia_nd = len;
+    for (int d = 0; d < len; ++d) s->dia_off[d] = o.off[d];
+}
+
+// the diagonal copy of the current operator; false where there is none
+bool dia_prepare(sfc_system *s)
+{
+    sfc_ctx *ctx = s->ctx;
+    if (!s->dia_tried) dia_pattern(s);
+    if (!s->dia_nd) return false;
+    if (s->dia_serial == s->op_serial) return s->dia_ok;
+    const bool block = s->has_bsr;
+    const int64_t rows = block ? s->nodes : s->N;
+    const int kept = s->dia_nd / 2 + 1;
+    try {
+        s->dia.reserve((size_t)kept * rows * (block ? 9 : 1));
+    } catch (const Error &) {  // no room for a second copy of the values
+        s->dia_nd = 0;
+        return false;
+    }
+    Offsets o{};
+    o.nd = s->dia_nd;
+    std::copy(s->dia_off, s->dia_off + o.nd, o.off);
+    const unsigned grid = grid_for(rows, 256);
+    DevInt bad = status_word(ctx, 4);
+    SFC_CK(cudaMemsetAsync(bad.p, 0, sizeof(int), ctx->stream));
+    if (block) {
+        k_dia_fill<9, false><<<grid, 256, 0, ctx->stream>>>(o, s->bptr.p, s->bcol.p, s->bval64.p, rows, s->dia.p, bad.p);
+        k_dia_fill<9, true><<<grid, 256, 0, ctx->stream>>>(o, s->bptr.p, s->bcol.p, s->bval64.p, rows, s->dia.p, bad.p);
+    } else {
+        k_dia_fill<1, false><<<grid, 256, 0, ctx->stream>>>(o, s->row_ptr.p, s->col.p, s->a_op.p, rows, s->dia.p, bad.p);
+        k_dia_fill<1, true><<<grid, 256, 0, ctx->stream>>>(o, s->row_ptr.p, s->col.p, s->a_op.p, rows, s->dia.p, bad.p);
+    }
+    count_launch(ctx, 2);
+    int hb = 1;
+    download(ctx, &hb, bad.p, 1);
+    s->dia_serial = s->op_serial;
+    s->dia_ok = hb == 0;
+    return s->dia_ok;
+}
+
+PcgArgs operator_args(sfc_system *s, bool dia)
+{
+    PcgArgs g{};
+    g.N = s->N;
+    g.nodes = s->nodes;
+    if (dia) {
+        g.a = s->dia.p;
+        const int h = s->dia_nd / 2;
+        g.nd = h + 1;
+        std::copy(s->dia_off + h, s->dia_off + s->dia_nd, g.off);
+    }
+    return g;
+}
+
+using PcgKernel = void (*)(PcgArgs);
+
+}  // namespace
+
+bool dia_spmv64(sfc_system *s, const double *x, double *y, double *dot, const int *done)
+{
+    // only the copy that a solve has made: a single product does not pay for it
+    if (!s->dia_nd || s->dia_serial != s->op_serial || !s->dia_ok) return false;
+    const PcgArgs g = operator_args(s, true);
+    const unsigned grid = grid_for(s->has_bsr ? s->nodes : s->N, 256, s->ctx->sm_count * 8);
+    if (s->has_bsr) k_dia_spmv64<true><<<grid, 256, 0, s->ctx->stream>>>(g, x, y, dot, done);
+    else k_dia_spmv64<false><<<grid, 256, 0, s->ctx->stream>>>(g, x, y, dot, done);
+    return true;
+}
+
+void dia_ensure(sfc_system *s) { dia_prepare(s); }
+
+PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_iter, bool two)
+{
+    sfc_ctx *ctx = s->ctx;
+    const int64_t N = s->N;
+    const CoarseSpace &cs = s->coarse;
+    const int pre = !two ? 0 : cs.dof == 1 ? 1 : 2;
+    const bool dia = dia_prepare(s);
+    PcgArgs g = operator_args(s, dia);
+    // node blocks where there are no diagonals, unless the tuner chose rows
+    const bool blocks = s->has_bsr && (dia || s->spmv_lanes == 0 || pre == 2);
+    const Format f = dia ? (s->has_bsr ? BDIA : DIA) : blocks ? BSR : CSR;
+    if (f == BSR) {
+        g.rp = s->bptr.p;
+        g.col = s->bcol.p;
+        g.a = s->bval64.p;
+    } else if (f == CSR) {
+        g.rp = s->row_ptr.p;
+        g.col = s->col.p;
+        g.a = s->a_op.p;
+        const double avg = (double)s->nnz / (double)std::max<int64_t>(N, 1);
+        g.lanes = s->spmv_lanes > 0 ? s->spmv_lanes : avg > 24 ? 32 : avg > 12 ? 16 : avg > 6 ? 8 : 4;
+    }
+    s->w64.reserve(3 * N);
+    g.b = b;
+    g.x = x;
+    g.r = s->w64.p;
+    g.p = g.r + N;
+    g.q = g.p + N;
+    g.dinv = s->dinv.p;
+    g.bdinv = s->bdinv32.p;
+    if (pre) {
+        s->coarse.c64.reserve(2 * cs.nc);
+        s->coarse.e64.reserve(cs.nc);
+        g.agg = pre == 1 ? cs.agg_free.p : cs.node_agg.p;
+        g.mode = cs.mode.p;
+        g.ac = cs.a64.p;
+        g.nc = cs.nc;
+        g.c = s->coarse.c64.p;
+        g.e = s->coarse.e64.p;
+        SFC_CK(cudaMemsetAsync(g.c, 0, 2 * cs.nc * sizeof(double), ctx->stream));
+    }
+    s->flags.reserve(4);
+    g.out = s->flags.p;
+    g.bar = reinterpret_cast<unsigned *>(s->flags.p + 3);
+    g.tol = tol;
+    g.max_iter = max_iter;
+    SFC_CK(cudaMemsetAsync(s->flags.p, 0, 4 * sizeof(int), ctx->stream));
+    // One cluster of up to 16 blocks while a thread has few rows: a barrier
+    // takes it 1.0 us and a sum 1.5, the grid 1.6 and 2.5.
+    static const PcgKernel table[2][4][3] = {
+        {{k_pcg64<CSR, 0, false>, k_pcg64<CSR, 1, false>, nullptr},
+         {k_pcg64<DIA, 0, false>, k_pcg64<DIA, 1, false>, nullptr},
+         {k_pcg64<BSR, 0, false>, nullptr, k_pcg64<BSR, 2, false>},
+         {k_pcg64<BDIA, 0, false>, nullptr, k_pcg64<BDIA, 2, false>}},
+        {{k_pcg64<CSR, 0, true>, k_pcg64<CSR, 1, true>, nullptr},
+         {k_pcg64<DIA, 0, true>, k_pcg64<DIA, 1, true>, nullptr},
+         {k_pcg64<BSR, 0, true>, nullptr, k_pcg64<BSR, 2, true>},
+         {k_pcg64<BDIA, 0, true>, nullptr, k_pcg64<BDIA, 2, true>}}};
+    SFC_REQUIRE(table[0][f][pre], "no PCG kernel for this operator and preconditioner");
+    const int64_t threads = f == BSR ? s->nodes * 32 : f == CSR ? N * g.lanes : f == BDIA ? s->nodes : N;
+    const double work = f == BSR || f == BDIA ? (double)s->nblocks * 9 : (double)s->nnz;
+    ProfScope ps(ctx, "pcg64", 0.0);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    cfg.stream = ctx->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    bool cluster = work <= kClusterWork;
+    if (cluster) {
+        unsigned blocks = 1;
+        while (blocks < 16 && (int64_t)blocks * 512 < threads) blocks *= 2;
+        const PcgKernel kernel = table[1][f][pre];
+        SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = blocks;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(512);
+        int fit = 0;
+        cluster = cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0;
+        if (cluster) SFC_CK(cudaLaunchKernelEx(&cfg, kernel, g));
+        else cudaGetLastError();
+    }
+    if (!cluster) {
+        const PcgKernel kernel = table[0][f][pre];
+        int occ = 0;
+        SFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 1024, 0));
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+        // blocks of 512 while they fit one to an SM, then one per SM of the
+        // size that spreads the rows over all of them
+        const int64_t sm = ctx->sm_count;
+        const unsigned block = threads <= 512 * sm ? 512 : (unsigned)std::min<int64_t>(1024, ((threads + sm - 1) / sm + 127) / 128 * 128);
+        cfg.blockDim = dim3(block);
+        cfg.gridDim = dim3(grid_for(threads, block, (int)sm * std::max(occ, 1)));
+        const size_t slots = 4 * ((size_t)max_iter + 2);
+        s->scal.reserve(slots);
+        g.sums = s->scal.p;
+        SFC_CK(cudaMemsetAsync(g.sums, 0, slots * sizeof(double), ctx->stream));
+        SFC_CK(cudaLaunchKernelEx(&cfg, kernel, g));
+    }
+    count_launch(ctx);
+    int h[3];
+    download(ctx, h, g.out, 3);
+    if (h[2] == 2) fail(SFC_ERR_TIMEOUT, "a grid barrier of the PCG kernel gave up");
+    if (h[2]) fail(SFC_ERR_NOT_SPD, "PCG breakdown: p^T A p <= 0");
+    return {h[0], h[1] != 0};
+}
+
+}  // namespace sfc

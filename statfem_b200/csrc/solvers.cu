@@ -9,9 +9,8 @@
 //
 // Two methods:
 //  * plain FP64 PCG, one right-hand side at a time (point Jacobi, the
-//    baseline method; or the two-level preconditioner of coarse.cu): CSR SpMV
-//    with sub-warp row groups, fused p.q reduction, fused x/r/z update with
-//    the r.r and r.z reductions;
+//    baseline method; or the two-level preconditioner of coarse.cu): one
+//    persistent kernel (pcg.cu);
 //  * mixed block PCG: up to 128 right-hand sides share each pass over the
 //    FP32 copy of the matrix (one warp per row, each lane owns 1-4 columns of
 //    an RHS-interleaved [N][K] block), iterations in FP32, and an outer FP64
@@ -20,7 +19,7 @@
 //    the FP64 relative-residual target.
 // All reductions accumulate in FP64.  Scalars are kept per iteration (and per
 // column) in device arrays, so no scalar kernel or host round trip sits
-// between the three launches of an iteration; the host checks convergence
+// between the launches of a block iteration; the host checks convergence
 // every `check_every` iterations.
 
 #include <algorithm>
@@ -146,98 +145,6 @@ __global__ void __launch_bounds__(kRedThreads) k_bspmv64(const int32_t *__restri
     if (dot) {
         d = block_sum(d, sh);
         if (threadIdx.x == 0) atomicAdd(dot, d);
-    }
-}
-
-// r = b' (lifted rhs), x = 0, p = z = D^-1 r; rz0 = r.z, bb = r.r
-__global__ void __launch_bounds__(kRedThreads) k_pcg_init(const double *__restrict__ b, const double *__restrict__ dinv,
-                                                           double *__restrict__ x, double *__restrict__ r,
-                                                           double *__restrict__ p, int64_t N, double *rz0, double *bb)
-{
-    __shared__ double sh[32];
-    double a = 0, c = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const double ri = b[i], zi = dinv[i] * ri;
-        x[i] = 0.0;
-        r[i] = ri;
-        p[i] = zi;
-        a += ri * zi;
-        c += ri * ri;
-    }
-    a = block_sum(a, sh);
-    c = block_sum(c, sh);
-    if (threadIdx.x == 0) {
-        atomicAdd(rz0, a);
-        atomicAdd(bb, c);
-    }
-}
-
-// alpha = rz/pq; x += alpha p; r -= alpha q; z = D^-1 r; rz' = r.z; rr' = r.r
-__global__ void __launch_bounds__(kRedThreads) k_pcg_update(double *__restrict__ x, double *__restrict__ r,
-                                                             const double *__restrict__ p, const double *__restrict__ q,
-                                                             const double *__restrict__ dinv, int64_t N,
-                                                             const double *pq, const double *rz, double *rz_next,
-                                                             double *rr_next, const int *done, int *err)
-{
-    __shared__ double sh[32];
-    if (*done) return;
-    const double den = *pq;
-    if (!(den > 0.0)) {
-        if (threadIdx.x == 0) atomicExch(err, 1);
-        return;
-    }
-    const double alpha = *rz / den;
-    double a = 0, c = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        x[i] += alpha * p[i];
-        const double ri = r[i] - alpha * q[i];
-        r[i] = ri;
-        const double zi = dinv[i] * ri;
-        a += ri * zi;
-        c += ri * ri;
-    }
-    a = block_sum(a, sh);
-    c = block_sum(c, sh);
-    if (threadIdx.x == 0) {
-        atomicAdd(rz_next, a);
-        atomicAdd(rr_next, c);
-    }
-}
-
-// convergence test on rr'; else beta = rz'/rz, p = D^-1 r + beta p
-__global__ void k_pcg_pupdate(double *__restrict__ p, const double *__restrict__ r, const double *__restrict__ dinv,
-                              int64_t N, const double *rz, const double *rz_next, const double *rr_next, double thr,
-                              int it_next, int *done, const int *err)
-{
-    if (*done || *err) return;
-    if (*rr_next <= thr) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *done = it_next;
-        return;
-    }
-    const double beta = *rz_next / *rz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = dinv[i] * r[i] + beta * p[i];
-}
-
-// scalar two-level variant: p = D^-1 r + e[agg(i)] + beta p (INIT: p = z)
-template <bool INIT>
-__global__ void k_pcg1_pupdate(double *__restrict__ p, const double *__restrict__ r, const double *__restrict__ dinv,
-                               const int32_t *__restrict__ node_agg, const float4 *__restrict__ mode,
-                               const double *__restrict__ e, int64_t N, const double *rz, const double *rz_next,
-                               const double *rr_next, double thr, int it_next, int *done, const int *err)
-{
-    double beta = 0.0;
-    if constexpr (!INIT) {
-        if (*done || *err) return;
-        if (*rr_next <= thr) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) *done = it_next;
-            return;
-        }
-        beta = *rz_next / *rz;
-    }
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const double z = dinv[i] * r[i] + (((int)mode[i].w & 1) ? 0.0 : e[node_agg[i]]);
-        p[i] = INIT ? z : z + beta * p[i];
     }
 }
 
@@ -1102,121 +1009,6 @@ __global__ void __launch_bounds__(256, 4) k_ncpupdate32(float *__restrict__ p, c
     }
 }
 
-// ---- FP64 two-level PCG (one vector, 3-dof nodes, thread per node) ---------
-__device__ __forceinline__ void bj_apply64(const float *__restrict__ D, const double (&r)[3], double (&z)[3])
-{
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-        z[i] = (double)D[3 * i] * r[0] + (double)D[3 * i + 1] * r[1] + (double)D[3 * i + 2] * r[2];
-}
-
-// r = b, x = 0; rz0 += r . Dinv r (block-Jacobi share), bb += r . r
-__global__ void __launch_bounds__(kRedThreads) k_pcg2_init(const double *__restrict__ b, const float *__restrict__ bdinv,
-                                                            double *__restrict__ x, double *__restrict__ r,
-                                                            int64_t nodes, double *rz0, double *bb)
-{
-    __shared__ double sh[32];
-    double a = 0, c = 0;
-    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nodes; n += (int64_t)gridDim.x * blockDim.x) {
-        double rv[3], zv[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            rv[i] = b[3 * n + i];
-            r[3 * n + i] = rv[i];
-            x[3 * n + i] = 0.0;
-        }
-        bj_apply64(bdinv + 9 * n, rv, zv);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            a += rv[i] * zv[i];
-            c += rv[i] * rv[i];
-        }
-    }
-    a = block_sum(a, sh);
-    c = block_sum(c, sh);
-    if (threadIdx.x == 0) {
-        atomicAdd(rz0, a);
-        atomicAdd(bb, c);
-    }
-}
-
-// alpha = rz/pq; x += alpha p; r -= alpha q; rz' += r . Dinv r; rr' += r . r
-__global__ void __launch_bounds__(kRedThreads) k_pcg2_update(double *__restrict__ x, double *__restrict__ r,
-                                                              const double *__restrict__ p, const double *__restrict__ q,
-                                                              const float *__restrict__ bdinv, int64_t nodes,
-                                                              const double *pq, const double *rz, double *rz_next,
-                                                              double *rr_next, const int *done, int *err)
-{
-    __shared__ double sh[32];
-    if (*done) return;
-    const double den = *pq;
-    if (!(den > 0.0)) {
-        if (threadIdx.x == 0) atomicExch(err, 1);
-        return;
-    }
-    const double alpha = *rz / den;
-    double a = 0, c = 0;
-    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nodes; n += (int64_t)gridDim.x * blockDim.x) {
-        double rv[3], zv[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const int64_t k = 3 * n + i;
-            x[k] += alpha * p[k];
-            rv[i] = r[k] - alpha * q[k];
-            r[k] = rv[i];
-        }
-        bj_apply64(bdinv + 9 * n, rv, zv);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            a += rv[i] * zv[i];
-            c += rv[i] * rv[i];
-        }
-    }
-    a = block_sum(a, sh);
-    c = block_sum(c, sh);
-    if (threadIdx.x == 0) {
-        atomicAdd(rz_next, a);
-        atomicAdd(rr_next, c);
-    }
-}
-
-// convergence test on rr'; else p = Dinv r + M e + beta p (INIT: p = z)
-template <bool INIT>
-__global__ void k_pcg2_pupdate(double *__restrict__ p, const double *__restrict__ r, const float *__restrict__ bdinv,
-                               const int32_t *__restrict__ node_agg, const float4 *__restrict__ mode,
-                               const double *__restrict__ e, int64_t nodes, const double *rz,
-                               const double *rz_next, const double *rr_next, double thr, int it_next, int *done,
-                               const int *err)
-{
-    double beta = 0.0;
-    if constexpr (!INIT) {
-        if (*done || *err) return;
-        if (*rr_next <= thr) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) *done = it_next;
-            return;
-        }
-        beta = *rz_next / *rz;
-    }
-    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nodes; n += (int64_t)gridDim.x * blockDim.x) {
-        double rv[3], zv[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) rv[i] = r[3 * n + i];
-        bj_apply64(bdinv + 9 * n, rv, zv);
-        const int64_t a = node_agg[n];
-        const float4 m = mode[n];
-        const int bits = (int)m.w;
-        const double *ea = e + 6 * a;
-        const double dx = m.x, dy = m.y, dz = m.z;
-        const double c[3] = {ea[0] + ea[4] * dz - ea[5] * dy, ea[1] + ea[5] * dx - ea[3] * dz,
-                             ea[2] + ea[3] * dy - ea[4] * dx};
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double z = zv[i] + (((bits >> i) & 1) ? 0.0 : c[i]);
-            p[3 * n + i] = INIT ? z : z + beta * p[3 * n + i];
-        }
-    }
-}
-
 // Convergence test after every inner iteration of a check interval: the
 // first iteration after which all columns are below their thresholds sets
 // *stop (every later kernel of the interval returns at once) and records in
@@ -1374,10 +1166,6 @@ __global__ void k_fix_apply(const int32_t *__restrict__ diag, const double *__re
 // ---------------------------------------------------------------------------
 // host drivers
 // ---------------------------------------------------------------------------
-struct PcgResult {
-    int iters;
-    bool converged;
-};
 
 void launch_spmv64(sfc_system *s, const double *x, double *y, double *dot, const int *done)
 {
@@ -1389,6 +1177,10 @@ void launch_spmv64(sfc_system *s, const double *x, double *y, double *dot, const
                                            : (double)s->nnz * 12 + 4.0 * (s->N + 1)) +
                      16.0 * s->N);
     const unsigned grid = (unsigned)(ctx->sm_count * 8);
+    if (lanes == 0 && dia_spmv64(s, x, y, dot, done)) {  // the diagonal copy of a lattice-numbered mesh
+        count_launch(ctx);
+        return;
+    }
     if (lanes == 0 && s->has_bsr) {  // 3-dof mesh: node blocks
         k_bspmv64<<<grid_for(s->nodes * 32, kRedThreads, grid), kRedThreads, 0, ctx->stream>>>(
             s->bptr.p, s->bcol.p, s->bval64.p, x, y, s->nodes, dot, done);
@@ -1415,102 +1207,6 @@ bool use_two_level(sfc_system *s)
     if (s->opt.precond != SFC_PRECOND_TWO_LEVEL) return false;
     if (s->has_bsr && !s->bdinv32.p) return false;  // 3-dof mesh without its block-Jacobi smoother
     return coarse_prepare(s);
-}
-
-// FP64 PCG on S x = b (device vectors, length N): point Jacobi, or with
-// `two` the two-level preconditioner (nodal block Jacobi + coarse correction;
-// the caller has run coarse_prepare)
-PcgResult pcg64(sfc_system *s, const double *b, double *x, double tol, int max_iter, int check, bool two)
-{
-    sfc_ctx *ctx = s->ctx;
-    const int64_t N = s->N;
-    s->w64.reserve(3 * N);
-    double *r = s->w64.p, *p = r + N, *q = p + N;
-    const int nsc = 3 * (max_iter + 2) + 1;
-    s->scal.reserve(nsc);
-    double *pq = s->scal.p, *rz = pq + (max_iter + 2), *rr = rz + (max_iter + 2), *bb = rr + (max_iter + 2);
-    s->flags.reserve(2);
-    int *done = s->flags.p, *err = s->flags.p + 1;
-    SFC_CK(cudaMemsetAsync(s->scal.p, 0, nsc * sizeof(double), ctx->stream));
-    SFC_CK(cudaMemsetAsync(s->flags.p, 0, 2 * sizeof(int), ctx->stream));
-    const unsigned g = grid_for(N, kRedThreads, ctx->sm_count * 4);
-    const int64_t nodes = s->nodes;
-    const unsigned gn = grid_for(nodes, kRedThreads, ctx->sm_count * 4);
-    const CoarseSpace &cs = s->coarse;
-    const bool two1 = two && cs.dof == 1;  // scalar mesh: point Jacobi + constant modes
-    two = two && cs.dof == 3;
-    if (two1) {
-        k_pcg_init<<<g, kRedThreads, 0, ctx->stream>>>(b, s->dinv.p, x, r, p, N, rz, bb);  // rz: Jacobi share
-        count_launch(ctx);
-        coarse_vec_apply(s, r, rz, nullptr);
-        k_pcg1_pupdate<true><<<g, kRedThreads, 0, ctx->stream>>>(p, r, s->dinv.p, cs.node_agg.p, cs.mode.p, cs.e64.p,
-                                                                 N, nullptr, nullptr, nullptr, 0.0, 0, done, err);
-    } else if (two) {
-        k_pcg2_init<<<gn, kRedThreads, 0, ctx->stream>>>(b, s->bdinv32.p, x, r, nodes, rz, bb);
-        count_launch(ctx);
-        coarse_vec_apply(s, r, rz, nullptr);
-        k_pcg2_pupdate<true><<<gn, kRedThreads, 0, ctx->stream>>>(p, r, s->bdinv32.p, cs.node_agg.p, cs.mode.p,
-                                                                  cs.e64.p, nodes, nullptr, nullptr, nullptr, 0.0, 0,
-                                                                  done, err);
-    } else {
-        k_pcg_init<<<g, kRedThreads, 0, ctx->stream>>>(b, s->dinv.p, x, r, p, N, rz, bb);
-    }
-    count_launch(ctx);
-    double hbb = 0;
-    download(ctx, &hbb, bb, 1);
-    if (hbb == 0.0) return {0, true};
-    const double thr = tol * tol * hbb;
-    int it = 0;
-    PcgResult res{max_iter, false};
-    for (it = 0; it < max_iter; ++it) {
-        launch_spmv64(s, p, q, pq + it, done);
-        if (two) {
-            {
-                ProfScope ps(ctx, "pcg_update", 56.0 * N + 36.0 * nodes);
-                k_pcg2_update<<<gn, kRedThreads, 0, ctx->stream>>>(x, r, p, q, s->bdinv32.p, nodes, pq + it, rz + it,
-                                                                   rz + it + 1, rr + it + 1, done, err);
-            }
-            count_launch(ctx);
-            coarse_vec_apply(s, r, rz + it + 1, done);
-            {
-                ProfScope ps(ctx, "pcg_pupdate", 32.0 * N + 56.0 * nodes);
-                k_pcg2_pupdate<false><<<gn, kRedThreads, 0, ctx->stream>>>(
-                    p, r, s->bdinv32.p, cs.node_agg.p, cs.mode.p, cs.e64.p, nodes, rz + it, rz + it + 1, rr + it + 1,
-                    thr, it + 1, done, err);
-            }
-            count_launch(ctx);
-        } else {
-            {
-                ProfScope ps(ctx, "pcg_update", 56.0 * N);
-                k_pcg_update<<<g, kRedThreads, 0, ctx->stream>>>(x, r, p, q, s->dinv.p, N, pq + it, rz + it,
-                                                                 rz + it + 1, rr + it + 1, done, err);
-            }
-            if (two1) {
-                count_launch(ctx);
-                coarse_vec_apply(s, r, rz + it + 1, done);
-                ProfScope ps(ctx, "pcg_pupdate", 32.0 * N + 12.0 * N);
-                k_pcg1_pupdate<false><<<g, kRedThreads, 0, ctx->stream>>>(p, r, s->dinv.p, cs.node_agg.p, cs.mode.p,
-                                                                          cs.e64.p, N, rz + it, rz + it + 1,
-                                                                          rr + it + 1, thr, it + 1, done, err);
-                count_launch(ctx);
-            } else {
-                ProfScope ps(ctx, "pcg_pupdate", 32.0 * N);
-                k_pcg_pupdate<<<g, kRedThreads, 0, ctx->stream>>>(p, r, s->dinv.p, N, rz + it, rz + it + 1,
-                                                                  rr + it + 1, thr, it + 1, done, err);
-                count_launch(ctx, 2);
-            }
-        }
-        if ((it + 1) % check == 0 || it + 1 == max_iter) {
-            int hf[2];
-            download(ctx, hf, s->flags.p, 2);
-            if (hf[1]) fail(SFC_ERR_NOT_SPD, "PCG breakdown: p^T A p <= 0");
-            if (hf[0]) {
-                res = {hf[0], true};
-                break;
-            }
-        }
-    }
-    return res;
 }
 
 double true_rel_residual(sfc_system *s, const double *b, const double *x)
@@ -1956,7 +1652,7 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             count_launch(ctx);
             const double bn = std::sqrt(hb[c]), r = std::sqrt(rn[c]);
             if (r > tol * bn) {
-                PcgResult pr = pcg64(s, s->tmpN.p, s->tmpN2.p, tol * bn / r, max_iter, check, two_any);
+                PcgStats pr = pcg64(s, s->tmpN.p, s->tmpN2.p, tol * bn / r, max_iter, two_any);
                 if (!pr.converged) all_conv = false;
                 if (debug)
                     std::fprintf(stderr, "[sfc block %d] column %d: FP64 fallback from rel %.3e, %d iterations%s\n", c0,
@@ -2021,12 +1717,6 @@ void lifted_rhs(sfc_system *s, double *b)
     k_lift<<<grid_for(s->N, 256), 256, 0, s->ctx->stream>>>(s->row_ptr.p, s->col.p, s->diag.p, s->a_ref.p, s->mask.p,
                                                            s->F.p, s->N, b);
     count_launch(s->ctx);
-}
-
-PcgStats pcg64_public(sfc_system *s, const double *b, double *x, double tol, int max_iter, int check)
-{
-    PcgResult r = pcg64(s, b, x, tol, max_iter, check, false);
-    return {r.iters, r.converged};
 }
 
 double device_dot(sfc_ctx *ctx, const double *a, const double *b, int64_t n)
@@ -2106,12 +1796,12 @@ void solve_forward(sfc_system *s, bool direct)
     s->solve_ev.ensure();
     cudaEvent_t e0 = s->solve_ev.a, e1 = s->solve_ev.b;
     SFC_CK(cudaEventRecord(e0, ctx->stream));
-    PcgResult r;
+    PcgStats r;
     bool two = false;
     {
         ProfScope ps(ctx, "phase:forward_solve", 0.0);
         two = use_two_level(s);
-        r = pcg64(s, b.p, s->X.p, tol, max_iter, check, two);
+        r = pcg64(s, b.p, s->X.p, tol, max_iter, two);
     }
     SFC_CK(cudaEventRecord(e1, ctx->stream));
     const double rel = true_rel_residual(s, b.p, s->X.p);
@@ -2162,7 +1852,7 @@ void solve_block(sfc_system *s, const double *B, double *X, int nrhs, int ld)
         for (int a = 0; a < nrhs; ++a) {
             k_gather_cols<<<grid_for(N, 256), 256, 0, ctx->stream>>>(B, ld, a, 1, 1, N, b.p);
             count_launch(ctx);
-            PcgResult r = pcg64(s, b.p, x.p, tol, max_iter, check, two);
+            PcgStats r = pcg64(s, b.p, x.p, tol, max_iter, two);
             st.iterations = std::max(st.iterations, r.iters);
             if (!r.converged) st.converged = 0;
             k_scatter_cols<<<grid_for(N, 256), 256, 0, ctx->stream>>>(x.p, ld, a, 1, 1, N, X);
