@@ -82,6 +82,26 @@ void transpose64(sfc_ctx *ctx, const double *in, double *out, int64_t rows, int6
     count_launch(ctx);
 }
 
+// Solves for host right-hand sides: the caller's [nrhs][N] columns go up as
+// they are and are transposed to the interleaved [N][nrhs] layout on the GPU
+// (and back).  The arrays stay with the system up to 256 MB, so that a
+// repeated call does not allocate.
+template <class F>
+void solve_host_columns(sfc_system *s, const double *rhs, double *u, int nrhs, F solve)
+{
+    const int64_t N = s->N;
+    const size_t n = (size_t)N * nrhs;
+    upload(s->ctx, s->host_cols[0], rhs, n);
+    s->host_cols[1].reserve(n);
+    transpose64(s->ctx, s->host_cols[0].p, s->host_cols[1].p, nrhs, N);
+    s->host_cols[2].reserve(n);
+    solve(s->host_cols[1].p, s->host_cols[2].p);
+    transpose64(s->ctx, s->host_cols[2].p, s->host_cols[0].p, N, nrhs);
+    download(s->ctx, u, s->host_cols[0].p, n);
+    if (3 * n * sizeof(double) > ((size_t)256 << 20))
+        for (auto &b : s->host_cols) b.release();
+}
+
 void ensure_vectors(sfc_system *s)
 {
     if (!s->F.p) {
@@ -452,18 +472,10 @@ int32_t sfc_solve_transpose(sfc_system_t *s, const double *rhs, double *u, int32
     if (!s || !rhs || !u || nrhs <= 0) return SFC_ERR_BAD_ARG;
     return guard(s->ctx, [&] {
         flush_staged(s);
-        const int64_t N = s->N;
-        std::vector<double> Bt((size_t)N * nrhs);
-        for (int a = 0; a < nrhs; ++a)
-            for (int64_t i = 0; i < N; ++i) Bt[(size_t)i * nrhs + a] = rhs[(size_t)a * N + i];
-        DBuf<double> B, X;
-        upload(s->ctx, B, Bt.data(), Bt.size());
-        X.alloc((size_t)N * nrhs);
-        solve_block(s, B.p, X.p, nrhs, nrhs);
-        transpose_fixup(s, B.p, X.p, nrhs, nrhs);
-        download(s->ctx, Bt.data(), X.p, Bt.size());
-        for (int a = 0; a < nrhs; ++a)
-            for (int64_t i = 0; i < N; ++i) u[(size_t)a * N + i] = Bt[(size_t)i * nrhs + a];
+        solve_host_columns(s, rhs, u, nrhs, [&](const double *B, double *X) {
+            solve_block(s, B, X, nrhs, nrhs);
+            transpose_fixup(s, B, X, nrhs, nrhs);
+        });
     });
 }
 
@@ -472,17 +484,7 @@ int32_t sfc_solve_multi(sfc_system_t *s, const double *rhs, double *u, int32_t n
     if (!s || !rhs || !u || nrhs <= 0) return SFC_ERR_BAD_ARG;
     return guard(s->ctx, [&] {
         flush_staged(s);
-        const int64_t N = s->N;
-        // the caller's [nrhs][N] columns go up as they are and are transposed
-        // to the interleaved [N][nrhs] layout on the GPU (and back)
-        DBuf<double> C, B, X;
-        upload(s->ctx, C, rhs, (size_t)N * nrhs);
-        B.alloc((size_t)N * nrhs);
-        transpose64(s->ctx, C.p, B.p, nrhs, N);
-        X.alloc((size_t)N * nrhs);
-        solve_multi(s, B.p, X.p, nrhs, nrhs);
-        transpose64(s->ctx, X.p, C.p, N, nrhs);
-        download(s->ctx, u, C.p, (size_t)N * nrhs);
+        solve_host_columns(s, rhs, u, nrhs, [&](const double *B, double *X) { solve_multi(s, B, X, nrhs, nrhs); });
     });
 }
 
@@ -501,6 +503,12 @@ static int give_vec(const sfc_system *s, const double *src, const uint32_t *dofs
     sfc_system *sm = const_cast<sfc_system *>(s);
     return guard(sm->ctx, [&] {
         SFC_REQUIRE(src, "vector not available (solve first)");
+        int64_t run = 0;  // the leading dofs in order, as most callers ask for all of them
+        while (run < n && run < s->N && dofs[run] == (uint64_t)run) ++run;
+        if (run == n) {
+            download(sm->ctx, out, src, n);
+            return;
+        }
         std::vector<double> h(s->N);
         download(sm->ctx, h.data(), src, s->N);
         for (int64_t t = 0; t < n; ++t) {
