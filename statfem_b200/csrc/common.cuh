@@ -452,7 +452,7 @@ struct sfc_system {
     sfc::DBuf<int> lat_err;   // bounded-wait status of the staged SpMM
     CUtensorMap pmap{};       // TMA view of the block operand P as (K, 3, nx, ny, nz)
     const float *pmap_ptr = nullptr;
-    int pmap_K = 0;
+    int pmap_K = 0, pmap_box = 0;
     // vectors
     sfc::DBuf<double> F, X;
     sfc::DBuf<unsigned char> mask;   // 1 for constrained dofs
@@ -568,7 +568,7 @@ void lattice_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, 
 void lattice_prepare(sfc_system *s, const float *P, int K);
 void lattice_check(sfc_system *s);
 void xline_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, const int *stop);
-void xline_prepare(int K);
+void xline_prepare(sfc_system *s, const float *P, int K);
 void xline_resid64(sfc_system *s, const double *X, const double *B, double *R, int K, double *rr);
 void xresid_prepare(int K);
 void coarse_block_reserve(sfc_system *s, int K);

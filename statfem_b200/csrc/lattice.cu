@@ -8,9 +8,8 @@
 // (dz, dy, dx) (zero where the lattice has no neighbour), rows padded to four
 // floats so a warp reads a block with three 16-byte broadcast loads.  P and Q
 // are the block solver's RHS-interleaved [N][K] FP32 arrays.  Two products
-// use this view: the streamed x-line kernel k_xspmm32 (the default; described
-// at the kernel) and the TMA-staged brick kernel k_lspmm32 below
-// (SFC_SPMM=lattice).
+// use this view: the streamed kernel k_tspmm32 (the default; described at the
+// kernel) and the TMA-staged brick kernel k_lspmm32 below (SFC_SPMM=lattice).
 //
 // Staged bricks.  A work item is a brick of 4 x 2 x 2 output nodes and a
 // 64-column slice of the block.  One elected thread issues a single 5-D TMA
@@ -101,6 +100,15 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                  "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
                  : "memory");
+}
+
+// the nine values of a block
+__device__ __forceinline__ void ld_block(const float *bp, float (&m)[9])
+{
+    const float4 a = *reinterpret_cast<const float4 *>(bp), b = *reinterpret_cast<const float4 *>(bp + 4);
+    m[0] = a.x, m[1] = a.y, m[2] = a.z, m[3] = a.w;
+    m[4] = b.x, m[5] = b.y, m[6] = b.z, m[7] = b.w;
+    m[8] = bp[8];
 }
 
 struct Brick {
@@ -214,15 +222,14 @@ __global__ void __launch_bounds__(128 * H, 2)
                         const int dx = cx - ox;  // lattice offset dx - 1
                         if (dx < 0 || dx > 2) continue;
                         const float *bp = bb + ox * NODE_FLOATS + (dz * 9 + dy * 3 + dx) * SLOT;
-                        const float4 bm[3] = {*reinterpret_cast<const float4 *>(bp),
-                                              *reinterpret_cast<const float4 *>(bp + 4),
-                                              *reinterpret_cast<const float4 *>(bp + 8)};
+                        float bm[9];
+                        ld_block(bp, bm);
 #pragma unroll
                         for (int r = 0; r < 3; ++r)
 #pragma unroll
                             for (int v = 0; v < V; ++v)
-                                acc[ox][r][v] =
-                                    fmaf(bm[r].z, p[2][v], fmaf(bm[r].y, p[1][v], fmaf(bm[r].x, p[0][v], acc[ox][r][v])));
+                                acc[ox][r][v] = fmaf(bm[3 * r + 2], p[2][v],
+                                                     fmaf(bm[3 * r + 1], p[1][v], fmaf(bm[3 * r], p[0][v], acc[ox][r][v])));
                     }
                 }
             }
@@ -282,38 +289,223 @@ __global__ void k_lattice_fill(const int32_t *__restrict__ bptr, const int32_t *
                 continue;
             }
             const int slot = (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1);
-            bq[i * NODE_FLOATS + slot * SLOT + (k / 3) * 4 + k % 3] = b32[(int64_t)(b0 + t) * 9 + k];
+            // FP32: nine values in a row (two 16-byte loads and one of four);
+            // FP64: rows padded to four
+            const int at = sizeof(T) == 4 ? k : (k / 3) * 4 + k % 3;
+            bq[i * NODE_FLOATS + slot * SLOT + at] = b32[(int64_t)(b0 + t) * 9 + k];
         }
     }
 }
 
-// Streamed lattice product (the default on lattices): one warp per
-// contiguous run of output nodes (numbered x fastest, so a run is a few x-line
-// segments), all K = 32 V columns of the block, V per lane.  The warp walks
-// each segment's column positions cx along x; at each it loads the P rows of
-// the nine neighbour lines (y + dy, z + dz) once and applies them to the
-// three output nodes cx - 1, cx, cx + 1 that couple to them, keeping a
-// sliding window of three output nodes' accumulators in registers.  Output
-// cx - 1 then has all its columns and is stored.  Every P row read from L1
-// therefore feeds three outputs (against one in the node-block kernel), and a
-// block's nine values (three 16-byte shared loads, the same address in every
-// lane) feed 9 V FMAs per lane.
+// Streamed lattice product (the default on lattices).  A CTA takes a tile of
+// TY x TZ x-lines, one per warp, and walks along x.  The tile's P rows with
+// its halo of neighbour lines (one 5-D TMA load, zero-filled outside the
+// lattice) and each line's 27 blocks of the next output (one bulk copy of
+// 1,296 bytes) are staged in shared memory one position ahead.  At position
+// cx a warp reads the three P rows of its nine neighbour lines once and
+// applies them to the three outputs cx - 1, cx, cx + 1 that couple to them,
+// in a sliding window of accumulators.
 //
-// Each block is read exactly once, so a load of it from global memory would
-// miss L1 and stall the FMAs that follow it.  Every output node's 27 blocks
-// (1296 bytes) are instead copied by cp.async into a per-warp ring of four
-// rows in shared memory one position before their first use (the three rows
-// in use and the one in flight), and the FMAs read them there.  Neighbour
-// lines outside the lattice are clamped to a line inside it: their blocks are
-// zero, so they add nothing; outputs outside the segment are computed from
-// stale ring rows and never stored.  p.q column dots in FP64.
-constexpr int XR = 4;  // block ring rows per warp
+// What bounds it: the issue of the FMAs (9 per block and column, 102 us at
+// 48^3 and 128 columns; FMA pipe 48 % active, issue slots 62 %, the rest the
+// two halo positions of a piece and the ragged tiles) with the shared-memory
+// loads beside them (50 % of their path: a 16-byte load takes four cycles
+// even when all lanes read one address, so a block is read as two of them and
+// one of 4 bytes).  Measured at 48^3 and 32^3 nodes, 128 columns, us:
+//   219, 74  this kernel
+//   231, 79  with a producer warp of its own (96 registers, spills)
+//   244, 84  with three 16-byte loads per block
+//   258, 85  a half-warp per line, eight columns per lane (half the block
+//            loads, but two warps per scheduler)
+//   260, 95  the same walk with the P rows loaded from L2 into registers:
+//            nine rows per output, 1.9 GB at 48^3; the tile moves three
+//
+// The lines of work are cut into equal contiguous pieces over the resident
+// CTAs (tiles in z-fastest order, so that CTAs next to one another share
+// their halo planes in L2 at about the same time).  Outputs outside a piece
+// are accumulated from stale ring rows and never stored.  p.q column dots in
+// FP64.  Waits on the mbarriers are bounded: one that gives up sets lat_err,
+// waits once more for the copies in flight and leaves (SFC_ERR_TIMEOUT).
+constexpr int TY = 4, TZ = 2, TL = TY * TZ;    // lines per tile
+constexpr int UY = TY + 2, UZ = TZ + 2;        // with the halo
+constexpr int TS = 2;                          // stages
+constexpr int TR = 4;                          // block ring rows per line: three in use, one in flight
 
-template <int V>
-constexpr size_t xsmem()
+template <int K>
+constexpr int tstage_floats()
 {
-    return (size_t)8 * 32 * V * sizeof(double) + (size_t)8 * XR * NODE_FLOATS * sizeof(float);
+    return UY * UZ * 3 * K;
 }
+template <int K>
+constexpr size_t tsmem()
+{
+    return (size_t)(TS * tstage_floats<K>() + TL * TR * NODE_FLOATS) * sizeof(float) + 2 * TS * sizeof(uint64_t) + 128;
+}
+
+// one piece of a CTA's range: outputs [x0, x1] of the lines of tile (y0, z0)
+struct Piece {
+    int y0, z0, x0, x1;
+};
+
+__device__ __forceinline__ Piece piece_at(int64_t g, int64_t g1, int nx, int tz_n)
+{
+    const int64_t t = g / nx;
+    Piece p;
+    p.x0 = (int)(g - t * nx);
+    p.x1 = (int)(min((t + 1) * nx, g1) - 1 - t * nx);
+    p.z0 = (int)(t % tz_n) * TZ;
+    p.y0 = (int)(t / tz_n) * TY;
+    return p;
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+template <int K>
+__global__ void __launch_bounds__(32 * TL, 2)
+    k_tspmm32(const __grid_constant__ CUtensorMap pmap, const float *__restrict__ bq, float *__restrict__ Q, int nx,
+              int ny, int nz, int64_t total, double *pq, const int *stop, int *err)
+{
+    constexpr int C = K / 32;  // columns per lane
+    constexpr int STAGE = tstage_floats<K>();
+    if (*stop) return;
+    extern __shared__ __align__(128) unsigned char traw[];
+    float *stage = reinterpret_cast<float *>(traw);
+    float *ring = stage + TS * STAGE;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(ring + TL * TR * NODE_FLOATS);
+    const uint32_t full = smem_u32(bars), empty = full + 8 * TS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < TS; ++k) {
+            mbar_init(full + 8 * k, TL);
+            mbar_init(empty + 8 * k, TL);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    const int tz_n = (nz + TZ - 1) / TZ;
+    const int64_t g1 = total * (blockIdx.x + 1) / gridDim.x;
+    const int wy = warp % TY, wz = warp / TY;
+    float *own_ring = ring + warp * TR * NODE_FLOATS;
+    // Staging of position t: every warp announces its line's blocks, the first
+    // one the tile's P rows too, once all warps have left the stage's last use.
+    auto produce = [&](const Piece &p, int cx, uint32_t t) -> bool {
+        const uint32_t st = t % TS, bar = full + 8 * st;
+        if (warp == 0 && t >= TS && !mbar_wait(empty + 8 * st, ((t / TS) - 1) & 1)) return false;
+        if (lane == 0) {
+            const int y = p.y0 + wy, z = p.z0 + wz;
+            const bool blocks = cx + 1 >= p.x0 && cx + 1 <= p.x1 && y < ny && z < nz;
+            mbar_expect_tx(bar, (warp == 0 ? STAGE * 4 : 0) + (blocks ? NODE_FLOATS * 4 : 0));
+            if (warp == 0) tma_load_5d(smem_u32(stage + st * STAGE), &pmap, bar, 0, 0, cx, p.y0 - 1, p.z0 - 1);
+            if (blocks)
+                bulk_load(smem_u32(own_ring + (t % TR) * NODE_FLOATS),
+                          bq + (((int64_t)z * ny + y) * nx + cx + 1) * NODE_FLOATS, NODE_FLOATS * 4, bar);
+        }
+        return true;
+    };
+    double dacc[C];
+#pragma unroll
+    for (int v = 0; v < C; ++v) dacc[v] = 0.0;
+    bool ok = true;
+    uint32_t t = 0;  // position counter of the CTA's whole walk
+    int64_t g = total * blockIdx.x / gridDim.x;
+    Piece p = piece_at(g, g1, nx, tz_n);
+    if (g < g1) produce(p, p.x0 - 1, 0);
+    while (g < g1 && ok) {
+        const int y = p.y0 + wy, z = p.z0 + wz;
+        const bool line = y < ny && z < nz;  // a warp past the face computes what it does not store
+        float *ql = Q + ((int64_t)z * ny + y) * nx * (3 * K) + lane * C;
+        g += p.x1 - p.x0 + 1;
+        float acc[3][3][C], pc[3][C];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int v = 0; v < C; ++v) acc[0][r][v] = acc[1][r][v] = acc[2][r][v] = pc[r][v] = 0.f;
+        for (int cx = p.x0 - 1; cx <= p.x1 + 1; ++cx, ++t) {
+            const uint32_t st = t % TS;
+            if (!mbar_wait(full + 8 * st, (t / TS) & 1)) {
+                ok = false;
+                break;
+            }
+            // neighbour line (dz, dy) lies (dz UY + dy) 3 K on
+            const float *base = stage + st * STAGE + (wz * UY + wy) * 3 * K + lane * C;
+            // output cx - 1 + o has its blocks in ring row t - 2 + o
+            const float *rows[3] = {own_ring + ((t - 2) % TR) * NODE_FLOATS, own_ring + ((t - 1) % TR) * NODE_FLOATS,
+                                    own_ring + (t % TR) * NODE_FLOATS};
+            auto plane = [&](int dz) {
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy) {
+                    const int l = dz * 3 + dy;
+                    const float *pj = base + (dz * UY + dy) * 3 * K;
+                    float pv[3][C];
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) ldv<C>(pj + r * K, pv[r]);
+#pragma unroll
+                    for (int o = 0; o < 3; ++o) {
+                        float m[9];
+                        ld_block(rows[o] + (l * 3 + 2 - o) * SLOT, m);
+#pragma unroll
+                        for (int r = 0; r < 3; ++r)
+#pragma unroll
+                            for (int v = 0; v < C; ++v)
+                                acc[o][r][v] = fmaf(m[3 * r + 2], pv[2][v],
+                                                    fmaf(m[3 * r + 1], pv[1][v], fmaf(m[3 * r], pv[0][v], acc[o][r][v])));
+                    }
+                }
+            };
+            plane(0);
+            // a third into the position the other warps have most likely left
+            // the stage of the last one
+            if (cx <= p.x1) ok = produce(p, cx + 1, t + 1);
+            else if (g < g1) {
+                const Piece q = piece_at(g, g1, nx, tz_n);
+                ok = produce(q, q.x0 - 1, t + 1);
+            }
+            if (!ok) break;
+            plane(1);
+            plane(2);
+            const bool store = line && cx - 1 >= p.x0 && cx - 1 <= p.x1;
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                if (store) {
+                    stv<C>(ql + (int64_t)(cx - 1) * (3 * K) + r * K, acc[0][r]);
+#pragma unroll
+                    for (int v = 0; v < C; ++v) dacc[v] += (double)pc[r][v] * (double)acc[0][r][v];
+                }
+                ldv<C>(base + (UY + 1) * 3 * K + r * K, pc[r]);
+#pragma unroll
+                for (int v = 0; v < C; ++v) {
+                    acc[0][r][v] = acc[1][r][v];
+                    acc[1][r][v] = acc[2][r][v];
+                    acc[2][r][v] = 0.f;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + 8 * st);
+        }
+        if (g < g1) p = piece_at(g, g1, nx, tz_n);
+    }
+    if (__syncthreads_or(!ok)) {
+        // no copy may outlive the CTA: the two positions that can be in flight
+        mbar_wait(full + 8 * (t % TS), (t / TS) & 1);
+        mbar_wait(full + 8 * ((t + 1) % TS), ((t + 1) / TS) & 1);
+        if (threadIdx.x == 0) atomicExch(err, 1);
+        return;
+    }
+    double *sh = reinterpret_cast<double *>(traw);
+#pragma unroll
+    for (int v = 0; v < C; ++v) sh[warp * K + lane * C + v] = dacc[v];
+    __syncthreads();
+    for (int c = threadIdx.x; c < K; c += blockDim.x) {
+        double sum = 0;
+        for (int j = 0; j < TL; ++j) sum += sh[j * K + c];
+        atomicAdd(pq + c, sum);
+    }
+}
+
+constexpr int XR = 4;  // block ring rows per warp (k_xresid64)
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src)
 {
@@ -322,130 +514,10 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-template <int V>
-__global__ void __launch_bounds__(256, 2)
-    k_xspmm32(const float *__restrict__ bq, const float *__restrict__ P, float *__restrict__ Q, int nx, int ny,
-              int nz, int64_t nodes, int64_t per_warp, double *pq, const int *stop)
-{
-    constexpr int K = 32 * V;
-    constexpr int64_t RS = 3 * (int64_t)K;  // floats per node of P and Q
-    extern __shared__ __align__(16) unsigned char xs[];
-    double *sh = reinterpret_cast<double *>(xs);
-    if (*stop) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *ring = reinterpret_cast<float *>(xs + 8 * K * sizeof(double)) + warp * XR * NODE_FLOATS;
-    const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    double dacc[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) dacc[v] = 0.0;
-    const int64_t end = min(nodes, (gw + 1) * per_warp);
-    const int64_t row = (int64_t)nx * RS;
-    for (int64_t a = gw * per_warp; a < end;) {
-        const int64_t line = a / nx;
-        const int x0 = (int)(a - line * nx);
-        const int x1 = (int)(min(end, (line + 1) * nx) - 1 - line * nx);
-        const int y = (int)(line % ny), z = (int)(line / ny);
-        // the nine neighbour lines (index z * ny + y), clamped into the lattice
-        int nl[9];
-#pragma unroll
-        for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-            for (int dy = 0; dy < 3; ++dy)
-                nl[dz * 3 + dy] = min(max(z + dz - 1, 0), nz - 1) * ny + min(max(y + dy - 1, 0), ny - 1);
-        const float *pb = P + lane * V;
-        const float *bl = bq + line * nx * NODE_FLOATS;
-        const float *own = P + line * row + lane * V;
-        float *ql = Q + line * row + lane * V;
-        const int c0 = max(0, x0 - 1), c1 = min(nx - 1, x1 + 1);
-        // output ox's blocks into ring row ox % XR (nothing outside the segment)
-        auto fetch = [&](int ox) {
-            if (ox < x0 || ox > x1) return;
-            const float4 *src = reinterpret_cast<const float4 *>(bl + (int64_t)ox * NODE_FLOATS);
-            float4 *dst = reinterpret_cast<float4 *>(ring + (ox % XR) * NODE_FLOATS);
-            for (int t = lane; t < NODE_FLOATS / 4; t += 32) cp_async16(dst + t, src + t);
-        };
-        // every lane is done with the previous segment's ring; the outputs
-        // that the first position needs
-        __syncwarp();
-        for (int ox = x0; ox <= c0 + 1; ++ox) fetch(ox);
-        cp_async_commit();
-        float acc[3][3][V];
-#pragma unroll
-        for (int o = 0; o < 3; ++o)
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                for (int v = 0; v < V; ++v) acc[o][r][v] = 0.f;
-        for (int cx = c0; cx <= c1; ++cx) {
-            // outputs up to cx + 1 have landed; then the copy for output cx + 2
-            // (into the row of output cx - 2, which no lane reads any more)
-            cp_async_wait_all();
-            __syncwarp();
-            fetch(cx + 2);
-            cp_async_commit();
-#pragma unroll
-            for (int l = 0; l < 9; ++l) {
-                const float *pj = pb + ((int64_t)nl[l] * nx + cx) * RS;
-                float p[3][V];
-                ldv<V>(pj, p[0]);
-                ldv<V>(pj + K, p[1]);
-                ldv<V>(pj + 2 * K, p[2]);
-#pragma unroll
-                for (int o = 0; o < 3; ++o) {
-                    // output cx - 1 + o couples to column cx at dx = 1 - o (slot 2 - o)
-                    const int slot = (cx - 1 + o + XR) % XR;  // cx - 1 + o >= -1
-                    const float4 *bp =
-                        reinterpret_cast<const float4 *>(ring + slot * NODE_FLOATS + (l * 3 + 2 - o) * SLOT);
-                    const float4 m[3] = {bp[0], bp[1], bp[2]};
-#pragma unroll
-                    for (int r = 0; r < 3; ++r)
-#pragma unroll
-                        for (int v = 0; v < V; ++v)
-                            acc[o][r][v] = fmaf(m[r].z, p[2][v], fmaf(m[r].y, p[1][v], fmaf(m[r].x, p[0][v], acc[o][r][v])));
-                }
-            }
-            // output cx - 1 has all three of its column positions
-            if (cx - 1 >= x0) {
-#pragma unroll
-                for (int r = 0; r < 3; ++r) {
-                    const int64_t off = (int64_t)(cx - 1) * RS + r * K;
-                    stv<V>(ql + off, acc[0][r]);
-                    float pv[V];
-                    ldv<V>(own + off, pv);
-#pragma unroll
-                    for (int v = 0; v < V; ++v) dacc[v] += (double)pv[v] * (double)acc[0][r][v];
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    acc[0][r][v] = acc[1][r][v];
-                    acc[1][r][v] = acc[2][r][v];
-                    acc[2][r][v] = 0.f;
-                }
-        }
-        if (c1 == x1) {
-            // the segment ends on the lattice face: its last output is in slot 0
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const int64_t off = (int64_t)x1 * RS + r * K;
-                stv<V>(ql + off, acc[0][r]);
-                float pv[V];
-                ldv<V>(own + off, pv);
-#pragma unroll
-                for (int v = 0; v < V; ++v) dacc[v] += (double)pv[v] * (double)acc[0][r][v];
-            }
-        }
-        a = line * nx + x1 + 1;
-    }
-    cp_async_wait_all();  // no copy outlives the kernel (they are all empty by now)
-    block_cols_add<V>(dacc, sh, pq);
-}
-
 // R = B - S X in FP64 on the lattice view (the true residual of the mixed
-// block solver's reliable updates; rr[c] += sum R^2 per column): the same
-// streamed x-line walk as k_xspmm32 over FP64 canonical blocks (12 doubles
+// block solver's reliable updates; rr[c] += sum R^2 per column): a streamed
+// x-line walk, a warp per run of output nodes with the P rows of its nine
+// neighbour lines loaded at each position, over FP64 canonical blocks (12 doubles
 // per 3x3 block, rows padded to four), each run of output nodes split over H
 // warps by columns (V doubles per lane) so that the FP64 accumulators fit two
 // CTAs per SM; the blocks of output cx + 2 are copied by cp.async into the
@@ -637,25 +709,32 @@ void build_lattice_blocks(sfc_system *s)
     s->lat_mode = want == "lattice" ? 1 : 2;
 }
 
-// the tensor map of P and the kernel's attributes, set up outside any
+// The tensor map of P as (K, 3, nx, ny, nz) for boxes of bc columns and bx x
+// by x bz nodes, cached with the operand and box it was made for.
+static void encode_map(sfc_system *s, const float *P, int K, int bc, int bx, int by, int bz)
+{
+    if (s->pmap_ptr == P && s->pmap_K == K && s->pmap_box == bx) return;
+    const int nx = s->lat[0], ny = s->lat[1], nz = s->lat[2];
+    const cuuint64_t dims[5] = {(cuuint64_t)K, 3, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
+    const cuuint64_t strides[4] = {(cuuint64_t)K * 4, (cuuint64_t)3 * K * 4, (cuuint64_t)3 * K * 4 * nx,
+                                   (cuuint64_t)3 * K * 4 * nx * ny};
+    const cuuint32_t box[5] = {(cuuint32_t)bc, 3, (cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = encode_fn()(&s->pmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float *>(P), dims, strides,
+                                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) fail(SFC_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+    s->pmap_ptr = P;
+    s->pmap_K = K;
+    s->pmap_box = bx;
+}
+
+// the tensor map of P and the brick kernel's attributes, set up outside any
 // stream capture
 void lattice_prepare(sfc_system *s, const float *P, int K)
 {
-    const int nx = s->lat[0], ny = s->lat[1], nz = s->lat[2];
     SFC_REQUIRE(K % CS == 0, "lattice SpMM needs a multiple of 64 columns");
-    if (s->pmap_ptr != P || s->pmap_K != K) {
-        const cuuint64_t dims[5] = {(cuuint64_t)K, 3, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
-        const cuuint64_t strides[4] = {(cuuint64_t)K * 4, (cuuint64_t)3 * K * 4, (cuuint64_t)3 * K * 4 * nx,
-                                       (cuuint64_t)3 * K * 4 * nx * ny};
-        const cuuint32_t box[5] = {CS, 3, HX, HY, HZ};
-        const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-        const CUresult r = encode_fn()(&s->pmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float *>(P), dims,
-                                       strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) fail(SFC_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
-        s->pmap_ptr = P;
-        s->pmap_K = K;
-    }
+    encode_map(s, P, K, CS, HX, HY, HZ);
     if (!g_groups) {
         const char *e = std::getenv("SFC_LATTICE_WARPS");
         g_groups = (e && std::string(e) == "4") ? 1 : 2;
@@ -690,47 +769,49 @@ void lattice_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, 
     count_launch(ctx);
 }
 
-// the streamed x-line product (k_xspmm32): contiguous runs of output nodes,
-// one per warp, of equal length, over every resident warp of the GPU
-template <int V>
-int xline_occ()
+// kernel attributes and the tensor map of P for the streamed product, set up
+// outside any stream capture
+template <int K>
+int tspmm_occ()
 {
     static int occ = 0;
     if (!occ) {
-        SFC_CK(cudaFuncSetAttribute(k_xspmm32<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xsmem<V>()));
-        SFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_xspmm32<V>, 256, xsmem<V>()));
+        SFC_CK(cudaFuncSetAttribute(k_tspmm32<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem<K>()));
+        SFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tspmm32<K>, 32 * TL, tsmem<K>()));
         if (occ < 1) occ = 1;
     }
     return occ;
 }
 
-template <int V>
-void xline_launch(sfc_system *s, const float *P, float *Q, double *pq, const int *stop)
+void xline_prepare(sfc_system *s, const float *P, int K)
 {
-    sfc_ctx *ctx = s->ctx;
-    const int64_t warps = (int64_t)xline_occ<V>() * ctx->sm_count * 8;
-    const int64_t per_warp = (s->nodes + warps - 1) / warps;
-    const unsigned grid = (unsigned)((s->nodes + per_warp * 8 - 1) / (per_warp * 8));
-    k_xspmm32<V><<<grid, 256, xsmem<V>(), ctx->stream>>>(s->bq.p, P, Q, s->lat[0], s->lat[1], s->lat[2], s->nodes,
-                                                           per_warp, pq, stop);
-    count_launch(ctx);
+    SFC_REQUIRE(K == 32 || K == 64 || K == 128, "streamed lattice SpMM needs 32, 64 or 128 columns");
+    if (K == 32) tspmm_occ<32>();
+    else if (K == 64) tspmm_occ<64>();
+    else tspmm_occ<128>();
+    encode_map(s, P, K, K, 1, UY, UZ);
 }
 
-// kernel attributes of the streamed product for K columns, set up outside any
-// stream capture
-void xline_prepare(int K)
+template <int K>
+void tspmm_launch(sfc_system *s, float *Q, double *pq, const int *stop)
 {
-    if (K == 32) xline_occ<1>();
-    else if (K == 64) xline_occ<2>();
-    else if (K == 128) xline_occ<4>();
+    sfc_ctx *ctx = s->ctx;
+    const int nx = s->lat[0], ny = s->lat[1], nz = s->lat[2];
+    const int64_t total = (int64_t)((ny + TY - 1) / TY) * ((nz + TZ - 1) / TZ) * nx;  // positions of all tiles
+    // equal pieces over the resident CTAs, of at least four positions (each
+    // piece walks two more)
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)tspmm_occ<K>() * ctx->sm_count, total / 4));
+    k_tspmm32<K><<<(unsigned)grid, 32 * TL, tsmem<K>(), ctx->stream>>>(s->pmap, s->bq.p, Q, nx, ny, nz, total, pq,
+                                                                           stop, s->lat_err.p);
+    count_launch(ctx);
 }
 
 void xline_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, const int *stop)
 {
-    SFC_REQUIRE(K == 32 || K == 64 || K == 128, "streamed lattice SpMM needs 32, 64 or 128 columns");
-    if (K == 32) xline_launch<1>(s, P, Q, pq, stop);
-    else if (K == 64) xline_launch<2>(s, P, Q, pq, stop);
-    else xline_launch<4>(s, P, Q, pq, stop);
+    xline_prepare(s, P, K);
+    if (K == 32) tspmm_launch<32>(s, Q, pq, stop);
+    else if (K == 64) tspmm_launch<64>(s, Q, pq, stop);
+    else tspmm_launch<128>(s, Q, pq, stop);
 }
 
 // the FP64 residual on the lattice view (k_xresid64): K = 128 as two

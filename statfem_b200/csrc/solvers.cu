@@ -1415,7 +1415,7 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
         // everything the captured launches allocate or set up, done outside the capture
         if (two_any) coarse_block_reserve(s, K);
         if (lattice) lattice_prepare(s, pp, K);
-        if (bsr && s->has_lattice && s->lat_mode == 2) xline_prepare(K);
+        if (bsr && s->has_lattice && s->lat_mode == 2) xline_prepare(s, pp, K);
         const std::vector<uintptr_t> key = {
             (uintptr_t)K, (uintptr_t)check, (uintptr_t)N, (uintptr_t)s->nodes, (uintptr_t)gw,
             (uintptr_t)(bsr | (bj << 1) | (two << 2) | (two1 << 3) | (lattice << 4) | (fuse_restrict << 5)),
