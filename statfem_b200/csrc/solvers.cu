@@ -204,6 +204,46 @@ __global__ void __launch_bounds__(kRedThreads) k_dot(const double *__restrict__ 
 // ---------------------------------------------------------------------------
 // block of K = 32*V right-hand sides, RHS-interleaved [N][K]
 // ---------------------------------------------------------------------------
+// Column sums of the r updates.  Eight CTAs form a cluster that adds its
+// partial sums through distributed shared memory before one atomic per
+// column: with one per CTA, 1,184 CTAs queued up on the 2 K addresses (52,728
+// dofs, 64 columns: 22.8 -> 18.4 us; the products, with K addresses and more
+// work behind them, were slower so).
+constexpr int kColCluster = 8;
+
+// out1[c] += a1, out2[c] += a2: per-lane column partials of the cluster's
+// 256-thread CTAs; sh: 8 K doubles
+template <int V>
+__device__ void cluster_cols_add(const double (&a1)[V], const double (&a2)[V], double *sh, double *out1, double *out2)
+{
+    constexpr int K = 32 * V;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, c = threadIdx.x;
+    double s[2] = {0.0, 0.0};
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        if (m) __syncthreads();
+#pragma unroll
+        for (int v = 0; v < V; ++v) sh[w * K + l * V + v] = m ? a2[v] : a1[v];
+        __syncthreads();
+        if (c < K)
+            for (int j = 0; j < 8; ++j) s[m] += sh[j * K + c];
+    }
+    __syncthreads();
+    if (c < K)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) sh[m * K + c] = s[m];
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    constexpr int per = 2 * K / kColCluster;
+    if (c < per) {
+        const int t = (int)cl.block_rank() * per + c;
+        double sum = 0.0;
+#pragma unroll
+        for (int r = 0; r < kColCluster; ++r) sum += cl.map_shared_rank(sh, r)[t];
+        atomicAdd(t < K ? out1 + t : out2 + t - K, sum);
+    }
+    cl.sync();  // the partial sums stay until every CTA has read them
+}
 // Q = S P (FP32 values, FP32 vectors, FP32 accumulate), warp per row;
 // pq[c] += sum_i P[i][c] Q[i][c] in FP64
 template <int V>
@@ -457,7 +497,7 @@ __global__ void __launch_bounds__(256) k_resid64(const int32_t *__restrict__ rp,
 
 // r32 = r64 * scale_c, x32 = 0, p = z = D^-1 r32 for restarted columns; rz0[c], rr0[c]
 template <int V, bool SETP = true>
-__global__ void __launch_bounds__(256) k_binit32(const double *__restrict__ R64, const double *__restrict__ scale,
+__global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(256) k_binit32(const double *__restrict__ R64, const double *__restrict__ scale,
                                                  const float *__restrict__ dinv, const int *__restrict__ restart,
                                                  float *__restrict__ r, float *__restrict__ x, float *__restrict__ p,
                                                  int64_t N, double *rz0, double *rr0)
@@ -483,15 +523,13 @@ __global__ void __launch_bounds__(256) k_binit32(const double *__restrict__ R64,
             a2[v] += (double)rv * rv;
         }
     }
-    block_cols_add<V>(a1, sh, rz0);
-    __syncthreads();
-    block_cols_add<V>(a2, sh, rr0);
+    cluster_cols_add<V>(a1, a2, sh, rz0, rr0);
 }
 
 // per column: frozen when rr[it][c] <= thr[c]; alpha = rz/pq; x += alpha p;
 // r -= alpha q; rz'[c], rr'[c]
 template <int V>
-__global__ void __launch_bounds__(256) k_bupdate32(float *__restrict__ x, float *__restrict__ r,
+__global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(256) k_bupdate32(float *__restrict__ x, float *__restrict__ r,
                                                    const float *__restrict__ p, const float *__restrict__ q,
                                                    const float *__restrict__ dinv, int64_t N, const double *pq,
                                                    const double *rz, const double *rr, const double *thr,
@@ -533,9 +571,7 @@ __global__ void __launch_bounds__(256) k_bupdate32(float *__restrict__ x, float 
         stv<V>(x + o, xv);
         stv<V>(r + o, rv);
     }
-    block_cols_add<V>(a1, sh, rz_next);
-    __syncthreads();
-    block_cols_add<V>(a2, sh, rr_next);
+    cluster_cols_add<V>(a1, a2, sh, rz_next, rr_next);
 }
 
 // p = D^-1 r + beta p for active columns (rr' > thr)
@@ -631,7 +667,7 @@ __device__ __forceinline__ void bj_apply(const float *__restrict__ D, const floa
 }
 
 template <int V, bool SETP = true>
-__global__ void __launch_bounds__(256) k_ninit32(const double *__restrict__ R64, const double *__restrict__ scale,
+__global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(256) k_ninit32(const double *__restrict__ R64, const double *__restrict__ scale,
                                                  const float *__restrict__ bdinv, const int *__restrict__ restart,
                                                  float *__restrict__ r, float *__restrict__ x, float *__restrict__ p,
                                                  int64_t nodes, double *rz0, double *rr0)
@@ -672,15 +708,13 @@ __global__ void __launch_bounds__(256) k_ninit32(const double *__restrict__ R64,
             }
         }
     }
-    block_cols_add<V>(a1, sh, rz0);
-    __syncthreads();
-    block_cols_add<V>(a2, sh, rr0);
+    cluster_cols_add<V>(a1, a2, sh, rz0, rr0);
 }
 
 // XUPD = false: x is left to the p update (k_npupdate32 / k_ncpupdate32 with
 // x given), so this pass reads r and q only
 template <int V, bool XUPD = true>
-__global__ void __launch_bounds__(256, 4) k_nupdate32(float *__restrict__ x, float *__restrict__ r,
+__global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(256, 4) k_nupdate32(float *__restrict__ x, float *__restrict__ r,
                                                    const float *__restrict__ p, const float *__restrict__ q,
                                                    const float *__restrict__ bdinv, int64_t nodes, const double *pq,
                                                    const double *rz, const double *rr, const double *thr,
@@ -732,9 +766,7 @@ __global__ void __launch_bounds__(256, 4) k_nupdate32(float *__restrict__ x, flo
                 a2[v] += (double)rv[i][v] * rv[i][v];
             }
     }
-    block_cols_add<V>(a1, sh, rz_next);
-    __syncthreads();
-    block_cols_add<V>(a2, sh, rr_next);
+    cluster_cols_add<V>(a1, a2, sh, rz_next, rr_next);
 }
 
 // Two-level r update fused with the coarse restriction: r -= alpha q, r.z and
@@ -1268,8 +1300,11 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     std::vector<int> hflags(2 + K), nbreak(K), fallback(K), nstall(K);
     int n_fallback = 0;
     const bool debug = std::getenv("SFC_DEBUG_SOLVER") != nullptr;
-    const unsigned gw = (unsigned)(ctx->sm_count * 8);  // warp-per-row kernels: 8 warps/block
     const bool bsr = s->has_bsr;
+    // warp-per-row (or node) kernels: 8 warps per block, whole clusters, no
+    // block without a row
+    const unsigned gw = (grid_for((bsr ? s->nodes : N) * 32, 256, ctx->sm_count * 8) + kColCluster - 1) / kColCluster *
+                        kColCluster;
     const bool two_any = use_two_level(s);
     const CoarseSpace &crs = s->coarse;
     const bool two = two_any && crs.dof == 3;   // block Jacobi + rigid-body modes
