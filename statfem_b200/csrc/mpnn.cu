@@ -502,7 +502,10 @@ __device__ __forceinline__ float2 bf16x2_to_f2(uint32_t u)
 }
 
 // x0 = rhat / s, H0 = BF16(relu(E [x0, Ahat x0] + e)) with Ahat x0 =
-// (Ahat rhat) / s; 8 lanes per node (8 features each), 4 nodes per warp trip
+// (Ahat rhat) / s; 8 lanes per node (8 features each), 4 nodes per warp trip.
+// Bound by the latency of row pointer -> column -> value, so the entries of a
+// row go out four per lane at a time (32 of a row in flight, the 27-entry rows
+// of a 3-D mesh in one go).
 __global__ void k_encoder_inf(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                               const float *__restrict__ v, const float *__restrict__ rhat, const double *scal,
                               const float *__restrict__ P, int64_t N, float *__restrict__ x0, uint4 *__restrict__ H0)
@@ -521,8 +524,22 @@ __global__ void k_encoder_inf(const int32_t *__restrict__ rp, const int32_t *__r
         const int64_t i = base + sub;
         const bool valid = i < N;
         float acc = 0.f;
-        if (valid)
-            for (int32_t k = rp[i] + fl; k < rp[i + 1]; k += 8) acc = fmaf(v[k], rhat[col[k]], acc);
+        const int32_t b = valid ? rp[i] : 0, e = valid ? rp[i + 1] : 0;
+        for (int32_t k = b + fl; k < e; k += 32) {
+            int32_t c[4];
+            float a[4], x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool in = k + 8 * u < e;
+                c[u] = in ? col[k + 8 * u] : -1;
+                a[u] = in ? v[k + 8 * u] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = c[u] >= 0 ? rhat[c[u]] : 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c[u] >= 0) acc = fmaf(a[u], x[u], acc);
+        }
         acc += __shfl_xor_sync(0xffffffffu, acc, 4);
         acc += __shfl_xor_sync(0xffffffffu, acc, 2);
         acc += __shfl_xor_sync(0xffffffffu, acc, 1);
@@ -663,7 +680,7 @@ __global__ void __launch_bounds__(128) k_layer_inf(const int32_t *__restrict__ r
 }
 
 // ---- inference on the 5th-generation tensor cores (tcgen05) ---------------------
-// A CTA of eight warps takes 128 nodes at a time: the warps gather the tile's
+// A CTA of eight warps takes up to 128 nodes at a time: the warps gather the tile's
 // [Hin | Ahat Hin] rows (BF16, K = 128) into shared memory in the canonical
 // K-major layout without swizzle (8-row x 16-byte core matrices: core (row
 // group g, K chunk c) at byte (16 g + c) * 128, so the next K chunk is 128
@@ -675,12 +692,22 @@ __global__ void __launch_bounds__(128) k_layer_inf(const int32_t *__restrict__ r
 // .. with tcgen05.ld, columns 0-31 and 32-63 respectively, add the bias, apply
 // relu and store BF16 rows (or, DECODE, the decoded correction z).  The mbarrier wait is bounded: on a timeout the
 // kernel sets *err, waits once more (bounded) for the MMAs in flight, frees
-// its tensor memory and leaves.
+// its tensor memory and leaves.  Bound by the gather: 128 bytes per matrix
+// entry through L1, about half of it from L2 (39,304 nodes of a cube, a layer
+// 32.6 -> 25.6 us with the next trip's indices prefetched, packed FP32 FMAs,
+// the tiles spread over all CTAs and neighbouring tiles on one SM).
 constexpr int kTcRows = 128;           // nodes per tile (MMA M)
 constexpr uint32_t kTcCols = 64;       // accumulator columns (MMA N), tensor-memory columns allocated
 constexpr int kTcBBytes = H * 2 * H * 2;      // W: 16 KiB
 constexpr int kTcABytes = kTcRows * 2 * H * 2;  // A tile: 32 KiB
-constexpr size_t kTcSmem = (size_t)kTcABytes + kTcBBytes + 16;  // + mbarrier + tensor-memory address
+// k_layer_tc: bytes from the tile's first row to W, and of the whole (+ mbarrier + tensor-memory address).  A tile of
+// fewer rows leaves the rest to L1, but W's end has to lie behind 128 rows
+__host__ __device__ constexpr int tc_layer_a(int rows)
+{
+    return (rows < kTcRows / 2 ? kTcRows / 2 : rows) * 2 * H * 2;
+}
+constexpr size_t tc_layer_smem(int rows) { return (size_t)tc_layer_a(rows) + kTcBBytes + 16; }
+static_assert(tc_layer_a(8) + kTcBBytes >= kTcABytes, "128 rows lie within the tile and W");
 constexpr uint32_t kTcWaitTries = 1u << 22;
 // instruction descriptor: FP32 accumulator (bits 4-5 = 1), A and B BF16 (bits
 // 7-9, 10-12 = 1), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
@@ -741,27 +768,66 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16])
     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(u[j]);
 }
 
+// two FP32 values in a 64-bit register (fma.rn.f32x2: each half rounds as fmaf)
+__device__ __forceinline__ unsigned long long f2_pack(float a)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+__device__ __forceinline__ unsigned long long bf16x2_to_f2b(uint32_t u)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(u << 16), "r"(u & 0xffff0000u));
+    return r;
+}
+
+__device__ __forceinline__ uint32_t f2_bf16(unsigned long long a)
+{
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+    return pack_bf16(lo, hi);
+}
+
 template <bool DECODE>
 __global__ void __launch_bounds__(256, 4) k_layer_tc(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                                                      const float *__restrict__ v, const uint32_t *__restrict__ Hin,
                                                      const __nv_bfloat16 *__restrict__ W,
-                                                     const float *__restrict__ bias, int64_t N,
+                                                     const float *__restrict__ bias, int64_t N, int rows, int sms,
                                                      uint32_t *__restrict__ Hout, const float *__restrict__ P,
                                                      const float *__restrict__ x0, const float *__restrict__ sdinv,
                                                      const unsigned char *__restrict__ mask, const double *scal,
-                                                     double *__restrict__ z, int *err)
+                                                     double *__restrict__ z, const double *__restrict__ q,
+                                                     double *zq, int *err)
 {
     extern __shared__ __align__(1024) unsigned char tsm[];
-    unsigned char *sA = tsm, *sB = tsm + kTcABytes;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(tsm + kTcABytes + kTcBBytes);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(tsm + kTcABytes + kTcBBytes + 8);
+    // the tile's rows, then W: the MMA's M = 128 reads on past `rows` into W,
+    // results that nobody takes
+    unsigned char *sA = tsm, *sB = tsm + tc_layer_a(rows);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sB + kTcBBytes);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sB + kTcBBytes + 8);
+    __shared__ __align__(16) float sbias[H], sdec[H];
+    if (threadIdx.x < H) {
+        sbias[threadIdx.x] = bias[threadIdx.x];
+        if constexpr (DECODE) sdec[threadIdx.x] = P[OFF_DW + threadIdx.x];
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t sA_u = (uint32_t)__cvta_generic_to_shared(sA), sB_u = (uint32_t)__cvta_generic_to_shared(sB);
     const uint32_t bar_u = (uint32_t)__cvta_generic_to_shared(bar);
     // W (row n = output feature, 16 chunks of 8 K values) into the canonical layout
     const uint4 *W4 = reinterpret_cast<const uint4 *>(W);
-    for (int t = threadIdx.x; t < H * 16; t += blockDim.x)
-        *reinterpret_cast<uint4 *>(sB + tc_off(t / 16, t % 16)) = W4[t];
+    for (int t = threadIdx.x; t < H * 16; t += blockDim.x) {
+        const int n = (t >> 7) * 8 + (t & 7), c = (t >> 3) & 15;
+        *reinterpret_cast<uint4 *>(sB + tc_off(n, c)) = W4[n * 16 + c];
+    }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          (uint32_t)__cvta_generic_to_shared(tslot)),
@@ -781,51 +847,69 @@ __global__ void __launch_bounds__(256, 4) k_layer_tc(const int32_t *__restrict__
     // warps w and w + 4 share TMEM lanes 32 (w % 4) ..: w < 4 reads columns 0-31, w >= 4 columns 32-63
     const int quad = warp & 3, half = warp >> 2;
     const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16) + 32u * half;
-    const int64_t tiles = (N + kTcRows - 1) / kTcRows;
+    const int64_t tiles = (N + rows - 1) / rows;
+    const int passes = rows >> 2;
     const uint4 *Hin4 = reinterpret_cast<const uint4 *>(Hin);
     const int sub = lane >> 3, fl = lane & 7;
     uint32_t parity = 0;
+    double dot = 0.0;  // DECODE: this thread's share of z . q
     bool ok = !(*err), pending = false;  // pending: MMAs committed and not yet waited for
-    for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        // gather: warp w fills rows 16 w .. 16 w + 15, four rows per pass, 8 lanes per row
-        for (int pass = 0; pass < 4; ++pass) {
-            const int rr = 16 * warp + pass * 4 + sub;
-            const int64_t i = tile * kTcRows + rr;
-            const bool valid = i < N;
-            const int32_t b = valid ? rp[i] : 0;
-            const int len = valid ? rp[i + 1] - b : 0;
-            int maxlen = len;
+    // consecutive tiles to the CTAs that the first wave puts on one SM: they
+    // share most of their neighbours' lines in L1
+    const int64_t per = gridDim.x / sms;  // the grid is a multiple of sms
+    for (int64_t t0 = 0; t0 < tiles && ok; t0 += gridDim.x) {
+        const int64_t tile = t0 + (blockIdx.x % sms) * per + blockIdx.x / sms;
+        if (tile >= tiles) break;
+        // gather: passes of four rows, 8 lanes per row, dealt to the warps in turn.
+        // A trip takes 8 neighbours: their 8 loads are independent, and the
+        // next trip's columns and weights (at a row's end the next pass's) are
+        // already on their way.
+        const int64_t first = tile * rows;
+        int32_t b, len;
+        auto row_at = [&](int pass, int32_t &rb, int32_t &rl) {
+            const int64_t i = first + 4 * pass + sub;
+            const bool in = pass < passes && i < N;
+            rb = in ? rp[i] : 0;
+            rl = in ? rp[i + 1] - rb : 0;
+        };
+        row_at(warp, b, len);
+        int32_t cv = fl < len ? col[b + fl] : 0;  // padding: row 0 with weight 0
+        float av = fl < len ? v[b + fl] : 0.f;
+        for (int pass = warp; pass < passes; pass += 8) {
+            const int rr = 4 * pass + sub;
+            const int64_t i = first + rr;
+            int32_t bn, lenn;
+            row_at(pass + 8, bn, lenn);
+            int maxlen = max(len, 1);
             maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, 8));
             maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, 16));
-            float acc[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) acc[q] = 0.f;
+            unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};  // pairs of FP32 sums
             for (int s0 = 0; s0 < maxlen; s0 += 8) {
-                const int sl = s0 + fl;
-                const int32_t cv = sl < len ? col[b + sl] : 0;  // padding: row 0 with weight 0
-                const float av = sl < len ? v[b + sl] : 0.f;
+                const bool more = s0 + 8 < maxlen;
+                const int sn = more ? s0 + 8 + fl : fl;
+                const int32_t nb = more ? b : bn, nl = more ? len : lenn;
+                const int32_t cvn = sn < nl ? col[nb + sn] : 0;
+                const float avn = sn < nl ? v[nb + sn] : 0.f;
+                uint4 u[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) u[j] = Hin4[(int64_t)__shfl_sync(0xffffffffu, cv, j, 8) * 8 + fl];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const int32_t cj = __shfl_sync(0xffffffffu, cv, j, 8);
-                    const float aj = __shfl_sync(0xffffffffu, av, j, 8);
-                    const uint4 u = Hin4[(int64_t)cj * 8 + fl];
-                    const float2 f0 = bf16x2_to_f2(u.x), f1 = bf16x2_to_f2(u.y), f2 = bf16x2_to_f2(u.z),
-                                 f3 = bf16x2_to_f2(u.w);
-                    acc[0] = fmaf(aj, f0.x, acc[0]);
-                    acc[1] = fmaf(aj, f0.y, acc[1]);
-                    acc[2] = fmaf(aj, f1.x, acc[2]);
-                    acc[3] = fmaf(aj, f1.y, acc[3]);
-                    acc[4] = fmaf(aj, f2.x, acc[4]);
-                    acc[5] = fmaf(aj, f2.y, acc[5]);
-                    acc[6] = fmaf(aj, f3.x, acc[6]);
-                    acc[7] = fmaf(aj, f3.y, acc[7]);
+                    const unsigned long long aj = f2_pack(__shfl_sync(0xffffffffu, av, j, 8));
+                    acc[0] = f2_fma(aj, bf16x2_to_f2b(u[j].x), acc[0]);
+                    acc[1] = f2_fma(aj, bf16x2_to_f2b(u[j].y), acc[1]);
+                    acc[2] = f2_fma(aj, bf16x2_to_f2b(u[j].z), acc[2]);
+                    acc[3] = f2_fma(aj, bf16x2_to_f2b(u[j].w), acc[3]);
                 }
+                cv = cvn;
+                av = avn;
             }
-            const uint4 hv = valid ? Hin4[i * 8 + fl] : make_uint4(0, 0, 0, 0);
+            const uint4 hv = i < N ? Hin4[i * 8 + fl] : make_uint4(0, 0, 0, 0);
             *reinterpret_cast<uint4 *>(sA + tc_off(rr, fl)) = hv;
             *reinterpret_cast<uint4 *>(sA + tc_off(rr, 8 + fl)) =
-                make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]),
-                           pack_bf16(acc[6], acc[7]));
+                make_uint4(f2_bf16(acc[0]), f2_bf16(acc[1]), f2_bf16(acc[2]), f2_bf16(acc[3]));
+            b = bn;
+            len = lenn;
         }
         // the tile is visible to the tensor cores, and every warp has read the
         // previous tile's accumulator
@@ -854,7 +938,8 @@ __global__ void __launch_bounds__(256, 4) k_layer_tc(const int32_t *__restrict__
         pending = false;
         parity ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int64_t i = tile * kTcRows + 32 * quad + lane;  // this thread's row
+        const int64_t i = first + 32 * quad + lane;  // this thread's row
+        const bool mine = 32 * quad + lane < rows && i < N;
         const int c0 = 32 * half;                              // and its first column
         float y = 0.f;
 #pragma unroll
@@ -867,26 +952,35 @@ __global__ void __launch_bounds__(256, 4) k_layer_tc(const int32_t *__restrict__
                 uint32_t w[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    w[j] = pack_bf16(fmaxf(d[2 * j] + bias[cb + 2 * j], 0.f),
-                                     fmaxf(d[2 * j + 1] + bias[cb + 2 * j + 1], 0.f));
-                if (i < N) {
+                    w[j] = pack_bf16(fmaxf(d[2 * j] + sbias[cb + 2 * j], 0.f),
+                                     fmaxf(d[2 * j + 1] + sbias[cb + 2 * j + 1], 0.f));
+                if (mine) {
                     uint4 *dst = reinterpret_cast<uint4 *>(Hout + i * (H / 2) + cb / 2);
                     dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
                     dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
                 }
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) y = fmaf(P[OFF_DW + cb + j], fmaxf(d[j] + bias[cb + j], 0.f), y);
+                for (int j = 0; j < 16; ++j) y = fmaf(sdec[cb + j], fmaxf(d[j] + sbias[cb + j], 0.f), y);
             }
         }
         if constexpr (DECODE) {
             if (half) ypart[32 * quad + lane] = y;
             __syncthreads();
-            if (!half && i < N) {
+            if (!half && mine) {
                 y += ypart[32 * quad + lane];
                 const double sc = sqrt(scal[0] / (double)N);
-                z[i] = sc * (double)sdinv[i] * (double)(mask[i] ? x0[i] : x0[i] + y + P[OFF_DB]);
+                const double zi = sc * (double)sdinv[i] * (double)(mask[i] ? x0[i] : x0[i] + y + P[OFF_DB]);
+                z[i] = zi;
+                if (q) dot += zi * q[i];
             }
+        }
+    }
+    if constexpr (DECODE) {
+        if (q && ok && !half) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+            if (lane == 0) atomicAdd(zq, dot);
         }
     }
     if (!ok && pending) {
@@ -1224,6 +1318,32 @@ __global__ void __launch_bounds__(256, 4) k_dense_bwd_w_tc(const float *__restri
     tc_finish<64>(tmem, bar_u, parity, ok, pending, err);
 }
 
+__device__ double block_sum_d(double v, double *sh)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
+    if (threadIdx.x < 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    return v;  // valid in thread 0
+}
+
+// *out += a . b
+__global__ void k_fdot(const double *__restrict__ a, const double *__restrict__ b, int64_t n, double *out)
+{
+    __shared__ double sh[32];
+    double v = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        v += a[i] * b[i];
+    v = block_sum_d(v, sh);
+    if (threadIdx.x == 0) atomicAdd(out, v);
+}
+
 // ---- host side -------------------------------------------------------------------
 // the tensor-core (tcgen05) kernels unless SFC_MPNN_TC=0 selects the mma.sync ones
 bool use_tc()
@@ -1248,14 +1368,15 @@ unsigned tc_grid(sfc_mpnn *m, int64_t N)
     }
     static bool attr = false;
     if (!attr) {
-        const std::pair<const void *, size_t> ks[] = {{(const void *)k_layer_tc<false>, kTcSmem},
-                                                      {(const void *)k_layer_tc<true>, kTcSmem},
+        const std::pair<const void *, size_t> ks[] = {{(const void *)k_layer_tc<false>, tc_layer_smem(kTcRows)},
+                                                      {(const void *)k_layer_tc<true>, tc_layer_smem(kTcRows)},
                                                       {(const void *)k_dense_fwd_tc, kTcFwdSmem},
                                                       {(const void *)k_dense_bwd_x_tc, kTcBwdSmem},
                                                       {(const void *)k_dense_bwd_w_tc, kTcFwdSmem}};
         for (const auto &k : ks) {
             SFC_CK(cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.second));
-            SFC_CK(cudaFuncSetAttribute(k.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+            const bool layer = k.first == (const void *)k_layer_tc<false> || k.first == (const void *)k_layer_tc<true>;
+            if (!layer) SFC_CK(cudaFuncSetAttribute(k.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         }
         attr = true;
     }
@@ -1422,34 +1543,56 @@ double loss_grad(sfc_mpnn *m, const double *r, const double *e, double w)
     return hl;
 }
 
-// z = M(r) (device FP64 vectors): the inference kernels, no host synchronisation
-void apply(sfc_mpnn *m, const double *r, double *z)
+// nodes per CTA of k_layer_tc: the MMA takes 128, but with N below 128 x the
+// CTAs the GPU holds (four per SM) tiles of 128 leave some SMs an extra tile,
+// and each warp a chain of four passes of gathers, so the nodes are spread
+// over all of them (a multiple of 8; at least 32, one pass per warp).  39,304
+// nodes, 27 entries per row: 32.6 us per layer with 128 (308 tiles), 25.6 with 72.
+int tc_layer_rows(const sfc_ctx *ctx, int64_t N)
+{
+    const int64_t slots = (int64_t)ctx->sm_count * 4, even = ((N + slots - 1) / slots + 7) / 8 * 8;
+    return (int)std::max<int64_t>(32, std::min<int64_t>(kTcRows, even));
+}
+
+// z = M(r) (device FP64 vectors): the inference kernels, no host
+// synchronisation.  With q, also *zq += z . q.  With `scaled`, scal[0] and ax0
+// already hold |D^-1/2 r|^2 and FP32(D^-1/2 r).
+void apply(sfc_mpnn *m, const double *r, double *z, const double *q = nullptr, double *zq = nullptr,
+           bool scaled = false)
 {
     sfc_ctx *ctx = m->ctx;
     const sfc_system *s = m->op_sys;
     const int64_t N = m->N;
     ProfScope ps(ctx, "mpnn_apply", 0.0);
-    SFC_CK(cudaMemsetAsync(m->scal.p, 0, sizeof(double), ctx->stream));
-    k_scaled_norm2<<<grid_for(N, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(r, m->sdinv.p, N, m->scal.p,
-                                                                                   m->ax0.p);
+    if (!scaled) {
+        SFC_CK(cudaMemsetAsync(m->scal.p, 0, sizeof(double), ctx->stream));
+        k_scaled_norm2<<<grid_for(N, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(r, m->sdinv.p, N, m->scal.p,
+                                                                                       m->ax0.p);
+        count_launch(ctx);
+    }
     k_encoder_inf<<<gwarp(ctx), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->ax0.p, m->scal.p,
                                                        m->params.p, N, m->x0.p, reinterpret_cast<uint4 *>(m->hb[0].p));
-    count_launch(ctx, 2);
+    count_launch(ctx);
     if (use_tc()) {
-        const unsigned gt = tc_grid(m, N);
+        tc_grid(m, N);
+        const int rows = tc_layer_rows(ctx, N);
+        const int64_t tiles = (N + rows - 1) / rows;
+        const unsigned gt =
+            (unsigned)(std::min<int64_t>((tiles + ctx->sm_count - 1) / ctx->sm_count, 4) * ctx->sm_count);
         for (int l = 0; l < LAYERS; ++l) {
             const uint32_t *hin = reinterpret_cast<const uint32_t *>(m->hb[l & 1].p);
             uint32_t *hout = reinterpret_cast<uint32_t *>(m->hb[(l + 1) & 1].p);
             const __nv_bfloat16 *W = m->wbf.p + l * H * 2 * H;
             const float *b = m->params.p + OFF_L + l * LSZ + H * 2 * H;
             if (l + 1 < LAYERS)
-                k_layer_tc<false><<<gt, 256, kTcSmem, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N,
-                                                                     hout, m->params.p, m->x0.p, m->sdinv.p,
-                                                                     s->mask.p, m->scal.p, nullptr, m->tc_err.p);
+                k_layer_tc<false><<<gt, 256, tc_layer_smem(rows), ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N,
+                                                                     rows, ctx->sm_count, hout, m->params.p, m->x0.p, m->sdinv.p,
+                                                                     s->mask.p, m->scal.p, nullptr, nullptr, nullptr,
+                                                                     m->tc_err.p);
             else
-                k_layer_tc<true><<<gt, 256, kTcSmem, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N,
-                                                                    nullptr, m->params.p, m->x0.p, m->sdinv.p,
-                                                                    s->mask.p, m->scal.p, z, m->tc_err.p);
+                k_layer_tc<true><<<gt, 256, tc_layer_smem(rows), ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N,
+                                                                    rows, ctx->sm_count, nullptr, m->params.p, m->x0.p, m->sdinv.p,
+                                                                    s->mask.p, m->scal.p, z, q, zq, m->tc_err.p);
             count_launch(ctx);
         }
         return;
@@ -1467,6 +1610,10 @@ void apply(sfc_mpnn *m, const double *r, double *z)
         else
             k_layer_inf<true><<<g, 128, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N, nullptr,
                                                           m->params.p, m->x0.p, m->sdinv.p, s->mask.p, m->scal.p, z);
+        count_launch(ctx);
+    }
+    if (q) {
+        k_fdot<<<grid_for(N, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(z, q, N, zq);
         count_launch(ctx);
     }
 }
@@ -1544,44 +1691,18 @@ __global__ void k_resid(const double *__restrict__ b, const double *__restrict__
         r[i] = b[i] - Sx[i];
 }
 
-__device__ double block_sum_d(double v, double *sh)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-    if (threadIdx.x < 32) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    }
-    return v;  // valid in thread 0
-}
-
-// *out += a . b unless *done
-__global__ void k_dot_done(const double *__restrict__ a, const double *__restrict__ b, int64_t n, double *out,
-                           const int *done)
-{
-    __shared__ double sh[32];
-    if (done && *done) return;
-    double v = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        v += a[i] * b[i];
-    v = block_sum_d(v, sh);
-    if (threadIdx.x == 0) atomicAdd(out, v);
-}
-
 __global__ void k_axpy(double *__restrict__ y, const double *__restrict__ x, double a, int64_t n)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] += a * x[i];
 }
 
-// alpha = (p.r)/(p.q); x += alpha p; r -= alpha q; rr' += r.r
+// alpha = (p.r)/(p.q); x += alpha p; r -= alpha q; rr' += r.r; and the
+// network's input: rhat = FP32(D^-1/2 r), scal += |D^-1/2 r|^2
 __global__ void k_fcg_update(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ p,
                              const double *__restrict__ q, int64_t n, const double *pq, const double *pr,
-                             double *rr_next, const int *done, int *err)
+                             double *rr_next, const float *__restrict__ sdinv, float *__restrict__ rhat, double *scal,
+                             const int *done, int *err)
 {
     __shared__ double sh[32];
     if (*done) return;
@@ -1591,29 +1712,36 @@ __global__ void k_fcg_update(double *__restrict__ x, double *__restrict__ r, con
         return;
     }
     const double alpha = *pr / den;
-    double c = 0;
+    double c = 0, c2 = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         x[i] += alpha * p[i];
         const double ri = r[i] - alpha * q[i];
         r[i] = ri;
         c += ri * ri;
+        const double t = ri * (double)sdinv[i];
+        c2 += t * t;
+        rhat[i] = (float)t;
     }
     c = block_sum_d(c, sh);
     if (threadIdx.x == 0) atomicAdd(rr_next, c);
+    c2 = block_sum_d(c2, sh);
+    if (threadIdx.x == 0) atomicAdd(scal, c2);
 }
 
-__global__ void k_fcg_check(const double *rr, double thr, int it, int *done, const int *err)
-{
-    if (!*done && !*err && *rr <= thr) *done = it;
-}
-
-// beta = -(z.q)/(p.q); p = z + beta p; pr' += p.r
+// beta = -(z.q)/(p.q); p = z + beta p; pr' += p.r; clears scal for the next
+// update.  Where the update brought rr to the threshold: *done = it instead.
 __global__ void k_fcg_pupdate(double *__restrict__ p, const double *__restrict__ z, const double *__restrict__ r,
-                              int64_t n, const double *zq, const double *pq, double *pr_next, const int *done,
-                              const int *err)
+                              int64_t n, const double *zq, const double *pq, double *pr_next, const double *rr,
+                              double thr, int it, double *scal, int *done, const int *err)
 {
     __shared__ double sh[32];
     if (*done || *err) return;
+    const bool last = *rr <= thr;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *scal = 0.0;
+        if (last) *done = it;
+    }
+    if (last) return;
     const double beta = -*zq / *pq;
     double c = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1640,6 +1768,7 @@ void solve_forward_fcg(sfc_system *s)
     SFC_REQUIRE(s->mpnn, "no learned preconditioner set (sfc_system_set_mpnn)");
     sfc_mpnn *m = s->mpnn;
     bind(m, s);  // the operator's values may have changed since the last use
+    dia_ensure(s);
     const int64_t N = s->N;
     const auto &o = s->opt;
     const int max_iter = o.max_iter > 0 ? o.max_iter : 20000;
@@ -1675,7 +1804,8 @@ void solve_forward_fcg(sfc_system *s)
         apply(m, r, z);
         SFC_CK(cudaMemcpyAsync(p, z, N * 8, cudaMemcpyDeviceToDevice, ctx->stream));
         spmv_op64_dot(s, p, q, pq + slot, nullptr);
-        k_dot_done<<<g, 256, 0, ctx->stream>>>(p, r, N, pr + slot, nullptr);
+        k_fdot<<<g, 256, 0, ctx->stream>>>(p, r, N, pr + slot);
+        SFC_CK(cudaMemsetAsync(m->scal.p, 0, sizeof(double), ctx->stream));  // for the next k_fcg_update
         count_launch(ctx);
     };
     int it = 0, iters = 0, fallback = 0, mark_it = 0;
@@ -1687,12 +1817,11 @@ void solve_forward_fcg(sfc_system *s)
         ProfScope ps(ctx, "fcg_iterations", 0.0);
         start(0);
         for (it = 0; it < max_iter; ++it) {
-            k_fcg_update<<<g, 256, 0, ctx->stream>>>(s->X.p, r, p, q, N, pq + it, pr + it, rr + it + 1, done, err);
-            k_fcg_check<<<1, 1, 0, ctx->stream>>>(rr + it + 1, thr, it + 1, done, err);
-            count_launch(ctx, 2);
-            apply(m, r, z);
-            k_dot_done<<<g, 256, 0, ctx->stream>>>(z, q, N, zq + it, done);
-            k_fcg_pupdate<<<g, 256, 0, ctx->stream>>>(p, z, r, N, zq + it, pq + it, pr + it + 1, done, err);
+            k_fcg_update<<<g, 256, 0, ctx->stream>>>(s->X.p, r, p, q, N, pq + it, pr + it, rr + it + 1, m->sdinv.p,
+                                                    m->ax0.p, m->scal.p, done, err);
+            apply(m, r, z, q, zq + it, true);
+            k_fcg_pupdate<<<g, 256, 0, ctx->stream>>>(p, z, r, N, zq + it, pq + it, pr + it + 1, rr + it + 1, thr,
+                                                      it + 1, m->scal.p, done, err);
             count_launch(ctx, 2);
             spmv_op64_dot(s, p, q, pq + it + 1, done);
             if ((it + 1) % check == 0 || it + 1 == max_iter) {
