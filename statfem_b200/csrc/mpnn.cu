@@ -37,7 +37,7 @@
 #include <random>
 #include <vector>
 
-#include "common.cuh"
+#include "pcg.cuh"
 
 namespace {
 
@@ -67,7 +67,9 @@ struct sfc_mpnn {
     sfc::DBuf<__nv_bfloat16> hb[2];  // inference activations (BF16, ping-pong)
     sfc::DBuf<int> tc_err;           // bounded-wait status of the tensor-core layers
     sfc::DBuf<double> fcg_sc;        // flexible-CG scalars, per iteration
-    sfc::DBuf<int> fcg_flags;        // done, breakdown
+    sfc::DBuf<int> fcg_flags;        // done, breakdown; k_fcg: its `out`
+    sfc::DBuf<float> win;            // scaled operator by windows of columns (k_fcg)
+    sfc::DBuf<__nv_bfloat16> hw[2];  // activations for those, with a margin of zeros
     sfc::DBuf<double> scal;  // [0]: N s^2 = |D^-1/2 r|^2, [1]: loss
     // training pairs (FP64, N each)
     sfc::DBuf<double> pr, pe;
@@ -1344,6 +1346,441 @@ __global__ void k_fdot(const double *__restrict__ a, const double *__restrict__ 
     if (threadIdx.x == 0) atomicAdd(out, v);
 }
 
+// ---- flexible CG with the network: one persistent kernel -------------------------
+// As launches an iteration took seven (24.0 ms for the 221 iterations of a
+// 33^3 cube), and of a layer's 23 us ten went into starting its CTAs: tensor
+// memory, W, first loads.  Here one CTA per SM, of a cooperative launch, keeps
+// all three W and its tensor memory, owns a run of consecutive rows and goes
+// through the phases of an iteration behind grid barriers (pcg.cuh; every wait
+// has a limit):
+//   x, r update with |r|^2, D^-1/2 r and its norm | encoder | layer | layer |
+//   layer and decoder with z.q | p update with p.r | q = S p with p.q
+//
+// A layer takes 320 rows a round (three MMA tiles of 128, the last one partly
+// behind the rows).  Its gather is the bulk of an iteration.  On meshes
+// numbered along a lattice (WIN) the columns of a row are runs of consecutive
+// nodes, the same for every row, so 8 lanes take four rows together: a window
+// of 6 activation rows serves 12 entries, no indices, the weights 16 bytes at
+// a time.  Sums stay in the order of the columns, as in k_layer_tc.
+constexpr int kFcgThreads = 640, kFcgWarps = kFcgThreads / 32;
+constexpr int kFcgRows = 4 * 4 * kFcgWarps;  // rows of a round: four per 8 lanes
+constexpr int kFcgABytes = kFcgRows * 2 * H * 2;
+constexpr size_t kFcgSmem = (size_t)kFcgABytes + LAYERS * kTcBBytes + 16;
+constexpr int kFcgTiles = (kFcgRows + kTcRows - 1) / kTcRows;
+constexpr uint32_t kFcgCols = 256;  // tensor-memory columns: kFcgTiles x 64, a power of two
+static_assert(kFcgTiles * kTcABytes <= kFcgABytes + LAYERS * kTcBBytes, "the last tile's 128 rows lie within A and W");
+static_assert(kFcgTiles * kTcCols <= kFcgCols, "accumulators");
+
+struct FcgArgs {
+    PcgArgs op;  // x, r, p, q; sums: pq, pr, rr, zq, |D^-1/2 r|^2, `slots` each; out: iterations, why, error, (barrier), mark_it
+    int64_t slots;
+    const int32_t *rp, *col;
+    const float *ahat;
+    const float4 *win;  // [run][quad of rows][3][4 rows]
+    int runs, woff[kDiaMax];
+    const float *sdinv;
+    const unsigned char *mask;
+    const __nv_bfloat16 *W;
+    const float *P;
+    float *rhat, *x0;
+    uint32_t *hb0, *hb1;  // WIN: with rows of zeros before and behind, for the windows that reach out of the matrix
+    double *z, *mark;  // mark: rr at the last 100-fold reduction
+    int64_t per;       // rows of a CTA, a multiple of 4
+    int it0, check, stall, mark_it;
+    double thr;
+};
+enum FcgWhy { FCG_CAP = 0, FCG_DONE = 1, FCG_BREAKDOWN = 2, FCG_STALL = 3 };
+
+struct FcgShared {
+    CommShared comm;
+    alignas(16) float bias[LAYERS][H];
+    alignas(16) float dec[H];
+    alignas(16) float enc[3][H];
+    float ypart[kFcgRows];
+};
+
+// rows r0 .. of the round -> [Hin | Ahat Hin] in sA
+template <bool WIN>
+__device__ __forceinline__ void fcg_gather(const FcgArgs &g, unsigned char *sA, const uint4 *Hin4, int64_t r0, int64_t row1)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane >> 3, fl = lane & 7;
+    const int64_t N = g.op.N;
+    if constexpr (WIN) {
+        const int rr = 4 * (4 * warp + sub);
+        const int64_t i = r0 + rr;
+        if (i >= row1) return;
+        unsigned long long acc[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[k][c] = 0ull;
+        const int64_t step = ((N + 3) >> 2) * 3;
+        const float4 *w4 = g.win + (i >> 2) * 3;
+        float w[3][4];
+        uint4 h[6];
+        const uint4 *row = Hin4 + i * 8 + fl, *hp = row + (int64_t)g.woff[0] * 8;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) h[j] = hp[8 * j];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) *reinterpret_cast<float4 *>(w[u]) = w4[u];
+#pragma unroll 1
+        for (int s = 1; s <= g.runs; ++s) {
+            // the next run's values are fetched as this run's are used up
+            const int sn = min(s, g.runs - 1);
+            w4 += s < g.runs ? step : 0;
+            hp = row + (int64_t)g.woff[sn] * 8;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const unsigned long long f[4] = {bf16x2_to_f2b(h[j].x), bf16x2_to_f2b(h[j].y), bf16x2_to_f2b(h[j].z),
+                                                 bf16x2_to_f2b(h[j].w)};
+                h[j] = hp[8 * j];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (j - k >= 0 && j - k < 3) {
+                        const unsigned long long a = f2_pack(w[j - k < 0 || j - k > 2 ? 0 : j - k][k]);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) acc[k][c] = f2_fma(a, f[c], acc[k][c]);
+                    }
+                if (j >= 3) *reinterpret_cast<float4 *>(w[j >= 3 ? j - 3 : 0]) = w4[j - 3];
+            }
+        }
+        // lane fl stores the rows in the order k ^ (fl & 3): the pieces of one
+        // row lie 128 bytes apart, in the same banks
+        uint4 y[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = make_uint4(f2_bf16(acc[k][0]), f2_bf16(acc[k][1]), f2_bf16(acc[k][2]), f2_bf16(acc[k][3]));
+        auto swap_if = [](bool c, uint4 &a, uint4 &b) {
+            const uint4 t = c ? b : a;
+            b = c ? a : b;
+            a = t;
+        };
+        swap_if(fl & 1, y[0], y[1]);
+        swap_if(fl & 1, y[2], y[3]);
+        swap_if(fl & 2, y[0], y[2]);
+        swap_if(fl & 2, y[1], y[3]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int kk = k ^ (fl & 3);
+            *reinterpret_cast<uint4 *>(sA + tc_off(rr + kk, fl)) = row[8 * kk];
+            *reinterpret_cast<uint4 *>(sA + tc_off(rr + kk, 8 + fl)) = y[k];
+        }
+    } else {
+        const int passes = (int)(min((int64_t)kFcgRows, row1 - r0) + 3) >> 2;
+        for (int pass = warp; pass < passes; pass += kFcgWarps) {
+            const int rr = 4 * pass + sub;
+            const int64_t i = r0 + rr;
+            const int32_t b = i < row1 ? g.rp[i] : 0;
+            const int len = i < row1 ? g.rp[i + 1] - b : 0;
+            int maxlen = len;
+            maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, 8));
+            maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, 16));
+            unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+            int32_t cv = fl < len ? g.col[b + fl] : 0;  // padding: row 0 with weight 0
+            float av = fl < len ? g.ahat[b + fl] : 0.f;
+            for (int s0 = 0; s0 < maxlen; s0 += 8) {
+                const int sn = s0 + 8 + fl;
+                const int32_t cvn = sn < len ? g.col[b + sn] : 0;
+                const float avn = sn < len ? g.ahat[b + sn] : 0.f;
+                uint4 u[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) u[j] = Hin4[(int64_t)__shfl_sync(0xffffffffu, cv, j, 8) * 8 + fl];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const unsigned long long aj = f2_pack(__shfl_sync(0xffffffffu, av, j, 8));
+                    acc[0] = f2_fma(aj, bf16x2_to_f2b(u[j].x), acc[0]);
+                    acc[1] = f2_fma(aj, bf16x2_to_f2b(u[j].y), acc[1]);
+                    acc[2] = f2_fma(aj, bf16x2_to_f2b(u[j].z), acc[2]);
+                    acc[3] = f2_fma(aj, bf16x2_to_f2b(u[j].w), acc[3]);
+                }
+                cv = cvn;
+                av = avn;
+            }
+            const uint4 hv = i < row1 ? Hin4[i * 8 + fl] : make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4 *>(sA + tc_off(rr, fl)) = hv;
+            *reinterpret_cast<uint4 *>(sA + tc_off(rr, 8 + fl)) =
+                make_uint4(f2_bf16(acc[0]), f2_bf16(acc[1]), f2_bf16(acc[2]), f2_bf16(acc[3]));
+        }
+    }
+}
+
+// one layer on the CTA's rows; false when a wait for the MMAs gave up (they
+// may still be in flight).  DECODE: z and this thread's share of z.q.
+template <bool WIN, bool DECODE>
+__device__ bool fcg_layer(const FcgArgs &g, FcgShared &sh, unsigned char *sA, uint32_t sB_u, uint32_t bar_u, uint32_t tmem,
+                          uint32_t &parity, const uint32_t *Hin, uint32_t *Hout, const float *bias, int64_t row0,
+                          int64_t row1, double nn, double &dot)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3;
+    const uint32_t sA_u = (uint32_t)__cvta_generic_to_shared(sA);
+    for (int64_t r0 = row0; r0 < row1; r0 += kFcgRows) {
+        const int rows = (int)min((int64_t)kFcgRows, row1 - r0), tiles = (rows + kTcRows - 1) / kTcRows;
+        fcg_gather<WIN>(g, sA, reinterpret_cast<const uint4 *>(Hin), r0, row1);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (threadIdx.x == 0) {
+            for (int tile = 0; tile < tiles; ++tile)
+#pragma unroll
+                for (int ks = 0; ks < 8; ++ks) {
+                    const uint64_t da = tc_desc(sA_u + (uint32_t)kTcABytes * tile + 256u * ks), db = tc_desc(sB_u + 256u * ks);
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+                        :
+                        : "r"(tmem + kTcCols * tile), "l"(da), "l"(db), "r"(kTcIdesc), "r"(ks), "r"(0u)
+                        : "memory");
+                }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_u)
+                         : "memory");
+        }
+        if (!__syncthreads_and(tc_wait(bar_u, parity))) return false;
+        parity ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // warps of one quarter of the TMEM lanes share out the tiles' halves of 32 columns
+        // (five such warps: a warp has at most one half of either parity)
+        static_assert(kFcgWarps / 4 % 2 == 1 && 2 * kFcgTiles <= kFcgWarps / 2, "one lower half to a warp");
+        float yown = 0.f;
+        int rown = rows;
+        for (int task = warp >> 2; task < 2 * tiles; task += kFcgWarps / 4) {
+            const int tile = task >> 1, half = task & 1, rr = kTcRows * tile + 32 * quad + lane;
+            const int64_t i = r0 + rr;
+            float y = 0.f;
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                float d[16];
+                const int cb = 32 * half + 16 * part;
+                float bv[16];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) *reinterpret_cast<float4 *>(bv + 4 * j) = *reinterpret_cast<const float4 *>(bias + cb + 4 * j);
+                tc_ld16(tmem + ((uint32_t)(32 * quad) << 16) + kTcCols * tile + cb, d);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if constexpr (!DECODE) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        w[j] = pack_bf16(fmaxf(d[2 * j] + bv[2 * j], 0.f),
+                                         fmaxf(d[2 * j + 1] + bv[2 * j + 1], 0.f));
+                    if (rr < rows) {
+                        uint4 *dst = reinterpret_cast<uint4 *>(Hout + i * (H / 2) + cb / 2);
+                        dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                        dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 w = *reinterpret_cast<const float4 *>(sh.dec + cb + 4 * j);
+                        y = fmaf(w.x, fmaxf(d[4 * j] + bv[4 * j], 0.f), y);
+                        y = fmaf(w.y, fmaxf(d[4 * j + 1] + bv[4 * j + 1], 0.f), y);
+                        y = fmaf(w.z, fmaxf(d[4 * j + 2] + bv[4 * j + 2], 0.f), y);
+                        y = fmaf(w.w, fmaxf(d[4 * j + 3] + bv[4 * j + 3], 0.f), y);
+                    }
+                }
+            }
+            if constexpr (DECODE) {
+                if (half && rr < rows) sh.ypart[rr] = y;
+                if (!half) {
+                    yown = y;
+                    rown = rr;
+                }
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if constexpr (DECODE) {
+            __syncthreads();
+            const double sc = sqrt(nn / (double)g.op.N);
+            if (rown < rows) {
+                const int64_t i = r0 + rown;
+                const float y = yown + sh.ypart[rown];
+                const double zi = sc * (double)g.sdinv[i] * (double)(g.mask[i] ? g.x0[i] : g.x0[i] + y + g.P[OFF_DB]);
+                g.z[i] = zi;
+                dot += zi * g.op.q[i];
+            }
+        }
+    }
+    return true;
+}
+
+template <int F, bool WIN>
+__global__ void __launch_bounds__(kFcgThreads, 1) k_fcg(const __grid_constant__ FcgArgs g)
+{
+    extern __shared__ __align__(1024) unsigned char tsm[];
+    __shared__ __align__(16) FcgShared sh;
+    unsigned char *sA = tsm, *sB = tsm + kFcgABytes;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sB + LAYERS * kTcBBytes);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sB + LAYERS * kTcBBytes + 8);
+    const uint32_t sB_u = (uint32_t)__cvta_generic_to_shared(sB), bar_u = (uint32_t)__cvta_generic_to_shared(bar);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int t = tid; t < LAYERS * H * 16; t += kFcgThreads) {
+        const int l = t >> 10, u = t & 1023, n = (u >> 7) * 8 + (u & 7), c = (u >> 3) & 15;
+        *reinterpret_cast<uint4 *>(sB + l * kTcBBytes + tc_off(n, c)) = reinterpret_cast<const uint4 *>(g.W)[l * H * 16 + n * 16 + c];
+    }
+    if (tid < H) {
+        for (int l = 0; l < LAYERS; ++l) sh.bias[l][tid] = g.P[OFF_L + l * LSZ + H * 2 * H + tid];
+        sh.dec[tid] = g.P[OFF_DW + tid];
+        sh.enc[0][tid] = g.P[OFF_EW + 2 * tid];
+        sh.enc[1][tid] = g.P[OFF_EW + 2 * tid + 1];
+        sh.enc[2][tid] = g.P[OFF_EB + tid];
+    }
+    const uint32_t tmem = tc_setup<kFcgCols>(tslot, bar_u);
+    uint32_t parity = 0;
+    bool tc_ok = true;
+    Comm<false> comm{g.op, sh.comm};
+    const int64_t N = g.op.N, S = g.slots, row0 = min(N, (int64_t)blockIdx.x * g.per), row1 = min(N, row0 + g.per);
+    const bool first = blockIdx.x == 0 && tid == 0;
+    double pq = g.op.sums[g.it0], pr = g.op.sums[S + g.it0], mark = *g.mark, none = 0.0;
+    int mark_it = g.mark_it, it = g.it0, why = FCG_CAP;
+    while (it < g.op.max_iter) {
+        if (!(pq > 0.0)) {
+            why = FCG_BREAKDOWN;
+            ++it;
+            break;
+        }
+        const double alpha = pr / pq;
+        double rr = 0.0, nn = 0.0;
+        for (int64_t i = row0 + tid; i < row1; i += kFcgThreads) {
+            g.op.x[i] += alpha * g.op.p[i];
+            const double ri = g.op.r[i] - alpha * g.op.q[i];
+            g.op.r[i] = ri;
+            rr += ri * ri;
+            const double t = ri * (double)g.sdinv[i];
+            nn += t * t;
+            g.rhat[i] = (float)t;
+        }
+        if (!comm.sum<2>(rr, nn, (int)(2 * S) + it + 1, (int)(4 * S) + it + 1)) break;
+        if (rr <= g.thr) {
+            why = FCG_DONE;
+            ++it;
+            break;
+        }
+        if ((it + 1) % g.check == 0) {  // no 10-fold reduction of |r| within `stall` iterations
+            if (rr < 0.01 * mark) {
+                mark = rr;
+                mark_it = it + 1;
+            } else if (it + 1 - mark_it > g.stall) {
+                why = FCG_STALL;
+                ++it;
+                break;
+            }
+        }
+        {  // encoder, 8 lanes per row
+            const int sub = lane >> 3, fl = lane & 7;
+            const float inv = nn > 0 ? (float)(1.0 / sqrt(nn / (double)N)) : 0.f;
+            constexpr int R = 4;  // rows of a lane group at a time: their chains of loads overlap
+            for (int64_t base = row0 + 4 * warp; base < row1; base += 4 * kFcgWarps * R) {
+                int32_t k0[R], e[R];
+                float acc[R], own[R];
+                int len = 0;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int64_t i = base + sub + 4 * kFcgWarps * r;
+                    k0[r] = i < row1 ? g.rp[i] + fl : 0;
+                    e[r] = i < row1 ? g.rp[i + 1] : 0;
+                    own[r] = i < row1 ? g.rhat[i] : 0.f;
+                    acc[r] = 0.f;
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) len = max(len, e[r] - k0[r]);
+                for (int k = 0; k < len; k += 32) {
+                    int32_t c[R][4];
+                    float a[R][4], x[R][4];
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int32_t at = k0[r] + k + 8 * u;
+                            c[r][u] = at < e[r] ? g.col[at] : -1;
+                            a[r][u] = at < e[r] ? g.ahat[at] : 0.f;
+                        }
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) x[r][u] = c[r][u] >= 0 ? g.rhat[c[r][u]] : 0.f;
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (c[r][u] >= 0) acc[r] = fmaf(a[r][u], x[r][u], acc[r]);
+                }
+                __syncwarp();
+                float ev[3][8];
+#pragma unroll
+                for (int w = 0; w < 3; ++w)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        *reinterpret_cast<float4 *>(ev[w] + 4 * q) = *reinterpret_cast<const float4 *>(&sh.enc[w][fl * 8 + 4 * q]);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    float s = acc[r];
+                    s += __shfl_xor_sync(0xffffffffu, s, 4);
+                    s += __shfl_xor_sync(0xffffffffu, s, 2);
+                    s += __shfl_xor_sync(0xffffffffu, s, 1);
+                    const int64_t i = base + sub + 4 * kFcgWarps * r;
+                    if (i < row1) {
+                        const float xi = own[r] * inv, ax = s * inv;
+                        uint32_t w[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            w[q] = pack_bf16(
+                                fmaxf(fmaf(ev[0][2 * q], xi, fmaf(ev[1][2 * q], ax, ev[2][2 * q])), 0.f),
+                                fmaxf(fmaf(ev[0][2 * q + 1], xi, fmaf(ev[1][2 * q + 1], ax, ev[2][2 * q + 1])), 0.f));
+                        reinterpret_cast<uint4 *>(g.hb0)[i * 8 + fl] = make_uint4(w[0], w[1], w[2], w[3]);
+                        if (fl == 0) g.x0[i] = xi;
+                    }
+                }
+            }
+        }
+        if (!comm.barrier()) break;
+        double zq = 0.0;
+        tc_ok = fcg_layer<WIN, false>(g, sh, sA, sB_u, bar_u, tmem, parity, g.hb0, g.hb1, sh.bias[0], row0, row1, nn, zq);
+        if (!tc_ok || !comm.barrier()) break;
+        tc_ok = fcg_layer<WIN, false>(g, sh, sA, sB_u + kTcBBytes, bar_u, tmem, parity, g.hb1, g.hb0, sh.bias[1], row0, row1, nn, zq);
+        if (!tc_ok || !comm.barrier()) break;
+        tc_ok = fcg_layer<WIN, true>(g, sh, sA, sB_u + 2 * kTcBBytes, bar_u, tmem, parity, g.hb0, nullptr, sh.bias[2], row0, row1, nn, zq);
+        if (!tc_ok || !comm.sum<1>(zq, none, (int)(3 * S) + it, 0)) break;
+        const double beta = -zq / pq;
+        pr = 0.0;
+        for (int64_t i = row0 + tid; i < row1; i += kFcgThreads) {
+            const double pi = g.z[i] + beta * g.op.p[i];
+            g.op.p[i] = pi;
+            pr += pi * g.op.r[i];
+        }
+        if (!comm.barrier()) break;
+        pq = product<F>(g.op, g.op.p, g.op.q);
+        if (!comm.sum<2>(pq, pr, it + 1, (int)S + it + 1)) break;
+        ++it;
+    }
+    if (first) {
+        g.op.out[0] = it;
+        g.op.out[1] = why;
+        g.op.out[4] = mark_it;
+        *g.mark = mark;
+    }
+    tc_finish<kFcgCols>(tmem, bar_u, parity, tc_ok, true, g.op.out + 5);
+}
+
+// windows of the layers' gather: runs of up to three consecutive columns
+struct FcgRuns {
+    int runs, off[kDiaMax];
+};
+
+__global__ void k_fcg_window(const __grid_constant__ FcgRuns o, const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
+                             const float *__restrict__ ahat, int64_t N, float *__restrict__ win)
+{
+    const int64_t quads = (N + 3) >> 2;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 4 * quads; i += (int64_t)gridDim.x * blockDim.x) {
+        int32_t k = i < N ? rp[i] : 0;
+        const int32_t e = i < N ? rp[i + 1] : 0;
+        for (int s = 0; s < o.runs; ++s)
+            for (int u = 0; u < 3; ++u) {
+                const bool hit = k < e && col[k] - (int)i == o.off[s] + u;
+                win[((s * quads + (i >> 2)) * 3 + u) * 4 + (i & 3)] = hit ? ahat[k] : 0.f;
+                k += hit;
+            }
+    }
+}
+
 // ---- host side -------------------------------------------------------------------
 // the tensor-core (tcgen05) kernels unless SFC_MPNN_TC=0 selects the mma.sync ones
 bool use_tc()
@@ -1753,6 +2190,111 @@ __global__ void k_fcg_pupdate(double *__restrict__ p, const double *__restrict__
     if (threadIdx.x == 0) atomicAdd(pr_next, c);
 }
 
+struct FcgRun {
+    double *x, *r, *z, *p, *q, *mark;
+    int64_t slots;
+    int it, max_iter, check, stall, mark_it;
+    double thr, mark_rr;
+};
+
+// k_fcg from slot run.it on
+FcgWhy fcg_run(sfc_mpnn *m, sfc_system *s, FcgRun &run)
+{
+    sfc_ctx *ctx = s->ctx;
+    const int64_t N = s->N;
+    FcgArgs g{};
+    const Format f = grid_operator(s, g.op, false);
+    FcgRuns o{};
+    // rows of a window outside the matrix, at most: its reach, and the rest of the four rows and the run
+    const int64_t margin = f == DIA ? s->dia_off[s->dia_nd - 1] + 8 : 0;
+    if (f == DIA) {
+        for (int d = 0; d < s->dia_nd;) {
+            const int first = s->dia_off[d];
+            o.off[o.runs++] = first;
+            while (d < s->dia_nd && s->dia_off[d] < first + 3) ++d;
+        }
+        try {
+            m->win.reserve((size_t)o.runs * 3 * ((N + 3) / 4 * 4));
+            for (auto &h : m->hw) h.reserve((size_t)(N + 2 * margin) * H);
+        } catch (const Error &) {  // no room: the gather reads the rows
+            o.runs = 0;
+        }
+    }
+    if (o.runs) {
+        k_fcg_window<<<grid_for(N, 256), 256, 0, ctx->stream>>>(o, s->row_ptr.p, s->col.p, m->ahat.p, N, m->win.p);
+        count_launch(ctx);
+        g.win = reinterpret_cast<const float4 *>(m->win.p);
+        g.runs = o.runs;
+        std::copy(o.off, o.off + o.runs, g.woff);
+    }
+    g.op.x = run.x;
+    g.op.r = run.r;
+    g.op.p = run.p;
+    g.op.q = run.q;
+    g.op.sums = m->fcg_sc.p;
+    g.op.max_iter = run.max_iter;
+    g.op.out = m->fcg_flags.p;
+    g.op.bar = reinterpret_cast<unsigned *>(m->fcg_flags.p + 3);
+    g.slots = run.slots;
+    g.rp = s->row_ptr.p;
+    g.col = s->col.p;
+    g.ahat = m->ahat.p;
+    g.sdinv = m->sdinv.p;
+    g.mask = s->mask.p;
+    g.W = m->wbf.p;
+    g.P = m->params.p;
+    g.rhat = m->ax0.p;
+    g.x0 = m->x0.p;
+    __nv_bfloat16 *hb[2] = {m->hb[0].p, m->hb[1].p};
+    if (o.runs)
+        for (int k = 0; k < 2; ++k) {
+            hb[k] = m->hw[k].p + margin * H;
+            SFC_CK(cudaMemsetAsync(m->hw[k].p, 0, margin * H * 2, ctx->stream));
+            SFC_CK(cudaMemsetAsync(hb[k] + N * H, 0, margin * H * 2, ctx->stream));
+        }
+    g.hb0 = reinterpret_cast<uint32_t *>(hb[0]);
+    g.hb1 = reinterpret_cast<uint32_t *>(hb[1]);
+    g.z = run.z;
+    g.mark = run.mark;
+    g.it0 = run.it;
+    g.check = run.check;
+    g.stall = run.stall;
+    g.mark_it = run.mark_it;
+    g.thr = run.thr;
+    // one CTA per SM, of at least 64 rows
+    const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(ctx->sm_count, N / 64));
+    g.per = ((N + ctas - 1) / ctas + 3) / 4 * 4;
+    using Kernel = void (*)(FcgArgs);
+    const Kernel kernel = f == CSR    ? k_fcg<CSR, false>
+                          : f == BSR  ? k_fcg<BSR, false>
+                          : f == BDIA ? k_fcg<BDIA, false>
+                          : o.runs    ? k_fcg<DIA, true>
+                                      : k_fcg<DIA, false>;
+    SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFcgSmem));
+    SFC_CK(cudaMemsetAsync(g.op.out, 0, 8 * sizeof(int), ctx->stream));
+    SFC_CK(cudaMemcpyAsync(run.mark, &run.mark_rr, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.stream = ctx->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)((N + g.per - 1) / g.per));
+    cfg.blockDim = dim3(kFcgThreads);
+    cfg.dynamicSmemBytes = kFcgSmem;
+    SFC_CK(cudaLaunchKernelEx(&cfg, kernel, g));
+    count_launch(ctx);
+    int h[6];
+    download(ctx, h, g.op.out, 6);
+    if (h[2]) fail(SFC_ERR_TIMEOUT, "learned preconditioner: a grid barrier gave up");
+    if (h[5]) fail(SFC_ERR_TIMEOUT, "learned preconditioner: a bounded wait for the tensor-core products gave up");
+    download(ctx, &run.mark_rr, run.mark, 1);
+    run.it = h[0];
+    run.mark_it = h[4];
+    return (FcgWhy)h[1];
+}
+
 }  // namespace
 
 // Flexible CG (FCG(1), Notay 2000) with z = M(r) from the network, with
@@ -1778,16 +2320,15 @@ void solve_forward_fcg(sfc_system *s)
     s->blk64.reserve(6 * N);
     double *b = s->blk64.p, *r = b + N, *z = r + N, *p = z + N, *q = p + N, *t = q + N;
     const int64_t slots = (int64_t)max_iter + 2;
-    m->fcg_sc.reserve(4 * slots);
-    double *pq = m->fcg_sc.p, *pr = pq + slots, *rr = pr + slots, *zq = rr + slots;
-    m->fcg_flags.reserve(2);
+    m->fcg_sc.reserve(5 * slots + 1);
+    double *pq = m->fcg_sc.p, *pr = pq + slots, *rr = pr + slots, *zq = rr + slots, *mark = zq + 2 * slots;
+    m->fcg_flags.reserve(8);
     int *done = m->fcg_flags.p, *err = done + 1;
     cudaEvent_t e0, e1;
     SFC_CK(cudaEventCreate(&e0));
     SFC_CK(cudaEventCreate(&e1));
     SFC_CK(cudaEventRecord(e0, ctx->stream));
-    SFC_CK(cudaMemsetAsync(m->fcg_sc.p, 0, 4 * slots * sizeof(double), ctx->stream));
-    SFC_CK(cudaMemsetAsync(done, 0, 2 * sizeof(int), ctx->stream));
+    SFC_CK(cudaMemsetAsync(m->fcg_sc.p, 0, (5 * slots + 1) * sizeof(double), ctx->stream));
     lifted_rhs(s, b);
     SFC_CK(cudaMemsetAsync(s->X.p, 0, N * 8, ctx->stream));
     SFC_CK(cudaMemcpyAsync(r, b, N * 8, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1805,7 +2346,6 @@ void solve_forward_fcg(sfc_system *s)
         SFC_CK(cudaMemcpyAsync(p, z, N * 8, cudaMemcpyDeviceToDevice, ctx->stream));
         spmv_op64_dot(s, p, q, pq + slot, nullptr);
         k_fdot<<<g, 256, 0, ctx->stream>>>(p, r, N, pr + slot);
-        SFC_CK(cudaMemsetAsync(m->scal.p, 0, sizeof(double), ctx->stream));  // for the next k_fcg_update
         count_launch(ctx);
     };
     int it = 0, iters = 0, fallback = 0, mark_it = 0;
@@ -1813,10 +2353,20 @@ void solve_forward_fcg(sfc_system *s)
     double mark_rr = bb;
     bool conv = bb == 0.0;
     double rel = 0.0;
-    if (!conv) {
-        ProfScope ps(ctx, "fcg_iterations", 0.0);
-        start(0);
-        for (it = 0; it < max_iter; ++it) {
+    // iterations from slot `it` on to convergence of the recurrence, breakdown
+    // (p.Sp <= 0), a stall or the cap; `it` ends at the iteration reached
+    auto iterate = [&]() -> FcgWhy {
+        if (use_tc()) {
+            FcgRun run{s->X.p, r, z, p, q, mark, slots, it, max_iter, check, kStall, mark_it, thr, mark_rr};
+            const FcgWhy why = fcg_run(m, s, run);
+            it = run.it;
+            mark_it = run.mark_it;
+            mark_rr = run.mark_rr;
+            return why;
+        }
+        SFC_CK(cudaMemsetAsync(done, 0, 2 * sizeof(int), ctx->stream));
+        SFC_CK(cudaMemsetAsync(m->scal.p, 0, sizeof(double), ctx->stream));  // for the next k_fcg_update
+        for (; it < max_iter; ++it) {
             k_fcg_update<<<g, 256, 0, ctx->stream>>>(s->X.p, r, p, q, N, pq + it, pr + it, rr + it + 1, m->sdinv.p,
                                                     m->ax0.p, m->scal.p, done, err);
             apply(m, r, z, q, zq + it, true);
@@ -1827,38 +2377,49 @@ void solve_forward_fcg(sfc_system *s)
             if ((it + 1) % check == 0 || it + 1 == max_iter) {
                 int hf[2];
                 download(ctx, hf, done, 2);
-                bool give_up = hf[1] != 0;  // breakdown (p^T S p <= 0)
-                if (!give_up && hf[0]) {
-                    iters = hf[0];
-                    rel = true_residual();
-                    if (rel <= tol) {
-                        conv = true;
-                        break;
-                    }
-                    // the recurrence drifted: restart from the true residual
-                    SFC_CK(cudaMemsetAsync(done, 0, sizeof(int), ctx->stream));
-                    if (it + 1 < max_iter) start(it + 1);
-                    mark_it = it + 1;
-                } else if (!give_up) {
-                    // stagnation: no 100-fold reduction of the recurrence
-                    // residual^2 (10-fold of the residual) within kStall iterations
-                    double rr_now = 0;
-                    download(ctx, &rr_now, rr + it + 1, 1);
-                    if (rr_now < 0.01 * mark_rr) {
-                        mark_rr = rr_now;
-                        mark_it = it + 1;
-                    } else if (it + 1 - mark_it > kStall) {
-                        give_up = true;
-                    }
+                if (hf[1]) {
+                    ++it;
+                    return FCG_BREAKDOWN;
                 }
-                if (give_up) break;
+                if (hf[0]) {
+                    it = hf[0];
+                    return FCG_DONE;
+                }
+                // stagnation: no 100-fold reduction of the recurrence
+                // residual^2 (10-fold of the residual) within kStall iterations
+                double rr_now = 0;
+                download(ctx, &rr_now, rr + it + 1, 1);
+                if (rr_now < 0.01 * mark_rr) {
+                    mark_rr = rr_now;
+                    mark_it = it + 1;
+                } else if (it + 1 - mark_it > kStall) {
+                    ++it;
+                    return FCG_STALL;
+                }
             }
+        }
+        return FCG_CAP;
+    };
+    if (!conv) {
+        ProfScope ps(ctx, "fcg_iterations", 0.0);
+        start(0);
+        while (iterate() == FCG_DONE) {
+            iters = it;
+            rel = true_residual();
+            conv = rel <= tol;
+            // counts go on from the end of the check interval
+            it = (int)std::min<int64_t>(max_iter, ((int64_t)it + check - 1) / check * check);
+            if (conv || it >= max_iter) break;
+            // the recurrence drifted: restart from the true residual
+            start(it);
+            mark_it = it;
         }
         if (!conv) {
             // the network failed this system (stagnation, breakdown or the
             // iteration cap): plain FP64 Jacobi-PCG finishes from the current
             // x on the true residual, S d = b - S x, x += d
-            iters = std::max(iters, std::min(it + 1, max_iter));
+            it = (int)std::min<int64_t>(max_iter, ((int64_t)it + check - 1) / check * check);
+            iters = std::max(iters, it);
             rel = true_residual();
             if (rel > tol) {
                 fallback = 1;

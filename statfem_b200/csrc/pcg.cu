@@ -20,252 +20,19 @@
 // Poisson: 60 MB against 172; all 27 diagonals, 115 MB, took 27 us a product,
 // the CSR 79).
 
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
-#include "common.cuh"
-
-namespace cg = cooperative_groups;
+#include "pcg.cuh"
 
 namespace sfc {
 namespace {
 
-constexpr int kDiaMax = 32;    // diagonals of the pattern
 // Nonzeros up to which one cluster of 16 blocks runs the solve.  An iteration
 // takes it 10.3 us at 29 thousand (64 x 64 square; the grid 11.7) and 19.5 at
 // 230 thousand (181 x 181; the grid 13).
 constexpr double kClusterWork = 1e5;
-
-enum Format { CSR = 0, DIA = 1, BSR = 2, BDIA = 3 };
-
-struct PcgArgs {
-    int64_t N, nodes;          // dofs; nodes of a 3-dof mesh
-    const int32_t *rp, *col;   // CSR rows, or node-block rows
-    const double *a;           // CSR values, diagonals or node blocks
-    int lanes;                 // lanes per CSR row
-    int nd;                    // diagonals kept: the main one, then those above it
-    int off[kDiaMax / 2 + 1];
-    const double *b, *dinv;
-    const float *bdinv;        // nodal block inverses
-    double *x, *r, *p, *q;
-    // coarse space
-    const int32_t *agg;        // aggregate of a node; scalar meshes: -1 where constrained
-    const float4 *mode;
-    const double *ac;          // nc x nc inverse
-    int64_t nc;
-    double *c, *e;             // [2][nc], [nc]
-    double *sums;              // [4][max_iter + 2]: zeroed slots of the sums
-    unsigned *bar;
-    double tol;
-    int max_iter;
-    int *out;                  // iterations, converged, error
-};
-
-__device__ __forceinline__ double warp_total(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-struct CommShared {
-    double warps[2][32], rows[32];
-    double part[2][2];
-    int ok;
-};
-
-// Sums over all blocks, each of them also a barrier.  CL: the blocks are one
-// cluster (hardware barrier, shares read through distributed shared memory).
-// Else a cooperative grid: an atomic per block into the sum's own slot and a
-// counter (2.3 us a sum; reading every block's share instead took 2.9, and
-// polling the shares themselves, without a counter, 4.3: the polls queue up
-// behind one another on a few lines of L2).  The counter's wait is bounded
-// (2^22 polls, seconds): a block that gives up reports it, and so does every
-// other in its turn.
-template <bool CL>
-struct Comm {
-    const PcgArgs &g;
-    CommShared &sh;
-    unsigned target = 0;
-    int turn = 0;
-
-    __device__ bool barrier()
-    {
-        if constexpr (CL) {
-            cg::this_cluster().sync();  // releases and acquires global memory too
-            return true;
-        } else {
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                target += gridDim.x;
-                __threadfence();
-                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.bar) : "memory");
-                unsigned v = 0;
-                int n = 0;
-                do {
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.bar) : "memory");
-                } while ((int)(v - target) < 0 && ++n < (1 << 22));
-                sh.ok = (int)(v - target) >= 0;
-                if (!sh.ok) atomicExch(g.out + 2, 2);
-                __threadfence();
-            }
-            __syncthreads();
-            return sh.ok != 0;
-        }
-    }
-
-    // a (and b, M = 2) <- the sum over all threads
-    template <int M>
-    __device__ bool sum(double &a, double &b, int slot0, int slot1)
-    {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        a = warp_total(a);
-        if (M == 2) b = warp_total(b);
-        if (lane == 0) {
-            sh.warps[0][warp] = a;
-            if (M == 2) sh.warps[1][warp] = b;
-        }
-        __syncthreads();
-        if (warp < M) {
-            const double t = warp_total(lane < nw ? sh.warps[warp][lane] : 0.0);
-            if (lane == 0) {
-                if (CL) sh.part[turn][warp] = t;
-                else atomicAdd(g.sums + (warp ? slot1 : slot0), t);
-            }
-        }
-        if (!barrier()) return false;
-        if constexpr (CL) {
-            cg::cluster_group cl = cg::this_cluster();
-            const bool in = lane < (int)cl.num_blocks();
-            const double *part = cl.map_shared_rank(&sh.part[turn][0], in ? lane : 0);
-            a = warp_total(in ? part[0] : 0.0);
-            if (M == 2) b = warp_total(in ? part[1] : 0.0);
-            turn ^= 1;
-        } else {
-            a = g.sums[slot0];
-            if (M == 2) b = g.sums[slot1];
-        }
-        return true;
-    }
-};
-
-// row i of S x
-__device__ __forceinline__ double dia_row(const double *a, const int *off, int nd, int64_t N, int64_t i, const double *x)
-{
-    double s = a[i] * x[i];
-    constexpr int U = 4;
-    for (int d0 = 1; d0 < nd; d0 += U) {
-        double v[2 * U], xv[2 * U];
-#pragma unroll
-        for (int d = 0; d < U; ++d) {
-            const bool in = d0 + d < nd;
-            const int64_t o = in ? off[d0 + d] : 0, up = i + o, dn = i - o;
-            const double *ad = a + (int64_t)(in ? d0 + d : 0) * N;
-            const bool u = in && up < N, l = in && dn >= 0;
-            v[2 * d] = u ? ad[i] : 0.0;
-            xv[2 * d] = u ? x[up] : 0.0;
-            v[2 * d + 1] = l ? ad[dn] : 0.0;
-            xv[2 * d + 1] = l ? x[dn] : 0.0;
-        }
-#pragma unroll
-        for (int d = 0; d < 2 * U; ++d) s += v[d] * xv[d];
-    }
-    return s;
-}
-
-// the three rows of node i, a thread per node: the operand's three values
-// serve three rows (a thread per row read them three times and was bound by
-// its L1 wavefronts: 63 us for 48^3 elasticity)
-__device__ __forceinline__ void bdia_node(const double *a, const int *off, int nd, int64_t nodes, int64_t i,
-                                          const double *x, double (&s)[3])
-{
-    s[0] = s[1] = s[2] = 0.0;
-    // block d of node at, times x of node j; below: the block's transpose
-    auto block = [&](int d, int64_t at, int64_t j, bool below) {
-        double v[9], xv[3];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) v[k] = a[((int64_t)d * 9 + k) * nodes + at];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) xv[k] = x[3 * j + k];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-            s[r] += below ? v[r] * xv[0] + v[3 + r] * xv[1] + v[6 + r] * xv[2]
-                          : v[3 * r] * xv[0] + v[3 * r + 1] * xv[1] + v[3 * r + 2] * xv[2];
-    };
-    block(0, i, i, false);
-#pragma unroll 1
-    for (int d = 1; d < nd; ++d) {
-        const int64_t up = i + off[d], dn = i - off[d];
-        if (up < nodes) block(d, i, up, false);
-        if (dn >= 0) block(d, dn, dn, true);
-    }
-}
-
-// q = S p over the grid's share of the rows; returns this thread's part of p.q
-template <int F>
-__device__ double product(const PcgArgs &g, const double *p, double *q)
-{
-    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    double dot = 0.0;
-    if constexpr (F == DIA) {
-        for (int64_t i = t0; i < g.N; i += nt) {
-            const double s = dia_row(g.a, g.off, g.nd, g.N, i, p);
-            q[i] = s;
-            dot += p[i] * s;
-        }
-    } else if constexpr (F == BDIA) {
-        for (int64_t i = t0; i < g.nodes; i += nt) {
-            double s[3];
-            bdia_node(g.a, g.off, g.nd, g.nodes, i, p, s);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                q[3 * i + k] = s[k];
-                dot += p[3 * i + k] * s[k];
-            }
-        }
-    } else if constexpr (F == BSR) {
-        for (int64_t i = t0 >> 5; i < g.nodes; i += nt >> 5) {
-            double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-            for (int32_t b = g.rp[i] + lane; b < g.rp[i + 1]; b += 32) {
-                const int64_t j = g.col[b];
-                const double *v = g.a + 9 * (int64_t)b;
-                const double x0 = p[3 * j], x1 = p[3 * j + 1], x2 = p[3 * j + 2];
-                s0 += v[0] * x0 + v[1] * x1 + v[2] * x2;
-                s1 += v[3] * x0 + v[4] * x1 + v[5] * x2;
-                s2 += v[6] * x0 + v[7] * x1 + v[8] * x2;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-                s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-                s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-            }
-            if (lane < 3) {
-                const double s = lane == 0 ? s0 : lane == 1 ? s1 : s2;
-                q[3 * i + lane] = s;
-                dot += p[3 * i + lane] * s;
-            }
-        }
-    } else {
-        const int G = g.lanes, per = 32 / G;
-        for (int64_t base = (t0 >> 5) * per; base < g.N; base += (nt >> 5) * per) {
-            const int64_t i = base + lane / G;
-            double s = 0.0;
-            if (i < g.N)
-                for (int32_t k = g.rp[i] + lane % G; k < g.rp[i + 1]; k += G) s += g.a[k] * p[g.col[k]];
-            for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
-            if (i < g.N && lane % G == 0) {
-                q[i] = s;
-                dot += p[i] * s;
-            }
-        }
-    }
-    return dot;
-}
 
 // Adds the M values of the warp's lanes to c[M agg ..]: lanes of consecutive
 // nodes of one aggregate (a run of the lattice's line) are summed first.
@@ -715,28 +482,34 @@ bool dia_spmv64(sfc_system *s, const double *x, double *y, double *dot, const in
 
 void dia_ensure(sfc_system *s) { dia_prepare(s); }
 
+Format grid_operator(sfc_system *s, PcgArgs &g, bool blocks)
+{
+    const bool dia = dia_prepare(s);
+    g = operator_args(s, dia);
+    if (dia) return s->has_bsr ? BDIA : DIA;
+    // node blocks where there are no diagonals, unless the tuner chose rows
+    if (s->has_bsr && (blocks || s->spmv_lanes == 0)) {
+        g.rp = s->bptr.p;
+        g.col = s->bcol.p;
+        g.a = s->bval64.p;
+        return BSR;
+    }
+    g.rp = s->row_ptr.p;
+    g.col = s->col.p;
+    g.a = s->a_op.p;
+    const double avg = (double)s->nnz / (double)std::max<int64_t>(s->N, 1);
+    g.lanes = s->spmv_lanes > 0 ? s->spmv_lanes : avg > 24 ? 32 : avg > 12 ? 16 : avg > 6 ? 8 : 4;
+    return CSR;
+}
+
 PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_iter, bool two)
 {
     sfc_ctx *ctx = s->ctx;
     const int64_t N = s->N;
     const CoarseSpace &cs = s->coarse;
     const int pre = !two ? 0 : cs.dof == 1 ? 1 : 2;
-    const bool dia = dia_prepare(s);
-    PcgArgs g = operator_args(s, dia);
-    // node blocks where there are no diagonals, unless the tuner chose rows
-    const bool blocks = s->has_bsr && (dia || s->spmv_lanes == 0 || pre == 2);
-    const Format f = dia ? (s->has_bsr ? BDIA : DIA) : blocks ? BSR : CSR;
-    if (f == BSR) {
-        g.rp = s->bptr.p;
-        g.col = s->bcol.p;
-        g.a = s->bval64.p;
-    } else if (f == CSR) {
-        g.rp = s->row_ptr.p;
-        g.col = s->col.p;
-        g.a = s->a_op.p;
-        const double avg = (double)s->nnz / (double)std::max<int64_t>(N, 1);
-        g.lanes = s->spmv_lanes > 0 ? s->spmv_lanes : avg > 24 ? 32 : avg > 12 ? 16 : avg > 6 ? 8 : 4;
-    }
+    PcgArgs g{};
+    const Format f = grid_operator(s, g, pre == 2);
     s->w64.reserve(3 * N);
     g.b = b;
     g.x = x;
