@@ -57,19 +57,20 @@ struct sfc_mpnn {
     sfc_ctx *ctx = nullptr;
     int64_t step = 0;
     sfc::DBuf<float> params, grads, adam_m, adam_v;
-    sfc::DBuf<__nv_bfloat16> wbf;  // LAYERS x [64][128] BF16 copies
+    sfc::DBuf<__nv_bfloat16> wbf;  // LAYERS x [64][128] BF16 copies, then their transposes
     // operator-dependent data (for the system the network was last used on)
     const sfc_system *op_sys = nullptr;
     int64_t N = 0;
     sfc::DBuf<float> ahat, sdinv;
     // activations and gradients
-    sfc::DBuf<float> x0, ax0, yhat, tgt, dvec, qvec, H[LAYERS + 1], Y[LAYERS + 1], dH0, dH1, dY;
+    sfc::DBuf<float> x0, ax0, yhat, dvec, qvec, H[LAYERS + 1], Y[LAYERS + 1], dH0, dH1, dY;
     sfc::DBuf<__nv_bfloat16> hb[2];  // inference activations (BF16, ping-pong)
     sfc::DBuf<int> tc_err;           // bounded-wait status of the tensor-core layers
     sfc::DBuf<double> fcg_sc;        // flexible-CG scalars, per iteration
     sfc::DBuf<int> fcg_flags;        // done, breakdown; k_fcg: its `out`
     sfc::DBuf<float> win;            // scaled operator by windows of columns (k_fcg)
     sfc::DBuf<__nv_bfloat16> hw[2];  // activations for those, with a margin of zeros
+    sfc::DBuf<double> io[2];  // operands of the host entry points, kept between calls
     sfc::DBuf<double> scal;  // [0]: N s^2 = |D^-1/2 r|^2, [1]: loss
     // training pairs (FP64, N each)
     sfc::DBuf<double> pr, pe;
@@ -106,64 +107,102 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
 }
 
 // ---- operator scaling --------------------------------------------------------
+// (8 lanes per row: a thread per row followed a chain of a square root and a
+// division per entry, 25 us for 15,625 nodes of a cube)
 __global__ void k_scale_op(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                            const int32_t *__restrict__ diag, const double *__restrict__ a, int64_t N,
                            float *__restrict__ ahat, float *__restrict__ sdinv)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+    const int fl = threadIdx.x & 7;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3; i < N; i += ((int64_t)gridDim.x * blockDim.x) >> 3) {
         const double si = 1.0 / sqrt(a[diag[i]]);
-        sdinv[i] = (float)si;
-        for (int32_t s = rp[i]; s < rp[i + 1]; ++s) {
-            const int32_t j = col[s];
-            ahat[s] = (float)(a[s] * si / sqrt(a[diag[j]]));
-        }
+        if (fl == 0) sdinv[i] = (float)si;
+        for (int32_t s = rp[i] + fl; s < rp[i + 1]; s += 8) ahat[s] = (float)(a[s] * si / sqrt(a[diag[col[s]]]));
     }
 }
 
-// y = Ahat x (one column), warp per row
-__global__ void k_spmv32(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
-                         const float *__restrict__ v, const float *__restrict__ x, float *__restrict__ y, int64_t N)
+// Ahat x (one column), warp per row, then what its value is for:
+// ENC: y = Ahat x and H0 = relu(E [x, y] + e), two features per lane;
+// else: y = g2 Ahat x with g2 = 2 w / N, *loss += w x . Ahat x / N
+template <bool ENC>
+__global__ void __launch_bounds__(256) k_spmv32(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
+                                                const float *__restrict__ v, const float *__restrict__ x,
+                                                float *__restrict__ y, int64_t N, const float *__restrict__ P,
+                                                float *__restrict__ H0, double w, double *loss)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const float g2 = (float)(2.0 * w / (double)N);
+    const double invn = w / (double)N;
+    double part = 0.0;
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < N; i += warps) {
         float s = 0.f;
         for (int32_t k = rp[i] + lane; k < rp[i + 1]; k += 32) s = fmaf(v[k], x[col[k]], s);
         s = warp_sumf(s);
-        if (lane == 0) y[i] = s;
+        if constexpr (ENC) {
+            if (lane == 0) y[i] = s;
+            const float xi = x[i];
+            const float *E = P + OFF_EW + 4 * lane, *e = P + OFF_EB + 2 * lane;
+            *reinterpret_cast<float2 *>(H0 + i * H + 2 * lane) =
+                make_float2(fmaxf(fmaf(E[0], xi, fmaf(E[1], s, e[0])), 0.f), fmaxf(fmaf(E[2], xi, fmaf(E[3], s, e[1])), 0.f));
+        } else if (lane == 0) {
+            part += (double)x[i] * (double)s * invn;
+            y[i] = s * g2;
+        }
+    }
+    if constexpr (!ENC) {
+        __shared__ double sh[8];
+        if (lane == 0) sh[threadIdx.x >> 5] = part;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < (int)(blockDim.x >> 5); ++k) part += sh[k];
+            atomicAdd(loss, part);
+        }
     }
 }
 
-// Y (+)= Ahat X for 64 feature columns, warp per row, two features per lane
-__global__ void k_agg64(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
-                        const float *__restrict__ v, const float *__restrict__ X, float *__restrict__ Y, int64_t N,
-                        int accumulate)
+// Y (+)= Ahat X for 64 feature columns: 16 lanes per row, four features each.
+// Bound by the latency of the activation rows' loads (256 bytes each): eight
+// are in flight at a time, and the next eight columns and weights on their way.
+__global__ void __launch_bounds__(1024, 1) k_agg64(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
+                                               const float *__restrict__ v, const float *__restrict__ X,
+                                               float *__restrict__ Y, int64_t N, int accumulate)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < N; i += warps) {
-        float2 acc = make_float2(0.f, 0.f);
-        const int32_t b = rp[i], e = rp[i + 1];
-        for (int32_t s0 = b; s0 < e; s0 += 32) {
-            const int32_t s = s0 + lane;
-            const float av = s < e ? v[s] : 0.f;
-            const int32_t cv = s < e ? col[s] : 0;
-            const int n = min(32, e - s0);
-            for (int j = 0; j < n; ++j) {
-                const float aj = __shfl_sync(0xffffffffu, av, j);
-                const int32_t cj = __shfl_sync(0xffffffffu, cv, j);
-                const float2 xv = *reinterpret_cast<const float2 *>(X + (int64_t)cj * H + 2 * lane);
-                acc.x = fmaf(aj, xv.x, acc.x);
-                acc.y = fmaf(aj, xv.y, acc.y);
+    const int lane = threadIdx.x & 31, fl = lane & 15;
+    // a CTA takes consecutive rows: they share most of their neighbours' lines
+    const int64_t per = ((N + gridDim.x - 1) / gridDim.x + 1) / 2 * 2, row0 = blockIdx.x * per, row1 = min(N, row0 + per);
+    const float4 *X4 = reinterpret_cast<const float4 *>(X);
+    // both rows of a warp take every trip: the columns are shuffled
+    for (int64_t base = row0 + (threadIdx.x >> 5) * 2; base < row1; base += blockDim.x >> 4) {
+        const int64_t i = base + (lane >> 4);
+        const int32_t b = i < row1 ? rp[i] : 0, len = i < row1 ? rp[i + 1] - b : 0;
+        const int maxlen = max(len, __shfl_xor_sync(0xffffffffu, len, 16));
+        float4 *out = reinterpret_cast<float4 *>(Y) + i * 16 + fl;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), old = acc;
+        if (accumulate && i < row1) old = *out;
+        int32_t cv = fl < min(len, 8) ? col[b + fl] : 0;  // padding: row 0 with weight 0
+        float av = fl < min(len, 8) ? v[b + fl] : 0.f;
+        for (int s0 = 0; s0 < maxlen; s0 += 8) {
+            const int sn = s0 + 8 + fl;
+            const int32_t cvn = fl < 8 && sn < len ? col[b + sn] : 0;
+            const float avn = fl < 8 && sn < len ? v[b + sn] : 0.f;
+            float4 u[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) u[j] = X4[(int64_t)__shfl_sync(0xffffffffu, cv, j, 16) * 16 + fl];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float aj = __shfl_sync(0xffffffffu, av, j, 16);
+                if (s0 + j < len) {
+                    acc.x = fmaf(aj, u[j].x, acc.x);
+                    acc.y = fmaf(aj, u[j].y, acc.y);
+                    acc.z = fmaf(aj, u[j].z, acc.z);
+                    acc.w = fmaf(aj, u[j].w, acc.w);
+                }
             }
+            cv = cvn;
+            av = avn;
         }
-        float2 *out = reinterpret_cast<float2 *>(Y + i * H + 2 * lane);
-        if (accumulate) {
-            const float2 o = *out;
-            acc.x += o.x;
-            acc.y += o.y;
-        }
-        *out = acc;
+        if (i < row1) *out = make_float4(acc.x + old.x, acc.y + old.y, acc.z + old.z, acc.w + old.w);
     }
 }
 
@@ -197,17 +236,6 @@ __global__ void k_scaled_norm2(const double *__restrict__ v, const float *__rest
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (threadIdx.x == 0) atomicAdd(out, s);
-    }
-}
-
-__global__ void k_encoder(const float *__restrict__ x0, const float *__restrict__ ax0, const float *__restrict__ P,
-                          int64_t N, float *__restrict__ H0)
-{
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N * H; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / H;
-        const int k = (int)(t - i * H);
-        const float z = fmaf(P[OFF_EW + 2 * k], x0[i], fmaf(P[OFF_EW + 2 * k + 1], ax0[i], P[OFF_EB + k]));
-        H0[t] = fmaxf(z, 0.f);
     }
 }
 
@@ -281,46 +309,19 @@ __global__ void k_decoder(const float *__restrict__ H3, const float *__restrict_
     }
 }
 
-// target t = D^1/2 e / s
-__global__ void k_target(const double *__restrict__ e, const float *__restrict__ sdinv, const double *scal, int64_t N,
-                         float *__restrict__ t)
+// d = yhat - t with the target t = D^1/2 e / s
+__global__ void k_target_diff(const double *__restrict__ e, const float *__restrict__ sdinv, const double *scal,
+                              const float *__restrict__ yhat, int64_t N, float *__restrict__ d)
 {
     const double inv = scal[0] > 0 ? 1.0 / sqrt(scal[0] / (double)N) : 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
-        t[i] = (float)(e[i] / (double)sdinv[i] * inv);
-}
-
-__global__ void k_sub(const float *__restrict__ a, const float *__restrict__ b, int64_t N, float *__restrict__ d)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
-        d[i] = a[i] - b[i];
-}
-
-// loss += w d . q / N ; g = 2 w q / N (in place)
-__global__ void k_loss(const float *__restrict__ d, float *__restrict__ q, int64_t N, double w, double *loss)
-{
-    __shared__ double sh[32];
-    double s = 0;
-    const float g2 = (float)(2.0 * w / (double)N);
-    const double invn = w / (double)N;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        s += (double)d[i] * (double)q[i] * invn;
-        q[i] *= g2;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) atomicAdd(loss, s);
-    }
+        d[i] = yhat[i] - (float)(e[i] / (double)sdinv[i] * inv);
 }
 
 // decoder backward: dH3 = g w ; dw += sum_i g_i H3_i ; dc += sum g_i
-__global__ void k_decoder_bwd(const float *__restrict__ g, const float *__restrict__ H3, const float *__restrict__ P,
+// (the block's sums first: an atomic per warp and parameter, on 65 addresses,
+// took 101 us for 15,625 nodes)
+__global__ void __launch_bounds__(256) k_decoder_bwd(const float *__restrict__ g, const float *__restrict__ H3, const float *__restrict__ P,
                               const unsigned char *__restrict__ mask, int64_t N, float *__restrict__ dH3,
                               float *__restrict__ G)
 {
@@ -336,9 +337,19 @@ __global__ void k_decoder_bwd(const float *__restrict__ g, const float *__restri
         a1 = fmaf(gi, h.y, a1);
         ac += gi;
     }
-    atomicAdd(&G[OFF_DW + 2 * lane], a0);
-    atomicAdd(&G[OFF_DW + 2 * lane + 1], a1);
-    if (lane == 0) atomicAdd(&G[OFF_DB], ac);
+    __shared__ float sh[8][H + 1];
+    const int warp = threadIdx.x >> 5;
+    sh[warp][2 * lane] = a0;
+    sh[warp][2 * lane + 1] = a1;
+    if (lane == 0) sh[warp][H] = ac;
+    __syncthreads();
+    static_assert(OFF_DB == OFF_DW + H, "weights, then the bias");
+    if (threadIdx.x <= H) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += sh[k][threadIdx.x];
+        atomicAdd(&G[OFF_DW + threadIdx.x], s);
+    }
 }
 
 // input gradient of a dense layer: dZ = dH * (Hl > 0) (BF16),
@@ -453,7 +464,8 @@ __global__ void __launch_bounds__(256) k_dense_bwd_w(const float *__restrict__ d
     if (jq == 0) atomicAdd(&Gb[o], accb);
 }
 
-__global__ void k_encoder_bwd(const float *__restrict__ dH0, const float *__restrict__ H0, const float *__restrict__ x0,
+// (the block's sums first, as above: 53 us with an atomic per thread)
+__global__ void __launch_bounds__(256) k_encoder_bwd(const float *__restrict__ dH0, const float *__restrict__ H0, const float *__restrict__ x0,
                               const float *__restrict__ ax0, int64_t N, float *__restrict__ G)
 {
     // thread owns feature k = threadIdx.x & 63 for its node stride
@@ -466,9 +478,16 @@ __global__ void k_encoder_bwd(const float *__restrict__ dH0, const float *__rest
         a1 = fmaf(z, ax0[i], a1);
         ab += z;
     }
-    atomicAdd(&G[OFF_EW + 2 * k], a0);
-    atomicAdd(&G[OFF_EW + 2 * k + 1], a1);
-    atomicAdd(&G[OFF_EB + k], ab);
+    __shared__ float sh[3][256];
+    sh[0][threadIdx.x] = a0;
+    sh[1][threadIdx.x] = a1;
+    sh[2][threadIdx.x] = ab;
+    __syncthreads();
+    const int w = threadIdx.x >> 6;
+    if (w < 3) {
+        const float s = (sh[w][k] + sh[w][k + H]) + (sh[w][k + 2 * H] + sh[w][k + 3 * H]);
+        atomicAdd(&G[w < 2 ? OFF_EW + 2 * k + w : OFF_EB + k], s);
+    }
 }
 
 __global__ void k_adam(float *__restrict__ P, const float *__restrict__ G, float *__restrict__ m,
@@ -487,7 +506,9 @@ __global__ void k_to_bf16(const float *__restrict__ P, __nv_bfloat16 *__restrict
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < LAYERS * H * 2 * H; t += gridDim.x * blockDim.x) {
         const int l = t / (H * 2 * H), r = t % (H * 2 * H);
-        wbf[t] = __float2bfloat16_rn(P[OFF_L + l * LSZ + r]);
+        const __nv_bfloat16 w = __float2bfloat16_rn(P[OFF_L + l * LSZ + r]);
+        wbf[t] = w;
+        wbf[LAYERS * H * 2 * H + l * H * 2 * H + (r % (2 * H)) * H + r / (2 * H)] = w;  // and its transpose
     }
 }
 
@@ -1069,34 +1090,39 @@ __device__ __forceinline__ void tc_finish(uint32_t tmem, uint32_t bar_u, uint32_
 // Hout = relu([Hin | Yin] W^T + b) on tcgen05: 128 nodes per tile, the FP32
 // inputs rounded to BF16 into the canonical K-major layout (K = 128), W
 // (64 x 128) staged once; M = 128, N = 64, eight K-steps into 64 TMEM columns.
-// Eight warps; warps w and w + 4 read back TMEM lanes 32 (w % 4) .., columns
-// 0-31 and 32-63.
+// A CTA takes `rows` <= 128 nodes at a time (tc_layer_rows): the time is that
+// of one tile's loads, so small meshes are spread over all CTAs.
+// Sixteen warps; warp w reads back TMEM lanes 32 (w % 4) .., columns 16 (w / 4) ...
 constexpr size_t kTcFwdSmem = (size_t)kTcABytes + kTcBBytes + 16;
 
-__global__ void __launch_bounds__(256, 4) k_dense_fwd_tc(const float *__restrict__ Hin, const float *__restrict__ Yin,
+__global__ void __launch_bounds__(512, 2) k_dense_fwd_tc(const float *__restrict__ Hin, const float *__restrict__ Yin,
                                                          const __nv_bfloat16 *__restrict__ W,
-                                                         const float *__restrict__ bias, int64_t N,
+                                                         const float *__restrict__ bias, int64_t N, int rows,
                                                          float *__restrict__ Hout, int *err)
 {
     extern __shared__ __align__(1024) unsigned char tsm[];
-    unsigned char *sA = tsm, *sB = tsm + kTcABytes;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(tsm + kTcABytes + kTcBBytes);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(tsm + kTcABytes + kTcBBytes + 8);
+    unsigned char *sA = tsm, *sB = tsm + tc_layer_a(rows);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sB + kTcBBytes);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sB + kTcBBytes + 8);
     const uint32_t sA_u = (uint32_t)__cvta_generic_to_shared(sA), sB_u = (uint32_t)__cvta_generic_to_shared(sB);
     const uint32_t bar_u = (uint32_t)__cvta_generic_to_shared(bar);
     const uint4 *W4 = reinterpret_cast<const uint4 *>(W);
-    for (int t = threadIdx.x; t < H * 16; t += blockDim.x) *reinterpret_cast<uint4 *>(sB + tc_off(t / 16, t % 16)) = W4[t];
+    for (int t = threadIdx.x; t < H * 16; t += blockDim.x) {
+        const int n = (t >> 7) * 8 + (t & 7), c = (t >> 3) & 15;
+        *reinterpret_cast<uint4 *>(sB + tc_off(n, c)) = W4[n * 16 + c];
+    }
     const uint32_t tmem = tc_setup<64>(tslot, bar_u);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, half = warp >> 2;
-    const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16) + 32u * half;
-    const int64_t tiles = (N + kTcRows - 1) / kTcRows;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, quarter = warp >> 2;
+    const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16) + 16u * quarter;
+    const int64_t tiles = (N + rows - 1) / rows;
     uint32_t parity = 0;
     bool ok = !(*err), pending = false;
     for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        // 128 rows x 16 pieces of 8 inputs: 8 pieces per thread
-        for (int t = threadIdx.x; t < kTcRows * 16; t += blockDim.x) {
-            const int rr = t >> 4, c = t & 15;
-            const int64_t i = tile * kTcRows + rr;
+        // rows x 16 pieces of 8 inputs, eight rows to eight lanes: their
+        // pieces lie side by side in shared memory
+        for (int t = threadIdx.x; t < rows * 16; t += blockDim.x) {
+            const int rr = (t >> 7) * 8 + (t & 7), c = (t >> 3) & 15;
+            const int64_t i = tile * rows + rr;
             uint4 u = make_uint4(0, 0, 0, 0);
             if (i < N) {
                 const float4 *src = reinterpret_cast<const float4 *>((c < 8 ? Hin : Yin) + i * H + (c & 7) * 8);
@@ -1110,22 +1136,19 @@ __global__ void __launch_bounds__(256, 4) k_dense_fwd_tc(const float *__restrict
         if (!ok) break;
         pending = false;
         parity ^= 1u;
-        const int64_t i = tile * kTcRows + 32 * quad + lane;
+        const int64_t i = tile * rows + 32 * quad + lane;
+        const bool mine = 32 * quad + lane < rows && i < N;
+        float d[16];
+        tc_ld16(trow, d);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const int cb = 16 * quarter;
+        if (mine) {
+            float4 *dst = reinterpret_cast<float4 *>(Hout + i * H + cb);
 #pragma unroll
-        for (int part = 0; part < 2; ++part) {
-            float d[16];
-            tc_ld16(trow + 16u * part, d);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int cb = 32 * half + 16 * part;
-            if (i < N) {
-                float4 *dst = reinterpret_cast<float4 *>(Hout + i * H + cb);
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    dst[q] = make_float4(fmaxf(d[4 * q] + bias[cb + 4 * q], 0.f),
-                                         fmaxf(d[4 * q + 1] + bias[cb + 4 * q + 1], 0.f),
-                                         fmaxf(d[4 * q + 2] + bias[cb + 4 * q + 2], 0.f),
-                                         fmaxf(d[4 * q + 3] + bias[cb + 4 * q + 3], 0.f));
-            }
+            for (int q = 0; q < 4; ++q)
+                dst[q] = make_float4(fmaxf(d[4 * q] + bias[cb + 4 * q], 0.f), fmaxf(d[4 * q + 1] + bias[cb + 4 * q + 1], 0.f),
+                                     fmaxf(d[4 * q + 2] + bias[cb + 4 * q + 2], 0.f),
+                                     fmaxf(d[4 * q + 3] + bias[cb + 4 * q + 3], 0.f));
         }
     }
     tc_finish<64>(tmem, bar_u, parity, ok, pending, err);
@@ -1133,46 +1156,43 @@ __global__ void __launch_bounds__(256, 4) k_dense_fwd_tc(const float *__restrict
 
 // [dHprev | dY] = dZ W with dZ = dH * (Hl > 0) on tcgen05: A = dZ rounded to
 // BF16 (128 x 64, K = 64 over the layer's outputs), B = W^T (128 x 64, staged
-// once from W by columns); M = 128, N = 128, four K-steps into 128 TMEM
-// columns.  Warps w and w + 4 read back TMEM lanes 32 (w % 4) .., columns
-// 0-63 (dHprev) and 64-127 (dY).
+// once from W's transposed copy); M = 128, N = 128, four K-steps into 128 TMEM
+// columns.  Warp w reads back TMEM lanes 32 (w % 4) .., columns 32 (w / 4) ..
+// (0-63: dHprev, 64-127: dY).
 constexpr int kTcXABytes = kTcRows * H * 2;   // 16 KiB
 constexpr int kTcXBBytes = 2 * H * H * 2;     // 16 KiB
-constexpr size_t kTcBwdSmem = (size_t)kTcXABytes + kTcXBBytes + 16;
+constexpr size_t kTcBwdSmem = (size_t)kTcXABytes + kTcXBBytes + 16;  // of 128 rows
+static_assert(kTcXBBytes >= kTcXABytes, "128 rows of A lie within a shorter tile and B");
 
-__global__ void __launch_bounds__(256, 4) k_dense_bwd_x_tc(const float *__restrict__ dH, const float *__restrict__ Hl,
-                                                           const __nv_bfloat16 *__restrict__ W, int64_t N,
+__global__ void __launch_bounds__(512, 2) k_dense_bwd_x_tc(const float *__restrict__ dH, const float *__restrict__ Hl,
+                                                           const __nv_bfloat16 *__restrict__ Wt, int64_t N, int rows,
                                                            float *__restrict__ dHprev, float *__restrict__ dY,
                                                            int *err)
 {
     extern __shared__ __align__(1024) unsigned char tsm[];
-    unsigned char *sA = tsm, *sB = tsm + kTcXABytes;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(tsm + kTcXABytes + kTcXBBytes);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(tsm + kTcXABytes + kTcXBBytes + 8);
+    unsigned char *sA = tsm, *sB = tsm + rows * H * 2;  // the MMA's 128 rows reach into B at most
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sB + kTcXBBytes);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sB + kTcXBBytes + 8);
     const uint32_t sA_u = (uint32_t)__cvta_generic_to_shared(sA), sB_u = (uint32_t)__cvta_generic_to_shared(sB);
     const uint32_t bar_u = (uint32_t)__cvta_generic_to_shared(bar);
-    // B[j][o] = W[o][j]: 128 rows j x 8 pieces of 8 outputs o
-    const uint16_t *W16 = reinterpret_cast<const uint16_t *>(W);
+    // B[j][o] = W[o][j]: 128 rows j x 8 pieces of 8 outputs o, from the transposed copy
+    const uint4 *Wt4 = reinterpret_cast<const uint4 *>(Wt);
     for (int t = threadIdx.x; t < 2 * H * 8; t += blockDim.x) {
-        const int j = t >> 3, c = t & 7;
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            w[q] = (uint32_t)W16[(8 * c + 2 * q) * 2 * H + j] | ((uint32_t)W16[(8 * c + 2 * q + 1) * 2 * H + j] << 16);
-        *reinterpret_cast<uint4 *>(sB + tc_off<8>(j, c)) = make_uint4(w[0], w[1], w[2], w[3]);
+        const int j = (t >> 6) * 8 + (t & 7), c = (t >> 3) & 7;
+        *reinterpret_cast<uint4 *>(sB + tc_off<8>(j, c)) = Wt4[j * 8 + c];
     }
     const uint32_t tmem = tc_setup<128>(tslot, bar_u);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, half = warp >> 2;
-    const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16) + 64u * half;
-    float *out = half ? dY : dHprev;
-    const int64_t tiles = (N + kTcRows - 1) / kTcRows;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, quarter = warp >> 2;
+    const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16) + 32u * quarter;
+    float *out = quarter >= 2 ? dY : dHprev;
+    const int64_t tiles = (N + rows - 1) / rows;
     uint32_t parity = 0;
     bool ok = !(*err), pending = false;
     for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        // 128 rows x 8 pieces of 8 outputs: 4 pieces per thread
-        for (int t = threadIdx.x; t < kTcRows * 8; t += blockDim.x) {
-            const int rr = t >> 3, c = t & 7;
-            const int64_t i = tile * kTcRows + rr;
+        // rows x 8 pieces of 8 outputs, eight rows to eight lanes
+        for (int t = threadIdx.x; t < rows * 8; t += blockDim.x) {
+            const int rr = (t >> 6) * 8 + (t & 7), c = (t >> 3) & 7;
+            const int64_t i = tile * rows + rr;
             uint4 u = make_uint4(0, 0, 0, 0);
             if (i < N) {
                 const float4 *d4 = reinterpret_cast<const float4 *>(dH + i * H + 8 * c);
@@ -1190,14 +1210,15 @@ __global__ void __launch_bounds__(256, 4) k_dense_bwd_x_tc(const float *__restri
         if (!ok) break;
         pending = false;
         parity ^= 1u;
-        const int64_t i = tile * kTcRows + 32 * quad + lane;
+        const int64_t i = tile * rows + 32 * quad + lane;
+        const bool mine = 32 * quad + lane < rows && i < N;
 #pragma unroll
-        for (int part = 0; part < 4; ++part) {
+        for (int part = 0; part < 2; ++part) {
             float d[16];
             tc_ld16(trow + 16u * part, d);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (i < N) {
-                float4 *dst = reinterpret_cast<float4 *>(out + i * H + 16 * part);
+            if (mine) {
+                float4 *dst = reinterpret_cast<float4 *>(out + i * H + 32 * (quarter & 1) + 16 * part);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) dst[q] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
             }
@@ -1226,50 +1247,48 @@ __global__ void __launch_bounds__(256, 4) k_dense_bwd_w_tc(const float *__restri
     unsigned char *sA = tsm, *sB = tsm + kTcABytes;  // Xc^T: 128 x 128 (32 KiB); dZ^T: 64 x 128 (16 KiB)
     uint64_t *bar = reinterpret_cast<uint64_t *>(tsm + kTcABytes + kTcBBytes);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(tsm + kTcABytes + kTcBBytes + 8);
-    __shared__ float sdb[H];
+    __shared__ float sdb[8][H];
     const uint32_t sA_u = (uint32_t)__cvta_generic_to_shared(sA), sB_u = (uint32_t)__cvta_generic_to_shared(sB);
     const uint32_t bar_u = (uint32_t)__cvta_generic_to_shared(bar);
-    for (int t = threadIdx.x; t < H; t += blockDim.x) sdb[t] = 0.f;
     const uint32_t tmem = tc_setup<64>(tslot, bar_u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, half = warp >> 2;
     const int64_t tiles = (N + kTcRows - 1) / kTcRows;
     uint32_t parity = 0;
     bool ok = !(*err), pending = false, any = false;
+    float db[8] = {};
     for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        // Xc: 128 nodes x 16 feature groups; dZ: 128 nodes x 8 output groups
-        for (int t = threadIdx.x; t < kTcRows * 24; t += blockDim.x) {
-            const int node = t / 24, g = t % 24;
+        // Xc: 128 nodes x 16 feature groups; dZ: 128 nodes x 8 output groups;
+        // eight nodes to eight lanes (their pieces lie side by side)
+        auto piece = [&](unsigned char *dst, int g, int node, const float4 &a, const float4 &b) {
+            *reinterpret_cast<uint4 *>(dst + (g * 16 + (node >> 3)) * 128 + (node & 7) * 16) =
+                make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+        };
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int t = threadIdx.x; t < kTcRows * 16; t += 256) {
+            const int node = (t >> 7) * 8 + (t & 7), g = (t >> 3) & 15;
             const int64_t i = tile * kTcRows + node;
-            uint4 u = make_uint4(0, 0, 0, 0);
+            const float4 *src = reinterpret_cast<const float4 *>((g < 8 ? Hin : Yin) + i * H + (g & 7) * 8);
+            piece(sA, g, node, i < N ? src[0] : zero, i < N ? src[1] : zero);
+        }
+#pragma unroll
+        for (int t = threadIdx.x; t < kTcRows * 8; t += 256) {
+            const int node = (t >> 6) * 8 + (t & 7), g = (t >> 3) & 7;  // g is the thread's in every trip
+            const int64_t i = tile * kTcRows + node;
+            float4 a = zero, b = zero;
             if (i < N) {
-                float4 a, b;
-                if (g < 16) {
-                    const float4 *src = reinterpret_cast<const float4 *>((g < 8 ? Hin : Yin) + i * H + (g & 7) * 8);
-                    a = src[0];
-                    b = src[1];
-                } else {
-                    const float4 *d4 = reinterpret_cast<const float4 *>(dH + i * H + (g - 16) * 8);
-                    const float4 *h4 = reinterpret_cast<const float4 *>(Hl + i * H + (g - 16) * 8);
-                    const float4 da = d4[0], dbv = d4[1], ha = h4[0], hb = h4[1];
-                    a = make_float4(ha.x > 0.f ? da.x : 0.f, ha.y > 0.f ? da.y : 0.f, ha.z > 0.f ? da.z : 0.f,
-                                    ha.w > 0.f ? da.w : 0.f);
-                    b = make_float4(hb.x > 0.f ? dbv.x : 0.f, hb.y > 0.f ? dbv.y : 0.f, hb.z > 0.f ? dbv.z : 0.f,
-                                    hb.w > 0.f ? dbv.w : 0.f);
-                    // db: unrounded dZ, one shared-memory add per output and piece
-                    const int o0 = (g - 16) * 8;
-                    atomicAdd(&sdb[o0], a.x);
-                    atomicAdd(&sdb[o0 + 1], a.y);
-                    atomicAdd(&sdb[o0 + 2], a.z);
-                    atomicAdd(&sdb[o0 + 3], a.w);
-                    atomicAdd(&sdb[o0 + 4], b.x);
-                    atomicAdd(&sdb[o0 + 5], b.y);
-                    atomicAdd(&sdb[o0 + 6], b.z);
-                    atomicAdd(&sdb[o0 + 7], b.w);
-                }
-                u = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+                const float4 *d4 = reinterpret_cast<const float4 *>(dH + i * H + g * 8);
+                const float4 *h4 = reinterpret_cast<const float4 *>(Hl + i * H + g * 8);
+                const float4 da = d4[0], dbv = d4[1], ha = h4[0], hb = h4[1];
+                a = make_float4(ha.x > 0.f ? da.x : 0.f, ha.y > 0.f ? da.y : 0.f, ha.z > 0.f ? da.z : 0.f,
+                                ha.w > 0.f ? da.w : 0.f);
+                b = make_float4(hb.x > 0.f ? dbv.x : 0.f, hb.y > 0.f ? dbv.y : 0.f, hb.z > 0.f ? dbv.z : 0.f,
+                                hb.w > 0.f ? dbv.w : 0.f);
             }
-            const uint32_t off = (uint32_t)((((g < 16 ? g : g - 16) * 16) + (node >> 3)) * 128 + (node & 7) * 16);
-            *reinterpret_cast<uint4 *>((g < 16 ? sA : sB) + off) = u;
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int q = 0; q < 8; ++q) db[q] += v[q];  // unrounded
+            piece(sB, g, node, a, b);
         }
         pending = true;
         // K-steps of 16 nodes: the descriptors advance by two node groups (256 B);
@@ -1314,9 +1333,21 @@ __global__ void __launch_bounds__(256, 4) k_dense_bwd_w_tc(const float *__restri
             for (int q = 0; q < 16; ++q) atomicAdd(&GW[(32 * half + 16 * part + q) * 2 * H + j], d[q]);
         }
     }
+    // db: the eight lanes of an output group, then the warps (group 4 (warp % 2) + lane / 8)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) db[q] += __shfl_xor_sync(0xffffffffu, db[q], o);
+        if ((lane & 7) == 0) sdb[warp][(4 * (warp & 1) + (lane >> 3)) * 8 + q] = db[q];
+    }
     __syncthreads();
-    if (ok && any)
-        for (int t = threadIdx.x; t < H; t += blockDim.x) atomicAdd(&Gb[t], sdb[t]);
+    if (ok && any && threadIdx.x < H) {
+        const int w0 = threadIdx.x >> 5;  // warps of this group's parity
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) s += sdb[2 * w + w0][threadIdx.x];
+        atomicAdd(&Gb[threadIdx.x], s);
+    }
     tc_finish<64>(tmem, bar_u, parity, ok, pending, err);
 }
 
@@ -1820,6 +1851,32 @@ unsigned tc_grid(sfc_mpnn *m, int64_t N)
     return (unsigned)std::min<int64_t>((N + kTcRows - 1) / kTcRows, (int64_t)ctx->sm_count * 4);
 }
 
+// nodes per CTA of k_layer_tc: the MMA takes 128, but with N below 128 x the
+// CTAs the GPU holds (four per SM) tiles of 128 leave some SMs an extra tile,
+// and each warp a chain of four passes of gathers, so the nodes are spread
+// over all of them (a multiple of 8; at least 32, one pass per warp).  39,304
+// nodes, 27 entries per row: 32.6 us per layer with 128 (308 tiles), 25.6 with 72.
+int tc_layer_rows(const sfc_ctx *ctx, int64_t N)
+{
+    const int64_t slots = (int64_t)ctx->sm_count * 4, even = ((N + slots - 1) / slots + 7) / 8 * 8;
+    return (int)std::max<int64_t>(32, std::min<int64_t>(kTcRows, even));
+}
+
+// nodes per tile of k_dense_fwd_tc and k_dense_bwd_x_tc, and the CTAs (two fit
+// an SM): as few rounds of one tile per SM as 128 nodes a tile allow, of equal
+// size.  More and smaller CTAs cost more to start (four per SM: 6 us until the
+// last one runs) than their loads take.
+int tc_dense_rows(const sfc_ctx *ctx, int64_t N)
+{
+    const int64_t sm = ctx->sm_count, rounds = (N + kTcRows * sm - 1) / (kTcRows * sm);
+    return (int)std::max<int64_t>(32, ((N + sm * rounds - 1) / (sm * rounds) + 7) / 8 * 8);
+}
+unsigned tc_tiles(sfc_mpnn *m, int64_t N, int rows)
+{
+    tc_grid(m, N);
+    return (unsigned)std::min<int64_t>((N + rows - 1) / rows, (int64_t)m->ctx->sm_count * 2);
+}
+
 // after a batch of applications: a tensor-core layer whose bounded wait gave
 // up fails the call
 void check_tc(sfc_mpnn *m)
@@ -1852,7 +1909,6 @@ void bind(sfc_mpnn *m, sfc_system *s)
         m->x0.alloc(N);
         m->ax0.alloc(N);
         m->yhat.alloc(N);
-        m->tgt.alloc(N);
         m->dvec.alloc(N);
         m->qvec.alloc(N);
         for (int l = 0; l <= LAYERS; ++l) {
@@ -1866,7 +1922,7 @@ void bind(sfc_mpnn *m, sfc_system *s)
         m->dY.alloc(N * H);
     }
     m->ahat.reserve(s->nnz);
-    k_scale_op<<<grid_for(N, 128), 128, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->diag.p, s->a_op.p, N, m->ahat.p,
+    k_scale_op<<<grid_for(8 * N, 256, ctx->sm_count * 16), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->diag.p, s->a_op.p, N, m->ahat.p,
                                                          m->sdinv.p);
     count_launch(ctx);
     m->op_sys = s;
@@ -1880,20 +1936,21 @@ void forward(sfc_mpnn *m, const double *r)
     sfc_ctx *ctx = m->ctx;
     const sfc_system *s = m->op_sys;
     const int64_t N = m->N;
+    const int rows = tc_dense_rows(ctx, N);
     ProfScope ps(ctx, "mpnn_forward", 0.0);
     SFC_CK(cudaMemsetAsync(m->scal.p, 0, sizeof(double), ctx->stream));
     k_scaled_norm2<<<grid_for(N, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(r, m->sdinv.p, N, m->scal.p);
     count_launch(ctx);
     k_x0<<<grid_for(N, 256), 256, 0, ctx->stream>>>(r, m->sdinv.p, m->scal.p, N, m->x0.p);
-    k_spmv32<<<gwarp(ctx), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->x0.p, m->ax0.p, N);
-    k_encoder<<<grid_for(N * H, 256), 256, 0, ctx->stream>>>(m->x0.p, m->ax0.p, m->params.p, N, m->H[0].p);
-    count_launch(ctx, 3);
+    k_spmv32<true><<<gwarp(ctx), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->x0.p, m->ax0.p, N,
+                                                       m->params.p, m->H[0].p, 0.0, nullptr);
+    count_launch(ctx, 2);
     for (int l = 1; l <= LAYERS; ++l) {
-        k_agg64<<<gwarp(ctx), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->H[l - 1].p, m->Y[l].p, N, 0);
+        k_agg64<<<ctx->sm_count, 1024, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->H[l - 1].p, m->Y[l].p, N, 0);
         if (use_tc())
-            k_dense_fwd_tc<<<tc_grid(m, N), 256, kTcFwdSmem, ctx->stream>>>(
+            k_dense_fwd_tc<<<tc_tiles(m, N, rows), 512, tc_layer_smem(rows), ctx->stream>>>(
                 m->H[l - 1].p, m->Y[l].p, m->wbf.p + (l - 1) * H * 2 * H, m->params.p + OFF_L + (l - 1) * LSZ + H * 2 * H,
-                N, m->H[l].p, m->tc_err.p);
+                N, rows, m->H[l].p, m->tc_err.p);
         else
             k_dense_fwd<<<gwarp(ctx), 256, 0, ctx->stream>>>(m->H[l - 1].p, m->Y[l].p, m->wbf.p + (l - 1) * H * 2 * H,
                                                             m->params.p + OFF_L + (l - 1) * LSZ + H * 2 * H, N,
@@ -1913,11 +1970,10 @@ void pair_residual(sfc_mpnn *m, const double *e, const float *yhat, double w)
     const sfc_system *s = m->op_sys;
     const int64_t N = m->N;
     SFC_CK(cudaMemsetAsync(m->scal.p + 1, 0, sizeof(double), ctx->stream));
-    k_target<<<grid_for(N, 256), 256, 0, ctx->stream>>>(e, m->sdinv.p, m->scal.p, N, m->tgt.p);
-    k_sub<<<grid_for(N, 256), 256, 0, ctx->stream>>>(yhat, m->tgt.p, N, m->dvec.p);
-    k_spmv32<<<gwarp(ctx), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->dvec.p, m->qvec.p, N);
-    k_loss<<<grid_for(N, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(m->dvec.p, m->qvec.p, N, w, m->scal.p + 1);
-    count_launch(ctx, 4);
+    k_target_diff<<<grid_for(N, 256), 256, 0, ctx->stream>>>(e, m->sdinv.p, m->scal.p, yhat, N, m->dvec.p);
+    k_spmv32<false><<<gwarp(ctx), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->dvec.p, m->qvec.p, N,
+                                                        nullptr, nullptr, w, m->scal.p + 1);
+    count_launch(ctx, 2);
 }
 
 // loss of the Jacobi preconditioner (zero network output) for pair (r, e)
@@ -1944,11 +2000,12 @@ double loss_grad(sfc_mpnn *m, const double *r, const double *e, double w)
     const sfc_system *s = m->op_sys;
     const int64_t N = m->N;
     forward(m, r);
+    const int rows = tc_dense_rows(ctx, N);
     ProfScope ps(ctx, "mpnn_backward", 0.0);
     pair_residual(m, e, m->yhat.p, w);
     // qvec = dL/dyhat
     float *dHa = m->dH0.p, *dHb = m->dH1.p;
-    k_decoder_bwd<<<gwarp(ctx), 256, 0, ctx->stream>>>(m->qvec.p, m->H[LAYERS].p, m->params.p, s->mask.p, N, dHa,
+    k_decoder_bwd<<<grid_for(N * 32, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(m->qvec.p, m->H[LAYERS].p, m->params.p, s->mask.p, N, dHa,
                                                        m->grads.p);
     count_launch(ctx);
     for (int l = LAYERS; l >= 1; --l) {
@@ -1962,33 +2019,22 @@ double loss_grad(sfc_mpnn *m, const double *r, const double *e, double w)
             k_dense_bwd_w<<<(unsigned)(ctx->sm_count * 2), 256, 0, ctx->stream>>>(dHa, m->H[l].p, m->H[l - 1].p,
                                                                                   m->Y[l].p, N, GW, GW + H * 2 * H);
         if (use_tc())
-            k_dense_bwd_x_tc<<<tc_grid(m, N), 256, kTcBwdSmem, ctx->stream>>>(dHa, m->H[l].p, W, N, dHb, m->dY.p,
-                                                                               m->tc_err.p);
+            k_dense_bwd_x_tc<<<tc_tiles(m, N, rows), 512, (size_t)rows * H * 2 + kTcXBBytes + 16, ctx->stream>>>(
+                dHa, m->H[l].p, W + LAYERS * H * 2 * H, N, rows, dHb, m->dY.p, m->tc_err.p);
         else
             k_dense_bwd_x<<<gwarp(ctx), 256, 0, ctx->stream>>>(dHa, m->H[l].p, W, N, dHb, m->dY.p);
         // dH(l-1) += Ahat^T dY (Ahat is symmetric)
-        k_agg64<<<gwarp(ctx), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->dY.p, dHb, N, 1);
+        k_agg64<<<ctx->sm_count, 1024, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, m->dY.p, dHb, N, 1);
         count_launch(ctx, 3);
         std::swap(dHa, dHb);
     }
-    k_encoder_bwd<<<grid_for(N * H, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(dHa, m->H[0].p, m->x0.p,
+    k_encoder_bwd<<<grid_for(N * H, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(dHa, m->H[0].p, m->x0.p,
                                                                                      m->ax0.p, N, m->grads.p);
     count_launch(ctx);
     double hl = 0;
     download(ctx, &hl, m->scal.p + 1, 1);
     check_tc(m);
     return hl;
-}
-
-// nodes per CTA of k_layer_tc: the MMA takes 128, but with N below 128 x the
-// CTAs the GPU holds (four per SM) tiles of 128 leave some SMs an extra tile,
-// and each warp a chain of four passes of gathers, so the nodes are spread
-// over all of them (a multiple of 8; at least 32, one pass per warp).  39,304
-// nodes, 27 entries per row: 32.6 us per layer with 128 (308 tiles), 25.6 with 72.
-int tc_layer_rows(const sfc_ctx *ctx, int64_t N)
-{
-    const int64_t slots = (int64_t)ctx->sm_count * 4, even = ((N + slots - 1) / slots + 7) / 8 * 8;
-    return (int)std::max<int64_t>(32, std::min<int64_t>(kTcRows, even));
 }
 
 // z = M(r) (device FP64 vectors): the inference kernels, no host
@@ -2495,7 +2541,7 @@ int32_t sfc_mpnn_create(sfc_ctx_t *ctx, uint64_t seed, sfc_mpnn_t **out)
         m->grads.alloc(NPARAM);
         m->adam_m.alloc(NPARAM);
         m->adam_v.alloc(NPARAM);
-        m->wbf.alloc(LAYERS * H * 2 * H);
+        m->wbf.alloc(2 * LAYERS * H * 2 * H);
         m->scal.alloc(4);
         upload(ctx, m->params, p.data(), NPARAM);
         SFC_CK(cudaMemsetAsync(m->adam_m.p, 0, NPARAM * 4, ctx->stream));
@@ -2580,7 +2626,7 @@ int32_t sfc_mpnn_loss_grad(sfc_mpnn_t *m, sfc_system_t *s, const double *r, cons
     if (!m || !s || !r || !e) return SFC_ERR_BAD_ARG;
     return mguard(m->ctx, [&] {
         bind(m, s);
-        DBuf<double> dr, de;
+        DBuf<double> &dr = m->io[0], &de = m->io[1];
         upload(m->ctx, dr, r, s->N);
         upload(m->ctx, de, e, s->N);
         SFC_CK(cudaMemsetAsync(m->grads.p, 0, NPARAM * 4, m->ctx->stream));
@@ -2595,9 +2641,9 @@ int32_t sfc_mpnn_apply(sfc_mpnn_t *m, sfc_system_t *s, const double *r, double *
     if (!m || !s || !r || !z) return SFC_ERR_BAD_ARG;
     return mguard(m->ctx, [&] {
         bind(m, s);
-        DBuf<double> dr, dz;
+        DBuf<double> &dr = m->io[0], &dz = m->io[1];
         upload(m->ctx, dr, r, s->N);
-        dz.alloc(s->N);
+        dz.reserve(s->N);
         apply(m, dr.p, dz.p);
         download(m->ctx, z, dz.p, s->N);
         check_tc(m);

@@ -83,3 +83,39 @@ def test_flexible_cg_forms_agree(ctx, kind, n):
         its.append(st["iterations"])
         net.close()
     assert abs(its[0] - its[1]) <= 2 + 0.05 * its[0]
+
+
+# a tile of 32 nodes mostly empty; ragged last tiles; 18,944 nodes are one tile of 128 per SM: two rounds
+@pytest.mark.parametrize("kind,shape", [(mg.TRI3_POISSON, (2, 3)), (mg.TRI3_POISSON, (68, 69)), (mg.HEX8_POISSON, (25,)),
+                                        (mg.TRI3_POISSON, (150, 149))])
+def test_gradient_matches_oracle(ctx, kind, shape):
+    """The training kernels at the sizes where their split changes, to the
+    bounds the small meshes are held to."""
+    rng = np.random.default_rng(sum(shape))
+    mesh = mg.unit_square_tri(*shape) if kind == mg.TRI3_POISSON else mg.unit_cube_hex(*shape)
+    gm = api.Mesh(ctx, kind, QPS[kind], mesh.coords, mesh.conn)
+    coeff = np.exp(0.5 * rng.standard_normal(mesh.num_elems))
+    gm.set_coefficients(coeff)
+    s = api.SystemSolveCuda(ctx, mesh.num_dofs)
+    s.assemble(gm)
+    s.assemble_load(gm, np.ones(1))
+    bc = mg.dirichlet_dofs(mesh, "all")
+    s.applyConstraints((bc, np.zeros(len(bc))))
+    rp, col, val, _ = O.fem(mesh, QPS[kind], np.ones(1), bc, coeff=coeff)
+    mask = np.zeros(mesh.num_dofs, dtype=np.uint8)
+    mask[bc] = 1
+    Ahat, sdinv = R.scaled_operator(R.symmetric_operator(rp, col, val, mask))
+    net = api.LearnedPreconditioner(ctx, seed=0)
+    p = R.init_params(5, decoder_scale=0.3)
+    net.set_params(p)
+    r = rng.standard_normal(mesh.num_dofs) * 1e3
+    e = rng.standard_normal(mesh.num_dofs) * 1e-2
+    loss, g = net.loss_grad(s, r, e)
+    loss_ref, g_ref = R.loss_grad(p, Ahat, sdinv, mask, r, e, bf16_ops=True)
+    assert abs(loss - loss_ref) <= 1e-4 * abs(loss_ref)
+    cuts = [R.OFF_EW, R.OFF_EB] + [R.OFF_L + l * R.LSZ + o for l in range(R.LAYERS) for o in (0, R.H * 2 * R.H)]
+    for a, b in zip(cuts, cuts[1:] + [R.OFF_DW]):
+        assert np.linalg.norm(g[a:b] - g_ref[a:b]) <= 1e-2 * np.linalg.norm(g_ref[a:b]) + 1e-6 * np.linalg.norm(g_ref), (a, b)
+    a, b = R.OFF_DW, R.NPARAM
+    assert np.linalg.norm(g[a:b] - g_ref[a:b]) <= 1e-2 * np.linalg.norm(g_ref[a:b]) + 1e-6 * np.linalg.norm(g_ref)
+    net.close()
