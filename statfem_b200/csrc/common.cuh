@@ -336,6 +336,17 @@ __device__ __forceinline__ void ldv(const float *p, float (&v)[V])
         v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
     }
 }
+// the same, zeros without `live`
+template <int V>
+__device__ __forceinline__ void ldv_if(bool live, const float *p, float (&v)[V])
+{
+    if (live) {
+        ldv<V>(p, v);
+    } else {
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = 0.f;
+    }
+}
 template <int V>
 __device__ __forceinline__ void stv(float *p, const float (&v)[V])
 {
@@ -486,7 +497,7 @@ struct sfc_system {
     sfc::CoarseSpace coarse;          // SFC_PRECOND_TWO_LEVEL
     // the mixed block solver's check interval of iterations, captured once
     // per launch configuration (block widths 32, 64, 128)
-    sfc::GraphExec blk_graph[3];
+    sfc::GraphExec blk_graph[7];  // by row width and columns in use (32s)
     sfc::EventPair solve_ev;  // device time of the last solve call
     sfc::DBuf<double> host_cols[3];  // host right-hand sides and solutions on the device
     sfc::BtdPlan btd;         // direct solve of small-bandwidth systems
@@ -567,8 +578,8 @@ void build_lattice_blocks(sfc_system *s);
 void lattice_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, const int *stop);
 void lattice_prepare(sfc_system *s, const float *P, int K);
 void lattice_check(sfc_system *s);
-void xline_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, const int *stop);
-void xline_prepare(sfc_system *s, const float *P, int K);
+void xline_spmm32(sfc_system *s, const float *P, float *Q, int K, int cols, double *pq, const double *thr, const int *stop);
+void xline_prepare(sfc_system *s, const float *P, int K, int cols);
 void xline_resid64(sfc_system *s, const double *X, const double *B, double *R, int K, double *rr);
 void xresid_prepare(int K);
 void coarse_block_reserve(sfc_system *s, int K);
@@ -598,6 +609,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
 // y = S x through the diagonal copy of the operator; false where there is none
 bool dia_spmv64(sfc_system *s, const double *x, double *y, double *dot, const int *done);
 void dia_ensure(sfc_system *s);  // makes the copy for the products that follow
+bool dia_offsets(sfc_system *s); // finds the pattern's diagonals (dia_nd, dia_off), if it has them
 // mpnn.cu
 void solve_forward_fcg(sfc_system *s);
 // solvers.cu: FP64 SpMV with a given number of lanes per row (4, 8, 16, 32)

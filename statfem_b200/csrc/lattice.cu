@@ -304,7 +304,12 @@ __global__ void k_lattice_fill(const int32_t *__restrict__ bptr, const int32_t *
 // 1,296 bytes) are staged in shared memory one position ahead.  At position
 // cx a warp reads the three P rows of its nine neighbour lines once and
 // applies them to the three outputs cx - 1, cx, cx + 1 that couple to them,
-// in a sliding window of accumulators.
+// in a sliding window of accumulators.  Of the K columns of a row it takes the
+// first 32 C: those in use, of a block that is not full (32^3 nodes, 128
+// columns 71 us, 96 of them 62; 64 columns 45, 32 of them 35).  At 64 columns
+// and less the block loads bound it; two or four lines per warp, which halve
+// or quarter them, took the same (45, 38: half the warps), and so did staging
+// two or three positions ahead.
 //
 // What bounds it: the issue of the FMAs (9 per block and column, 102 us at
 // 48^3 and 128 columns; FMA pipe 48 % active, issue slots 62 %, the rest the
@@ -363,13 +368,15 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-template <int K>
+template <int K, int C>
 __global__ void __launch_bounds__(32 * TL, 2)
     k_tspmm32(const __grid_constant__ CUtensorMap pmap, const float *__restrict__ bq, float *__restrict__ Q, int nx,
-              int ny, int nz, int64_t total, double *pq, const int *stop, int *err)
+              int ny, int nz, int64_t total, double *pq, const double *thr, const int *stop, int *err)
 {
-    constexpr int C = K / 32;  // columns per lane
-    constexpr int STAGE = tstage_floats<K>();
+    constexpr int KC = 32 * C;  // columns taken of the K
+    constexpr int STAGE = tstage_floats<KC>();
+    // this lane's columns: consecutive, but three of them 32 apart (there are no loads of 12 bytes)
+    constexpr int CS0 = C == 3 ? 1 : C, CS1 = C == 3 ? 32 : 1;
     if (*stop) return;
     extern __shared__ __align__(128) unsigned char traw[];
     float *stage = reinterpret_cast<float *>(traw);
@@ -405,6 +412,30 @@ __global__ void __launch_bounds__(32 * TL, 2)
         }
         return true;
     };
+    auto ldc = [&](const float *at, float (&v)[C]) {
+        if constexpr (C == 3) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) v[j] = at[32 * j];
+        } else {
+            ldv<C>(at, v);
+        }
+    };
+    auto stc = [&](float *at, const float (&v)[C]) {
+        if constexpr (C == 3) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) at[32 * j] = v[j];
+        } else {
+            stv<C>(at, v);
+        }
+    };
+    // the updates read Q by lanes of K / 32 columns, each with all of its
+    // columns or none: a column is stored if that lane has an open one
+    constexpr int VU = K / 32;
+    bool live = false;
+#pragma unroll
+    for (int v = 0; v < C; ++v)
+#pragma unroll
+        for (int u = 0; u < VU; ++u) live |= thr[(lane * CS0 + v * CS1) / VU * VU + u] < INFINITY;
     double dacc[C];
 #pragma unroll
     for (int v = 0; v < C; ++v) dacc[v] = 0.0;
@@ -416,7 +447,7 @@ __global__ void __launch_bounds__(32 * TL, 2)
     while (g < g1 && ok) {
         const int y = p.y0 + wy, z = p.z0 + wz;
         const bool line = y < ny && z < nz;  // a warp past the face computes what it does not store
-        float *ql = Q + ((int64_t)z * ny + y) * nx * (3 * K) + lane * C;
+        float *ql = Q + ((int64_t)z * ny + y) * nx * (3 * K) + lane * CS0;
         g += p.x1 - p.x0 + 1;
         float acc[3][3][C], pc[3][C];
 #pragma unroll
@@ -429,8 +460,8 @@ __global__ void __launch_bounds__(32 * TL, 2)
                 ok = false;
                 break;
             }
-            // neighbour line (dz, dy) lies (dz UY + dy) 3 K on
-            const float *base = stage + st * STAGE + (wz * UY + wy) * 3 * K + lane * C;
+            // neighbour line (dz, dy) lies (dz UY + dy) 3 KC on
+            const float *base = stage + st * STAGE + (wz * UY + wy) * 3 * KC + lane * CS0;
             // output cx - 1 + o has its blocks in ring row t - 2 + o
             const float *rows[3] = {own_ring + ((t - 2) % TR) * NODE_FLOATS, own_ring + ((t - 1) % TR) * NODE_FLOATS,
                                     own_ring + (t % TR) * NODE_FLOATS};
@@ -438,10 +469,10 @@ __global__ void __launch_bounds__(32 * TL, 2)
 #pragma unroll
                 for (int dy = 0; dy < 3; ++dy) {
                     const int l = dz * 3 + dy;
-                    const float *pj = base + (dz * UY + dy) * 3 * K;
+                    const float *pj = base + (dz * UY + dy) * 3 * KC;
                     float pv[3][C];
 #pragma unroll
-                    for (int r = 0; r < 3; ++r) ldv<C>(pj + r * K, pv[r]);
+                    for (int r = 0; r < 3; ++r) ldc(pj + r * KC, pv[r]);
 #pragma unroll
                     for (int o = 0; o < 3; ++o) {
                         float m[9];
@@ -466,15 +497,15 @@ __global__ void __launch_bounds__(32 * TL, 2)
             if (!ok) break;
             plane(1);
             plane(2);
-            const bool store = line && cx - 1 >= p.x0 && cx - 1 <= p.x1;
+            const bool store = line && live && cx - 1 >= p.x0 && cx - 1 <= p.x1;
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
                 if (store) {
-                    stv<C>(ql + (int64_t)(cx - 1) * (3 * K) + r * K, acc[0][r]);
+                    stc(ql + (int64_t)(cx - 1) * (3 * K) + r * K, acc[0][r]);
 #pragma unroll
                     for (int v = 0; v < C; ++v) dacc[v] += (double)pc[r][v] * (double)acc[0][r][v];
                 }
-                ldv<C>(base + (UY + 1) * 3 * K + r * K, pc[r]);
+                ldc(base + (UY + 1) * 3 * KC + r * KC, pc[r]);
 #pragma unroll
                 for (int v = 0; v < C; ++v) {
                     acc[0][r][v] = acc[1][r][v];
@@ -496,11 +527,11 @@ __global__ void __launch_bounds__(32 * TL, 2)
     }
     double *sh = reinterpret_cast<double *>(traw);
 #pragma unroll
-    for (int v = 0; v < C; ++v) sh[warp * K + lane * C + v] = dacc[v];
+    for (int v = 0; v < C; ++v) sh[warp * KC + lane * CS0 + v * CS1] = dacc[v];
     __syncthreads();
-    for (int c = threadIdx.x; c < K; c += blockDim.x) {
+    for (int c = threadIdx.x; c < KC; c += blockDim.x) {
         double sum = 0;
-        for (int j = 0; j < TL; ++j) sum += sh[j * K + c];
+        for (int j = 0; j < TL; ++j) sum += sh[j * KC + c];
         atomicAdd(pq + c, sum);
     }
 }
@@ -664,9 +695,35 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 
 }  // namespace
 
+namespace {
+
+// Nodes from which a mesh that is only numbered like a lattice (its nodes
+// moved) gets the lattice view too.  The product by node blocks and by the
+// streamed kernel, us, with 32, 64 and 128 columns: 6,859 nodes 18.0, 23.1,
+// 34.9 and 20.1, 25.0, 35.3; 12,167 nodes 27.2, 30.7, 45.4 and 23.1, 29.1,
+// 43.6; 50,653 nodes 93, 114, 154 and 54, 68, 109.
+constexpr int64_t kNumberedLattice = 8192;
+
+// the sides of the lattice that the pattern is numbered along, if its 27
+// diagonals are those of lattice neighbours (k_lattice_fill checks the entries)
+bool numbered_lattice(sfc_system *s, int &nx, int &ny, int &nz)
+{
+    if (!s->has_bsr || s->nodes < kNumberedLattice || !dia_offsets(s) || s->dia_nd != 27) return false;
+    nx = s->dia_off[16];
+    const int plane = s->dia_off[22];
+    if (nx < 2 || plane % nx || s->nodes % plane) return false;
+    ny = plane / nx;
+    nz = (int)(s->nodes / plane);
+    for (int d = 0; d < 27; ++d)
+        if (s->dia_off[d] != (d / 9 - 1) * plane + (d / 3 % 3 - 1) * nx + d % 3 - 1) return false;
+    return ny >= 2 && nz >= 2;
+}
+
+}  // namespace
+
 // Installs the lattice view when the system's pattern comes from a 3-dof
-// mesh whose nodes form a lattice (numbered x fastest) and every block couples
-// lattice neighbours, and picks the product that uses it: the streamed
+// mesh whose nodes form a lattice (numbered x fastest), or is numbered like
+// one, and every block couples lattice neighbours, and picks the product that uses it: the streamed
 // x-line kernel by default, the TMA-staged brick kernel with SFC_SPMM=lattice
 // in the environment.  SFC_SPMM=bsr, and every other mesh, keep the
 // node-block (BSR) kernels.
@@ -679,10 +736,24 @@ void build_lattice_blocks(sfc_system *s)
     const char *e = std::getenv("SFC_SPMM");
     const std::string want = e ? e : "";
     if (want == "bsr") return;
-    if (!s->has_bsr || !m || !m->is_grid || m->dim != 3 || m->dof != 3) return;
-    const int nx = m->gn[0], ny = m->gn[1], nz = m->gn[2];
-    if ((int64_t)nx * ny * nz != s->nodes || nx < 2 || ny < 2 || nz < 2) return;
-    s->bq.alloc((size_t)s->nodes * NODE_FLOATS);  // same size on every rebuild: no reallocation
+    if (!s->has_bsr || !m || m->dim != 3 || m->dof != 3) return;
+    int nx, ny, nz;
+    if (m->is_grid) {
+        nx = m->gn[0], ny = m->gn[1], nz = m->gn[2];
+        if ((int64_t)nx * ny * nz != s->nodes || nx < 2 || ny < 2 || nz < 2) return;
+        s->bq.alloc((size_t)s->nodes * NODE_FLOATS);  // same size on every rebuild: no reallocation
+        s->bq64.alloc((size_t)s->nodes * NODE_FLOATS);
+    } else {
+        if (want == "lattice" || !numbered_lattice(s, nx, ny, nz)) return;
+        try {
+            s->bq.alloc((size_t)s->nodes * NODE_FLOATS);
+            s->bq64.alloc((size_t)s->nodes * NODE_FLOATS);
+        } catch (const Error &) {  // no room for the views: the node blocks do
+            s->bq.release();
+            s->bq64.release();
+            return;
+        }
+    }
     if (!s->lat_err.p) {
         s->lat_err.alloc(1);
         SFC_CK(cudaMemsetAsync(s->lat_err.p, 0, sizeof(int), ctx->stream));
@@ -694,7 +765,6 @@ void build_lattice_blocks(sfc_system *s)
     k_lattice_fill<float><<<grid_for(s->nodes * 32, 256), 256, 0, ctx->stream>>>(s->bptr.p, s->bcol.p, s->bval32.p,
                                                                               s->nodes, nx, ny, s->bq.p, err.p);
     // the FP64 view for the true residual (k_xresid64)
-    s->bq64.alloc((size_t)s->nodes * NODE_FLOATS);
     SFC_CK(cudaMemsetAsync(s->bq64.p, 0, (size_t)s->nodes * NODE_FLOATS * 8, ctx->stream));
     k_lattice_fill<double><<<grid_for(s->nodes * 32, 256), 256, 0, ctx->stream>>>(s->bptr.p, s->bcol.p, s->bval64.p,
                                                                                s->nodes, nx, ny, s->bq64.p, err.p);
@@ -713,7 +783,8 @@ void build_lattice_blocks(sfc_system *s)
 // by x bz nodes, cached with the operand and box it was made for.
 static void encode_map(sfc_system *s, const float *P, int K, int bc, int bx, int by, int bz)
 {
-    if (s->pmap_ptr == P && s->pmap_K == K && s->pmap_box == bx) return;
+    const int shape = bc * 256 + bx;
+    if (s->pmap_ptr == P && s->pmap_K == K && s->pmap_box == shape) return;
     const int nx = s->lat[0], ny = s->lat[1], nz = s->lat[2];
     const cuuint64_t dims[5] = {(cuuint64_t)K, 3, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
     const cuuint64_t strides[4] = {(cuuint64_t)K * 4, (cuuint64_t)3 * K * 4, (cuuint64_t)3 * K * 4 * nx,
@@ -726,7 +797,7 @@ static void encode_map(sfc_system *s, const float *P, int K, int bc, int bx, int
     if (r != CUDA_SUCCESS) fail(SFC_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
     s->pmap_ptr = P;
     s->pmap_K = K;
-    s->pmap_box = bx;
+    s->pmap_box = shape;
 }
 
 // the tensor map of P and the brick kernel's attributes, set up outside any
@@ -771,47 +842,62 @@ void lattice_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, 
 
 // kernel attributes and the tensor map of P for the streamed product, set up
 // outside any stream capture
-template <int K>
+template <int K, int C>
 int tspmm_occ()
 {
     static int occ = 0;
     if (!occ) {
-        SFC_CK(cudaFuncSetAttribute(k_tspmm32<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem<K>()));
-        SFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tspmm32<K>, 32 * TL, tsmem<K>()));
+        constexpr size_t smem = tsmem<32 * C>();
+        SFC_CK(cudaFuncSetAttribute(k_tspmm32<K, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tspmm32<K, C>, 32 * TL, smem));
         if (occ < 1) occ = 1;
     }
     return occ;
 }
 
-void xline_prepare(sfc_system *s, const float *P, int K)
+namespace {
+// f(K, C) for the columns per row and per lane
+template <class F>
+void tspmm_pick(int K, int cols, F &&f)
 {
+    using std::integral_constant;
     SFC_REQUIRE(K == 32 || K == 64 || K == 128, "streamed lattice SpMM needs 32, 64 or 128 columns");
-    if (K == 32) tspmm_occ<32>();
-    else if (K == 64) tspmm_occ<64>();
-    else tspmm_occ<128>();
-    encode_map(s, P, K, K, 1, UY, UZ);
+    const int C = (std::min(cols, K) + 31) / 32;
+    if (K == 32) f(integral_constant<int, 32>(), integral_constant<int, 1>());
+    else if (K == 64 && C == 1) f(integral_constant<int, 64>(), integral_constant<int, 1>());
+    else if (K == 64) f(integral_constant<int, 64>(), integral_constant<int, 2>());
+    else if (C == 1) f(integral_constant<int, 128>(), integral_constant<int, 1>());
+    else if (C == 2) f(integral_constant<int, 128>(), integral_constant<int, 2>());
+    else if (C == 3) f(integral_constant<int, 128>(), integral_constant<int, 3>());
+    else f(integral_constant<int, 128>(), integral_constant<int, 4>());
+}
+}  // namespace
+
+void xline_prepare(sfc_system *s, const float *P, int K, int cols)
+{
+    tspmm_pick(K, cols, [&](auto k, auto c) {
+        tspmm_occ<k.value, c.value>();
+        encode_map(s, P, K, 32 * c.value, 1, UY, UZ);
+    });
 }
 
-template <int K>
-void tspmm_launch(sfc_system *s, float *Q, double *pq, const int *stop)
+// Q = S P of the first cols columns (of K to a row), pq: column dots; columns
+// whose threshold is infinite are not stored
+void xline_spmm32(sfc_system *s, const float *P, float *Q, int K, int cols, double *pq, const double *thr, const int *stop)
 {
+    xline_prepare(s, P, K, cols);
     sfc_ctx *ctx = s->ctx;
     const int nx = s->lat[0], ny = s->lat[1], nz = s->lat[2];
     const int64_t total = (int64_t)((ny + TY - 1) / TY) * ((nz + TZ - 1) / TZ) * nx;  // positions of all tiles
-    // equal pieces over the resident CTAs, of at least four positions (each
-    // piece walks two more)
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)tspmm_occ<K>() * ctx->sm_count, total / 4));
-    k_tspmm32<K><<<(unsigned)grid, 32 * TL, tsmem<K>(), ctx->stream>>>(s->pmap, s->bq.p, Q, nx, ny, nz, total, pq,
-                                                                           stop, s->lat_err.p);
+    tspmm_pick(K, cols, [&](auto k, auto c) {
+        // equal pieces over the resident CTAs, of at least four positions (each
+        // piece walks two more)
+        const int64_t grid =
+            std::max<int64_t>(1, std::min<int64_t>((int64_t)tspmm_occ<k.value, c.value>() * ctx->sm_count, total / 4));
+        k_tspmm32<k.value, c.value><<<(unsigned)grid, 32 * TL, tsmem<32 * c.value>(), ctx->stream>>>(
+            s->pmap, s->bq.p, Q, nx, ny, nz, total, pq, thr, stop, s->lat_err.p);
+    });
     count_launch(ctx);
-}
-
-void xline_spmm32(sfc_system *s, const float *P, float *Q, int K, double *pq, const int *stop)
-{
-    xline_prepare(s, P, K);
-    if (K == 32) tspmm_launch<32>(s, Q, pq, stop);
-    else if (K == 64) tspmm_launch<64>(s, Q, pq, stop);
-    else tspmm_launch<128>(s, Q, pq, stop);
 }
 
 // the FP64 residual on the lattice view (k_xresid64): K = 128 as two

@@ -482,6 +482,12 @@ bool dia_spmv64(sfc_system *s, const double *x, double *y, double *dot, const in
 
 void dia_ensure(sfc_system *s) { dia_prepare(s); }
 
+bool dia_offsets(sfc_system *s)
+{
+    if (!s->dia_tried) dia_pattern(s);
+    return s->dia_nd > 0;
+}
+
 Format grid_operator(sfc_system *s, PcgArgs &g, bool blocks)
 {
     const bool dia = dia_prepare(s);

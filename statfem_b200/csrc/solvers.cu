@@ -244,17 +244,33 @@ __device__ void cluster_cols_add(const double (&a1)[V], const double (&a2)[V], d
     }
     cl.sync();  // the partial sums stay until every CTA has read them
 }
+
+// Whether a lane has a column to work on: the others' (past the right-hand
+// sides, converged, or left to FP64) have an infinite threshold, and nothing
+// of theirs is read or written, so that a block costs the bytes of its open
+// columns (72 of 128, 98,304 dofs: p update 46 -> 37 us).  Their sums stay zero.
+template <int V>
+__device__ __forceinline__ bool live_lane(const double *thr)
+{
+    bool l = false;
+#pragma unroll
+    for (int v = 0; v < V; ++v) l |= thr[(threadIdx.x & 31) * V + v] < INFINITY;
+    return l;
+}
+
 // Q = S P (FP32 values, FP32 vectors, FP32 accumulate), warp per row;
 // pq[c] += sum_i P[i][c] Q[i][c] in FP64
 template <int V>
 __global__ void __launch_bounds__(256) k_spmm32(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                                                 const float *__restrict__ a, const float *__restrict__ P,
-                                                float *__restrict__ Q, int64_t N, double *pq, const int *stop)
+                                                float *__restrict__ Q, int64_t N, double *pq, const double *thr,
+                                                const int *stop)
 {
     constexpr int K = 32 * V;
     __shared__ double sh[8 * K];
     if (*stop) return;
     const int lane = threadIdx.x & 31;
+    const bool live = live_lane<V>(thr);
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     double dacc[V];
 #pragma unroll
@@ -273,14 +289,14 @@ __global__ void __launch_bounds__(256) k_spmm32(const int32_t *__restrict__ rp, 
                 const float aj = __shfl_sync(0xffffffffu, av, j);
                 const int32_t cj = __shfl_sync(0xffffffffu, cv, j);
                 float pv[V];
-                ldv<V>(P + (int64_t)cj * K + lane * V, pv);
+                ldv_if<V>(live, P + (int64_t)cj * K + lane * V, pv);
 #pragma unroll
                 for (int v = 0; v < V; ++v) acc[v] = fmaf(aj, pv[v], acc[v]);
             }
         }
-        stv<V>(Q + i * K + lane * V, acc);
+        if (live) stv<V>(Q + i * K + lane * V, acc);
         float pi[V];
-        ldv<V>(P + i * K + lane * V, pi);
+        ldv_if<V>(live, P + i * K + lane * V, pi);
 #pragma unroll
         for (int v = 0; v < V; ++v) dacc[v] += (double)pi[v] * (double)acc[v];
     }
@@ -295,7 +311,8 @@ __global__ void __launch_bounds__(256) k_spmm32(const int32_t *__restrict__ rp, 
 template <int V>
 __global__ void __launch_bounds__(256) k_bspmm32(const int32_t *__restrict__ bptr, const int32_t *__restrict__ bcol,
                                                  const float *__restrict__ bval, const float *__restrict__ P,
-                                                 float *__restrict__ Q, int64_t nodes, double *pq, const int *stop)
+                                                 float *__restrict__ Q, int64_t nodes, double *pq, const double *thr,
+                                                 const int *stop)
 {
     constexpr int K = 32 * V;
     __shared__ double sh[8 * K];
@@ -303,6 +320,7 @@ __global__ void __launch_bounds__(256) k_bspmm32(const int32_t *__restrict__ bpt
     __shared__ int sc[8][32];
     if (*stop) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool live = live_lane<V>(thr);
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     double dacc[V];
 #pragma unroll
@@ -329,9 +347,9 @@ __global__ void __launch_bounds__(256) k_bspmm32(const int32_t *__restrict__ bpt
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const float *pj = P + (int64_t)(3 * sc[w][t + u]) * K + lane * V;
-                    ldv<V>(pj, pv[u][0]);
-                    ldv<V>(pj + K, pv[u][1]);
-                    ldv<V>(pj + 2 * K, pv[u][2]);
+                    ldv_if<V>(live, pj, pv[u][0]);
+                    ldv_if<V>(live, pj + K, pv[u][1]);
+                    ldv_if<V>(live, pj + 2 * K, pv[u][2]);
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
@@ -349,9 +367,9 @@ __global__ void __launch_bounds__(256) k_bspmm32(const int32_t *__restrict__ bpt
             for (; t < nbk; ++t) {
                 const float *pj = P + (int64_t)(3 * sc[w][t]) * K + lane * V;
                 float p0[V], p1[V], p2[V];
-                ldv<V>(pj, p0);
-                ldv<V>(pj + K, p1);
-                ldv<V>(pj + 2 * K, p2);
+                ldv_if<V>(live, pj, p0);
+                ldv_if<V>(live, pj + K, p1);
+                ldv_if<V>(live, pj + 2 * K, p2);
                 const float *bv = &sv[w][t * 9];
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
@@ -365,9 +383,9 @@ __global__ void __launch_bounds__(256) k_bspmm32(const int32_t *__restrict__ bpt
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
             const int64_t o = (3 * i + r) * K + lane * V;
-            stv<V>(Q + o, acc[r]);
+            if (live) stv<V>(Q + o, acc[r]);
             float pi[V];
-            ldv<V>(P + o, pi);
+            ldv_if<V>(live, P + o, pi);
 #pragma unroll
             for (int v = 0; v < V; ++v) dacc[v] += (double)pi[v] * (double)acc[r][v];
         }
@@ -552,7 +570,8 @@ __global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(256) k_bup
     double a1[V], a2[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) a1[v] = a2[v] = 0.0;
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < N; i += warps) {
+    const int64_t end = live_lane<V>(thr) ? N : 0;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < end; i += warps) {
         const int64_t o = i * K + lane * V;
         float xv[V], rv[V], pv[V], qv[V];
         ldv<V>(x + o, xv);
@@ -574,12 +593,47 @@ __global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(256) k_bup
     cluster_cols_add<V>(a1, a2, sh, rz_next, rr_next);
 }
 
+// The end of an inner iteration, by the last block of its p update (a launch
+// of its own and the memset of the next slots took 5 of 59 us at 52,728 dofs
+// and 40 columns): clears the slots of the iteration after next, and the first
+// iteration after which all columns are below their thresholds sets *stop
+// (every later kernel of the check interval returns at once) and records in
+// *ran how many of the interval's iterations ran.  A block counts itself in
+// when it is done, so that none still reads what the last one changes.
+struct IterEnd {
+    const double *rr, *thr;
+    double *clear;  // 3 K sums
+    int *stop, *ran, *count;
+    int it;  // within the interval
+};
+
+template <int K>
+__device__ void iteration_end(const IterEnd &e)
+{
+    __shared__ int last;
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(e.count, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    bool open = false;
+    for (int c = threadIdx.x; c < K; c += blockDim.x) open |= e.rr[c] > e.thr[c];
+    for (int c = threadIdx.x; c < 3 * K; c += blockDim.x) e.clear[c] = 0.0;
+    open = __syncthreads_or(open);
+    if (threadIdx.x == 0) {
+        *e.count = 0;
+        if (!open) {
+            *e.stop = 1;
+            *e.ran = e.it + 1;
+        }
+    }
+}
+
 // p = D^-1 r + beta p for active columns (rr' > thr)
 template <int V>
 __global__ void __launch_bounds__(256) k_bpupdate32(float *__restrict__ p, const float *__restrict__ r,
                                                     const float *__restrict__ dinv, int64_t N, const double *rz,
                                                     const double *rz_next, const double *rr_next, const double *thr,
-                                                    const int *stop, const int *brk)
+                                                    const int *stop, const int *brk, IterEnd end_of)
 {
     constexpr int K = 32 * V;
     if (*stop) return;
@@ -593,7 +647,8 @@ __global__ void __launch_bounds__(256) k_bpupdate32(float *__restrict__ p, const
         beta[v] = act[v] ? (float)(rz_next[c] / rz[c]) : 0.f;
     }
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < N; i += warps) {
+    const int64_t end = live_lane<V>(thr) ? N : 0;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < end; i += warps) {
         const int64_t o = i * K + lane * V;
         float pv[V], rv[V];
         ldv<V>(p + o, pv);
@@ -604,6 +659,7 @@ __global__ void __launch_bounds__(256) k_bpupdate32(float *__restrict__ p, const
             if (act[v]) pv[v] = fmaf(beta[v], pv[v], di * rv[v]);
         stv<V>(p + o, pv);
     }
+    iteration_end<K>(end_of);
 }
 
 // scalar two-level p update: z = D^-1 r + e[agg(i)] (0 on constrained dofs),
@@ -615,7 +671,7 @@ __global__ void __launch_bounds__(256) k_cbpupdate32(float *__restrict__ p, cons
                                                      const float4 *__restrict__ mode, const float *__restrict__ e,
                                                      int64_t N, const double *rz, const double *rz_next,
                                                      const double *rr_next, const double *thr, const int *stop,
-                                                     const int *brk, const int *restart)
+                                                     const int *brk, const int *restart, IterEnd end_of)
 {
     constexpr int K = 32 * V;
     if (!INIT && *stop) return;
@@ -634,7 +690,8 @@ __global__ void __launch_bounds__(256) k_cbpupdate32(float *__restrict__ p, cons
         }
     }
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < N; i += warps) {
+    const int64_t end = INIT || live_lane<V>(thr) ? N : 0;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < end; i += warps) {
         const int64_t o = i * K + lane * V;
         float pv[V], rv[V], ev[V];
         ldv<V>(p + o, pv);
@@ -649,6 +706,7 @@ __global__ void __launch_bounds__(256) k_cbpupdate32(float *__restrict__ p, cons
         }
         stv<V>(p + o, pv);
     }
+    if constexpr (!INIT) iteration_end<K>(end_of);
 }
 
 // ---- nodal 3x3 block-Jacobi variants of the three vector kernels -------------
@@ -737,7 +795,8 @@ __global__ void __cluster_dims__(kColCluster, 1, 1) __launch_bounds__(256, 4) k_
     double a1[V], a2[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) a1[v] = a2[v] = 0.0;
-    for (int64_t n = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; n < nodes; n += warps) {
+    const int64_t end = live_lane<V>(thr) ? nodes : 0;
+    for (int64_t n = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; n < end; n += warps) {
         float rv[3][V], zv[3][V];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -802,6 +861,7 @@ __global__ void __cluster_dims__(S, 1, 1) __launch_bounds__(32 * W, 24 / W)
         if (!frozen && !(den > 0.0) && rank == 0 && a == 0) err[col] = 1;
         alpha[v] = (frozen || !(den > 0.0)) ? 0.f : (float)(rz[col] / den);
     }
+    const bool live = live_lane<V>(thr);
     // r.z and r.r over this warp's nodes (a few dozen) in FP32, then FP64
     // across warps and CTAs
     float a1f[V], a2f[V];
@@ -830,6 +890,7 @@ __global__ void __cluster_dims__(S, 1, 1) __launch_bounds__(32 * W, 24 / W)
             const float mx = __shfl_sync(0xffffffffu, lm.x, k), my = __shfl_sync(0xffffffffu, lm.y, k),
                         mz = __shfl_sync(0xffffffffu, lm.z, k);
             const int bits = (int)__shfl_sync(0xffffffffu, lm.w, k);
+            if (!live) continue;  // the shuffles are behind
             float rv[3][V], zv[3][V];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -912,7 +973,7 @@ __global__ void __launch_bounds__(256) k_npupdate32(float *__restrict__ p, const
                                                     const float *__restrict__ bdinv, int64_t nodes, const double *rz,
                                                     const double *rz_next, const double *rr_next, const double *thr,
                                                     const int *stop, const int *brk, float *__restrict__ x,
-                                                    const double *pq, const double *rr)
+                                                    const double *pq, const double *rr, IterEnd end_of)
 {
     constexpr int K = 32 * V;
     if (*stop) return;
@@ -927,7 +988,8 @@ __global__ void __launch_bounds__(256) k_npupdate32(float *__restrict__ p, const
         alpha[v] = x ? iter_alpha(c, pq, rz, rr, thr, brk) : 0.f;
     }
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t n = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; n < nodes; n += warps) {
+    const int64_t end = live_lane<V>(thr) ? nodes : 0;
+    for (int64_t n = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; n < end; n += warps) {
         float rv[3][V], zv[3][V];
 #pragma unroll
         for (int i = 0; i < 3; ++i) ldv<V>(r + (3 * n + i) * K + lane * V, rv[i]);
@@ -950,6 +1012,7 @@ __global__ void __launch_bounds__(256) k_npupdate32(float *__restrict__ p, const
             stv<V>(p + o, pv);
         }
     }
+    iteration_end<K>(end_of);
 }
 
 // two-level variant of the p update: z = Dinv_n r_n + M_n e_a (the coarse
@@ -965,7 +1028,7 @@ __global__ void __launch_bounds__(256, 4) k_ncpupdate32(float *__restrict__ p, c
                                                      int64_t nodes, const double *rz, const double *rz_next,
                                                      const double *rr_next, const double *thr, const int *stop,
                                                      const int *brk, const int *restart, float *__restrict__ x,
-                                                     const double *pq, const double *rr)
+                                                     const double *pq, const double *rr, IterEnd end_of)
 {
     constexpr int K = 32 * V;
     if (!INIT && *stop) return;
@@ -986,7 +1049,8 @@ __global__ void __launch_bounds__(256, 4) k_ncpupdate32(float *__restrict__ p, c
         }
     }
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t n = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; n < nodes; n += warps) {
+    const int64_t end = INIT || live_lane<V>(thr) ? nodes : 0;
+    for (int64_t n = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; n < end; n += warps) {
         float rv[3][V], zv[3][V];
 #pragma unroll
         for (int i = 0; i < 3; ++i) ldv<V>(r + (3 * n + i) * K + lane * V, rv[i]);
@@ -1039,26 +1103,7 @@ __global__ void __launch_bounds__(256, 4) k_ncpupdate32(float *__restrict__ p, c
             stv<V>(p + o, pv);
         }
     }
-}
-
-// Convergence test after every inner iteration of a check interval: the
-// first iteration after which all columns are below their thresholds sets
-// *stop (every later kernel of the interval returns at once) and records in
-// *ran how many of the interval's iterations ran (it_local + 1).
-template <int K>
-__global__ void k_bcheck_it(const double *rr, const double *thr, int *stop, int *ran, int it_local)
-{
-    __shared__ int any;
-    if (*stop) return;  // uniform: only check kernels set it, and none runs beside this one
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    for (int c = threadIdx.x; c < K; c += blockDim.x)
-        if (rr[c] > thr[c]) any = 1;
-    __syncthreads();
-    if (threadIdx.x == 0 && !any) {
-        *stop = 1;
-        *ran = it_local + 1;
-    }
+    if constexpr (!INIT) iteration_end<K>(end_of);
 }
 
 // x64 += norm_c * x32
@@ -1282,10 +1327,10 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     } b64{s->blk64.p}, x64{s->blk64.p + N * K}, r64{s->blk64.p + 2 * N * K}, cs{s->colsc.p};
     float *xr = s->blk32.p, *rr32 = xr + N * K, *pp = rr32 + N * K, *qq = pp + N * K;
     // Per-iteration column scalars in a ring of R slots of 3K doubles
-    // (p.q | r.z | r.r).  Iteration it reads r.z and r.r of slot it % R and
-    // accumulates its p.q, the new r.z and the new r.r into slot (it+1) % R,
-    // which it zeroes first (the slot's last reader, iteration it+1-R, is
-    // done).  With R = check every check interval uses the same slots, so
+    // (p.q | r.z | r.r).  Iteration it reads r.z and r.r of slot it % R,
+    // accumulates its p.q, the new r.z and the new r.r into slot (it+1) % R
+    // and zeroes slot (it+2) % R in the end (whose last reader is done: an
+    // earlier iteration, or with R = 2 this one).  With R = check every check interval uses the same slots, so
     // one captured graph serves every interval.
     const int R = check >= 2 ? check : 2;
     const int64_t nsc = 3 * (int64_t)R * K;
@@ -1294,8 +1339,9 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     double *bn2 = cs.p, *rn2 = bn2 + K, *scale = rn2 + K, *norm = scale + K, *thr = norm + K;
     // flags[0]: all columns below their thresholds; flags[1 + c]: breakdown
     // (p^T A p <= 0) in column c; flags[1 + K]: iterations of the current
-    // check interval that ran before flags[0] was set (0: all of them)
-    s->flags.reserve(2 + K);
+    // check interval that ran before flags[0] was set (0: all of them);
+    // flags[2 + K]: blocks of the p update that are done
+    s->flags.reserve(3 + K);
     int *stop = s->flags.p, *err = s->flags.p + 1, *ran = s->flags.p + 1 + K;
     std::vector<int> hflags(2 + K), nbreak(K), fallback(K), nstall(K);
     int n_fallback = 0;
@@ -1305,6 +1351,12 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     // block without a row
     const unsigned gw = (grid_for((bsr ? s->nodes : N) * 32, 256, ctx->sm_count * 8) + kColCluster - 1) / kColCluster *
                         kColCluster;
+    // The updates start, and add up their columns, once per CTA: r updates two
+    // to an SM, p updates (no sums) four, which is one wave.  52,728 dofs, 40
+    // columns, us with 8, 4, 2: r update 18.4, 16.4, 13.7, p update 16.8, 16.3,
+    // 20.8; 151,959 dofs, 128 columns, r update with 6, 4, 2: 49, 54, 46.
+    const unsigned gu = std::min<unsigned>(gw, (unsigned)ctx->sm_count / 4 * kColCluster),
+                   gp = std::min<unsigned>(gw, (unsigned)ctx->sm_count * 4);
     const bool two_any = use_two_level(s);
     const CoarseSpace &crs = s->coarse;
     const bool two = two_any && crs.dof == 3;   // block Jacobi + rigid-body modes
@@ -1333,12 +1385,13 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             k_resid64<V><<<gw, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op.p, X, Bm, R, N, out);
         count_launch(ctx);
     };
+    int cols = K;  // of the block at hand
     auto spmm = [&](const float *Pm, float *Qm, double *out) {
         ProfScope ps(ctx, "spmm32",
                      bsr ? (double)s->nblocks * 40 + 4.0 * (s->nodes + 1) + 2.0 * N * K * 4
                          : (double)s->nnz * 8 + 4.0 * (N + 1) + 2.0 * N * K * 4);
         if (bsr && s->has_lattice && s->lat_mode == 2) {
-            xline_spmm32(s, Pm, Qm, K, out, stop);
+            xline_spmm32(s, Pm, Qm, K, cols, out, thr, stop);
             return;
         }
         if (bsr && s->has_lattice && s->lat_mode == 1 && K >= 64) {
@@ -1346,9 +1399,9 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             return;
         }
         if (bsr)
-            k_bspmm32<V><<<gw, 256, 0, ctx->stream>>>(s->bptr.p, s->bcol.p, s->bval32.p, Pm, Qm, s->nodes, out, stop);
+            k_bspmm32<V><<<gw, 256, 0, ctx->stream>>>(s->bptr.p, s->bcol.p, s->bval32.p, Pm, Qm, s->nodes, out, thr, stop);
         else
-            k_spmm32<V><<<gw, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op32.p, Pm, Qm, N, out, stop);
+            k_spmm32<V><<<gw, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op32.p, Pm, Qm, N, out, thr, stop);
         count_launch(ctx);
     };
     s->restart.reserve(K);
@@ -1364,7 +1417,7 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             k_ncpupdate32<V, true><<<gw, 256, 0, ctx->stream>>>(pp, rr32, s->bdinv32.p, crs.node_agg.p, crs.mode.p,
                                                                 crs.e32.p, s->nodes, nullptr, nullptr, nullptr,
                                                                 nullptr, nullptr, nullptr, restart.p, nullptr, nullptr,
-                                                                nullptr);
+                                                                nullptr, IterEnd{});
         } else if (two1) {
             k_binit32<V, false><<<gw, 256, 0, ctx->stream>>>(r64.p, scale, s->dinv32.p, restart.p, rr32, xr, pp, N,
                                                              rz_slot, rr_slot);
@@ -1372,7 +1425,7 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             coarse_block_apply<V>(s, rr32, rz_slot, nullptr);
             k_cbpupdate32<V, true><<<gw, 256, 0, ctx->stream>>>(pp, rr32, s->dinv32.p, crs.node_agg.p, crs.mode.p,
                                                                 crs.e32.p, N, nullptr, nullptr, nullptr, nullptr,
-                                                                nullptr, nullptr, restart.p);
+                                                                nullptr, nullptr, restart.p, IterEnd{});
         } else if (bj)
             k_ninit32<V><<<gw, 256, 0, ctx->stream>>>(r64.p, scale, s->bdinv32.p, restart.p, rr32, xr, pp, s->nodes,
                                                       rz_slot, rr_slot);
@@ -1385,17 +1438,28 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     // coarse correction, beta and the p update
     auto iterate = [&](int it) {
         double *cur = sl(it), *nxt = sl(it + 1);
-        SFC_CK(cudaMemsetAsync(nxt, 0, (size_t)3 * K * 8, ctx->stream));
+        const IterEnd end_of{nxt + 2 * K, thr, sl(it + 2), stop, ran, ran + 1, it % check};
         double *pqi = nxt, *rz0 = cur + K, *rr0 = cur + 2 * K, *rz1 = nxt + K, *rr1 = nxt + 2 * K;
         spmm(pp, qq, pqi);
         if (fuse_restrict) {
             coarse_block_reserve(s, K);  // no-op once reserved (always, inside a capture)
             {
                 ProfScope ps(ctx, "nrupdate32", 3.0 * N * K * 4 + 52.0 * s->nodes + 4.0 * crs.nc * K);
-                constexpr int W = 8, S = 2;  // 16 warps per aggregate
-                k_nrupdate32<V, W, S><<<(unsigned)(crs.nagg * S), 32 * W, 0, ctx->stream>>>(
-                    rr32, qq, s->bdinv32.p, crs.agg_ptr.p, crs.agg_nodes.p, crs.mode.p, crs.c32.p, pqi, rz0, rr0,
-                    thr, rz1, rr1, stop, err);
+                constexpr int W = 8;
+                auto launch = [&](auto size) {
+                    constexpr int S = decltype(size)::value;
+                    k_nrupdate32<V, W, S><<<(unsigned)(crs.nagg * S), 32 * W, 0, ctx->stream>>>(
+                        rr32, qq, s->bdinv32.p, crs.agg_ptr.p, crs.agg_nodes.p, crs.mode.p, crs.c32.p, pqi, rz0, rr0,
+                        thr, rz1, rr1, stop, err);
+                };
+                // as many CTAs per aggregate as one wave holds (three of W warps
+                // to an SM), two at least.  64 aggregates (31^3 cells, 128
+                // columns) with 2, 4, 8: 61, 41, 52 us; 27 (24^3): 70, 43, 30;
+                // 1 (8^3): 42, 26, 19; 343 (48^3): 114, 139, 140.
+                const int64_t room = 3 * (int64_t)ctx->sm_count / std::max<int64_t>(crs.nagg, 1);
+                if (room >= 8) launch(std::integral_constant<int, 8>());
+                else if (room >= 4) launch(std::integral_constant<int, 4>());
+                else launch(std::integral_constant<int, 2>());
             }
             count_launch(ctx);
             coarse_block_gemm<V>(s, rz1, stop);
@@ -1403,10 +1467,10 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             {
                 ProfScope ps(ctx, "bupdate32", (bj ? 3.0 : 6.0) * N * K * 4 + (bj ? 12.0 : 4.0) * N);
                 if (bj)
-                    k_nupdate32<V, false><<<gw, 256, 0, ctx->stream>>>(xr, rr32, pp, qq, s->bdinv32.p, s->nodes,
+                    k_nupdate32<V, false><<<gu, 256, 0, ctx->stream>>>(xr, rr32, pp, qq, s->bdinv32.p, s->nodes,
                                                                        pqi, rz0, rr0, thr, rz1, rr1, stop, err);
                 else
-                    k_bupdate32<V><<<gw, 256, 0, ctx->stream>>>(xr, rr32, pp, qq, s->dinv32.p, N, pqi, rz0,
+                    k_bupdate32<V><<<gu, 256, 0, ctx->stream>>>(xr, rr32, pp, qq, s->dinv32.p, N, pqi, rz0,
                                                                 rr0, thr, rz1, rr1, stop, err);
             }
             count_launch(ctx);
@@ -1416,27 +1480,24 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             ProfScope ps(ctx, "bpupdate32",
                          (bj ? 5.0 : 3.0) * N * K * 4 + (bj ? 12.0 : 4.0) * N + (two ? 8.0 * s->nodes : 0.0));
             if (two)
-                k_ncpupdate32<V, false><<<gw, 256, 0, ctx->stream>>>(pp, rr32, s->bdinv32.p, crs.node_agg.p,
+                k_ncpupdate32<V, false><<<gp, 256, 0, ctx->stream>>>(pp, rr32, s->bdinv32.p, crs.node_agg.p,
                                                                      crs.mode.p, crs.e32.p, s->nodes, rz0, rz1,
                                                                      rr1, thr, stop, err, nullptr, xr, pqi,
-                                                                     rr0);
+                                                                     rr0, end_of);
             else if (bj)
-                k_npupdate32<V><<<gw, 256, 0, ctx->stream>>>(pp, rr32, s->bdinv32.p, s->nodes, rz0, rz1,
-                                                             rr1, thr, stop, err, xr, pqi, rr0);
+                k_npupdate32<V><<<gp, 256, 0, ctx->stream>>>(pp, rr32, s->bdinv32.p, s->nodes, rz0, rz1,
+                                                             rr1, thr, stop, err, xr, pqi, rr0, end_of);
             else if (two1)
-                k_cbpupdate32<V, false><<<gw, 256, 0, ctx->stream>>>(pp, rr32, s->dinv32.p, crs.node_agg.p,
+                k_cbpupdate32<V, false><<<gp, 256, 0, ctx->stream>>>(pp, rr32, s->dinv32.p, crs.node_agg.p,
                                                                      crs.mode.p, crs.e32.p, N, rz0, rz1,
-                                                                     rr1, thr, stop, err, nullptr);
+                                                                     rr1, thr, stop, err, nullptr, end_of);
             else
-                k_bpupdate32<V><<<gw, 256, 0, ctx->stream>>>(pp, rr32, s->dinv32.p, N, rz0, rz1, rr1,
-                                                             thr, stop, err);
+                k_bpupdate32<V><<<gp, 256, 0, ctx->stream>>>(pp, rr32, s->dinv32.p, N, rz0, rz1, rr1,
+                                                             thr, stop, err, end_of);
         }
-        // convergence after every iteration: the rest of the interval returns
-        // at once when all columns are below their thresholds
-        k_bcheck_it<K><<<1, 128, 0, ctx->stream>>>(rr1, thr, stop, ran, it % check);
-        count_launch(ctx, 2);
+        count_launch(ctx);
     };
-    // A whole check interval as one CUDA graph: the ring's zeroing, `check`
+    // A whole check interval as one CUDA graph: `check`
     // iterations and the convergence flag, captured once per launch
     // configuration (the key lists every pointer and size baked into the
     // launches) and replayed for every later interval.  Not used while kernel
@@ -1446,11 +1507,12 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     const bool use_graph = !ctx->prof && check >= 2 && !(genv && genv[0] == '0');
     const bool lattice = bsr && s->has_lattice && s->lat_mode == 1 && K >= 64;
     auto launch_chunk_graph = [&]() -> bool {
-        GraphExec &g = s->blk_graph[V == 1 ? 0 : V == 2 ? 1 : 2];
+        const int in_use = (cols + 31) / 32;
+        GraphExec &g = s->blk_graph[(V == 1 ? 0 : V == 2 ? 1 : 3) + in_use - 1];
         // everything the captured launches allocate or set up, done outside the capture
         if (two_any) coarse_block_reserve(s, K);
         if (lattice) lattice_prepare(s, pp, K);
-        if (bsr && s->has_lattice && s->lat_mode == 2) xline_prepare(s, pp, K);
+        if (bsr && s->has_lattice && s->lat_mode == 2) xline_prepare(s, pp, K, cols);
         const std::vector<uintptr_t> key = {
             (uintptr_t)K, (uintptr_t)check, (uintptr_t)N, (uintptr_t)s->nodes, (uintptr_t)gw,
             (uintptr_t)(bsr | (bj << 1) | (two << 2) | (two1 << 3) | (lattice << 4) | (fuse_restrict << 5)),
@@ -1461,7 +1523,7 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             (uintptr_t)s->lat_err.p, (uintptr_t)s->lat_mode, (uintptr_t)s->lat[0], (uintptr_t)s->lat[1], (uintptr_t)s->lat[2],
             (uintptr_t)s->pmap_ptr, (uintptr_t)crs.agg_ptr.p, (uintptr_t)crs.agg_nodes.p, (uintptr_t)crs.mode.p,
             (uintptr_t)crs.c32.p, (uintptr_t)crs.e32.p, (uintptr_t)crs.a32.p, (uintptr_t)crs.node_agg.p,
-            (uintptr_t)crs.nagg, (uintptr_t)crs.nc, (uintptr_t)crs.dof};
+            (uintptr_t)crs.nagg, (uintptr_t)crs.nc, (uintptr_t)crs.dof, (uintptr_t)in_use};
         if (!g.exec || g.key != key) {
             g.reset();
             if (g.failed_key == key) return false;  // this configuration could not be captured: eager
@@ -1531,11 +1593,12 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     bool all_conv = true;
     for (int c0 = 0; c0 < nrhs; c0 += K) {
         const int kb = std::min(K, nrhs - c0);
+        cols = kb;
         k_gather_cols<<<grid_for(N * K, 256), 256, 0, ctx->stream>>>(B, ld, c0, kb, K, N, b64.p);
         SFC_CK(cudaMemsetAsync(x64.p, 0, N * K * 8, ctx->stream));
         SFC_CK(cudaMemsetAsync(cs.p, 0, 6 * K * 8, ctx->stream));
         SFC_CK(cudaMemsetAsync(s->scal.p, 0, nsc * 8, ctx->stream));
-        SFC_CK(cudaMemsetAsync(s->flags.p, 0, (2 + K) * sizeof(int), ctx->stream));
+        SFC_CK(cudaMemsetAsync(s->flags.p, 0, (3 + K) * sizeof(int), ctx->stream));
         std::fill(nbreak.begin(), nbreak.end(), 0);
         std::fill(fallback.begin(), fallback.end(), 0);
         std::fill(nstall.begin(), nstall.end(), 0);
@@ -1670,7 +1733,8 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             SFC_CK(cudaMemcpyAsync(thr, ht.data(), K * 8, cudaMemcpyHostToDevice, ctx->stream));
             SFC_CK(cudaMemcpyAsync(restart.p, hrestart.data(), K * 4, cudaMemcpyHostToDevice, ctx->stream));
             SFC_CK(cudaMemsetAsync(sl(it), 0, (size_t)3 * K * 8, ctx->stream));
-            SFC_CK(cudaMemsetAsync(s->flags.p, 0, (2 + K) * sizeof(int), ctx->stream));
+            SFC_CK(cudaMemsetAsync(sl(it + 1), 0, (size_t)3 * K * 8, ctx->stream));
+            SFC_CK(cudaMemsetAsync(s->flags.p, 0, (3 + K) * sizeof(int), ctx->stream));
             // r32 <- scaled true residual, x32 <- 0, p kept (restarted columns: p = z)
             init32(rz1, rr1);
         }
