@@ -105,92 +105,103 @@ __global__ void __launch_bounds__(256) k_kw_dense(const double *__restrict__ coo
     }
 }
 
-// one axis of the Kronecker product: for every node, column a:
-// out[node(m)] = sum_k Kd[m][k] in[node(k)]  along axis d (stride sd, length nd)
-// STAGE: the nd x nd factor is staged in shared memory (it fits); else it
-// is read through the cache
-template <bool STAGE>
-__global__ void k_kron_axis(const double *__restrict__ Kd, int nd, int64_t sd, int64_t nodes, int dof, int c,
-                            int64_t ns, const double *__restrict__ in, double *__restrict__ out)
+// D (8 x 8) += A (8 x 4) B (4 x 8): lane l holds A[l / 4][l % 4], B[l % 4][l / 4], D[l / 4][2 (l % 4) + 0, 1]
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
 {
-    extern __shared__ double sKd[];
-    const double *sK = Kd;
-    if (STAGE) {
-        for (int t = threadIdx.x; t < nd * nd; t += blockDim.x) sKd[t] = Kd[t];
-        __syncthreads();
-        sK = sKd;
-    }
-    const int64_t total = nodes * ns;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t node = t / ns;
-        const int64_t a = t - node * ns;
-        const int64_t m = (node / sd) % nd;
-        const int64_t base = node - m * sd;
-        double s = 0.0;
-        for (int k = 0; k < nd; ++k) s = fma(sK[m * nd + k], in[((base + k * sd) * dof + c) * ns + a], s);
-        out[(node * dof + c) * ns + a] = s;
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// 1-D SE correlation factor along one grid axis: scale exp(-d^2/(2 l^2)) of the
+// n coordinates behind it (the host took 0.4 ms for two axes of 182)
+__global__ void k_se_axis(double *__restrict__ K, int n, double length, double scale)
+{
+    const double *x = K + (int64_t)n * n;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n * n; t += (int64_t)gridDim.x * blockDim.x) {
+        const double d = x[t / n] - x[t % n];
+        K[t] = scale * exp(-(d * d) / (2. * length * length));
     }
 }
 
-// The same axis product as a batch of small dense products, for nd <= 64
-// points per line: one CTA per (line, 128 columns) stages the line's input
-// rows and the factor in shared memory; warp w computes the output points
-// m = w, w + 8, ... and lane l the columns l, l + 32, l + 64, l + 96, so each
-// staged value feeds up to 8 multiply-adds from registers.
-constexpr int kLineCols = 128;
+// One axis of the Kronecker product: out[m] = sum_k Kd[m][k] in[k] along axis d
+// (length nd, stride sd nodes) of every lattice line, for all cols = dof ns
+// values of a node.  One product of the nd x nd factor with all lines' values
+// side by side (a line's cols columns after the other's), FP64 matrix
+// instructions (m8n8k4): a CTA of four warps takes 64 rows by 64 columns,
+// whichever lines these belong to, 16 x 64 to a warp, and passes over k in
+// steps of 16, the next step's values on their way while one is multiplied.
+// Bound by the multiplications (the lane layouts and the odd multiples of four
+// as row lengths keep shared memory free of conflicts).  182 x 182 nodes, 75
+// columns: 50 us an axis (a thread per value, reading a line per value,
+// took 345; the matrix units' time is 27); 49^3 nodes, 768 columns: 534 (three
+// launches of a line per CTA in FMAs took 957).
+constexpr int kKronTile = 64, kKronStep = 16;
 
-__global__ void __launch_bounds__(256) k_kron_line(const double *__restrict__ Kd, int nd, int64_t sd, int dof, int c,
-                                                   int64_t ns, const double *__restrict__ in, double *__restrict__ out)
+__global__ void __launch_bounds__(128) k_kron_axis(const double *__restrict__ Kd, int nd, int64_t sd, int64_t cols,
+                                                   int64_t total, const double *__restrict__ in, double *__restrict__ out)
 {
-    extern __shared__ double sm[];
-    double *sK = sm, *sIn = sm + nd * nd;
-    const int64_t L = blockIdx.x;  // line: nodes base + k sd, k < nd
-    const int64_t base = (L / sd) * sd * nd + L % sd;
-    const int64_t col0 = (int64_t)blockIdx.y * kLineCols;
-    const int ncols = (int)(ns - col0 < kLineCols ? ns - col0 : kLineCols);
-    for (int t = threadIdx.x; t < nd * nd; t += blockDim.x) sK[t] = Kd[t];
-    // eight loads in flight per thread before they are stored
-    const int total = nd * kLineCols;
-    for (int t0 = threadIdx.x; t0 < total; t0 += 8 * blockDim.x) {
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int t = t0 + u * blockDim.x, k = t / kLineCols, j = t % kLineCols;
-            v[u] = (t < total && j < ncols) ? in[((base + k * sd) * dof + c) * ns + col0 + j] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int t = t0 + u * blockDim.x;
-            if (t < total) sIn[t] = v[u];
-        }
+    constexpr int T = kKronTile, S = kKronStep, LA = S + 4, LB = T + 4;
+    __shared__ double sA[T * LA], sB[S * LB];
+    __shared__ int64_t off[T];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
+    const int m0 = blockIdx.y * T;
+    const int64_t stride = sd * cols;
+    if (threadIdx.x < T) {
+        const int64_t n = (int64_t)blockIdx.x * T + threadIdx.x, line = n / cols;
+        off[threadIdx.x] = n < total ? ((line / sd) * sd * nd + line % sd) * cols + n % cols : -1;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double acc[8][4];
+    double acc[2][T / 8][2];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[u][q] = 0.0;
-    for (int k = 0; k < nd; ++k) {
-        double v[4];
+        for (int j = 0; j < T / 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    // this thread's values of a step: A (row t / 16, k = t % 16), B (k = t / 64, column t % 64)
+    const int bc = threadIdx.x % T;
+    const int64_t bo = off[bc];
+    double va[T * S / 128], vb[T * S / 128];
+    auto fetch = [&](int k0) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = sIn[k * kLineCols + lane + 32 * q];
+        for (int u = 0; u < T * S / 128; ++u) {
+            const int t = threadIdx.x + 128 * u, m = m0 + t / S, k = k0 + t % S, kb = k0 + t / T;
+            va[u] = m < nd && k < nd ? Kd[(int64_t)m * nd + k] : 0.0;
+            vb[u] = kb < nd && bo >= 0 ? in[bo + kb * stride] : 0.0;
+        }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < nd; k0 += S) {
+        __syncthreads();
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int m = w + 8 * u;
-            const double kv = m < nd ? sK[m * nd + k] : 0.0;
+        for (int u = 0; u < T * S / 128; ++u) {
+            const int t = threadIdx.x + 128 * u;
+            sA[(t / S) * LA + t % S] = va[u];
+            sB[(t / T) * LB + bc] = vb[u];
+        }
+        __syncthreads();
+        if (k0 + S < nd) fetch(k0 + S);
+        const int steps = min(S / 4, (nd - k0 + 3) / 4);
+        for (int s = 0; s < steps; ++s) {
+            const double a0 = sA[(16 * warp + r) * LA + 4 * s + q], a1 = sA[(16 * warp + 8 + r) * LA + 4 * s + q];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[u][q] = fma(kv, v[q], acc[u][q]);
+            for (int j = 0; j < T / 8; ++j) {
+                const double b = sB[(4 * s + q) * LB + 8 * j + r];
+                dmma(acc[0][j], a0, b);
+                dmma(acc[1][j], a1, b);
+            }
         }
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int m = w + 8 * u;
+    for (int i = 0; i < 2; ++i) {
+        const int m = m0 + 16 * warp + 8 * i + r;
         if (m >= nd) continue;
-        double *o = out + ((base + m * sd) * dof + c) * ns + col0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (lane + 32 * q < ncols) o[lane + 32 * q] = acc[u][q];
+        for (int j = 0; j < T / 8; ++j)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int64_t o = off[8 * j + 2 * q + v];
+                if (o >= 0) out[o + m * stride] = acc[i][j][v];
+            }
     }
 }
 
@@ -464,19 +475,6 @@ void gemm(sfc_ctx *ctx, int ta, int tb, int64_t M, int64_t N, int64_t K, double 
     count_launch(ctx);
 }
 
-// 1-D SE correlation factor along one grid axis: exp(-d^2/(2 l^2))
-std::vector<double> se_axis(const std::vector<double> &x, double length)
-{
-    const int n = (int)x.size();
-    std::vector<double> K((size_t)n * n);
-    for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j) {
-            const double d = x[i] - x[j];
-            K[(size_t)i * n + j] = std::exp(-(d * d) / (2. * length * length));
-        }
-    return K;
-}
-
 }  // namespace
 
 // T = K W (per component); W, T, tmp: num_dofs x ns device arrays
@@ -492,47 +490,27 @@ void kernel_times(sfc_ctx *ctx, sfc_covar_forcing *cf, double sigma, double leng
         const int nax = m->dim;
         DBuf<double> *dK = cf->kron;
         for (int a = 0; a < nax; ++a) {
-            std::vector<double> Kd = se_axis(m->gaxis[a], length);
-            if (a == 0)
-                for (double &v : Kd) v *= sigma * sigma;
-            upload(ctx, dK[a], Kd.data(), Kd.size());
+            const size_t n = m->gaxis[a].size();
+            dK[a].reserve(n * n + n);
+            SFC_CK(cudaMemcpyAsync(dK[a].p + n * n, m->gaxis[a].data(), n * 8, cudaMemcpyHostToDevice, ctx->stream));
+            k_se_axis<<<grid_for(n * n, 256), 256, 0, ctx->stream>>>(dK[a].p, (int)n, length,
+                                                                     a == 0 ? sigma * sigma : 1.0);
+            count_launch(ctx);
         }
-        for (int c = 0; c < dof; ++c) {
-            const double *src = W;
-            double *bufs[2] = {T, tmp};
-            int64_t sd = 1;
-            int cur = 0;
-            for (int a = 0; a < nax; ++a) {
-                const int nd = m->gn[a];
-                double *dst = bufs[cur];
-                ProfScope ps(ctx, "kron_axis", 2.0 * nodes * ns * 8);
-                const size_t kb = (size_t)nd * nd * 8;
-                if (nd <= 64) {
-                    const size_t smem = (size_t)(nd * nd + nd * kLineCols) * 8;
-                    SFC_CK(cudaFuncSetAttribute(k_kron_line, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                    const dim3 g((unsigned)(nodes / nd), (unsigned)((ns + kLineCols - 1) / kLineCols));
-                    k_kron_line<<<g, 256, smem, ctx->stream>>>(dK[a].p, nd, sd, dof, c, ns, src, dst);
-                } else if (kb <= 48 * 1024) {
-                    k_kron_axis<true><<<grid_for(nodes * ns, 256), 256, kb, ctx->stream>>>(dK[a].p, nd, sd, nodes, dof,
-                                                                                         c, ns, src, dst);
-                } else if (kb <= 200 * 1024) {
-                    SFC_CK(cudaFuncSetAttribute(k_kron_axis<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)kb));
-                    k_kron_axis<true><<<grid_for(nodes * ns, 256), 256, kb, ctx->stream>>>(dK[a].p, nd, sd, nodes, dof,
-                                                                                         c, ns, src, dst);
-                } else {
-                    k_kron_axis<false><<<grid_for(nodes * ns, 256), 256, 0, ctx->stream>>>(dK[a].p, nd, sd, nodes,
-                                                                                         dof, c, ns, src, dst);
-                }
-                count_launch(ctx);
-                src = dst;
-                cur ^= 1;
-                sd *= nd;
-            }
-            if (src != T)  // strided copy of this component's rows back into T
-                SFC_CK(cudaMemcpy2DAsync(T + (int64_t)c * ns, (size_t)dof * ns * 8, src + (int64_t)c * ns,
-                                         (size_t)dof * ns * 8, (size_t)ns * 8, (size_t)nodes, cudaMemcpyDeviceToDevice,
-                                         ctx->stream));
+        // the last axis ends in T
+        const double *src = W;
+        int64_t sd = 1;
+        const int64_t cols = dof * ns;
+        for (int a = 0; a < nax; ++a) {
+            const int nd = m->gn[a];
+            double *dst = (nax - a) % 2 ? T : tmp;
+            ProfScope ps(ctx, "kron_axis", 2.0 * nodes * cols * 8);
+            const int64_t total = nodes / nd * cols;
+            const dim3 g((unsigned)((total + kKronTile - 1) / kKronTile), (unsigned)((nd + kKronTile - 1) / kKronTile));
+            k_kron_axis<<<g, 128, 0, ctx->stream>>>(dK[a].p, nd, sd, cols, total, src, dst);
+            count_launch(ctx);
+            src = dst;
+            sd *= nd;
         }
         SFC_CK(cudaStreamSynchronize(ctx->stream));
     } else {
@@ -549,10 +527,14 @@ void kernel_times(sfc_ctx *ctx, sfc_covar_forcing *cf, double sigma, double leng
 
 // C = A^T B for a symmetric product (A^T B = B^T A, as W^T K W): only the
 // 128 x 128 tiles on and above the diagonal are formed, over a slice of the
-// K rows per CTA (8 x 8 outputs per thread, 8-row chunks double-buffered in
-// shared memory); partial tiles go to part[split][tile] and k_atb_sym_reduce
-// adds them in split order and mirrors the upper tiles (deterministic, exactly
-// symmetric).
+// K rows per CTA; partial tiles go to part[split][tile] and k_atb_sym_reduce
+// adds them in split order and mirrors the upper half (deterministic, exactly
+// symmetric).  FP64 matrix instructions, 32 x 64 outputs to a warp, 8-row
+// chunks double-buffered in shared memory.  Bound by the multiplications:
+// 352,947 rows, 256 columns 1,520 us (8 x 8 outputs per thread in FMAs 2,920,
+// the units' time is 960).  Tiles of 8 x 8 past the M columns are neither
+// multiplied nor stored nor read back: with 16 columns the partial tiles'
+// padding was most of 74 us, now 22.
 constexpr int kSymT = 128;
 constexpr int kSymK = 8;
 
@@ -560,35 +542,39 @@ __global__ void __launch_bounds__(256) k_atb_sym(const double *__restrict__ A, c
                                                  int64_t M, int64_t rows_per_split, const int2 *__restrict__ tiles,
                                                  int ntiles, double *__restrict__ part)
 {
-    __shared__ __align__(16) double sa[2][kSymK][kSymT];
-    __shared__ __align__(16) double sb[2][kSymK][kSymT];
+    constexpr int LD = kSymT + 4;  // an odd multiple of four: no bank conflicts
+    __shared__ __align__(16) double sa[2][kSymK][LD];
+    __shared__ __align__(16) double sb[2][kSymK][LD];
     const int2 tile = tiles[blockIdx.y];
     const int64_t a0 = (int64_t)tile.x * kSymT, b0 = (int64_t)tile.y * kSymT;
     const int64_t k0 = (int64_t)blockIdx.x * rows_per_split;
     const int64_t k1 = k0 + rows_per_split < K ? k0 + rows_per_split : K;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    double acc[8][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
+    const int am = 32 * (warp & 3), bn = 64 * (warp >> 2);  // the warp's outputs
+    const int mi = (int)max((int64_t)0, min((int64_t)4, (M - a0 - am + 7) / 8)),
+              nj = (int)max((int64_t)0, min((int64_t)8, (M - b0 - bn + 7) / 8));  // 8 x 8 tiles with columns
+    double acc[4][8][2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
+        for (int j = 0; j < 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
     // each thread stages 4 values of each operand per chunk: row t / 128, column t % 128
     double ra[4], rb[4];
     auto fetch = [&](int64_t kk) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int t = threadIdx.x + 256 * q, r = t / kSymT, c = t % kSymT;
-            const int64_t k = kk + r;
-            ra[q] = (k < k1 && a0 + c < M) ? A[k * M + a0 + c] : 0.0;
-            rb[q] = (k < k1 && b0 + c < M) ? B[k * M + b0 + c] : 0.0;
+        for (int u = 0; u < 4; ++u) {
+            const int t = threadIdx.x + 256 * u, row = t / kSymT, c = t % kSymT;
+            const int64_t k = kk + row;
+            ra[u] = (k < k1 && a0 + c < M) ? A[k * M + a0 + c] : 0.0;
+            rb[u] = (k < k1 && b0 + c < M) ? B[k * M + b0 + c] : 0.0;
         }
     };
     auto stash = [&](int buf) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int t = threadIdx.x + 256 * q, r = t / kSymT, c = t % kSymT;
-            sa[buf][r][c] = ra[q];
-            sb[buf][r][c] = rb[q];
+        for (int u = 0; u < 4; ++u) {
+            const int t = threadIdx.x + 256 * u, row = t / kSymT, c = t % kSymT;
+            sa[buf][row][c] = ra[u];
+            sb[buf][row][c] = rb[u];
         }
     };
     int buf = 0;
@@ -600,20 +586,21 @@ __global__ void __launch_bounds__(256) k_atb_sym(const double *__restrict__ A, c
     for (int64_t kk = k0; kk < k1; kk += kSymK) {
         const bool more = kk + kSymK < k1;
         if (more) fetch(kk + kSymK);  // in flight during the products
+        if (mi > 0) {
 #pragma unroll
-        for (int r = 0; r < kSymK; ++r) {
-            double av[8], bv[8];
+            for (int s = 0; s < kSymK / 4; ++s) {
+                double av[4];
 #pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                const double2 x = *reinterpret_cast<const double2 *>(&sa[buf][r][ty * 8 + i]);
-                const double2 y = *reinterpret_cast<const double2 *>(&sb[buf][r][tx * 8 + i]);
-                av[i] = x.x; av[i + 1] = x.y;
-                bv[i] = y.x; bv[i + 1] = y.y;
+                for (int i = 0; i < 4; ++i) av[i] = sa[buf][4 * s + q][am + 8 * i + r];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < nj) {
+                        const double bv = sb[buf][4 * s + q][bn + 8 * j + r];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (i < mi) dmma(acc[i][j], av[i], bv);
+                    }
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
         }
         if (more) stash(buf ^ 1);
         __syncthreads();
@@ -621,22 +608,38 @@ __global__ void __launch_bounds__(256) k_atb_sym(const double *__restrict__ A, c
     }
     double *o = part + ((int64_t)blockIdx.x * ntiles + blockIdx.y) * kSymT * kSymT;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[(ty * 8 + i) * kSymT + tx * 8 + j] = acc[i][j];
+        for (int j = 0; j < 8; ++j)
+            if (i < mi && j < nj)
+                *reinterpret_cast<double2 *>(o + (am + 8 * i + r) * kSymT + bn + 8 * j + 2 * q) =
+                    make_double2(acc[i][j][0], acc[i][j][1]);
 }
 
-__global__ void k_atb_sym_reduce(const double *__restrict__ part, int splits, const int2 *__restrict__ tiles,
-                                 int ntiles, int64_t M, double alpha, double *__restrict__ C)
+// 32 entries of a row of C's tiles per block, the splits over its eight rows
+// of threads
+__global__ void __launch_bounds__(256) k_atb_sym_reduce(const double *__restrict__ part, int splits,
+                                                        const int2 *__restrict__ tiles, int ntiles, int64_t M,
+                                                        double alpha, double *__restrict__ C)
 {
-    const int64_t total = (int64_t)ntiles * kSymT * kSymT;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int ti = (int)(t / (kSymT * kSymT));
-        const int e = (int)(t % (kSymT * kSymT)), i = e / kSymT, j = e % kSymT;
-        const int64_t a = (int64_t)tiles[ti].x * kSymT + i, b = (int64_t)tiles[ti].y * kSymT + j;
-        if (a >= M || b >= M) continue;
-        double sum = 0.0;
-        for (int sp = 0; sp < splits; ++sp) sum += part[((int64_t)sp * ntiles + ti) * kSymT * kSymT + e];
+    __shared__ double sh[8][32];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int ti = blockIdx.y, e = blockIdx.x * 32 + x, i = e / kSymT, j = e % kSymT;
+    const int64_t a = (int64_t)tiles[ti].x * kSymT + i, b = (int64_t)tiles[ti].y * kSymT + j;
+    const bool in = a < M && b < M;
+    if (!__syncthreads_or(in)) return;
+    // below the diagonal: the entry above it
+    const int from = tiles[ti].x == tiles[ti].y && i > j ? j * kSymT + i : e;
+    const int first = splits * y / 8, last = splits * (y + 1) / 8;
+    double sum = 0.0;
+    if (in)
+#pragma unroll 4
+        for (int sp = first; sp < last; ++sp) sum += part[((int64_t)sp * ntiles + ti) * kSymT * kSymT + from];
+    sh[y][x] = sum;
+    __syncthreads();
+    if (y == 0 && in) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) sum += sh[k][x];
         sum *= alpha;
         C[a * M + b] = sum;
         if (tiles[ti].x != tiles[ti].y) C[b * M + a] = sum;
@@ -676,8 +679,10 @@ void atb_symmetric(sfc_ctx *ctx, const double *A, const double *B, int64_t K, in
     SFC_CK(cudaMemcpyAsync(dtiles, ht.data(), ntiles * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
     k_atb_sym<<<dim3((unsigned)splits, (unsigned)ntiles), 256, 0, ctx->stream>>>(A, B, K, M, rows, dtiles, ntiles,
                                                                                   part.p);
-    k_atb_sym_reduce<<<grid_for((int64_t)ntiles * kSymT * kSymT, 256), 256, 0, ctx->stream>>>(part.p, (int)splits,
-                                                                                               dtiles, ntiles, M, 1.0, C);
+    // the rows of a tile that has any
+    const unsigned rows32 = (unsigned)(std::min<int64_t>(M, kSymT) * kSymT / 32);
+    k_atb_sym_reduce<<<dim3(rows32, (unsigned)ntiles), 256, 0, ctx->stream>>>(part.p, (int)splits, dtiles, ntiles, M, 1.0,
+                                                                             C);
     count_launch(ctx, 2);
 }
 
