@@ -403,12 +403,14 @@ __global__ void k_koh_system(int ns, int n_o, const double *__restrict__ mean, c
                              double *__restrict__ C, double *__restrict__ D)
 {
     const int64_t nn = (int64_t)ns * ns;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nn; t += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < max(nn, (int64_t)ns * n_o);
+         t += (int64_t)gridDim.x * blockDim.x) {
+        if (t < (int64_t)ns * n_o) D[t] = Y[t] - hp.rho * mean[t / n_o];
+        if (t >= nn) continue;
         const int k = (int)(t / ns), l = (int)(t % ns);
         double v = se_value(xs + 3 * k, xs + 3 * l, dim, hp.mismatch_sigma, hp.mismatch_length);
         if (k == l) v += hp.mismatch_sensor_eps * hp.mismatch_sensor_eps;
         C[t] = v + hp.rho * hp.rho * Cs[t];
-        if (t < (int64_t)ns * n_o) D[t] = Y[t] - hp.rho * mean[t / n_o];
     }
 }
 
