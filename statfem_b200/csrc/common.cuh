@@ -216,7 +216,7 @@ struct sfc_mesh;
 namespace sfc {
 // scratch of spd_inverse_gj (dense.cu)
 struct GjScratch {
-    DBuf<double> diag, rowp, colp;
+    DBuf<double> diag, other, dinv;  // pivots' thresholds; the matrix's second copy; inverses of diagonal blocks
     DBuf<int> word;
     struct Graph {  // captured launch sequence of one (matrix, size)
         const double *A;

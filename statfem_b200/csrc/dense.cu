@@ -2,8 +2,8 @@
 // Gauss-Jordan elimination without pivoting, on the GPU: the in-place form
 //     A[k,k] <- D^-1,  A[k,j] <- D^-1 A[k,j],  A[i,k] <- -A[i,k] D^-1,
 //     A[i,j] <- A[i,j] - A[i,k] D^-1 A[k,j]
-// for 32-wide panels k (D the panel's diagonal block), two launches per
-// panel.  Used for the coarse matrix of the two-level preconditioner (with
+// for 32-wide panels k (D the panel's diagonal block), one launch per panel
+// that reads one copy of A and writes the other.  Used for the coarse matrix of the two-level preconditioner (with
 // dependent pivots dropped: a generalised inverse on the independent modes)
 // and for the sensor-space matrices of the KOH likelihood and posterior
 // (LikelihoodKOH.ipp:75-120, 311-361), where a non-positive pivot is the
@@ -18,159 +18,224 @@ namespace sfc {
 
 namespace {
 
-constexpr int kGJ = 32;         // panel width
-constexpr int kPanelCols = 64;  // columns per CTA of the panel kernel
+constexpr int kGJ = 32;     // panel width
+constexpr int kGjTile = 64; // tile of A per CTA
 
-__global__ void k_diag_of(const double *__restrict__ A, int64_t n, double *__restrict__ d)
+// D (8 x 8) += A (8 x 4) B (4 x 8): lane l holds A[l / 4][l % 4], B[l % 4][l / 4], D[l / 4][2 (l % 4) + 0, 1]
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        d[i] = A[i * n + i];
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
 }
 
-// Gauss-Jordan step, part 1: invert the kb x kb diagonal block D of panel k0
-// (in shared memory, every CTA redundantly; a pivot that is not above
-// rel x the dof's original diagonal is dropped: its row and column are
-// zeroed), save the old column panel colp[i][m] = A[i][k0+m] and form the new
-// row panel rowp[m][j] = (D^-1 A[k0.., j])[m] (= D^-1 itself inside the block).
-__global__ void __launch_bounds__(256) k_gj_panel(const double *__restrict__ A, int64_t n, int64_t k0, int kb,
-                                                  const double *__restrict__ adiag, double rel, double *__restrict__ rowp,
-                                                  double *__restrict__ colp, int *dropped, double *pivots)
+// 1 / d by Newton's iteration on the hardware's approximation (about 20 bits,
+// two steps): no branch in the chain of pivots
+__device__ __forceinline__ double recip(double d)
 {
-    // launched with 256 threads
-    __shared__ double D[2][kGJ][kGJ + 1];
-    __shared__ double T[kGJ][kPanelCols + 1];
-    __shared__ double sad[kGJ];
-    const int64_t j0 = (int64_t)blockIdx.x * kPanelCols;
-    if (threadIdx.x < kGJ) sad[threadIdx.x] = threadIdx.x < kb ? adiag[k0 + threadIdx.x] : 0.0;
-    // stage the diagonal block, this CTA's 64 columns of the row panel and its
-    // 64 rows of the column panel, every load of a thread in flight together
-    {
-        double vd[kGJ * kGJ / 256], vt[kPanelCols * kGJ / 256], vc[kPanelCols * kGJ / 256];
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+    x = fma(x, fma(-d, x, 1.0), x);
+    return fma(x, fma(-d, x, 1.0), x);
+}
+
+// Inverse of the kb x kb symmetric block in D (row stride LD) by the first
+// four warps, written to out (32 x 32, zero outside): the symmetric sweep,
+// warp w holding rows 8 w .., lane j column j, with the next row published
+// before the rest of a step.  A pivot not above rel x the dof's original
+// diagonal (thr) is dropped: its row and column are zeroed.  buf: 2 x 32.
+template <int LD>
+__device__ void gj_block_inverse(const double *D, int kb, const double *thr, double *buf, double *out, int *dropped,
+                                 double *pivots)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[8];
 #pragma unroll
-        for (int u = 0; u < kGJ * kGJ / 256; ++u) {
-            const int t = threadIdx.x + 256 * u, r = t / kGJ, c = t % kGJ;
-            vd[u] = (r < kb && c < kb) ? A[(k0 + r) * n + k0 + c] : 0.0;
-        }
+    for (int i = 0; i < 8; ++i) {
+        const int r = 8 * warp + i;
+        v[i] = r < kb && lane < kb ? D[r * LD + lane] : (r == lane ? 1.0 : 0.0);
+    }
+    if (warp == 0) buf[lane] = v[0];
+    int ndrop = 0;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll 1
+    for (int b = 0; b < 4; ++b) {
 #pragma unroll
-        for (int u = 0; u < kPanelCols * kGJ / 256; ++u) {
-            const int t = threadIdx.x + 256 * u;
-            const int l = t / kPanelCols, c = t % kPanelCols;
-            vt[u] = (l < kb && j0 + c < n) ? A[(k0 + l) * n + j0 + c] : 0.0;
-            const int jj = t / kGJ, m = t % kGJ;  // m fastest: row j0 + jj of A read contiguously
-            vc[u] = (j0 + jj < n && m < kb) ? A[(j0 + jj) * n + k0 + m] : 0.0;
-        }
+        for (int t = 0; t < 8; ++t) {
+            const int k = 8 * b + t, t1 = (t + 1) & 7;
+            const bool own = warp == b, next = warp == (t == 7 ? b + 1 : b);
+            const double *sh = buf + 32 * (t & 1);
+            double *nx = buf + 32 * (t1 & 1);
+            double row[8];
 #pragma unroll
-        for (int u = 0; u < kGJ * kGJ / 256; ++u) {
-            const int t = threadIdx.x + 256 * u;
-            D[0][t / kGJ][t % kGJ] = vd[u];
-        }
+            for (int i = 0; i < 8; ++i) row[i] = sh[8 * warp + i];
+            const double piv = sh[k], mine = sh[lane];
+            const bool drop = k < kb && !(piv > thr[k]);
+            if (threadIdx.x == 0 && k < kb) {
+                if (pivots) pivots[k] = piv;
+                ndrop += drop;
+            }
+            const double inv = drop ? 0.0 : recip(piv);
+            const bool me = lane == k;
+            const double f = me ? inv : drop ? 0.0 : -mine * inv;
+            if (next) {
+                v[t1] = drop ? (me ? 0.0 : v[t1]) : fma(row[t1], f, me ? 0.0 : v[t1]);
+                nx[lane] = v[t1];
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
-        for (int u = 0; u < kPanelCols * kGJ / 256; ++u) {
-            const int t = threadIdx.x + 256 * u;
-            T[t / kPanelCols][t % kPanelCols] = vt[u];
-            const int jj = t / kGJ, m = t % kGJ;
-            if (j0 + jj < n && m < kb) colp[(j0 + jj) * kGJ + m] = vc[u];
+            for (int i = 0; i < 8; ++i) {
+                if (next && i == t1) continue;
+                if (own && i == t) v[i] = me ? -inv : -f;
+                else v[i] = drop ? (me ? 0.0 : v[i]) : fma(row[i], f, me ? 0.0 : v[i]);
+            }
         }
     }
-    __syncthreads();
-    // Gauss-Jordan on the diagonal block: every thread owns 4 entries, reads
-    // buffer cur and writes the other, one barrier per pivot; the drop test
-    // is evaluated identically by every thread
-    int cur = 0, ndrop = 0;
-    for (int p = 0; p < kb; ++p) {
-        const double piv = D[cur][p][p];
-        const bool drop = !(piv > rel * sad[p]);
-        if (pivots && blockIdx.x == 0 && threadIdx.x == 0) pivots[k0 + p] = piv;
-        ndrop += drop;
-        const double ip = drop ? 0.0 : 1.0 / piv;
 #pragma unroll
-        for (int u = 0; u < kGJ * kGJ / 256; ++u) {
-            const int t = threadIdx.x + 256 * u, r = t / kGJ, c = t % kGJ;
-            double v;
-            if (drop)
-                v = (r == p || c == p) ? 0.0 : D[cur][r][c];
-            else if (r == p && c == p)
-                v = ip;
-            else if (r == p)
-                v = D[cur][p][c] * ip;
-            else if (c == p)
-                v = -D[cur][r][p] * ip;
-            else
-                v = D[cur][r][c] - D[cur][r][p] * (D[cur][p][c] * ip);
-            D[cur ^ 1][r][c] = v;
+    for (int i = 0; i < 8; ++i) {
+        const int r = 8 * warp + i;
+        out[r * kGJ + lane] = r < kb && lane < kb ? -v[i] : 0.0;
+    }
+    if (threadIdx.x == 0 && ndrop) atomicAdd(dropped, ndrop);
+}
+
+// The original diagonal (x rel: the thresholds of the pivots) and the inverse
+// of the first diagonal block
+__global__ void __launch_bounds__(256) k_gj_first(const double *__restrict__ A, int64_t n, double rel,
+                                                  double *__restrict__ thr, double *__restrict__ dinv, int *dropped,
+                                                  double *pivots)
+{
+    __shared__ double D[kGJ * (kGJ + 1)], buf[2 * kGJ], st[kGJ];
+    const int kb = (int)min((int64_t)kGJ, n);
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) thr[i] = rel * A[i * n + i];
+    for (int t = threadIdx.x; t < kGJ * kGJ; t += blockDim.x) {
+        const int r = t / kGJ, c = t % kGJ;
+        D[r * (kGJ + 1) + c] = r < kb && c < kb ? A[r * n + c] : 0.0;
+    }
+    if (threadIdx.x < kGJ) st[threadIdx.x] = threadIdx.x < kb ? rel * A[threadIdx.x * (n + 1)] : 0.0;
+    __syncthreads();
+    if (threadIdx.x < 128) gj_block_inverse<kGJ + 1>(D, kb, st, buf, dinv, dropped, pivots);
+}
+
+// One panel, a 64 x 64 tile of the result per CTA, with D^-1 of the panel's
+// diagonal block in dinv:
+//   rows of the panel:     out = rowp[i - k0][j],  rowp = D^-1 A[k0.., j] (D^-1 itself inside the block)
+//   columns of the panel:  out = -A[i, k0..] rowp[:, j]
+//   elsewhere:             out = A[i][j] - A[i, k0..] rowp[:, j]
+// on FP64 matrix instructions, every CTA forming the rowp of its columns
+// itself.  The first CTA takes the tile with the next panel's diagonal block
+// and inverts that too, while the others are at their products: the chain
+// from panel to panel is a launch, a tile and an inverse of 3 us.  1,000 x
+// 1,000: 468 us; 1,202 as two launches per panel, the inverse (with a barrier
+// of the whole CTA and a division per pivot) before the panel's products.
+__global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ A, double *__restrict__ out, int64_t n,
+                                                 int64_t k0, int kb, const double *__restrict__ thr,
+                                                 const double *__restrict__ dinv, double *__restrict__ dnext,
+                                                 int *dropped, double *pivots)
+{
+    constexpr int T = kGjTile, LC = kGJ + 4, LR = T + 4;  // odd multiples of four: no bank conflicts
+    __shared__ double sD[kGJ * LC], sC[T * LC], sR[kGJ * LR];
+    __shared__ double buf[2 * kGJ], st[kGJ];
+    const int gt = (int)((n + T - 1) / T);
+    const int64_t kn = k0 + kGJ;  // the next panel
+    const int crit = (int)(min(kn, n - 1) / T);
+    int b = blockIdx.x;
+    b = b == 0 ? crit * gt + crit : b == crit * gt + crit ? 0 : b;
+    const int64_t i0 = (int64_t)(b / gt) * T, j0 = (int64_t)(b % gt) * T;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, q = lane & 3;
+    const int wi = 16 * (warp & 3), wj = 32 * (warp >> 2);  // the warp's 16 x 32 of the tile
+    double own[2][4][2];
+    {  // every load of a thread in flight before the stores
+        double vd[4], vc[8], vr[8];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) vd[u] = dinv[threadIdx.x + 256 * u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int t = threadIdx.x + 256 * u;
+            const int i = t / kGJ, m = t % kGJ, l = t / T, j = t % T;
+            vc[u] = (i0 + i < n && m < kb) ? A[(i0 + i) * n + k0 + m] : 0.0;
+            vr[u] = (l < kb && j0 + j < n) ? A[(k0 + l) * n + j0 + j] : 0.0;
         }
-        cur ^= 1;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const int64_t i = i0 + wi + 8 * x + r, j = j0 + wj + 8 * y + 2 * q + v;
+                    own[x][y][v] = i < n && j < n ? A[i * n + j] : 0.0;
+                }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int t = threadIdx.x + 256 * u;
+            sD[(t / kGJ) * LC + t % kGJ] = vd[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int t = threadIdx.x + 256 * u;
+            sC[(t / kGJ) * LC + t % kGJ] = vc[u];
+            sR[(t / T) * LR + t % T] = vr[u];
+        }
+        if (threadIdx.x < kGJ) st[threadIdx.x] = kn + threadIdx.x < n ? thr[kn + threadIdx.x] : 0.0;
+    }
+    __syncthreads();
+    {  // rowp: rows 8 (warp % 4) .., columns wj .. of it
+        double p[4][2];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) p[y][0] = p[y][1] = 0.0;
+        const int m0 = 8 * (warp & 3);
+#pragma unroll
+        for (int k = 0; k < kGJ; k += 4) {
+            const double a = sD[(m0 + r) * LC + k + q];
+#pragma unroll
+            for (int y = 0; y < 4; ++y) dmma(p[y], a, sR[(k + q) * LR + wj + 8 * y + r]);
+        }
         __syncthreads();
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && ndrop) atomicAdd(dropped, ndrop);
-    const int c = threadIdx.x % kPanelCols, mg = threadIdx.x / kPanelCols;  // 4 groups of 8 rows of D^-1
-    const int64_t j = j0 + c;
-    if (j < n) {
-        const bool inside = j >= k0 && j < k0 + kb;
 #pragma unroll
-        for (int u = 0; u < kGJ / 4; ++u) {
-            const int m = mg * (kGJ / 4) + u;
-            if (m >= kb) continue;
-            double v;
-            if (inside) {
-                v = D[cur][m][j - k0];
-            } else {
-                v = 0.0;
-#pragma unroll 8
-                for (int l = 0; l < kGJ; ++l) v += D[cur][m][l] * T[l][c];
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int m = m0 + r, j = wj + 8 * y + 2 * q + v;
+                const int64_t in = j0 + j - k0;  // column of the block
+                sR[m * LR + j] = in >= 0 && in < kb ? sD[m * LC + in] : p[y][v];
             }
-            rowp[m * n + j] = v;
-        }
-    }
-}
-
-// Gauss-Jordan step, part 2 (64 x 64 tile per CTA):
-//   rows of the panel:     A[i][j] = rowp[i-k0][j]
-//   columns of the panel:  A[i][j] = -colp[i] . rowp[:, j]   (= -A[i,k] D^-1)
-//   elsewhere:             A[i][j] -= colp[i] . rowp[:, j]
-__global__ void __launch_bounds__(256) k_gj_update(double *__restrict__ A, int64_t n, int64_t k0, int kb,
-                                                   const double *__restrict__ rowp, const double *__restrict__ colp)
-{
-    __shared__ double cp[64][kGJ + 1];
-    __shared__ double rp[kGJ][64 + 1];
-    const int64_t i0 = (int64_t)blockIdx.y * 64, j0 = (int64_t)blockIdx.x * 64;
-    {  // all 16 loads of a thread in flight before the stores (launched with 256 threads)
-        double vc[64 * kGJ / 256], vr[64 * kGJ / 256];
-#pragma unroll
-        for (int u = 0; u < 64 * kGJ / 256; ++u) {
-            const int t = threadIdx.x + 256 * u;
-            const int r = t / kGJ, m = t % kGJ;
-            vc[u] = (i0 + r < n && m < kb) ? colp[(i0 + r) * kGJ + m] : 0.0;
-            const int mm = t / 64, c = t % 64;
-            vr[u] = (j0 + c < n && mm < kb) ? rowp[mm * n + j0 + c] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 64 * kGJ / 256; ++u) {
-            const int t = threadIdx.x + 256 * u;
-            cp[t / kGJ][t % kGJ] = vc[u];
-            rp[t / 64][t % 64] = vr[u];
-        }
     }
     __syncthreads();
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    for (int u = 0; u < 4; ++u) {
-        const int64_t i = i0 + ty + 16 * u;
-        if (i >= n) continue;
-        for (int v = 0; v < 4; ++v) {
-            const int64_t j = j0 + tx + 16 * v;
-            if (j >= n) continue;
-            if (i >= k0 && i < k0 + kb) {
-                A[i * n + j] = rp[i - k0][tx + 16 * v];
-                continue;
-            }
-            double s = 0.0;
+    double s[2][4][2];
 #pragma unroll
-            for (int m = 0; m < kGJ; ++m) s += cp[ty + 16 * u][m] * rp[m][tx + 16 * v];
-            A[i * n + j] = (j >= k0 && j < k0 + kb) ? -s : A[i * n + j] - s;
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) s[x][y][0] = s[x][y][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < kGJ; k += 4) {
+        const double a0 = sC[(wi + r) * LC + k + q], a1 = sC[(wi + 8 + r) * LC + k + q];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const double bv = sR[(k + q) * LR + wj + 8 * y + r];
+            dmma(s[0][y], a0, bv);
+            dmma(s[1][y], a1, bv);
         }
     }
+    __syncthreads();  // sD is free for the next block
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int ti = wi + 8 * x + r, tj = wj + 8 * y + 2 * q + v;
+                const int64_t i = i0 + ti, j = j0 + tj;
+                const bool in_r = i >= k0 && i < k0 + kb, in_c = j >= k0 && j < k0 + kb;
+                const double w = in_r ? sR[(i - k0) * LR + tj] : in_c ? -s[x][y][v] : own[x][y][v] - s[x][y][v];
+                if (i < n && j < n) out[i * n + j] = w;
+                if (blockIdx.x == 0 && i >= kn && i < kn + kGJ && j >= kn && j < kn + kGJ)
+                    sD[(i - kn) * LC + j - kn] = w;
+            }
+    if (blockIdx.x != 0 || kn >= n) return;
+    __syncthreads();
+    if (threadIdx.x < 128)
+        gj_block_inverse<LC>(sD, (int)min((int64_t)kGJ, n - kn), st, buf, dnext, dropped, pivots ? pivots + kn : nullptr);
 }
-
 
 }  // namespace
 
@@ -185,34 +250,38 @@ GjScratch::~GjScratch() { drop_graphs(); }
 
 void GjScratch::reserve(int64_t n)
 {
-    if ((size_t)n > diag.n || (size_t)(kGJ * n) > rowp.n || !word.p) drop_graphs();  // buffers move
+    if ((size_t)n > diag.n || (size_t)(n * n) > other.n || !word.p) drop_graphs();  // buffers move
     diag.reserve(n);
-    rowp.reserve(kGJ * n);
-    colp.reserve(kGJ * n);
+    other.reserve(n * n);
+    dinv.reserve(2 * kGJ * kGJ);
     word.reserve(1);
 }
 
 namespace {
 void gj_enqueue(cudaStream_t st, double *A, int64_t n, double rel, GjScratch &w, double *pivots)
 {
-    k_diag_of<<<grid_for(n, 256), 256, 0, st>>>(A, n, w.diag.p);
     cudaMemsetAsync(w.word.p, 0, sizeof(int), st);
-    const unsigned gp = (unsigned)((n + kPanelCols - 1) / kPanelCols), gt = (unsigned)((n + 63) / 64);
-    for (int64_t k0 = 0; k0 < n; k0 += kGJ) {
+    k_gj_first<<<1, 256, 0, st>>>(A, n, rel, w.diag.p, w.dinv.p, w.word.p, pivots);
+    const unsigned gt = (unsigned)((n + kGjTile - 1) / kGjTile);
+    double *from = A, *to = w.other.p;
+    int p = 0;
+    for (int64_t k0 = 0; k0 < n; k0 += kGJ, ++p) {
         const int kb = (int)std::min<int64_t>(kGJ, n - k0);
-        k_gj_panel<<<gp, 256, 0, st>>>(A, n, k0, kb, w.diag.p, rel, w.rowp.p, w.colp.p, w.word.p, pivots);
-        k_gj_update<<<dim3(gt, gt), 256, 0, st>>>(A, n, k0, kb, w.rowp.p, w.colp.p);
+        k_gj_step<<<gt * gt, 256, 0, st>>>(from, to, n, k0, kb, w.diag.p, w.dinv.p + (p & 1) * kGJ * kGJ,
+                                           w.dinv.p + (~p & 1) * kGJ * kGJ, w.word.p, pivots);
+        std::swap(from, to);
     }
+    if (from != A) cudaMemcpyAsync(A, from, n * n * sizeof(double), cudaMemcpyDeviceToDevice, st);
 }
 }  // namespace
 
 // The launch sequence of one inverse depends only on (A, n, rel, pivots) and
 // the scratch buffers, so it is captured once into a CUDA graph and replayed
-// (2 n / 32 + 1 short launches would otherwise be host-bound).
+// (n / 32 + 1 short launches would otherwise be host-bound).
 void spd_inverse_gj(sfc_ctx *ctx, double *A, int64_t n, double rel, GjScratch &w, double *pivots, int *dropped)
 {
     w.reserve(n);
-    const int nlaunch = 1 + 2 * (int)((n + kGJ - 1) / kGJ);
+    const int nlaunch = 1 + (int)((n + kGJ - 1) / kGJ);
     GjScratch::Graph *g = nullptr;
     for (auto &e : w.graphs)
         if (e.A == A && e.n == n && e.rel == rel && e.pivots == pivots) g = &e;
