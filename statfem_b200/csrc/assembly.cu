@@ -281,6 +281,12 @@ __device__ __forceinline__ double jacobian(const double (*X)[3], const double (*
 // element matrices
 // ---------------------------------------------------------------------------
 
+// four doubles, a whole 32-byte sector, in one store (p 32-byte aligned)
+__device__ __forceinline__ void store4(double *p, double a, double b, double c, double d)
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
 // Poisson element matrix, one thread per element (L = NN <= 8):
 // Ke = 0; per quadrature point Ke += ((kappa*detJ)*w) * (dphiDx^T dphiDx)
 // (del2/fem/ElementPotential.ipp:58-74, corlib/ComputeElementMatrix.hpp:62-77,
@@ -323,15 +329,22 @@ __global__ void __launch_bounds__(128) k_elem_poisson(const double *__restrict__
                 }
         }
         double *out = ke + e * (NN * NN);
-        int u = 0;
+        // upper triangle at (m, n): row m starts at m NN - m (m - 1) / 2
+        auto at = [&](int m, int n) -> double {
+            const int a = m < n ? m : n, b = m < n ? n : m;
+            return Ke[a * NN - a * (a - 1) / 2 + b - a];
+        };
+        if constexpr (NN % 4 == 0) {
 #pragma unroll
-        for (int m = 0; m < NN; ++m)
+            for (int m = 0; m < NN; ++m)
 #pragma unroll
-            for (int n = m; n < NN; ++n) {
-                out[m * NN + n] = Ke[u];
-                out[n * NN + m] = Ke[u];
-                ++u;
-            }
+                for (int n = 0; n < NN; n += 4) store4(out + m * NN + n, at(m, n), at(m, n + 1), at(m, n + 2), at(m, n + 3));
+        } else {
+#pragma unroll
+            for (int m = 0; m < NN; ++m)
+#pragma unroll
+                for (int n = 0; n < NN; ++n) out[m * NN + n] = at(m, n);
+        }
     }
 }
 
@@ -451,11 +464,31 @@ __global__ void k_gather(const int32_t *__restrict__ slot_ptr, const int32_t *__
 // ((w*detJ)*factor) * (f_c*phi_n)  (del2/fem/ElementPotential.ipp:149-176;
 // solid/fem/ElementStatic.ipp:441-466), factor = 1.
 // ---------------------------------------------------------------------------
+// On hexahedra a node has eight elements of eight points, so each point's
+// w*detJ is computed once, by k_load_points, and read from sw (80^3 cells:
+// 166 us; 352 with the determinants in this kernel, bound by the arithmetic).
+template <int D, int NN>
+__global__ void __launch_bounds__(128) k_load_points(const double *__restrict__ coords, const uint32_t *__restrict__ conn,
+                                                     const QuadTable qt, int64_t E, double *__restrict__ sw)
+{
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+        double X[NN][3];
+#pragma unroll
+        for (int K = 0; K < NN; ++K) {
+            const double *p = coords + 3 * (int64_t)conn[e * NN + K];
+            X[K][0] = p[0];
+            X[K][1] = p[1];
+            X[K][2] = p[2];
+        }
+        for (int q = 0; q < qt.nq; ++q) sw[e * qt.nq + q] = MUL(MUL(qt.w[q], jacobian<D, NN>(X, qt.dphi[q])), 1.0);
+    }
+}
+
 template <int D, int NN>
 __global__ void k_load(const double *__restrict__ coords, const uint32_t *__restrict__ conn,
                        const int32_t *__restrict__ node_ptr, const int32_t *__restrict__ node_elem,
                        const QuadTable qt, int64_t num_nodes, int dof, double f0, double f1, double f2,
-                       double *__restrict__ F)
+                       const double *__restrict__ sw, double *__restrict__ F)
 {
     const double f[3] = {f0, f1, f2};
     for (int64_t nd = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; nd < num_nodes;
@@ -465,6 +498,13 @@ __global__ void k_load(const double *__restrict__ coords, const uint32_t *__rest
             const int32_t ek = node_elem[t];
             const int64_t e = ek / NN;
             const int k = ek - (int)(e * NN);
+            if (sw) {
+                for (int q = 0; q < qt.nq; ++q) {
+                    const double s = sw[e * qt.nq + q];
+                    for (int c = 0; c < dof; ++c) acc[c] = ADD(acc[c], MUL(s, MUL(f[c], qt.phi[q][k])));
+                }
+                continue;
+            }
             double X[NN][3];
 #pragma unroll
             for (int K = 0; K < NN; ++K) {
@@ -911,16 +951,29 @@ void assemble_load(sfc_ctx *ctx, const sfc_mesh *m, const double *f, double *F_d
     switch (m->kind) {
     case SFC_ELEM_LINE2_POISSON:
         k_load<1, 2><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->conn.p, m->node_ptr.p, m->node_elem.p, m->quad,
-                                                  m->num_nodes, m->dof, f0, f1, f2, F_dev);
+                                                  m->num_nodes, m->dof, f0, f1, f2, nullptr, F_dev);
         break;
     case SFC_ELEM_TRI3_POISSON:
         k_load<2, 3><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->conn.p, m->node_ptr.p, m->node_elem.p, m->quad,
-                                                  m->num_nodes, m->dof, f0, f1, f2, F_dev);
+                                                  m->num_nodes, m->dof, f0, f1, f2, nullptr, F_dev);
         break;
-    default:
+    default: {
+        DBuf<double> &sw = const_cast<sfc_mesh *>(m)->load_w;
+        const double *points = nullptr;
+        try {
+            sw.reserve(m->num_elems * m->quad.nq);
+            points = sw.p;
+        } catch (const Error &) {  // no room: every node computes its points
+        }
+        if (points) {
+            k_load_points<3, 8><<<grid_for(m->num_elems, 128), 128, 0, ctx->stream>>>(m->coords.p, m->conn.p, m->quad,
+                                                                                    m->num_elems, sw.p);
+            count_launch(ctx);
+        }
         k_load<3, 8><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->conn.p, m->node_ptr.p, m->node_elem.p, m->quad,
-                                                  m->num_nodes, m->dof, f0, f1, f2, F_dev);
+                                                  m->num_nodes, m->dof, f0, f1, f2, points, F_dev);
         break;
+    }
     }
     count_launch(ctx);
 }

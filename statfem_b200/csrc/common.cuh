@@ -416,6 +416,7 @@ struct sfc_mesh {
     sfc::DBuf<int32_t> node_ptr;   // num_nodes + 1
     sfc::DBuf<int32_t> node_elem;  // num_elems * nn
     // element matrices of the last assembly (num_elems * L * L)
+    sfc::DBuf<double> load_w;  // hexahedra: w*detJ of every quadrature point (assemble_load)
     sfc::DBuf<double> ke;
     // tensor-grid description of the node set (for the Kronecker covariance)
     bool is_grid = false;
