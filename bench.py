@@ -97,7 +97,7 @@ class ClockSampler:
 
 
 # the CUDA kernel behind the solver's "spmm32" step, by last_stats()["spmm_kernel"]
-SPMM_KERNELS = {1: "k_spmm32", 2: "k_bspmm32", 3: "k_lspmm32", 4: "k_xspmm32"}
+SPMM_KERNELS = {1: "k_spmm32", 2: "k_bspmm32", 3: "k_lspmm32", 4: "k_tspmm32"}
 
 
 def ncu_traffic(kernel, block_width, impl=None):
@@ -561,6 +561,25 @@ def run_batch(args, ws, rank, local):
     alg_bytes = float(np.sum(res["iterations"].astype(np.float64) * dofs) * C3_BYTES_PER_DOF_ITER)
     peak, peak_kind = peaks()
     achieved = alg_bytes / (kern_ms / 1e3) / 1e9
+    roofline = {"kernel": "k_batch (persistent)", "bound": "hbm", "achieved": round(achieved, 1),
+                "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": None,
+                "peak_source": peak_kind, "bytes_per_launch": alg_bytes,
+                "avg_launch_us": round(kern_ms * 1e3, 1),
+                "algorithmic_bytes": "%d B per dof per inner iteration x sum(iterations x dofs)"
+                                     % C3_BYTES_PER_DOF_ITER}
+    if not res["iterations"].any():
+        # block elimination: a banded factorisation and the solves with its two factors
+        band = np.asarray(wl["sides"], dtype=np.float64) + 1
+        flops = float(np.sum(dofs * band ** 2 + 4.0 * dofs * band * wl["ns"]))
+        achieved = flops / (kern_ms / 1e3) / 1e12
+        fp64 = 148 * 64 * 2 * 1.965e9 / 1e12
+        roofline = {"kernel": "block elimination (btd.cu) and k_batch", "bound": "fp64",
+                    "achieved": round(achieved, 2), "peak": round(fp64, 1), "unit": "TFLOP/s",
+                    "frac": round(achieved / fp64, 4), "traffic": None,
+                    "peak_source": "nominal (148 SMs x 64 FP64 FMA per clock at 1,965 MHz)",
+                    "avg_launch_us": round(kern_ms * 1e3, 1),
+                    "algorithmic_flops": "sum over instances of dofs x (side + 1)^2 (banded factor) + "
+                                         "4 x dofs x (side + 1) x sensors (solves)"}
     # end to end: coefficients and readings from host memory, results back
     ctx.synchronize()
     ctx.mark(2)
@@ -590,12 +609,7 @@ def run_batch(args, ws, rank, local):
         "e2e": {"value": round(n_total * args.steps / (e2e_ms / 1e3), 3), "unit": "posterior solves/s",
                 "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": int(launches),
-        "roofline": {"kernel": "k_batch (persistent)", "bound": "hbm", "achieved": round(achieved, 1),
-                     "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": None,
-                     "peak_source": peak_kind, "bytes_per_launch": alg_bytes,
-                     "avg_launch_us": round(kern_ms * 1e3, 1),
-                     "algorithmic_bytes": "%d B per dof per inner iteration x sum(iterations x dofs)"
-                                          % C3_BYTES_PER_DOF_ITER},
+        "roofline": roofline,
         "phases_ms_per_step": {"assembly": round(asm_ms, 2), "solve_likelihood_kernel": round(kern_ms, 2)},
         "iterations": {"mean": float(res["iterations"].mean()), "max": int(res["iterations"].max())},
         "status_ok": int((status_all == 0).sum()),

@@ -117,7 +117,8 @@ typedef struct sfc_solve_stats {
                                  meshes), 3 lattice bricks staged by TMA
                                  (SFC_SPMM=lattice), 4 streamed lattice
                                  x-lines (the default on 3-dof structured
-                                 lattices)                                    */
+                                 lattices, and from 8,192 nodes on meshes
+                                 numbered like one)                           */
     int32_t reserved;
 } sfc_solve_stats_t;
 
