@@ -2345,11 +2345,12 @@ FcgWhy fcg_run(sfc_mpnn *m, sfc_system *s, FcgRun &run)
 
 // Flexible CG (FCG(1), Notay 2000) with z = M(r) from the network, with
 // plain Jacobi-PCG as the fallback when the network stalls or breaks down:
-// alpha = p.r / p.Sp, p' = z - (z.Sp / p.Sp) p.  The scalars live on the
-// device (one slot per iteration) and the host reads the flags every
-// check_every iterations, so the iteration issues no synchronisation.  When
-// the recurrence residual meets tol, the true FP64 residual ||b - S x|| is
-// computed; if it misses tol, the method restarts from it.
+// alpha = p.r / p.Sp, p' = z - (z.Sp / p.Sp) p.  The iterations are one
+// persistent kernel (k_fcg); with SFC_MPNN_TC=0 they are launches whose scalars
+// live on the device, one slot per iteration, and whose flags the host reads
+// every check_every iterations.  When the recurrence residual meets tol, the
+// true FP64 residual ||b - S x|| is computed; if it misses tol, the method
+// restarts from it.
 void solve_forward_fcg(sfc_system *s)
 {
     sfc_ctx *ctx = s->ctx;

@@ -1497,9 +1497,8 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
         }
         count_launch(ctx);
     };
-    // A whole check interval as one CUDA graph: `check`
-    // iterations and the convergence flag, captured once per launch
-    // configuration (the key lists every pointer and size baked into the
+    // A whole check interval as one CUDA graph: `check` iterations with their
+    // convergence tests, captured once per launch configuration (the key lists every pointer and size baked into the
     // launches) and replayed for every later interval.  Not used while kernel
     // profiling records events around each launch, nor with
     // SFC_BLOCK_GRAPH=0 in the environment.
