@@ -94,6 +94,7 @@ struct BatchArgs {
     double tol, itol;
     int max_iter, max_cycles;
     int warm;  // x64 holds the direct solution (btd.cu)
+    const int *bad;  // per instance: a pivot of it was not positive
     // outputs
     double *loglik, *mean_s, *cov_s, *pmean, *pcov;
     int *status, *iters;
@@ -263,7 +264,8 @@ __global__ void __launch_bounds__(BT, OCC) k_batch(BatchArgs a)
         float4 *X4 = reinterpret_cast<float4 *>(a.x32), *R4 = reinterpret_cast<float4 *>(a.r32);
         float4 *P4 = reinterpret_cast<float4 *>(a.p32), *Q4 = reinterpret_cast<float4 *>(a.q32);
         // right-hand sides b = P^T, dense in W (W is free until the statistics)
-        bool warm = a.warm != 0;
+        // (of a matrix that is not positive definite none: the iteration reports it)
+        bool warm = a.warm && !a.bad[inst];
         for (int64_t i = my0 + warp; i < my1; i += BW) {
             if (!warm) a.x64[i * BK + lane] = 0.0;
             a.W[i * BK + lane] = 0.0;
@@ -317,8 +319,8 @@ __global__ void __launch_bounds__(BT, OCC) k_batch(BatchArgs a)
                 lost = lost || !(rr0[q] <= bb[q]);
             }
             if (warm && cycle == 0 && __any_sync(0xffffffffu, lost)) {
-                // a matrix the direct elimination cannot take (not positive
-                // definite, not finite): from zero, as without it
+                // not finite, or further off than zero: from zero, as without
+                // the elimination
                 warm = false;
                 for (int64_t i = my0 + warp; i < my1; i += BW) a.x64[i * BK + lane] = 0.0;
                 cluster_barrier(cl);
@@ -879,6 +881,7 @@ void batch_build_args(sfc_batch *b)
     a.max_iter = b->max_iter;
     a.max_cycles = b->max_cycles;
     a.warm = batch_direct(b);
+    a.bad = b->btd.bad.p;
     a.loglik = b->loglik.p;
     a.mean_s = b->mean_s.p;
     a.cov_s = b->cov_s.p;

@@ -104,8 +104,8 @@ __device__ __forceinline__ int line_at(const Inst &q, int chain, int st)
 
 // 1 / d by Newton's iteration on the hardware's approximation (about 20 bits;
 // two steps reach rounding): no branch, so the compiler can place the other
-// rows' updates inside its latency.  d outside the approximation's range
-// gives a non-finite pivot, which the residual check of the caller sees.
+// rows' updates inside its latency.  For d and 1 / d normal numbers
+// (pivot_ok): both are flushed to zero below.
 __device__ __forceinline__ double recip(double d)
 {
     double x;
@@ -114,6 +114,9 @@ __device__ __forceinline__ double recip(double d)
     return fma(x, fma(-d, x, 1.0), x);
 }
 
+// A pivot of a positive definite matrix, within the range of recip
+__device__ __forceinline__ bool pivot_ok(double d) { return d >= 0x1p-1022 && d <= 0x1p1022; }
+
 // In-place inverse of the kw x kw symmetric positive definite block at P (row
 // stride ld) by the first four warps (warp w holds rows 8 w .. 8 w + 7, lane j
 // column j).  The symmetric sweep (its result is the negative inverse) makes
@@ -121,9 +124,12 @@ __device__ __forceinline__ double recip(double d)
 // through shared memory; the next row is updated and published before the
 // rest of a step, which runs inside the next pivot's latency.  2.9 us for 32
 // columns; 7.0 us with 256 threads, a division and a full barrier per step,
-// 6.9 us with one warp (its 31 updates per step bound it).
-__device__ void pivot_inverse(double *P, int ld, int kw, double *buf)
+// 6.9 us with one warp (its 31 updates per step bound it).  Whether all pivots
+// were positive: the pivots of an elimination in any symmetric order are, if
+// and only if the matrix is positive definite.
+__device__ bool pivot_inverse(double *P, int ld, int kw, double *buf)
 {
+    bool ok = true;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double v[8];
 #pragma unroll
@@ -145,6 +151,7 @@ __device__ void pivot_inverse(double *P, int ld, int kw, double *buf)
 #pragma unroll
             for (int i = 0; i < 8; ++i) row[i] = sh[8 * warp + i];
             const double inv = recip(sh[k]), mine = sh[lane];
+            ok = ok && pivot_ok(sh[k]);
             const bool me = lane == k;
             const double f = me ? inv : -mine * inv;
             if (next) {
@@ -165,6 +172,7 @@ __device__ void pivot_inverse(double *P, int ld, int kw, double *buf)
         const int r = 8 * warp + i;
         if (r < kw && lane < kw) P[(size_t)r * ld + lane] = -v[i];
     }
+    return ok;
 }
 
 // the entries of this chain's own rows of `line` into shared memory
@@ -240,7 +248,7 @@ __device__ void build_block(const Inst &q, const Sm &s, int line, int c, int C, 
 // against 3.3 us through distributed shared memory at 182 columns on eight
 // CTAs, whose owners serve every reader in turn, and one cluster barrier
 // instead of two (factor of the 182 x 182 grid 6.5 -> 5.1 ms).
-__device__ void invert_block(const Inst &q, const Sm &s, bool have, int c, int C, int nloc, double *G)
+__device__ void invert_block(const Inst &q, const Sm &s, bool have, int c, int C, int nloc, double *G, int *bad)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lr4 = lane >> 2, lk4 = lane & 3;
@@ -256,7 +264,8 @@ __device__ void invert_block(const Inst &q, const Sm &s, bool have, int c, int C
                 cp_async16(s.P + (size_t)r * ld + 2 * j, Gp + (size_t)r * q.mp + 2 * j);
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        if (warp < PW / 8) pivot_inverse(s.P + c0, ld, kw, s.buf);
+        // every CTA of the chain takes the same pivots: the first one reports
+        if (warp < PW / 8 && !pivot_inverse(s.P + c0, ld, kw, s.buf) && c == 0 && threadIdx.x == 0) *bad = 1;
         __syncthreads();
         const int g0 = c0 >> 3, g1 = g0 + (kw >> 3), nk = kw >> 2, nt = kw >> 3;
         // panel columns: -A V for the other rows, V for the pivot rows; two
@@ -435,7 +444,7 @@ __device__ __forceinline__ int local_groups(const Inst &q, int c, int C)
 }
 
 __device__ void factor(const BtdArgs &a, const Inst &q, const Sm &s, int chain, int c, int C,
-                       double *X, double *Y)
+                       double *X, double *Y, int *bad)
 {
     const int nloc = local_groups(q, c, C);
     const size_t ysz = (size_t)q.m * q.mp;
@@ -459,7 +468,7 @@ __device__ void factor(const BtdArgs &a, const Inst &q, const Sm &s, int chain, 
         Couple cp;
         if (have && !last) load_couple(a, q, line, chain, cp);
         __syncthreads();
-        invert_block(q, s, have, c, C, nloc, G);
+        invert_block(q, s, have, c, C, nloc, G, bad);
         if (have) store_block(q, s, line, c, C, nloc, X, Y + chain * ysz, cp, !last);
         if (!last) stage_entries(a, q, s, line_at(q, chain, st + 1), c, C, nloc);
     }
@@ -617,8 +626,9 @@ __global__ void __launch_bounds__(TT, 2) k_btd_batch(BtdArgs a)
         const int qi = *cl.map_shared_rank(s.word, 0);
         cl.sync();
         if (qi >= a.n_inst) break;
-        const Inst q = load_inst(a, a.order[qi]);
-        factor(a, q, s, chain, c, C, X, Y);
+        const int inst = a.order[qi];
+        const Inst q = load_inst(a, inst);
+        factor(a, q, s, chain, c, C, X, Y, a.bad + inst);
         for (int c0 = 0; c0 < a.ncols; c0 += kBtdCols) solve_tile(cl, a, q, s, c0, chain, c, C, X);
     }
 }
@@ -629,7 +639,7 @@ __global__ void __launch_bounds__(TT) k_btd_factor(BtdArgs a)
     const int C = a.chain, rank = (int)cg::this_cluster().block_rank();
     Sm s = carve(raw, a.lmax, C);
     const Inst q = load_inst(a, 0);
-    factor(a, q, s, rank / C, rank % C, C, a.X, a.Y);
+    factor(a, q, s, rank / C, rank % C, C, a.X, a.Y, a.bad);
 }
 
 // one cluster per tile of 32 columns
@@ -720,12 +730,12 @@ __global__ void k_bandwidth(const int32_t *__restrict__ rp, const int32_t *__res
 }
 
 // per column: |b - S x|^2, |b|^2, |x|^2 (out[3][ncols]) and the largest
-// absolute row sum of S (out[3 ncols], the bits of a non-negative double).
-// A block takes 32 columns (a lane each) and a share of the rows.
+// absolute row sum of S (out[3 ncols], the bits of a non-negative double);
+// behind it whether the factor is *bad.  A block takes 32 columns (a lane each) and a share of the rows.
 __global__ void __launch_bounds__(256) k_btd_check(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                                                    const double *__restrict__ a, const double *__restrict__ B,
                                                    const double *__restrict__ X, int64_t N, int ld, int ncols,
-                                                   double *out)
+                                                   const int *bad, double *out)
 {
     __shared__ double sh[3][8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 32 + lane;
@@ -753,6 +763,7 @@ __global__ void __launch_bounds__(256) k_btd_check(const int32_t *__restrict__ r
         for (int w = 0; w < 8; ++w) t += sh[warp][w][lane];
         atomicAdd(out + (int64_t)warp * ncols + c, t);
     }
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) out[3 * (int64_t)ncols + 1] = *bad;
     if (blockIdx.y == 0 && lane == 0)
         atomicMax(reinterpret_cast<unsigned long long *>(out + 3 * (int64_t)ncols),
                   (unsigned long long)__double_as_longlong(big));
@@ -807,6 +818,7 @@ bool btd_plan(sfc_ctx *ctx, BtdPlan &p, const int32_t *rp, const int32_t *col, i
     upload(ctx, p.line, line, n_inst);
     upload(ctx, p.order, order, n_inst);
     p.word.reserve(2);
+    p.bad.reserve(n_inst);
     BtdArgs a{};
     a.rp = rp;
     a.col = col;
@@ -872,6 +884,7 @@ BtdArgs btd_args(BtdPlan &p, const int32_t *rp, const int32_t *col, const double
     a.xstride = (int64_t)(p.X.n / p.slots);
     a.ystride = (int64_t)(p.Y.n / p.slots);
     a.queue = p.word.p;
+    a.bad = p.bad.p;
     a.chain = p.chain;
     a.lmax = p.lmax;
     return a;
@@ -882,6 +895,7 @@ void btd_launch_batch(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a, cudaStre
     k_btd_entries<true><<<grid_for(a.N, 256), 256, 0, st>>>(a, nullptr);
     SFC_CK(cudaGetLastError());
     SFC_CK(cudaMemsetAsync(a.queue, 0, sizeof(int), st));
+    SFC_CK(cudaMemsetAsync(a.bad, 0, a.n_inst * sizeof(int), st));
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = btd_config(k_btd_batch, p, p.slots, st, &attr);
     SFC_CK(cudaLaunchKernelEx(&cfg, k_btd_batch, a));
@@ -890,6 +904,7 @@ void btd_launch_batch(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a, cudaStre
 void btd_launch_factor(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a)
 {
     k_btd_entries<true><<<grid_for(a.N, 256), 256, 0, ctx->stream>>>(a, nullptr);
+    SFC_CK(cudaMemsetAsync(a.bad, 0, sizeof(int), ctx->stream));
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = btd_config(k_btd_factor, p, 1, ctx->stream, &attr);
     SFC_CK(cudaLaunchKernelEx(&cfg, k_btd_factor, a));
@@ -950,14 +965,16 @@ bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int l
         p.factored = s->op_serial;
     }
     btd_launch_solve(ctx, p, a);
-    const size_t nn = 3 * (size_t)nrhs + 1;
+    const size_t nn = 3 * (size_t)nrhs + 2;
     p.norms.reserve(nn);
     SFC_CK(cudaMemsetAsync(p.norms.p, 0, nn * sizeof(double), ctx->stream));
     const dim3 grid((unsigned)std::min<int64_t>((s->N + 31) / 32, 2 * ctx->sm_count), (unsigned)((nrhs + 31) / 32));
-    k_btd_check<<<grid, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op.p, B, X, s->N, ld, nrhs, p.norms.p);
+    k_btd_check<<<grid, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op.p, B, X, s->N, ld, nrhs, a.bad,
+                                              p.norms.p);
     count_launch(ctx);
     std::vector<double> h(nn);
     download(ctx, h.data(), p.norms.p, nn);
+    if (h[nn - 1] != 0.0) return false;  // not positive definite: for the iteration to report
     double worst = 0.0;
     for (int c = 0; c < nrhs; ++c) {
         const double r = std::sqrt(h[c]), b = std::sqrt(h[nrhs + c]), x = std::sqrt(h[2 * (size_t)nrhs + c]);

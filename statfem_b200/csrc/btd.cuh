@@ -30,6 +30,7 @@ struct BtdArgs {
     double *U;
     int ld, ncols;
     int *queue;
+    int *bad;    // per instance: 1 where a pivot was not a positive number the reciprocal takes
     int chain;   // CTAs per elimination chain; a cluster has two chains
     int lmax;    // longest line
 };

@@ -286,6 +286,7 @@ struct BtdPlan {
     DBuf<double> vals;
     DBuf<double> X, Y;
     DBuf<int> word;
+    DBuf<int> bad;           // per instance: a pivot was not positive
     DBuf<double> norms;      // residual check
     uint64_t factored = 0;  // operator serial of the inverse blocks in X (single systems)
 };
