@@ -105,7 +105,8 @@ typedef struct sfc_solve_stats {
                                  meshes)                                      */
     int32_t refinements;      /* FP64 refinement cycles (mixed solver)         */
     int32_t num_rhs;
-    int32_t converged;        /* 1 when every RHS met tol                      */
+    int32_t converged;        /* 1 when every RHS met tol (the FP64 methods: by
+                                 their recurrence residual)                   */
     double max_rel_residual;  /* max over RHS of the true FP64 ||b-Ax||/||b||  */
     double device_ms;         /* device time of the last solve call            */
     int32_t fallback_columns; /* mixed solver: columns finished by FP64

@@ -731,11 +731,12 @@ __global__ void k_bandwidth(const int32_t *__restrict__ rp, const int32_t *__res
 
 // per column: |b - S x|^2, |b|^2, |x|^2 (out[3][ncols]) and the largest
 // absolute row sum of S (out[3 ncols], the bits of a non-negative double);
-// behind it whether the factor is *bad.  A block takes 32 columns (a lane each) and a share of the rows.
+// behind it whether the factor is *bad.  With R, b - S x goes there too
+// ([row][ncols]).  A block takes 32 columns (a lane each) and a share of the rows.
 __global__ void __launch_bounds__(256) k_btd_check(const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                                                    const double *__restrict__ a, const double *__restrict__ B,
                                                    const double *__restrict__ X, int64_t N, int ld, int ncols,
-                                                   const int *bad, double *out)
+                                                   const int *bad, double *out, double *__restrict__ R)
 {
     __shared__ double sh[3][8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 32 + lane;
@@ -749,6 +750,7 @@ __global__ void __launch_bounds__(256) k_btd_check(const int32_t *__restrict__ r
             sum += fabs(v);
             if (ok) r -= v * X[(int64_t)col[k] * ld + c];
         }
+        if (R && ok) R[i * ncols + c] = r;
         rr += r * r;
         bb += b * b;
         xx += x * x;
@@ -767,6 +769,13 @@ __global__ void __launch_bounds__(256) k_btd_check(const int32_t *__restrict__ r
     if (blockIdx.y == 0 && lane == 0)
         atomicMax(reinterpret_cast<unsigned long long *>(out + 3 * (int64_t)ncols),
                   (unsigned long long)__double_as_longlong(big));
+}
+
+// X += D (D: [row][ncols])
+__global__ void k_btd_correct(double *__restrict__ X, const double *__restrict__ D, int64_t N, int ld, int ncols)
+{
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N * ncols; t += (int64_t)gridDim.x * blockDim.x)
+        X[t / ncols * ld + t % ncols] += D[t];
 }
 
 template <class K>
@@ -949,7 +958,8 @@ void plan_system(sfc_system *s)
 
 }  // namespace
 
-bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int ld, double tol, double *max_rel)
+bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int ld, double tol, bool recurrence,
+                      double *max_rel)
 {
     sfc_ctx *ctx = s->ctx;
     BtdPlan &p = s->btd;
@@ -967,25 +977,55 @@ bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int l
     btd_launch_solve(ctx, p, a);
     const size_t nn = 3 * (size_t)nrhs + 2;
     p.norms.reserve(nn);
-    SFC_CK(cudaMemsetAsync(p.norms.p, 0, nn * sizeof(double), ctx->stream));
-    const dim3 grid((unsigned)std::min<int64_t>((s->N + 31) / 32, 2 * ctx->sm_count), (unsigned)((nrhs + 31) / 32));
-    k_btd_check<<<grid, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op.p, B, X, s->N, ld, nrhs, a.bad,
-                                              p.norms.p);
-    count_launch(ctx);
     std::vector<double> h(nn);
-    download(ctx, h.data(), p.norms.p, nn);
+    const dim3 grid((unsigned)std::min<int64_t>((s->N + 31) / 32, 2 * ctx->sm_count), (unsigned)((nrhs + 31) / 32));
+    auto check = [&](double *R) {
+        SFC_CK(cudaMemsetAsync(p.norms.p, 0, nn * sizeof(double), ctx->stream));
+        k_btd_check<<<grid, 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->a_op.p, B, X, s->N, ld, nrhs, a.bad,
+                                                  p.norms.p, R);
+        count_launch(ctx);
+        if (!R) download(ctx, h.data(), p.norms.p, nn);
+    };
+    // every column within tol; with `floor` one whose residual is at the
+    // rounding of its own terms, on a system that rounding does not swamp,
+    // will do (a nearly singular one has solutions so large that any residual
+    // is at theirs)
+    auto within = [&](bool floor) {
+        double worst = 0.0;
+        for (int c = 0; c < nrhs; ++c) {
+            const double r = std::sqrt(h[c]), b = std::sqrt(h[nrhs + c]), x = std::sqrt(h[2 * (size_t)nrhs + c]);
+            const double terms = 8.0 * 2.2e-16 * (h[3 * (size_t)nrhs] * x + b);
+            if (!(r <= tol * b || (floor && r <= terms && terms <= 1e-8 * b))) return false;
+            if (b > 0) worst = std::max(worst, r / b);
+        }
+        *max_rel = worst;
+        return true;
+    };
+    check(nullptr);
     if (h[nn - 1] != 0.0) return false;  // not positive definite: for the iteration to report
-    double worst = 0.0;
-    for (int c = 0; c < nrhs; ++c) {
-        const double r = std::sqrt(h[c]), b = std::sqrt(h[nrhs + c]), x = std::sqrt(h[2 * (size_t)nrhs + c]);
-        // tol, or a residual at the rounding of its own terms, which the
-        // recurrence residual of FP64 PCG does not see
-        const double floor = 8.0 * 2.2e-16 * (h[3 * (size_t)nrhs] * x + b);
-        if (!(r <= tol * b || r <= floor)) return false;
-        if (b > 0) worst = std::max(worst, r / b);
+    if (within(recurrence)) return true;
+    // a residual above tol: once more on it with the same factor, twice at most
+    const size_t n = (size_t)s->N * nrhs;
+    DBuf<double> R, D;
+    try {
+        R.alloc(n);
+        D.alloc(n);
+    } catch (const Error &) {
+        return false;
     }
-    *max_rel = worst;
-    return true;
+    BtdArgs e = a;
+    e.B = R.p;
+    e.U = D.p;
+    e.ld = nrhs;
+    for (int step = 0; step < 2; ++step) {
+        check(R.p);
+        btd_launch_solve(ctx, p, e);
+        k_btd_correct<<<grid_for((int64_t)n, 256), 256, 0, ctx->stream>>>(X, D.p, s->N, ld, nrhs);
+        count_launch(ctx);
+        check(nullptr);
+        if (within(recurrence)) return true;
+    }
+    return false;
 }
 
 }  // namespace sfc

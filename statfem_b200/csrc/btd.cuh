@@ -45,8 +45,13 @@ void btd_launch_batch(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a, cudaStre
 // one system: the inverse blocks, then any number of columns
 void btd_launch_factor(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a);
 void btd_launch_solve(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a);
-// S X = B of a system whose operator is built; false (X undefined) where the
-// elimination does not apply or a column misses tol
-bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int ld, double tol, double *max_rel);
+// S X = B of a system whose operator is built, refined with FP64 residuals
+// where the first solution misses tol; false (X undefined) where the
+// elimination does not apply, the operator is not positive definite or a
+// column's true residual still misses tol.  `recurrence`: in place of a solver
+// that stops by its recurrence residual, which does not see the rounding of
+// the true one; a residual at that rounding is then accepted too.
+bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int ld, double tol, bool recurrence,
+                      double *max_rel);
 
 }  // namespace sfc

@@ -1850,7 +1850,7 @@ bool solve_direct(sfc_system *s, const double *B, double *X, int nrhs, int ld)
     s->solve_ev.ensure();
     SFC_CK(cudaEventRecord(s->solve_ev.a, ctx->stream));
     double worst = 0.0;
-    if (!btd_solve_system(s, B, X, nrhs, ld, tol, &worst)) return false;
+    if (!btd_solve_system(s, B, X, nrhs, ld, tol, o.method != SFC_SOLVER_PCG_MIXED, &worst)) return false;
     SFC_CK(cudaEventRecord(s->solve_ev.b, ctx->stream));
     SFC_CK(cudaEventSynchronize(s->solve_ev.b));
     float ms = 0;
