@@ -342,8 +342,8 @@ __global__ void k_dia_check(const __grid_constant__ Offsets o, const int32_t *__
 }
 
 // BELOW = false: the diagonals on and above the main one (W values per
-// entry).  BELOW = true: compares the entries below with them, *bad where
-// they differ by more than rounding of the main diagonal.
+// entry).  BELOW = true: compares the entries below, stored or not, with them,
+// *bad where they differ by more than rounding of the main diagonal.
 template <int W, bool BELOW>
 __global__ void k_dia_fill(const __grid_constant__ Offsets o, const int32_t *__restrict__ rp,
                            const int32_t *__restrict__ col, const double *__restrict__ a, int64_t rows,
@@ -355,14 +355,14 @@ __global__ void k_dia_fill(const __grid_constant__ Offsets o, const int32_t *__r
         const int32_t e = rp[i + 1];
         for (int d = 0; d < (BELOW ? h : o.nd); ++d) {
             const bool hit = k < e && col[k] - (int)i == o.off[d];
-            if (BELOW && hit) {
-                const int64_t at = i + o.off[d];
+            const int64_t at = i + o.off[d];
+            if (BELOW && at >= 0) {  // an entry that is not stored is zero
                 const double tol = 1e-12 * (fabs(dia[i]) + fabs(dia[at]));
 #pragma unroll
                 for (int w = 0; w < W; ++w) {
                     const int t = W == 9 ? (w % 3) * 3 + w / 3 : 0;  // transposed block
                     const double up = dia[((int64_t)(h - d) * W + t) * rows + at];
-                    if (!(fabs(a[(int64_t)k * W + w] - up) <= tol)) atomicExch(bad, 1);
+                    if (!(fabs((hit ? a[(int64_t)k * W + w] : 0.0) - up) <= tol)) atomicExch(bad, 1);
                 }
             }
             if (!BELOW && d >= h)
