@@ -1403,8 +1403,7 @@ static_assert(kFcgTiles * kTcABytes <= kFcgABytes + LAYERS * kTcBBytes, "the las
 static_assert(kFcgTiles * kTcCols <= kFcgCols, "accumulators");
 
 struct FcgArgs {
-    PcgArgs op;  // x, r, p, q; sums: pq, pr, rr, zq, |D^-1/2 r|^2, `slots` each; out: iterations, why, error, (barrier), mark_it
-    int64_t slots;
+    PcgArgs op;  // x, r, p, q; sums: p.q, p.r, r.r, z.q, |D^-1/2 r|^2; out: iterations, why, error, (barrier), mark_it
     const int32_t *rp, *col;
     const float *ahat;
     const float4 *win;  // [run][quad of rows][3][4 rows]
@@ -1658,9 +1657,10 @@ __global__ void __launch_bounds__(kFcgThreads, 1) k_fcg(const __grid_constant__ 
     uint32_t parity = 0;
     bool tc_ok = true;
     Comm<false> comm{g.op, sh.comm};
-    const int64_t N = g.op.N, S = g.slots, row0 = min(N, (int64_t)blockIdx.x * g.per), row1 = min(N, row0 + g.per);
+    enum { PQ, PR, RR, ZQ, NN, SUMS };
+    const int64_t N = g.op.N, row0 = min(N, (int64_t)blockIdx.x * g.per), row1 = min(N, row0 + g.per);
     const bool first = blockIdx.x == 0 && tid == 0;
-    double pq = g.op.sums[g.it0], pr = g.op.sums[S + g.it0], mark = *g.mark, none = 0.0;
+    double pq = g.op.sums[sum_slot(PQ, g.it0)], pr = g.op.sums[sum_slot(PR, g.it0)], mark = *g.mark, none = 0.0;
     int mark_it = g.mark_it, it = g.it0, why = FCG_CAP;
     while (it < g.op.max_iter) {
         if (!(pq > 0.0)) {
@@ -1679,7 +1679,8 @@ __global__ void __launch_bounds__(kFcgThreads, 1) k_fcg(const __grid_constant__ 
             nn += t * t;
             g.rhat[i] = (float)t;
         }
-        if (!comm.sum<2>(rr, nn, (int)(2 * S) + it + 1, (int)(4 * S) + it + 1)) break;
+        if (!comm.sum<2>(rr, nn, sum_slot(RR, it + 1), sum_slot(NN, it + 1))) break;
+        if (first) clear_slots<SUMS>(g.op.sums, it);
         if (rr <= g.thr) {
             why = FCG_DONE;
             ++it;
@@ -1769,7 +1770,7 @@ __global__ void __launch_bounds__(kFcgThreads, 1) k_fcg(const __grid_constant__ 
         tc_ok = fcg_layer<WIN, false>(g, sh, sA, sB_u + kTcBBytes, bar_u, tmem, parity, g.hb1, g.hb0, sh.bias[1], row0, row1, nn, zq);
         if (!tc_ok || !comm.barrier()) break;
         tc_ok = fcg_layer<WIN, true>(g, sh, sA, sB_u + 2 * kTcBBytes, bar_u, tmem, parity, g.hb0, nullptr, sh.bias[2], row0, row1, nn, zq);
-        if (!tc_ok || !comm.sum<1>(zq, none, (int)(3 * S) + it, 0)) break;
+        if (!tc_ok || !comm.sum<1>(zq, none, sum_slot(ZQ, it), 0)) break;
         const double beta = -zq / pq;
         pr = 0.0;
         for (int64_t i = row0 + tid; i < row1; i += kFcgThreads) {
@@ -1779,7 +1780,7 @@ __global__ void __launch_bounds__(kFcgThreads, 1) k_fcg(const __grid_constant__ 
         }
         if (!comm.barrier()) break;
         pq = product<F>(g.op, g.op.p, g.op.q);
-        if (!comm.sum<2>(pq, pr, it + 1, (int)S + it + 1)) break;
+        if (!comm.sum<2>(pq, pr, sum_slot(PQ, it + 1), sum_slot(PR, it + 1))) break;
         ++it;
     }
     if (first) {
@@ -2238,7 +2239,6 @@ __global__ void k_fcg_pupdate(double *__restrict__ p, const double *__restrict__
 
 struct FcgRun {
     double *x, *r, *z, *p, *q, *mark;
-    int64_t slots;
     int it, max_iter, check, stall, mark_it;
     double thr, mark_rr;
 };
@@ -2281,7 +2281,6 @@ FcgWhy fcg_run(sfc_mpnn *m, sfc_system *s, FcgRun &run)
     g.op.max_iter = run.max_iter;
     g.op.out = m->fcg_flags.p;
     g.op.bar = reinterpret_cast<unsigned *>(m->fcg_flags.p + 3);
-    g.slots = run.slots;
     g.rp = s->row_ptr.p;
     g.col = s->col.p;
     g.ahat = m->ahat.p;
@@ -2366,7 +2365,9 @@ void solve_forward_fcg(sfc_system *s)
     s->X.alloc(N);
     s->blk64.reserve(6 * N);
     double *b = s->blk64.p, *r = b + N, *z = r + N, *p = z + N, *q = p + N, *t = q + N;
-    const int64_t slots = (int64_t)max_iter + 2;
+    // a slot per iteration for the launches; the persistent kernel goes round a few
+    const bool ring = use_tc();
+    const int64_t slots = ring ? kSumRing : (int64_t)max_iter + 2;
     m->fcg_sc.reserve(5 * slots + 1);
     double *pq = m->fcg_sc.p, *pr = pq + slots, *rr = pr + slots, *zq = rr + slots, *mark = zq + 2 * slots;
     m->fcg_flags.reserve(8);
@@ -2388,7 +2389,9 @@ void solve_forward_fcg(sfc_system *s)
         count_launch(ctx);
         return std::sqrt(device_dot(ctx, r, r, N) / bb);
     };
-    auto start = [&](int slot) {  // direction from the current residual
+    auto start = [&](int at) {  // direction from the current residual
+        const int64_t slot = ring ? at % kSumRing : at;
+        if (ring) SFC_CK(cudaMemsetAsync(m->fcg_sc.p, 0, 5 * slots * sizeof(double), ctx->stream));
         apply(m, r, z);
         SFC_CK(cudaMemcpyAsync(p, z, N * 8, cudaMemcpyDeviceToDevice, ctx->stream));
         spmv_op64_dot(s, p, q, pq + slot, nullptr);
@@ -2404,7 +2407,7 @@ void solve_forward_fcg(sfc_system *s)
     // (p.Sp <= 0), a stall or the cap; `it` ends at the iteration reached
     auto iterate = [&]() -> FcgWhy {
         if (use_tc()) {
-            FcgRun run{s->X.p, r, z, p, q, mark, slots, it, max_iter, check, kStall, mark_it, thr, mark_rr};
+            FcgRun run{s->X.p, r, z, p, q, mark, it, max_iter, check, kStall, mark_it, thr, mark_rr};
             const FcgWhy why = fcg_run(m, s, run);
             it = run.it;
             mark_it = run.mark_it;

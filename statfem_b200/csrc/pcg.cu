@@ -221,16 +221,16 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
     Comm<CL> comm{g, sh};
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
     double rz, rr, none = 0.0;
-    const int len = g.max_iter + 2;  // slots of one sum
+    enum { PQ, RZ, RR, CE, SUMS };
     update<PRE, true>(g, 0.0, g.c, rz, rr);
-    if (!comm.template sum<2>(rz, rr, len, 2 * len)) return;
+    if (!comm.template sum<2>(rz, rr, sum_slot(RZ, 0), sum_slot(RR, 0))) return;
     if (rr == 0.0) {
         for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x) g.x[i] = 0.0;
         if (first) g.out[1] = 1;
     } else {
         if constexpr (PRE > 0) {
             double ce = coarse_product(g, g.c, sh.rows);
-            if (!comm.template sum<1>(ce, none, 3 * len, 0)) return;
+            if (!comm.template sum<1>(ce, none, sum_slot(CE, 0), 0)) return;
             rz += ce;
         }
         direction<PRE, true>(g, 0.0, 0.0);
@@ -239,7 +239,8 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
         int it = 0;
         for (; it < g.max_iter; ++it) {
             double pq = product<F>(g, g.p, g.q);
-            if (!comm.template sum<1>(pq, none, it, 0)) return;
+            if (!comm.template sum<1>(pq, none, sum_slot(PQ, it), 0)) return;
+            if (!CL && first) clear_slots<SUMS>(g.sums, it);
             if (!(pq > 0.0)) {
                 if (first) g.out[2] = 1;
                 break;
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
             const double alpha = rz / pq;
             double rzn;
             update<PRE, false>(g, alpha, c, rzn, rr);
-            if (!comm.template sum<2>(rzn, rr, len + it + 1, 2 * len + it + 1)) return;
+            if (!comm.template sum<2>(rzn, rr, sum_slot(RZ, it + 1), sum_slot(RR, it + 1))) return;
             if (rr <= thr) {
                 for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x)
                     g.x[i] += alpha * g.p[i];
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
                 double *other = g.c + (it & 1) * g.nc;
                 for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < g.nc; k += (int64_t)gridDim.x * blockDim.x)
                     other[k] = 0.0;
-                if (!comm.template sum<1>(ce, none, 3 * len + it + 1, 0)) return;
+                if (!comm.template sum<1>(ce, none, sum_slot(CE, it + 1), 0)) return;
                 rzn += ce;
             }
             direction<PRE, false>(g, alpha, rzn / rz);
@@ -589,7 +590,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
         const unsigned block = threads <= 512 * sm ? 512 : (unsigned)std::min<int64_t>(1024, ((threads + sm - 1) / sm + 127) / 128 * 128);
         cfg.blockDim = dim3(block);
         cfg.gridDim = dim3(grid_for(threads, block, (int)sm * std::max(occ, 1)));
-        const size_t slots = 4 * ((size_t)max_iter + 2);
+        constexpr size_t slots = 4 * kSumRing;
         s->scal.reserve(slots);
         g.sums = s->scal.p;
         SFC_CK(cudaMemsetAsync(g.sums, 0, slots * sizeof(double), ctx->stream));

@@ -30,14 +30,30 @@ struct PcgArgs {
     const double *ac;          // nc x nc inverse
     int64_t nc;
     double *c, *e;             // [2][nc], [nc]
-    double *sums;              // [4][max_iter + 2]: zeroed slots of the sums
+    double *sums;              // [sum][kSumRing]: slots of the sums, zero at the start
     unsigned *bar;
     double tol;
     int max_iter;
     int *out;                  // iterations, converged, error
 };
 
+// Slots of a sum over the grid, by iteration: the one in use, those whose last
+// readers and first writers lie a barrier apart from its own, and the one that
+// an iteration clears for the third one after it.
+constexpr int kSumRing = 4;
+
 namespace {
+
+// slot of sum k in iteration it, and the clearing: by one thread of the grid,
+// behind the first barrier of iteration it (every block has then read what
+// iteration it - 1 and those before it added up)
+__device__ __forceinline__ int sum_slot(int k, int it) { return k * kSumRing + (it & (kSumRing - 1)); }
+template <int SUMS>
+__device__ __forceinline__ void clear_slots(double *sums, int it)
+{
+#pragma unroll
+    for (int k = 0; k < SUMS; ++k) sums[sum_slot(k, it + 3)] = 0.0;
+}
 
 __device__ __forceinline__ double warp_total(double v)
 {
