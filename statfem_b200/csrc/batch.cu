@@ -759,7 +759,7 @@ void batch_configure(sfc_batch *b, int want_cluster)
 {
     const BatchKernel kernel = batch_kernel(b);
     const size_t smem = batch_smem(b->smax);
-    SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(kernel);
     SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     const int tries[] = {want_cluster, 8, 4, 2, 1};
     for (int cs : tries) {

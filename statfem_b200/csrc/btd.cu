@@ -781,7 +781,7 @@ __global__ void k_btd_correct(double *__restrict__ X, const double *__restrict__
 template <class K>
 cudaLaunchConfig_t btd_config(K kernel, const BtdPlan &p, int clusters, cudaStream_t st, cudaLaunchAttribute *attr)
 {
-    SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    allow_shared(kernel);
     SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     attr->id = cudaLaunchAttributeClusterDimension;
@@ -818,7 +818,7 @@ bool btd_plan(sfc_ctx *ctx, BtdPlan &p, const int32_t *rp, const int32_t *col, i
     // CTAs per chain: the fewest that leave room for two CTAs on an SM (two
     // instances then hide each other's pivot inverses), more while the
     // clusters do not fill the device and each CTA keeps two row groups
-    const size_t lim = 227 * 1024;
+    const size_t lim = kMaxShared;
     int C = 1;
     while (C < 8 && btd_smem(p.lmax, C) > 112 * 1024) C *= 2;
     while (C < 8 && 2 * C * n_inst < ctx->sm_count && (p.lmax + 7) / 8 >= 4 * C) C *= 2;

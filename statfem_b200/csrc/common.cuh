@@ -158,6 +158,17 @@ inline unsigned grid_for(int64_t work, int block, int max_blocks = 148 * 32)
     return (unsigned)g;
 }
 
+// The dynamic shared memory that a kernel may ask for is the device's, one
+// value for all contexts and threads: it is set to the same bound on every
+// call (at most 227 KB with the kernel's static part), not to the size of the
+// launch at hand, which another thread's smaller one would take back.
+constexpr int kMaxShared = 227 * 1024;
+template <class K>
+void allow_shared(K *kernel, int bound = kMaxShared)
+{
+    SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bound));
+}
+
 // copy host -> device on the context stream (synchronous w.r.t. the host
 // buffer: the call returns once the data has been consumed)
 template <class T>

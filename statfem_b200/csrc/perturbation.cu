@@ -246,8 +246,7 @@ int material_factor(sfc_ctx *ctx, const DBuf<double> &cent, int64_t E, int dim, 
     const int64_t chunks = (E + 31) / 32;
     int G = 1;
     while (G < kFacWarps && 2 * G * chunks <= (int64_t)kFacWarps * kFacCtas) G *= 2;
-    SFC_CK(cudaFuncSetAttribute(k_material_factor<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                std::min(most, kFacRow) * 8 + 16));
+    allow_shared(k_material_factor<true>, kFacRow * 8 + 16);
     for (;;) {
         DevInt out = status_word(ctx, 2);
         const bool staged = cap <= kFacRow;

@@ -518,7 +518,7 @@ void kernel_times(sfc_ctx *ctx, sfc_covar_forcing *cf, double sigma, double leng
     } else {
         const size_t smem = (size_t)(kTI * kTJ + kTJ * ns) * 8;
         SFC_REQUIRE(ns <= 256, "dense forcing covariance supports at most 256 projection rows");
-        SFC_CK(cudaFuncSetAttribute(k_kw_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared(k_kw_dense);
         for (int c = 0; c < dof; ++c) {
             k_kw_dense<<<(unsigned)((nodes + kTI - 1) / kTI), 256, smem, ctx->stream>>>(m->coords.p, nodes, m->dim, dof,
                                                                                      c, ns, W, T, sigma, length);
@@ -797,9 +797,9 @@ void koh_loglik_batch(sfc_koh *k, const sfc_hparams_t *hps, int n, double *out)
     const int ns = (int)k->ns;
     // in shared memory where the item's system fits a block
     const size_t smem = (size_t)(ns + k->n_o) * (ns | 1) * sizeof(double);
-    if (smem <= 200 * 1024) {
-        if (smem > 48 * 1024)
-            SFC_CK(cudaFuncSetAttribute(k_koh_loglik_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr int bound = 200 * 1024;
+    if (smem <= bound) {
+        if (smem > 48 * 1024) allow_shared(k_koh_loglik_shared, bound);
         k->bres.reserve(n);
         k->bhp.reserve(n);
         SFC_CK(cudaMemcpyAsync(k->bhp.p, hps, n * sizeof(*hps), cudaMemcpyHostToDevice, ctx->stream));
