@@ -98,7 +98,7 @@ void solve_host_columns(sfc_system *s, const double *rhs, double *u, int nrhs, F
     solve(s->host_cols[1].p, s->host_cols[2].p);
     transpose64(s->ctx, s->host_cols[2].p, s->host_cols[0].p, N, nrhs);
     download(s->ctx, u, s->host_cols[0].p, n);
-    if (3 * n * sizeof(double) > ((size_t)256 << 20))
+    if (3 * n * sizeof(double) > kKeptScratch)
         for (auto &b : s->host_cols) b.release();
 }
 

@@ -958,7 +958,7 @@ void assemble_load(sfc_ctx *ctx, const sfc_mesh *m, const double *f, double *F_d
                                                   m->num_nodes, m->dof, f0, f1, f2, nullptr, F_dev);
         break;
     default: {
-        DBuf<double> &sw = const_cast<sfc_mesh *>(m)->load_w;
+        DBuf<double> &sw = ctx->load_w;
         const double *points = nullptr;
         try {
             sw.reserve(m->num_elems * m->quad.nq);
@@ -972,6 +972,7 @@ void assemble_load(sfc_ctx *ctx, const sfc_mesh *m, const double *f, double *F_d
         }
         k_load<3, 8><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->conn.p, m->node_ptr.p, m->node_elem.p, m->quad,
                                                   m->num_nodes, m->dof, f0, f1, f2, points, F_dev);
+        if (sw.n * sizeof(double) > kKeptScratch) sw.release();
         break;
     }
     }

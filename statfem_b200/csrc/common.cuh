@@ -45,6 +45,9 @@ struct Error {
         if (!(cond)) ::sfc::fail(SFC_ERR_TOO_LARGE, msg);                              \
     } while (0)
 
+// Scratch beyond this many bytes is given back after the call
+constexpr size_t kKeptScratch = (size_t)256 << 20;
+
 // Device buffer with RAII ownership.
 template <class T>
 struct DBuf {
@@ -104,6 +107,10 @@ struct sfc_ctx {
     // synchronisation) on the repeated-solve path
     sfc::DBuf<int> ierr;       // >= 16 ints
     sfc::DBuf<double> dsmall;  // >= 16 doubles
+    // w*detJ of every quadrature point of a hexahedral mesh (assemble_load).
+    // Here and not with the mesh, which calls on other contexts may read at
+    // the same time; kept up to kKeptScratch bytes
+    sfc::DBuf<double> load_w;
     // kernel timing (off by default): an event pair around each profiled launch
     bool prof = false;
     struct ProfRec {
@@ -428,7 +435,6 @@ struct sfc_mesh {
     sfc::DBuf<int32_t> node_ptr;   // num_nodes + 1
     sfc::DBuf<int32_t> node_elem;  // num_elems * nn
     // element matrices of the last assembly (num_elems * L * L)
-    sfc::DBuf<double> load_w;  // hexahedra: w*detJ of every quadrature point (assemble_load)
     sfc::DBuf<double> ke;
     // tensor-grid description of the node set (for the Kronecker covariance)
     bool is_grid = false;

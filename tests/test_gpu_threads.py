@@ -77,3 +77,27 @@ def test_material_factors(ctx):
         hp = dict(HP, **{"material.sigma": 0.3, "material.length": 0.4})
         return (lambda: pt.updateSolution(hp, factor_tol=1e-6)), pt.giveProjectedCovarU
     assert together(works_of(make, [14, 5])) == []
+
+
+@pytest.mark.parametrize("kind,n", [(mg.HEX8_POISSON, 12), (mg.HEX8_ELASTIC, 7)])
+def test_loads_from_one_mesh(ctx, kind, n):
+    """Systems of several contexts take their loads from the same mesh, the
+    first calls among them: each allocates for itself."""
+    prob = statfem_problem(kind, n, 1, seed=n)
+    mesh = prob["mesh"]
+    f = np.arange(1.0, 1.0 + mesh.dof)
+    gm = api.Mesh(ctx, kind, 8, mesh.coords, mesh.conn)
+    s = api.SystemSolveCuda(ctx, mesh.num_dofs)
+    s.assemble_load(gm, f)
+    want = s.giveForce()
+    shared = api.Mesh(ctx, kind, 8, mesh.coords, mesh.conn)
+    works = []
+    for _ in range(4):
+        t = api.SystemSolveCuda(api.Context(0), mesh.num_dofs)
+
+        def call(t=t):
+            t.clearRhs()
+            t.assemble_load(shared, f)
+
+        works.append((call, lambda t=t: np.testing.assert_array_equal(t.giveForce(), want)))
+    assert together(works) == []
