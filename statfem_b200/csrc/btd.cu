@@ -947,6 +947,7 @@ void plan_system(sfc_system *s)
     count_launch(ctx);
     int bw = 0;
     download(ctx, &bw, p.word.p, 1);
+    p.width = std::max(bw - 1, 1);
     const int64_t row0[2] = {0, s->N};
     const int32_t order = 0;
     for (const int m : {s->N <= 64 ? (int)s->N : 32, bw - 1, bw}) {
@@ -958,13 +959,32 @@ void plan_system(sfc_system *s)
 
 }  // namespace
 
+bool btd_applies(sfc_system *s)
+{
+    if (!s->btd.tried) plan_system(s);
+    return s->btd.usable;
+}
+
+// A chain's step takes a factor of 6 + 0.1 m + 0.0009 m^2 us and, there and back,
+// a solve of 7 + 0.07 m (m dofs to a line; fitted to the times at direct_pays,
+// within 15 %), 1.3 times that in chains of a few CTAs with three row groups and
+// more each; the clusters of a wave beside one another, 32 columns to a cluster.
+double btd_estimate(const sfc_system *s, int nrhs)
+{
+    const BtdPlan &p = s->btd;
+    const double m = p.lmax, steps = std::ceil((double)p.N / m) / 2 + 1;
+    const int tiles = (nrhs + kBtdCols - 1) / kBtdCols, wave = std::max(1, s->ctx->sm_count / (2 * p.chain));
+    const double factor = p.factored == s->op_serial ? 0.0 : 6 + 0.1 * m + 0.0009 * m * m;
+    const double full = p.chain < 8 && btd_rows(p.lmax, p.chain) >= 24 ? 1.3 : 1.0;
+    return 60 + full * steps * (factor + (7 + 0.07 * m) * ((tiles + wave - 1) / wave));
+}
+
 bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int ld, double tol, bool recurrence,
                       double *max_rel)
 {
     sfc_ctx *ctx = s->ctx;
     BtdPlan &p = s->btd;
-    if (!p.tried) plan_system(s);
-    if (!p.usable) return false;
+    if (!btd_applies(s)) return false;
     BtdArgs a = btd_args(p, s->row_ptr.p, s->col.p, s->a_op.p);
     a.B = B;
     a.U = X;

@@ -45,6 +45,10 @@ void btd_launch_batch(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a, cudaStre
 // one system: the inverse blocks, then any number of columns
 void btd_launch_factor(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a);
 void btd_launch_solve(sfc_ctx *ctx, const BtdPlan &p, const BtdArgs &a);
+// Whether the system's pattern has the form (planned on the first call), and an
+// estimate of a solve for nrhs columns in us (with the factor, unless it is there)
+bool btd_applies(sfc_system *s);
+double btd_estimate(const sfc_system *s, int nrhs);
 // S X = B of a system whose operator is built, refined with FP64 residuals
 // where the first solution misses tol; false (X undefined) where the
 // elimination does not apply, the operator is not positive definite or a

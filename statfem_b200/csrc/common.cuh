@@ -296,6 +296,7 @@ struct EventPair {
 struct BtdPlan {
     bool tried = false, usable = false;  // for the pattern at hand
     int n = 0, lmax = 0, chain = 0, slots = 0;
+    int width = 0;  // single systems: dofs of a grid line, by the bandwidth
     size_t smem = 0;
     int64_t N = 0;
     DBuf<int64_t> row0;

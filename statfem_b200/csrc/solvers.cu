@@ -1830,16 +1830,69 @@ double device_dot(sfc_ctx *ctx, const double *a, const double *b, int64_t n)
     return h;
 }
 
+// constrained dofs
+__global__ void k_count_mask(const unsigned char *__restrict__ mask, int64_t N, int *count)
+{
+    int c = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
+        c += mask[i] != 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) atomicAdd(count, c);
+}
+
+// Whether the elimination is worth its time against the iteration: its chain
+// grows with the lines and their length, the iteration with the dofs and the
+// columns.  The two-level one takes 115 iterations to 1e-11, more once the
+// boxes, whose number is bounded, grow; point Jacobi 5 per dof of a square's
+// side and 11 across a strip that is held along its edges (one that is not, or
+// a bar, takes them along its length: eliminated).  Adjoint solves,
+// elimination / iteration in ms, for 8, 75 and 200 columns (cells of 1 x 1):
+//                 two-level                             point Jacobi, 8 and 75
+//   64^2          1.12 / 3.15  1.15 / 3.84  1.14 / 8.52  1.12 / 5.63  1.15 / 7.25
+//   128^2         3.31 / 4.53  3.36 / 6.01  3.39 / 13.0  3.31 / 17.6  3.36 / 23.1
+//   181^2         6.66 / 6.00  6.76 / 9.99  6.85 / 20.2  6.67 / 27.7  6.77 / 51.6
+//   230^2         12.0 / 7.67  12.2 / 14.1  12.2 / 28.1  12.0 / 42.6  12.2 / 80.1
+//   318^2         26.8 / 12.2  27.1 / 25.7  27.0 / 51.2  26.8 / 75.7  27.1 / 223
+//   150 x 600     17.6 / 11.0  18.0 / 24.8  18.0 / 48.9  17.6 / 60.3  18.0 / 181
+//   60 x 2,000    25.9 / 14.1  26.9 / 29.8  26.9 / 57.5  25.9 / 40.3  26.9 / 115
+//   20 x 2,000    11.3 / 5.47  11.9 / 8.57  12.3 / 17.7  11.3 / 8.48  11.9 / 13.8
+//   8 x 3,000     7.08 / 3.50  7.28 / 4.98  7.43 / 9.82  7.08 / 3.07  7.28 / 4.81
+//   255 x 1,000   54.2 / 31.5  55.0 / 71.7  54.8 / 145   54.2 / 274   55.0 / 740
+// The choice is the faster one of these, or within 12 % of it.
+bool direct_pays(sfc_system *s, int nrhs, bool forward)
+{
+    const auto &o = s->opt;
+    const double N = (double)s->N, tol = o.tol > 0 ? o.tol : 1e-8;
+    const double decades = std::max(0.1, -std::log10(tol) / 11), direct = btd_estimate(s, nrhs);
+    const int blocks = (nrhs + 127) / 128;
+    if (o.precond == SFC_PRECOND_TWO_LEVEL && s->pattern_mesh) {
+        const double its = 115 * std::max(1.0, std::sqrt(N / 130000)) * decades;
+        // the forward solve's alternative is the FP64 kernel of pcg.cu
+        const double us = forward ? 10 + 8e-5 * N : 24 + N * (nrhs <= 32 ? 7.5e-4 : nrhs <= 64 ? 1.1e-3 : 1.75e-3);
+        return direct <= its * us * blocks;
+    }
+    const double w = s->btd.width, l = N / w, side = 1 / std::sqrt(1 / (w * w) + 1 / (l * l));
+    const double its = (std::max(w, l) >= 4 * std::min(w, l) ? 11 : 7.4) * side * decades;
+    const double us = forward ? 8 + 3e-5 * N : 18 + N * (nrhs <= 32 ? 5e-4 : 1.3e-3);
+    if (direct <= its * us * blocks) return true;
+    sfc_ctx *ctx = s->ctx;
+    DevInt held = status_word(ctx, 5);
+    SFC_CK(cudaMemsetAsync(held.p, 0, sizeof(int), ctx->stream));
+    k_count_mask<<<grid_for(s->N, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(s->mask.p, s->N, held.p);
+    count_launch(ctx);
+    int h = 0;
+    download(ctx, &h, held.p, 1);
+    return h < 1.5 * l;  // two edges of a strip are 2 l
+}
+
 // Block elimination for the statX objects' own solves (the explicit solve
-// entry points keep the PCG they name).  With SFC_SOLVER_PCG_MIXED wherever it
-// applies: the adjoint solve of 75 sensors on the 182 x 182 grid 10.3 -> 6.9 ms,
-// of 16 on 65 x 65 5.1 -> 1.2 ms.  SFC_SOLVER_PCG_FP64 is the plain method
-// that others are compared with and keeps its iterations, except where a
-// solve is no more than its launches (up to 1,024 dofs: the full-field
-// posterior of the 33-dof bar, 44 solves, 19.5 -> 0.63 ms).  A cap below the
-// number of dofs (CG's own bound on its iterations) and below the default
-// asks for an early stop and keeps them too.
-bool solve_direct(sfc_system *s, const double *B, double *X, int nrhs, int ld)
+// entry points keep the PCG they name).  With SFC_SOLVER_PCG_MIXED where it
+// pays.  SFC_SOLVER_PCG_FP64 is the plain method that others are compared with
+// and keeps its iterations, except where a solve is no more than its launches
+// (up to 1,024 dofs: the full-field posterior of the 33-dof bar, 44 solves,
+// 19.5 -> 0.63 ms).  A cap below the number of dofs (CG's own bound on its
+// iterations) and below the default asks for an early stop and keeps them too.
+bool solve_direct(sfc_system *s, const double *B, double *X, int nrhs, int ld, bool forward = false)
 {
     sfc_ctx *ctx = s->ctx;
     const auto &o = s->opt;
@@ -1847,6 +1900,7 @@ bool solve_direct(sfc_system *s, const double *B, double *X, int nrhs, int ld)
     const int max_iter = o.max_iter > 0 ? o.max_iter : 20000;
     const double tol = o.tol > 0 ? o.tol : 1e-8;
     if (max_iter < s->N && max_iter < 20000) return false;
+    if (!btd_applies(s) || (o.method == SFC_SOLVER_PCG_MIXED && !direct_pays(s, nrhs, forward))) return false;
     s->solve_ev.ensure();
     SFC_CK(cudaEventRecord(s->solve_ev.a, ctx->stream));
     double worst = 0.0;
@@ -1886,7 +1940,7 @@ void solve_forward(sfc_system *s, bool direct)
     k_lift<<<grid_for(N, 256), 256, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, s->diag.p, s->a_ref.p, s->mask.p, s->F.p,
                                                       N, b.p);
     count_launch(ctx);
-    if (direct && solve_direct(s, b.p, s->X.p, 1, 1)) return;
+    if (direct && solve_direct(s, b.p, s->X.p, 1, 1, true)) return;
     const auto &o = s->opt;
     const int max_iter = o.max_iter > 0 ? o.max_iter : 20000;
     const int check = o.check_every > 0 ? o.check_every : 16;
