@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "btd.cuh"
+#include "tile64.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -56,13 +57,6 @@ __host__ __device__ inline size_t btd_smem(int m, int C)
     const size_t panel = (size_t)PW * ld > (size_t)mp * ZLD ? (size_t)PW * ld : (size_t)mp * ZLD;
     return 8 * ((size_t)rows * ld + panel + 4 * PW + (size_t)rows * (kBtdSide + kBtdSide + kBtdMid)) +
            4 * (size_t)rows * (kBtdSide + kBtdSide + kBtdMid) + 64;
-}
-
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
 }
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
@@ -102,34 +96,13 @@ __device__ __forceinline__ int line_at(const Inst &q, int chain, int st)
     return l > q.mid ? l : -1;
 }
 
-// 1 / d by Newton's iteration on the hardware's approximation (about 20 bits;
-// two steps reach rounding): no branch, so the compiler can place the other
-// rows' updates inside its latency.  For d and 1 / d normal numbers
-// (pivot_ok): both are flushed to zero below.
-__device__ __forceinline__ double recip(double d)
-{
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-    x = fma(x, fma(-d, x, 1.0), x);
-    return fma(x, fma(-d, x, 1.0), x);
-}
-
-// A pivot of a positive definite matrix, within the range of recip
-__device__ __forceinline__ bool pivot_ok(double d) { return d >= 0x1p-1022 && d <= 0x1p1022; }
-
 // In-place inverse of the kw x kw symmetric positive definite block at P (row
-// stride ld) by the first four warps (warp w holds rows 8 w .. 8 w + 7, lane j
-// column j).  The symmetric sweep (its result is the negative inverse) makes
-// the pivot column equal to the pivot row, so a step exchanges one row
-// through shared memory; the next row is updated and published before the
-// rest of a step, which runs inside the next pivot's latency.  2.9 us for 32
-// columns; 7.0 us with 256 threads, a division and a full barrier per step,
-// 6.9 us with one warp (its 31 updates per step bound it).  Whether all pivots
-// were positive: the pivots of an elimination in any symmetric order are, if
-// and only if the matrix is positive definite.
+// stride ld) by the first four warps (sweep_inverse).  Returns whether every
+// pivot was positive and in the reciprocal's range: the pivots of an elimination
+// in any symmetric order are positive if and only if the matrix is positive
+// definite.
 __device__ bool pivot_inverse(double *P, int ld, int kw, double *buf)
 {
-    bool ok = true;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double v[8];
 #pragma unroll
@@ -137,36 +110,12 @@ __device__ bool pivot_inverse(double *P, int ld, int kw, double *buf)
         const int r = 8 * warp + i;
         v[i] = r < kw && lane < kw ? P[(size_t)r * ld + lane] : (r == lane ? 1.0 : 0.0);
     }
-    if (warp == 0) buf[lane] = v[0];
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll 1
-    for (int kb = 0; 8 * kb < kw; ++kb) {
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int k = 8 * kb + t, t1 = (t + 1) & 7;
-            const bool own = warp == kb, next = warp == (t == 7 ? kb + 1 : kb);
-            const double *sh = buf + PW * (t & 1);
-            double *nx = buf + PW * (t1 & 1);
-            double row[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) row[i] = sh[8 * warp + i];
-            const double inv = recip(sh[k]), mine = sh[lane];
-            ok = ok && pivot_ok(sh[k]);
-            const bool me = lane == k;
-            const double f = me ? inv : -mine * inv;
-            if (next) {
-                v[t1] = fma(row[t1], f, me ? 0.0 : v[t1]);
-                nx[lane] = v[t1];
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (next && i == t1) continue;
-                if (own && i == t) v[i] = me ? -inv : -f;
-                else v[i] = fma(row[i], f, me ? 0.0 : v[i]);
-            }
-        }
-    }
+    bool ok = true;
+    sweep_inverse(v, kw, buf, [&](int, double d, double &inv) {
+        ok = ok && recip_takes(d);
+        inv = recip(d);
+        return true;
+    });
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int r = 8 * warp + i;

@@ -13,6 +13,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "tile64.cuh"
 
 namespace sfc {
 
@@ -21,29 +22,10 @@ namespace {
 constexpr int kGJ = 32;     // panel width
 constexpr int kGjTile = 64; // tile of A per CTA
 
-// D (8 x 8) += A (8 x 4) B (4 x 8): lane l holds A[l / 4][l % 4], B[l % 4][l / 4], D[l / 4][2 (l % 4) + 0, 1]
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
-// 1 / d by Newton's iteration on the hardware's approximation (about 20 bits,
-// two steps): no branch in the chain of pivots
-__device__ __forceinline__ double recip(double d)
-{
-    double x;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-    x = fma(x, fma(-d, x, 1.0), x);
-    return fma(x, fma(-d, x, 1.0), x);
-}
-
 // Inverse of the kb x kb symmetric block in D (row stride LD) by the first
-// four warps, written to out (32 x 32, zero outside): the symmetric sweep,
-// warp w holding rows 8 w .., lane j column j, with the next row published
-// before the rest of a step.  A pivot not above rel x the dof's original
-// diagonal (thr) is dropped: its row and column are zeroed.  buf: 2 x 32.
+// four warps (sweep_inverse), written to out (32 x 32, zero outside).  A pivot
+// not above rel x the dof's original diagonal (thr) is dropped: its row and
+// column are zeroed.  buf: 2 x 32.
 template <int LD>
 __device__ void gj_block_inverse(const double *D, int kb, const double *thr, double *buf, double *out, int *dropped,
                                  double *pivots)
@@ -55,42 +37,16 @@ __device__ void gj_block_inverse(const double *D, int kb, const double *thr, dou
         const int r = 8 * warp + i;
         v[i] = r < kb && lane < kb ? D[r * LD + lane] : (r == lane ? 1.0 : 0.0);
     }
-    if (warp == 0) buf[lane] = v[0];
     int ndrop = 0;
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll 1
-    for (int b = 0; b < 4; ++b) {
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int k = 8 * b + t, t1 = (t + 1) & 7;
-            const bool own = warp == b, next = warp == (t == 7 ? b + 1 : b);
-            const double *sh = buf + 32 * (t & 1);
-            double *nx = buf + 32 * (t1 & 1);
-            double row[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) row[i] = sh[8 * warp + i];
-            const double piv = sh[k], mine = sh[lane];
-            const bool drop = k < kb && !(piv > thr[k]);
-            if (threadIdx.x == 0 && k < kb) {
-                if (pivots) pivots[k] = piv;
-                ndrop += drop;
-            }
-            const double inv = drop ? 0.0 : recip(piv);
-            const bool me = lane == k;
-            const double f = me ? inv : drop ? 0.0 : -mine * inv;
-            if (next) {
-                v[t1] = drop ? (me ? 0.0 : v[t1]) : fma(row[t1], f, me ? 0.0 : v[t1]);
-                nx[lane] = v[t1];
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (next && i == t1) continue;
-                if (own && i == t) v[i] = me ? -inv : -f;
-                else v[i] = drop ? (me ? 0.0 : v[i]) : fma(row[i], f, me ? 0.0 : v[i]);
-            }
+    sweep_inverse(v, kGJ, buf, [&](int k, double d, double &inv) {
+        const bool drop = k < kb && !(d > thr[k]);
+        if (threadIdx.x == 0 && k < kb) {
+            if (pivots) pivots[k] = d;
+            ndrop += drop;
         }
-    }
+        if (!drop) inv = recip_takes(d) ? recip(d) : 1.0 / d;
+        return !drop;
+    });
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int r = 8 * warp + i;

@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "koh_dev.cuh"
+#include "tile64.cuh"
 
 namespace sfc {
 
@@ -103,14 +104,6 @@ __global__ void __launch_bounds__(256) k_kw_dense(const double *__restrict__ coo
         const int64_t i = i0 + ii;
         if (i < nodes) T[(i * dof + c) * ns + a] = acc[u];
     }
-}
-
-// D (8 x 8) += A (8 x 4) B (4 x 8): lane l holds A[l / 4][l % 4], B[l % 4][l / 4], D[l / 4][2 (l % 4) + 0, 1]
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
 }
 
 // 1-D SE correlation factor along one grid axis: scale exp(-d^2/(2 l^2)) of the
