@@ -234,7 +234,7 @@ struct sfc_mesh;
 namespace sfc {
 // scratch of spd_inverse_gj (dense.cu)
 struct GjScratch {
-    DBuf<double> diag, other, dinv;  // pivots' thresholds; the matrix's second copy; inverses of diagonal blocks
+    DBuf<double> diag, rowp, colp, dinv;  // pivots' thresholds; copies of two panels' rows and columns; inverses of diagonal blocks
     DBuf<int> word;
     struct Graph {  // captured launch sequence of one (matrix, size)
         const double *A;

@@ -2,13 +2,16 @@
 // Gauss-Jordan elimination without pivoting, on the GPU: the in-place form
 //     A[k,k] <- D^-1,  A[k,j] <- D^-1 A[k,j],  A[i,k] <- -A[i,k] D^-1,
 //     A[i,j] <- A[i,j] - A[i,k] D^-1 A[k,j]
-// for 32-wide panels k (D the panel's diagonal block), one launch per panel
-// that reads one copy of A and writes the other.  Used for the coarse matrix of the two-level preconditioner (with
+// for 32-wide panels k (D the panel's diagonal block), one launch per panel: a
+// tile's own values are read and written by one CTA, and the panel's rows and
+// columns, which the others read, were copied by the launch before.  Used for the coarse matrix of the two-level preconditioner (with
 // dependent pivots dropped: a generalised inverse on the independent modes)
 // and for the sensor-space matrices of the KOH likelihood and posterior
 // (LikelihoodKOH.ipp:75-120, 311-361), where a non-positive pivot is the
 // reference's failed LLT.  The Schur-complement pivots are the squared
 // diagonal of the Cholesky factor, so their logarithms sum to log det A.
+
+#include <algorithm>
 
 #include <algorithm>
 
@@ -56,13 +59,25 @@ __device__ void gj_block_inverse(const double *D, int kb, const double *thr, dou
 }
 
 // The original diagonal (x rel: the thresholds of the pivots) and the inverse
-// of the first diagonal block
+// of the first diagonal block; the other CTAs copy the first panel's rows
+// (rowp[m][j]) and columns (colp[i][m]), kGjTile of either
 __global__ void __launch_bounds__(256) k_gj_first(const double *__restrict__ A, int64_t n, double rel,
-                                                  double *__restrict__ thr, double *__restrict__ dinv, int *dropped,
+                                                  double *__restrict__ thr, double *__restrict__ dinv,
+                                                  double *__restrict__ rowp, double *__restrict__ colp, int *dropped,
                                                   double *pivots)
 {
     __shared__ double D[kGJ * (kGJ + 1)], buf[2 * kGJ], st[kGJ];
     const int kb = (int)min((int64_t)kGJ, n);
+    if (blockIdx.x > 0) {
+        const int64_t j0 = (int64_t)(blockIdx.x - 1) * kGjTile;
+#pragma unroll
+        for (int u = 0; u < kGjTile * kGJ / 256; ++u) {
+            const int t = threadIdx.x + 256 * u, l = t / kGjTile, j = t % kGjTile, i = t / kGJ, m = t % kGJ;
+            if (l < kb && j0 + j < n) rowp[l * n + j0 + j] = A[l * n + j0 + j];
+            if (m < kb && j0 + i < n) colp[(j0 + i) * kGJ + m] = A[(j0 + i) * n + m];
+        }
+        return;
+    }
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) thr[i] = rel * A[i * n + i];
     for (int t = threadIdx.x; t < kGJ * kGJ; t += blockDim.x) {
         const int r = t / kGJ, c = t % kGJ;
@@ -73,21 +88,22 @@ __global__ void __launch_bounds__(256) k_gj_first(const double *__restrict__ A, 
     if (threadIdx.x < 128) gj_block_inverse<kGJ + 1>(D, kb, st, buf, dinv, dropped, pivots);
 }
 
-// One panel, a 64 x 64 tile of the result per CTA, with D^-1 of the panel's
-// diagonal block in dinv:
-//   rows of the panel:     out = rowp[i - k0][j],  rowp = D^-1 A[k0.., j] (D^-1 itself inside the block)
-//   columns of the panel:  out = -A[i, k0..] rowp[:, j]
-//   elsewhere:             out = A[i][j] - A[i, k0..] rowp[:, j]
-// on FP64 matrix instructions, every CTA forming the rowp of its columns
-// itself.  The first CTA takes the tile with the next panel's diagonal block
+// One panel, a 64 x 64 tile of A per CTA, in place, with D^-1 of the panel's
+// diagonal block in dinv and its rows and columns as they were in rowp, colp:
+//   rows of the panel:     A[i][j] = r[i - k0][j],  r = D^-1 rowp[:, j] (D^-1 itself inside the block)
+//   columns of the panel:  A[i][j] = -colp[i] r[:, j]
+//   elsewhere:             A[i][j] -= colp[i] r[:, j]
+// on FP64 matrix instructions, every CTA forming the r of its columns itself
+// and copying what it has of the next panel's rows and columns.  The first CTA takes the tile with the next panel's diagonal block
 // and inverts that too, while the others are at their products: the chain
 // from panel to panel is a launch, a tile and an inverse of 3 us.  1,000 x
 // 1,000: 468 us; 1,202 as two launches per panel, the inverse (with a barrier
 // of the whole CTA and a division per pivot) before the panel's products.
-__global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ A, double *__restrict__ out, int64_t n,
-                                                 int64_t k0, int kb, const double *__restrict__ thr,
-                                                 const double *__restrict__ dinv, double *__restrict__ dnext,
-                                                 int *dropped, double *pivots)
+__global__ void __launch_bounds__(256) k_gj_step(double *__restrict__ A, int64_t n, int64_t k0, int kb,
+                                                 const double *__restrict__ thr, const double *__restrict__ rowp,
+                                                 const double *__restrict__ colp, double *__restrict__ rown,
+                                                 double *__restrict__ coln, const double *__restrict__ dinv,
+                                                 double *__restrict__ dnext, int *dropped, double *pivots)
 {
     constexpr int T = kGjTile, LC = kGJ + 4, LR = T + 4;  // odd multiples of four: no bank conflicts
     __shared__ double sD[kGJ * LC], sC[T * LC], sR[kGJ * LR];
@@ -109,8 +125,8 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ A, d
         for (int u = 0; u < 8; ++u) {
             const int t = threadIdx.x + 256 * u;
             const int i = t / kGJ, m = t % kGJ, l = t / T, j = t % T;
-            vc[u] = (i0 + i < n && m < kb) ? A[(i0 + i) * n + k0 + m] : 0.0;
-            vr[u] = (l < kb && j0 + j < n) ? A[(k0 + l) * n + j0 + j] : 0.0;
+            vc[u] = (i0 + i < n && m < kb) ? colp[(i0 + i) * kGJ + m] : 0.0;
+            vr[u] = (l < kb && j0 + j < n) ? rowp[l * n + j0 + j] : 0.0;
         }
 #pragma unroll
         for (int x = 0; x < 2; ++x)
@@ -135,7 +151,7 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ A, d
         if (threadIdx.x < kGJ) st[threadIdx.x] = kn + threadIdx.x < n ? thr[kn + threadIdx.x] : 0.0;
     }
     __syncthreads();
-    {  // rowp: rows 8 (warp % 4) .., columns wj .. of it
+    {  // r: rows 8 (warp % 4) .., columns wj .. of it
         double p[4][2];
 #pragma unroll
         for (int y = 0; y < 4; ++y) p[y][0] = p[y][1] = 0.0;
@@ -183,9 +199,12 @@ __global__ void __launch_bounds__(256) k_gj_step(const double *__restrict__ A, d
                 const int64_t i = i0 + ti, j = j0 + tj;
                 const bool in_r = i >= k0 && i < k0 + kb, in_c = j >= k0 && j < k0 + kb;
                 const double w = in_r ? sR[(i - k0) * LR + tj] : in_c ? -s[x][y][v] : own[x][y][v] - s[x][y][v];
-                if (i < n && j < n) out[i * n + j] = w;
-                if (blockIdx.x == 0 && i >= kn && i < kn + kGJ && j >= kn && j < kn + kGJ)
-                    sD[(i - kn) * LC + j - kn] = w;
+                if (i >= n || j >= n) continue;
+                const bool nr = i >= kn && i < kn + kGJ, nc = j >= kn && j < kn + kGJ;
+                A[i * n + j] = w;
+                if (nr) rown[(i - kn) * n + j] = w;
+                if (nc) coln[i * kGJ + j - kn] = w;
+                if (blockIdx.x == 0 && nr && nc) sD[(i - kn) * LC + j - kn] = w;
             }
     if (blockIdx.x != 0 || kn >= n) return;
     __syncthreads();
@@ -206,9 +225,10 @@ GjScratch::~GjScratch() { drop_graphs(); }
 
 void GjScratch::reserve(int64_t n)
 {
-    if ((size_t)n > diag.n || (size_t)(n * n) > other.n || !word.p) drop_graphs();  // buffers move
+    if ((size_t)n > diag.n || (size_t)(2 * kGJ * n) > std::min(rowp.n, colp.n) || !word.p) drop_graphs();  // buffers move
     diag.reserve(n);
-    other.reserve(n * n);
+    rowp.reserve(2 * kGJ * n);
+    colp.reserve(2 * kGJ * n);
     dinv.reserve(2 * kGJ * kGJ);
     word.reserve(1);
 }
@@ -217,17 +237,16 @@ namespace {
 void gj_enqueue(cudaStream_t st, double *A, int64_t n, double rel, GjScratch &w, double *pivots)
 {
     cudaMemsetAsync(w.word.p, 0, sizeof(int), st);
-    k_gj_first<<<1, 256, 0, st>>>(A, n, rel, w.diag.p, w.dinv.p, w.word.p, pivots);
     const unsigned gt = (unsigned)((n + kGjTile - 1) / kGjTile);
-    double *from = A, *to = w.other.p;
+    double *D[2] = {w.dinv.p, w.dinv.p + kGJ * kGJ}, *R[2] = {w.rowp.p, w.rowp.p + kGJ * n},
+           *C[2] = {w.colp.p, w.colp.p + kGJ * n};
+    k_gj_first<<<1 + gt, 256, 0, st>>>(A, n, rel, w.diag.p, D[0], R[0], C[0], w.word.p, pivots);
     int p = 0;
-    for (int64_t k0 = 0; k0 < n; k0 += kGJ, ++p) {
+    for (int64_t k0 = 0; k0 < n; k0 += kGJ, p ^= 1) {
         const int kb = (int)std::min<int64_t>(kGJ, n - k0);
-        k_gj_step<<<gt * gt, 256, 0, st>>>(from, to, n, k0, kb, w.diag.p, w.dinv.p + (p & 1) * kGJ * kGJ,
-                                           w.dinv.p + (~p & 1) * kGJ * kGJ, w.word.p, pivots);
-        std::swap(from, to);
+        k_gj_step<<<gt * gt, 256, 0, st>>>(A, n, k0, kb, w.diag.p, R[p], C[p], R[p ^ 1], C[p ^ 1], D[p], D[p ^ 1],
+                                           w.word.p, pivots);
     }
-    if (from != A) cudaMemcpyAsync(A, from, n * n * sizeof(double), cudaMemcpyDeviceToDevice, st);
 }
 }  // namespace
 
