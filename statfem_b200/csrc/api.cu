@@ -84,22 +84,30 @@ void transpose64(sfc_ctx *ctx, const double *in, double *out, int64_t rows, int6
 
 // Solves for host right-hand sides: the caller's [nrhs][N] columns go up as
 // they are and are transposed to the interleaved [N][nrhs] layout on the GPU
-// (and back).  The arrays stay with the system up to 256 MB, so that a
-// repeated call does not allocate.
+// (and back).  The two arrays stay with the system up to kKeptScratch bytes, so
+// that a repeated call does not allocate; beyond that they are given back, by a
+// call that fails too.
 template <class F>
 void solve_host_columns(sfc_system *s, const double *rhs, double *u, int nrhs, F solve)
 {
     const int64_t N = s->N;
     const size_t n = (size_t)N * nrhs;
-    upload(s->ctx, s->host_cols[0], rhs, n);
-    s->host_cols[1].reserve(n);
-    transpose64(s->ctx, s->host_cols[0].p, s->host_cols[1].p, nrhs, N);
-    s->host_cols[2].reserve(n);
-    solve(s->host_cols[1].p, s->host_cols[2].p);
-    transpose64(s->ctx, s->host_cols[2].p, s->host_cols[0].p, N, nrhs);
-    download(s->ctx, u, s->host_cols[0].p, n);
-    if (3 * n * sizeof(double) > kKeptScratch)
-        for (auto &b : s->host_cols) b.release();
+    DBuf<double> &a = s->host_cols[0], &b = s->host_cols[1];
+    struct GiveBack {
+        DBuf<double> &a, &b;
+        ~GiveBack()
+        {
+            if ((a.n + b.n) * sizeof(double) <= kKeptScratch) return;
+            a.release();
+            b.release();
+        }
+    } give_back{a, b};
+    upload(s->ctx, a, rhs, n);
+    b.reserve(n);
+    transpose64(s->ctx, a.p, b.p, nrhs, N);
+    solve(b.p, a.p);
+    transpose64(s->ctx, a.p, b.p, N, nrhs);
+    download(s->ctx, u, b.p, n);
 }
 
 void ensure_vectors(sfc_system *s)

@@ -519,7 +519,7 @@ struct sfc_system {
     // per launch configuration (block widths 32, 64, 128)
     sfc::GraphExec blk_graph[7];  // by row width and columns in use (32s)
     sfc::EventPair solve_ev;  // device time of the last solve call
-    sfc::DBuf<double> host_cols[3];  // host right-hand sides and solutions on the device
+    sfc::DBuf<double> host_cols[2];  // host right-hand sides and solutions on the device
     sfc::BtdPlan btd;         // direct solve of small-bandwidth systems
     // diagonal copy of the operator (pcg.cu): [offset][row], or
     // [offset][3 x 3][node] on 3-dof meshes, from the main diagonal up
