@@ -306,6 +306,17 @@ void perturbation_update(sfc_perturbation *pt, const sfc_hparams_t *hp, double m
     const double add = pt->reg * msigma;
     k_add_scaled2<<<grid_for(ns * ns, 256), 256, 0, ctx->stream>>>(pt->cov.p, fg->d_ppt.p, add * add, ns * ns);
     count_launch(ctx);
+    struct GiveBack {  // the workspaces stay up to kKeptScratch bytes
+        sfc_perturbation *pt;
+        ~GiveBack()
+        {
+            DBuf<double> *all[] = {&pt->factor, &pt->vals, &pt->Bt, &pt->Y, &pt->W, &pt->T, &pt->V, &pt->work};
+            size_t n = 0;
+            for (auto *b : all) n += b->n;
+            if (n * sizeof(double) > kKeptScratch)
+                for (auto *b : all) b->release();
+        }
+    } give_back{pt};
     // chunks of kc factor columns: kc * ns right-hand sides per block solve
     int64_t kcap = std::min<int64_t>(4096 / std::max<int64_t>(ns, 1), (int64_t)(64e6 / std::max<int64_t>(N * ns, 1)));
     if (!m->is_grid) kcap = std::min<int64_t>(kcap, 256 / std::max<int64_t>(ns, 1));  // dense kernel: <= 256 columns

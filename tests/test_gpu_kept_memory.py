@@ -44,3 +44,20 @@ def test_host_columns(ctx, call):
     assert before - free_bytes() <= 64 << 20
     s.close()
     gm.close()
+
+
+def test_material_workspaces(ctx):
+    """56 x 56 cells, chunks of 256 factor columns by 16 sensors: 106 MB an array, five of them."""
+    prob = statfem_problem(mg.TRI3_POISSON, 56, 16, seed=2)
+    g = gpu_prior(ctx, prob, HP, 1e-3, 1.0, api.SFC_SOLVER_PCG_MIXED, tol=1e-9)
+    pt = api.ForwardPerturbation(g["fg"])
+    hp = dict(HP, **{"material.sigma": 0.3, "material.length": 0.05})
+    before = free_bytes()
+    pt.updateSolution(hp, max_rank=300)
+    first = pt.giveProjectedCovarU()
+    assert before - free_bytes() <= 512 << 20  # what it keeps, and the solver's workspaces
+    pt.updateSolution(hp, max_rank=300)
+    assert np.abs(pt.giveProjectedCovarU() - first).max() <= 1e-10 * np.abs(first).max()
+    pt.close()
+    for k in ("fg", "cf", "s", "gm"):
+        g[k].close()
