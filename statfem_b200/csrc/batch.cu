@@ -1143,8 +1143,9 @@ int32_t sfc_batch_autotune(sfc_batch_t *b, int32_t remeasure, int32_t *cluster)
         for (int v = b->smax; v > 1; v >>= 1) ++smax_log;
         int nlog = 0;
         for (int v = b->n; v > 1; v >>= 1) ++nlog;
+        // the elimination and the iteration have kernels and costs of their own
         const std::string key = "batch:" + tune_device_key(b->ctx) + ":i" + std::to_string(nlog) + ":s" +
-                                std::to_string(smax_log);
+                                std::to_string(smax_log) + (batch_direct(b) ? ":direct" : "");
         std::string v;
         if (!remeasure && tune_lookup(key, v)) {
             batch_release_graph(b);
