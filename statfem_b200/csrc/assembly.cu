@@ -959,12 +959,8 @@ void assemble_load(sfc_ctx *ctx, const sfc_mesh *m, const double *f, double *F_d
         break;
     default: {
         DBuf<double> &sw = ctx->load_w;
-        const double *points = nullptr;
-        try {
-            sw.reserve(m->num_elems * m->quad.nq);
-            points = sw.p;
-        } catch (const Error &) {  // no room: every node computes its points
-        }
+        // without room every node computes its points
+        const double *points = reserve_spare(spare(sw, (size_t)m->num_elems * m->quad.nq)) ? sw.p : nullptr;
         if (points) {
             k_load_points<3, 8><<<grid_for(m->num_elems, 128), 128, 0, ctx->stream>>>(m->coords.p, m->conn.p, m->quad,
                                                                                     m->num_elems, sw.p);

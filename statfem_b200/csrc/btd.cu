@@ -804,12 +804,9 @@ bool btd_plan(sfc_ctx *ctx, BtdPlan &p, const int32_t *rp, const int32_t *col, i
     if (clusters == 0) return false;
     p.slots = keep_blocks ? 1 : std::min(clusters, n_inst);
     const int mp = (p.lmax + 7) & ~7;
-    try {
-        p.cols.reserve(N * (2 * kBtdSide + kBtdMid));
-        p.vals.reserve(N * (2 * kBtdSide + kBtdMid));
-        p.X.reserve((size_t)p.slots * xmax);
-        p.Y.reserve((size_t)p.slots * 2 * (p.lmax + 2 * PW) * mp);
-    } catch (const Error &) {  // no room: the iterative solver needs less
+    const size_t entries = N * (2 * kBtdSide + kBtdMid);
+    if (!reserve_spare(spare(p.cols, entries), spare(p.vals, entries), spare(p.X, (size_t)p.slots * xmax),
+                       spare(p.Y, (size_t)p.slots * 2 * (p.lmax + 2 * PW) * mp))) {  // the iterative solver needs less
         p.cols.release();
         p.vals.release();
         p.X.release();
@@ -976,12 +973,7 @@ bool btd_solve_system(sfc_system *s, const double *B, double *X, int nrhs, int l
     // a residual above tol: once more on it with the same factor, twice at most
     const size_t n = (size_t)s->N * nrhs;
     DBuf<double> R, D;
-    try {
-        R.alloc(n);
-        D.alloc(n);
-    } catch (const Error &) {
-        return false;
-    }
+    if (!reserve_spare(spare(R, n), spare(D, n))) return false;
     BtdArgs e = a;
     e.B = R.p;
     e.U = D.p;

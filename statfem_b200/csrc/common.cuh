@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "statfem_cuda.h"
@@ -84,6 +85,33 @@ struct DBuf {
     }
     T *get() const { return p; }
 };
+
+// Room for copies and factors that a call can do without: false where they
+// would take more than half of what is free, so that what cannot be done
+// without finds room after them.
+template <class... T>
+bool reserve_spare(std::pair<DBuf<T> &, size_t>... want)
+{
+    const size_t more = (((want.second > want.first.n) ? want.second * sizeof(T) : (size_t)0) + ... + (size_t)0);
+    if (more) {
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) != cudaSuccess || more > free / 2) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    try {
+        (want.first.reserve(want.second), ...);
+    } catch (const Error &) {
+        return false;
+    }
+    return true;
+}
+template <class T>
+std::pair<DBuf<T> &, size_t> spare(DBuf<T> &b, size_t count)
+{
+    return {b, count};
+}
 
 }  // namespace sfc
 

@@ -745,10 +745,8 @@ void build_lattice_blocks(sfc_system *s)
         s->bq64.alloc((size_t)s->nodes * NODE_FLOATS);
     } else {
         if (want == "lattice" || !numbered_lattice(s, nx, ny, nz)) return;
-        try {
-            s->bq.alloc((size_t)s->nodes * NODE_FLOATS);
-            s->bq64.alloc((size_t)s->nodes * NODE_FLOATS);
-        } catch (const Error &) {  // no room for the views: the node blocks do
+        const size_t view = (size_t)s->nodes * NODE_FLOATS;
+        if (!reserve_spare(spare(s->bq, view), spare(s->bq64, view))) {  // no room: the node blocks do
             s->bq.release();
             s->bq64.release();
             return;

@@ -2259,12 +2259,10 @@ FcgWhy fcg_run(sfc_mpnn *m, sfc_system *s, FcgRun &run)
             o.off[o.runs++] = first;
             while (d < s->dia_nd && s->dia_off[d] < first + 3) ++d;
         }
-        try {
-            m->win.reserve((size_t)o.runs * 3 * ((N + 3) / 4 * 4));
-            for (auto &h : m->hw) h.reserve((size_t)(N + 2 * margin) * H);
-        } catch (const Error &) {  // no room: the gather reads the rows
+        const size_t rows = (size_t)(N + 2 * margin) * H;
+        // without room the gather reads the rows
+        if (!reserve_spare(spare(m->win, (size_t)o.runs * 3 * ((N + 3) / 4 * 4)), spare(m->hw[0], rows), spare(m->hw[1], rows)))
             o.runs = 0;
-        }
     }
     if (o.runs) {
         k_fcg_window<<<grid_for(N, 256), 256, 0, ctx->stream>>>(o, s->row_ptr.p, s->col.p, m->ahat.p, N, m->win.p);

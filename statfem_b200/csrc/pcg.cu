@@ -425,9 +425,7 @@ bool dia_prepare(sfc_system *s)
     const bool block = s->has_bsr;
     const int64_t rows = block ? s->nodes : s->N;
     const int kept = s->dia_nd / 2 + 1;
-    try {
-        s->dia.reserve((size_t)kept * rows * (block ? 9 : 1));
-    } catch (const Error &) {  // no room for a second copy of the values
+    if (!reserve_spare(spare(s->dia, (size_t)kept * rows * (block ? 9 : 1)))) {  // no room for a second copy
         s->dia_nd = 0;
         return false;
     }
