@@ -1737,8 +1737,8 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             // r32 <- scaled true residual, x32 <- 0, p kept (restarted columns: p = z)
             init32(rz1, rr1);
         }
-        // FP64 fallback: S d = r_c (the column's true residual) by Jacobi-PCG
-        // to tol ||b_c|| / ||r_c||, then x_c += d
+        // FP64 fallback: S d = r_c (the column's true residual) by PCG to
+        // tol ||b_c|| / ||r_c||, then x_c += d
         bool any_fb = false;
         for (int c = 0; c < kb; ++c) {
             if (!fallback[c]) continue;
@@ -1746,11 +1746,14 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
             ++n_fallback;
             s->tmpN.reserve(N);
             s->tmpN2.reserve(N);
-            k_gather_cols<<<grid_for(N, 256), 256, 0, ctx->stream>>>(r64.p, K, c, 1, 1, N, s->tmpN.p);
-            count_launch(ctx);
             const double bn = std::sqrt(hb[c]), r = std::sqrt(rn[c]);
-            if (r > tol * bn) {
-                PcgStats pr = pcg64(s, s->tmpN.p, s->tmpN2.p, tol * bn / r, max_iter, two_any);
+            // a column that the FP32 iteration left further off than zero, or not finite, starts again there
+            const bool afresh = !(r <= bn);
+            if (afresh) SFC_CK(cudaMemset2DAsync(x64.p + c, K * 8, 0, 8, N, ctx->stream));
+            k_gather_cols<<<grid_for(N, 256), 256, 0, ctx->stream>>>(afresh ? b64.p : r64.p, K, c, 1, 1, N, s->tmpN.p);
+            count_launch(ctx);
+            if (afresh || r > tol * bn) {
+                PcgStats pr = pcg64(s, s->tmpN.p, s->tmpN2.p, afresh ? tol : tol * bn / r, max_iter, two_any);
                 if (!pr.converged) all_conv = false;
                 if (debug)
                     std::fprintf(stderr, "[sfc block %d] column %d: FP64 fallback from rel %.3e, %d iterations%s\n", c0,
@@ -1767,6 +1770,7 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
         for (int c = 0; c < kb; ++c) {
             const double bn = std::sqrt(hb[c]);
             if (bn > 0) worst = std::max(worst, std::sqrt(rn[c]) / bn);
+            if (!(rn[c] < INFINITY)) all_conv = false;
         }
         if (nactive > 0) {
             all_conv = false;
