@@ -828,8 +828,7 @@ __global__ void __launch_bounds__(256, 4) k_layer_tc(const int32_t *__restrict__
                                                      uint32_t *__restrict__ Hout, const float *__restrict__ P,
                                                      const float *__restrict__ x0, const float *__restrict__ sdinv,
                                                      const unsigned char *__restrict__ mask, const double *scal,
-                                                     double *__restrict__ z, const double *__restrict__ q,
-                                                     double *zq, int *err)
+                                                     double *__restrict__ z, int *err)
 {
     extern __shared__ __align__(1024) unsigned char tsm[];
     // the tile's rows, then W: the MMA's M = 128 reads on past `rows` into W,
@@ -875,7 +874,6 @@ __global__ void __launch_bounds__(256, 4) k_layer_tc(const int32_t *__restrict__
     const uint4 *Hin4 = reinterpret_cast<const uint4 *>(Hin);
     const int sub = lane >> 3, fl = lane & 7;
     uint32_t parity = 0;
-    double dot = 0.0;  // DECODE: this thread's share of z . q
     bool ok = !(*err), pending = false;  // pending: MMAs committed and not yet waited for
     // consecutive tiles to the CTAs that the first wave puts on one SM: they
     // share most of their neighbours' lines in L1
@@ -993,17 +991,8 @@ __global__ void __launch_bounds__(256, 4) k_layer_tc(const int32_t *__restrict__
             if (!half && mine) {
                 y += ypart[32 * quad + lane];
                 const double sc = sqrt(scal[0] / (double)N);
-                const double zi = sc * (double)sdinv[i] * (double)(mask[i] ? x0[i] : x0[i] + y + P[OFF_DB]);
-                z[i] = zi;
-                if (q) dot += zi * q[i];
+                z[i] = sc * (double)sdinv[i] * (double)(mask[i] ? x0[i] : x0[i] + y + P[OFF_DB]);
             }
-        }
-    }
-    if constexpr (DECODE) {
-        if (q && ok && !half) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-            if (lane == 0) atomicAdd(zq, dot);
         }
     }
     if (!ok && pending) {
@@ -2039,10 +2028,9 @@ double loss_grad(sfc_mpnn *m, const double *r, const double *e, double w)
 }
 
 // z = M(r) (device FP64 vectors): the inference kernels, no host
-// synchronisation.  With q, also *zq += z . q.  With `scaled`, scal[0] and ax0
-// already hold |D^-1/2 r|^2 and FP32(D^-1/2 r).
-void apply(sfc_mpnn *m, const double *r, double *z, const double *q = nullptr, double *zq = nullptr,
-           bool scaled = false)
+// synchronisation.  With `scaled`, scal[0] and ax0 already hold |D^-1/2 r|^2
+// and FP32(D^-1/2 r).
+void apply(sfc_mpnn *m, const double *r, double *z, bool scaled = false)
 {
     sfc_ctx *ctx = m->ctx;
     const sfc_system *s = m->op_sys;
@@ -2071,12 +2059,11 @@ void apply(sfc_mpnn *m, const double *r, double *z, const double *q = nullptr, d
             if (l + 1 < LAYERS)
                 k_layer_tc<false><<<gt, 256, tc_layer_smem(rows), ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N,
                                                                      rows, ctx->sm_count, hout, m->params.p, m->x0.p, m->sdinv.p,
-                                                                     s->mask.p, m->scal.p, nullptr, nullptr, nullptr,
-                                                                     m->tc_err.p);
+                                                                     s->mask.p, m->scal.p, nullptr, m->tc_err.p);
             else
                 k_layer_tc<true><<<gt, 256, tc_layer_smem(rows), ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N,
                                                                     rows, ctx->sm_count, nullptr, m->params.p, m->x0.p, m->sdinv.p,
-                                                                    s->mask.p, m->scal.p, z, q, zq, m->tc_err.p);
+                                                                    s->mask.p, m->scal.p, z, m->tc_err.p);
             count_launch(ctx);
         }
         return;
@@ -2094,10 +2081,6 @@ void apply(sfc_mpnn *m, const double *r, double *z, const double *q = nullptr, d
         else
             k_layer_inf<true><<<g, 128, 0, ctx->stream>>>(s->row_ptr.p, s->col.p, m->ahat.p, hin, W, b, N, nullptr,
                                                           m->params.p, m->x0.p, m->sdinv.p, s->mask.p, m->scal.p, z);
-        count_launch(ctx);
-    }
-    if (q) {
-        k_fdot<<<grid_for(N, 256, ctx->sm_count * 4), 256, 0, ctx->stream>>>(z, q, N, zq);
         count_launch(ctx);
     }
 }
@@ -2417,10 +2400,11 @@ void solve_forward_fcg(sfc_system *s)
         for (; it < max_iter; ++it) {
             k_fcg_update<<<g, 256, 0, ctx->stream>>>(s->X.p, r, p, q, N, pq + it, pr + it, rr + it + 1, m->sdinv.p,
                                                     m->ax0.p, m->scal.p, done, err);
-            apply(m, r, z, q, zq + it, true);
+            apply(m, r, z, true);
+            k_fdot<<<g, 256, 0, ctx->stream>>>(z, q, N, zq + it);
             k_fcg_pupdate<<<g, 256, 0, ctx->stream>>>(p, z, r, N, zq + it, pq + it, pr + it + 1, rr + it + 1, thr,
                                                       it + 1, m->scal.p, done, err);
-            count_launch(ctx, 2);
+            count_launch(ctx, 3);
             spmv_op64_dot(s, p, q, pq + it + 1, done);
             if ((it + 1) % check == 0 || it + 1 == max_iter) {
                 int hf[2];

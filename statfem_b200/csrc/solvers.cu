@@ -1947,7 +1947,6 @@ void solve_forward(sfc_system *s, bool direct)
     if (direct && solve_direct(s, b.p, s->X.p, 1, 1, true)) return;
     const auto &o = s->opt;
     const int max_iter = o.max_iter > 0 ? o.max_iter : 20000;
-    const int check = o.check_every > 0 ? o.check_every : 16;
     const double tol = o.tol > 0 ? o.tol : 1e-8;
     s->solve_ev.ensure();
     cudaEvent_t e0 = s->solve_ev.a, e1 = s->solve_ev.b;
@@ -1997,7 +1996,6 @@ void solve_block(sfc_system *s, const double *B, double *X, int nrhs, int ld)
             block_mixed<4>(s, B, X, nrhs, ld, st);
     } else {
         const int max_iter = o.max_iter > 0 ? o.max_iter : 20000;
-        const int check = o.check_every > 0 ? o.check_every : 16;
         const double tol = o.tol > 0 ? o.tol : 1e-8;
         s->tmpN.reserve(N);
         s->blk64.reserve(N);
