@@ -33,6 +33,14 @@ namespace {
 // takes it 10.3 us at 29 thousand (64 x 64 square; the grid 11.7) and 19.5 at
 // 230 thousand (181 x 181; the grid 13).
 constexpr double kClusterWork = 1e5;
+// The same for rows of indices (renumbered squares, us: 57 thousand 14.9, the
+// grid 8.8; 26 thousand 9.6), and from where those of 16 lanes go as launches,
+// shorter ones from twice as many (renumbered cubes: 0.77 million 16.4, as
+// launches 18; 2.5 million 32.5 and 28.5; 13.8 million 148 and 111; squares of
+// 2.5 million 31 and 38)
+constexpr double kClusterRows = 4e4, kLaunchRows = 2e6;
+
+enum { PQ, RZ, RR, CE, SUMS };  // p.q, r.z (the smoother's share), r.r, c.e
 
 // Adds the M values of the warp's lanes to c[M agg ..]: lanes of consecutive
 // nodes of one aggregate (a run of the lattice's line) are summed first.
@@ -221,7 +229,6 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
     Comm<CL> comm{g, sh};
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
     double rz, rr, none = 0.0;
-    enum { PQ, RZ, RR, CE, SUMS };
     update<PRE, true>(g, 0.0, g.c, rz, rr);
     if (!comm.template sum<2>(rz, rr, sum_slot(RZ, 0), sum_slot(RR, 0))) return;
     if (rr == 0.0) {
@@ -275,6 +282,84 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
         if (first && it == g.max_iter) g.out[0] = it;
     }
     if constexpr (CL) cg::this_cluster().sync();  // shared memory stays until the others have read it
+}
+
+// ---- the same as launches ---------------------------------------------------
+// For large matrices of rows of indices, whose product wants all the warps that
+// an SM can hold, in blocks that finish at their own pace: of an iteration's 82
+// us on 274,625 renumbered nodes of a cube the persistent kernel's product took
+// 70 and the wait for its last block 9; as a kernel of its own it takes 51.  The
+// sums' slots and what they hold are those of k_pcg64; kernel boundaries are its
+// barriers.  out[1] is set in iteration out[0] and stops every later one.
+__device__ void add_sums(double a, double b, double *sa, double *sb)
+{
+    __shared__ double sh[2][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    a = warp_total(a);
+    b = warp_total(b);
+    if (lane == 0) {
+        sh[0][warp] = a;
+        sh[1][warp] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[threadIdx.x][w];
+        double *to = threadIdx.x ? sb : sa;
+        if (to) atomicAdd(to, t);
+    }
+}
+
+template <int PRE, bool INIT>
+__global__ void __launch_bounds__(256) k_step_update(const __grid_constant__ PcgArgs g, int it)
+{
+    if (g.out[1] | g.out[2]) return;
+    double alpha = 0.0, rz, rr;
+    if (!INIT) {
+        const double pq = g.sums[sum_slot(PQ, it)];
+        if (!(pq > 0.0)) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) g.out[2] = 1;
+            return;
+        }
+        alpha = (g.sums[sum_slot(RZ, it)] + g.sums[sum_slot(CE, it)]) / pq;
+    }
+    const int to = INIT ? 0 : it + 1;
+    update<PRE, INIT>(g, alpha, g.c + (to & 1) * g.nc, rz, rr);
+    add_sums(rz, rr, g.sums + sum_slot(RZ, to), g.sums + sum_slot(RR, to));
+}
+
+// the coarse correction of slot `to`; clears the other restriction
+__global__ void __launch_bounds__(256) k_step_coarse(const __grid_constant__ PcgArgs g, int to)
+{
+    if (g.out[1] | g.out[2]) return;
+    __shared__ double rows[32];
+    const double ce = coarse_product(g, g.c + (to & 1) * g.nc, rows);
+    double *other = g.c + ((to + 1) & 1) * g.nc;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < g.nc; k += (int64_t)gridDim.x * blockDim.x) other[k] = 0.0;
+    add_sums(ce, 0.0, g.sums + sum_slot(CE, to), nullptr);
+}
+
+template <int PRE, bool INIT>
+__global__ void __launch_bounds__(256) k_step_direction(const __grid_constant__ PcgArgs g, int it, double thr)
+{
+    if (g.out[2] || (!INIT && g.out[1] && g.out[0] != it + 1)) return;
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (INIT) {
+        direction<PRE, true>(g, 0.0, 0.0);
+        return;
+    }
+    const double rz = g.sums[sum_slot(RZ, it)] + g.sums[sum_slot(CE, it)], alpha = rz / g.sums[sum_slot(PQ, it)];
+    if (g.sums[sum_slot(RR, it + 1)] <= thr) {
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x)
+            g.x[i] += alpha * g.p[i];
+        if (first) {
+            g.out[0] = it + 1;
+            g.out[1] = 1;
+        }
+        return;
+    }
+    direction<PRE, false>(g, alpha, (g.sums[sum_slot(RZ, it + 1)] + g.sums[sum_slot(CE, it + 1)]) / rz);
+    if (first) clear_slots<SUMS>(g.sums, it);
 }
 
 // y = S x by diagonals; dot += x.y; skipped when *done
@@ -466,6 +551,42 @@ PcgArgs operator_args(sfc_system *s, bool dia)
 
 using PcgKernel = void (*)(PcgArgs);
 
+template <int PRE>
+PcgStats pcg64_launches(sfc_system *s, const PcgArgs &g)
+{
+    sfc_ctx *ctx = s->ctx;
+    constexpr int kCheck = 16;
+    const unsigned grid = grid_for(g.N, 256, ctx->sm_count * 8), rows = grid_for(g.nc * 32, 256, ctx->sm_count * 8);
+    cudaStream_t st = ctx->stream;
+    auto coarse = [&](int to) {
+        if constexpr (PRE > 0) {
+            k_step_coarse<<<rows, 256, 0, st>>>(g, to);
+            count_launch(ctx);
+        }
+    };
+    k_step_update<PRE, true><<<grid, 256, 0, st>>>(g, 0);
+    coarse(0);
+    k_step_direction<PRE, true><<<grid, 256, 0, st>>>(g, 0, 0.0);
+    count_launch(ctx, 2);
+    double rr = 0.0;
+    download(ctx, &rr, g.sums + sum_slot(RR, 0), 1);
+    if (rr == 0.0) return {0, true};
+    const double thr = g.tol * g.tol * rr;
+    for (int it = 0; it < g.max_iter; ++it) {
+        spmv_op64_dot(s, g.p, g.q, g.sums + sum_slot(PQ, it), g.out + 1);
+        k_step_update<PRE, false><<<grid, 256, 0, st>>>(g, it);
+        coarse(it + 1);
+        k_step_direction<PRE, false><<<grid, 256, 0, st>>>(g, it, thr);
+        count_launch(ctx, 2);
+        if ((it + 1) % kCheck && it + 1 < g.max_iter) continue;
+        int h[3];
+        download(ctx, h, g.out, 3);
+        if (h[2]) fail(SFC_ERR_NOT_SPD, "PCG breakdown: p^T A p <= 0");
+        if (h[1]) return {h[0], true};
+    }
+    return {g.max_iter, false};
+}
+
 }  // namespace
 
 bool dia_spmv64(sfc_system *s, const double *x, double *y, double *dot, const int *done)
@@ -540,6 +661,14 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
     g.tol = tol;
     g.max_iter = max_iter;
     SFC_CK(cudaMemsetAsync(s->flags.p, 0, 4 * sizeof(int), ctx->stream));
+    if (f == CSR && (double)s->nnz > (g.lanes >= 16 ? 1 : 2) * kLaunchRows) {
+        constexpr size_t slots = SUMS * kSumRing;
+        s->scal.reserve(slots);
+        g.sums = s->scal.p;
+        SFC_CK(cudaMemsetAsync(g.sums, 0, slots * sizeof(double), ctx->stream));
+        ProfScope ps(ctx, "pcg64", 0.0);
+        return pre ? pcg64_launches<1>(s, g) : pcg64_launches<0>(s, g);
+    }
     // One cluster of up to 16 blocks while a thread has few rows: a barrier
     // takes it 1.0 us and a sum 1.5, the grid 1.6 and 2.5.
     static const PcgKernel table[2][4][3] = {
@@ -552,7 +681,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
          {k_pcg64<BSR, 0, true>, nullptr, k_pcg64<BSR, 2, true>},
          {k_pcg64<BDIA, 0, true>, nullptr, k_pcg64<BDIA, 2, true>}}};
     SFC_REQUIRE(table[0][f][pre], "no PCG kernel for this operator and preconditioner");
-    const int64_t threads = f == BSR ? s->nodes * 32 : f == CSR ? N * g.lanes : f == BDIA ? s->nodes : N;
+    const int64_t threads = f == BSR ? s->nodes * 32 : f == BDIA ? s->nodes : f == CSR ? N * g.lanes : N;
     const double work = f == BSR || f == BDIA ? (double)s->nblocks * 9 : (double)s->nnz;
     ProfScope ps(ctx, "pcg64", 0.0);
     cudaLaunchConfig_t cfg = {};
@@ -560,7 +689,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
     cfg.stream = ctx->stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    bool cluster = work <= kClusterWork;
+    bool cluster = work <= (f == CSR ? kClusterRows : kClusterWork);
     if (cluster) {
         unsigned blocks = 1;
         while (blocks < 16 && (int64_t)blocks * 512 < threads) blocks *= 2;
@@ -588,7 +717,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
         const unsigned block = threads <= 512 * sm ? 512 : (unsigned)std::min<int64_t>(1024, ((threads + sm - 1) / sm + 127) / 128 * 128);
         cfg.blockDim = dim3(block);
         cfg.gridDim = dim3(grid_for(threads, block, (int)sm * std::max(occ, 1)));
-        constexpr size_t slots = 4 * kSumRing;
+        constexpr size_t slots = SUMS * kSumRing;
         s->scal.reserve(slots);
         g.sums = s->scal.p;
         SFC_CK(cudaMemsetAsync(g.sums, 0, slots * sizeof(double), ctx->stream));

@@ -47,7 +47,7 @@ namespace {
 // slot of sum k in iteration it, and the clearing: by one thread of the grid,
 // behind the first barrier of iteration it (every block has then read what
 // iteration it - 1 and those before it added up)
-__device__ __forceinline__ int sum_slot(int k, int it) { return k * kSumRing + (it & (kSumRing - 1)); }
+__host__ __device__ __forceinline__ int sum_slot(int k, int it) { return k * kSumRing + (it & (kSumRing - 1)); }
 template <int SUMS>
 __device__ __forceinline__ void clear_slots(double *sums, int it)
 {
@@ -241,16 +241,50 @@ __device__ double product(const PcgArgs &g, const double *p, double *q)
             }
         }
     } else {
+        // two groups of rows at a time (row bounds, columns and operands of one are
+        // a chain of loads), the matrix past L1, which the operand may keep
+        constexpr int U = 2;
         const int G = g.lanes, per = 32 / G;
-        for (int64_t base = (t0 >> 5) * per; base < g.N; base += (nt >> 5) * per) {
-            const int64_t i = base + lane / G;
-            double s = 0.0;
-            if (i < g.N)
-                for (int32_t k = g.rp[i] + lane % G; k < g.rp[i + 1]; k += G) s += g.a[k] * p[g.col[k]];
-            for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
-            if (i < g.N && lane % G == 0) {
-                q[i] = s;
-                dot += p[i] * s;
+        const int64_t step = (nt >> 5) * per;
+        for (int64_t base = (t0 >> 5) * per; base < g.N; base += U * step) {
+            const int64_t i0 = base + lane / G;
+            int32_t k[U], e[U];
+            double s[U];
+            bool more = false;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int64_t i = i0 + u * step;
+                k[u] = i < g.N ? g.rp[i] + lane % G : 0;
+                e[u] = i < g.N ? g.rp[i + 1] : 0;
+                s[u] = 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) more |= k[u] < e[u];
+            while (more) {
+                int32_t c[U];
+                double a[U];
+                more = false;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    c[u] = k[u] < e[u] ? __ldcs(g.col + k[u]) : -1;
+                    a[u] = k[u] < e[u] ? __ldcs(g.a + k[u]) : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (c[u] >= 0) s[u] += a[u] * p[c[u]];
+                    k[u] += G;
+                    more |= k[u] < e[u];
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                for (int o = G / 2; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o, G);
+                const int64_t i = i0 + u * step;
+                if (i < g.N && lane % G == 0) {
+                    q[i] = s[u];
+                    dot += p[i] * s[u];
+                }
             }
         }
     }
