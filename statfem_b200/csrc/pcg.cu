@@ -635,7 +635,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
     const CoarseSpace &cs = s->coarse;
     const int pre = !two ? 0 : cs.dof == 1 ? 1 : 2;
     PcgArgs g{};
-    const Format f = grid_operator(s, g, pre == 2);
+    Format f = grid_operator(s, g, pre == 2);
     s->w64.reserve(3 * N);
     g.b = b;
     g.x = x;
@@ -671,18 +671,24 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
     }
     // One cluster of up to 16 blocks while a thread has few rows: a barrier
     // takes it 1.0 us and a sum 1.5, the grid 1.6 and 2.5.
-    static const PcgKernel table[2][4][3] = {
+    static const PcgKernel table[2][5][3] = {
         {{k_pcg64<CSR, 0, false>, k_pcg64<CSR, 1, false>, nullptr},
          {k_pcg64<DIA, 0, false>, k_pcg64<DIA, 1, false>, nullptr},
          {k_pcg64<BSR, 0, false>, nullptr, k_pcg64<BSR, 2, false>},
-         {k_pcg64<BDIA, 0, false>, nullptr, k_pcg64<BDIA, 2, false>}},
+         {k_pcg64<BDIA, 0, false>, nullptr, k_pcg64<BDIA, 2, false>},
+         {k_pcg64<BDIA8, 0, false>, nullptr, k_pcg64<BDIA8, 2, false>}},
         {{k_pcg64<CSR, 0, true>, k_pcg64<CSR, 1, true>, nullptr},
          {k_pcg64<DIA, 0, true>, k_pcg64<DIA, 1, true>, nullptr},
          {k_pcg64<BSR, 0, true>, nullptr, k_pcg64<BSR, 2, true>},
-         {k_pcg64<BDIA, 0, true>, nullptr, k_pcg64<BDIA, 2, true>}}};
+         {k_pcg64<BDIA, 0, true>, nullptr, k_pcg64<BDIA, 2, true>},
+         {k_pcg64<BDIA8, 0, true>, nullptr, k_pcg64<BDIA8, 2, true>}}};
+    // Eight lanes per node while that leaves every warp with one piece of work: a
+    // thread per node uses a tenth of the SMs at a few thousand nodes (an iteration
+    // on 1,331, 6,859 and 17,576 nodes: 22.9, 23.3, 23.7 us; 8.5, 10.2, 13.2 so).
+    if (f == BDIA && s->nodes * 8 <= 1024 * (int64_t)ctx->sm_count) f = BDIA8;
     SFC_REQUIRE(table[0][f][pre], "no PCG kernel for this operator and preconditioner");
-    const int64_t threads = f == BSR ? s->nodes * 32 : f == BDIA ? s->nodes : f == CSR ? N * g.lanes : N;
-    const double work = f == BSR || f == BDIA ? (double)s->nblocks * 9 : (double)s->nnz;
+    const int64_t threads = f == BSR ? s->nodes * 32 : f == BDIA8 ? s->nodes * 8 : f == BDIA ? s->nodes : f == CSR ? N * g.lanes : N;
+    const double work = f == BSR || f == BDIA || f == BDIA8 ? (double)s->nblocks * 9 : (double)s->nnz;
     ProfScope ps(ctx, "pcg64", 0.0);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr;
@@ -714,7 +720,8 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
         // blocks of 512 while they fit one to an SM, then one per SM of the
         // size that spreads the rows over all of them
         const int64_t sm = ctx->sm_count;
-        const unsigned block = threads <= 512 * sm ? 512 : (unsigned)std::min<int64_t>(1024, ((threads + sm - 1) / sm + 127) / 128 * 128);
+        const unsigned block = f == BDIA8 ? (unsigned)std::max<int64_t>(128, std::min<int64_t>(1024, ((threads + sm - 1) / sm + 127) / 128 * 128))
+                               : threads <= 512 * sm ? 512 : (unsigned)std::min<int64_t>(1024, ((threads + sm - 1) / sm + 127) / 128 * 128);
         cfg.blockDim = dim3(block);
         cfg.gridDim = dim3(grid_for(threads, block, (int)sm * std::max(occ, 1)));
         constexpr size_t slots = SUMS * kSumRing;

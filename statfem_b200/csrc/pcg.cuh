@@ -12,7 +12,8 @@ namespace sfc {
 namespace cg = cooperative_groups;
 
 constexpr int kDiaMax = 32;    // diagonals of the pattern
-enum Format { CSR = 0, DIA = 1, BSR = 2, BDIA = 3 };
+// BDIA8: block diagonals, eight lanes to a node
+enum Format { CSR = 0, DIA = 1, BSR = 2, BDIA = 3, BDIA8 = 4 };
 
 struct PcgArgs {
     int64_t N, nodes;          // dofs; nodes of a 3-dof mesh
@@ -166,6 +167,35 @@ __device__ __forceinline__ double dia_row(const double *a, const int *off, int n
     return s;
 }
 
+// s += block d of node at (below: its transpose) times x of node j
+__device__ __forceinline__ void bdia_block(const double *a, int64_t nodes, int d, int64_t at, int64_t j, bool below,
+                                           const double *x, double (&s)[3])
+{
+    double v[9], xv[3];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = a[((int64_t)d * 9 + k) * nodes + at];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) xv[k] = x[3 * j + k];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        s[r] += below ? v[r] * xv[0] + v[3 + r] * xv[1] + v[6 + r] * xv[2]
+                      : v[3 * r] * xv[0] + v[3 * r + 1] * xv[1] + v[3 * r + 2] * xv[2];
+}
+
+// share `sub` of eight of the three rows of node i
+__device__ __forceinline__ void bdia_share(const double *a, const int *off, int nd, int64_t nodes, int64_t i, int sub,
+                                           const double *x, double (&s)[3])
+{
+    if (sub == 0) bdia_block(a, nodes, 0, i, i, false, x, s);
+#pragma unroll 1
+    for (int b = sub + 1; b < 2 * nd; b += 8) {  // 1, 2: above and below on the first diagonal, and so on
+        if (b == 2 * nd - 1) break;
+        const int d = (b + 1) >> 1;
+        const int64_t j = b & 1 ? i + off[d] : i - off[d];
+        if (j >= 0 && j < nodes) bdia_block(a, nodes, d, b & 1 ? i : j, j, !(b & 1), x, s);
+    }
+}
+
 // the three rows of node i, a thread per node: the operand's three values
 // serve three rows (a thread per row read them three times and was bound by
 // its L1 wavefronts: 63 us for 48^3 elasticity)
@@ -173,24 +203,12 @@ __device__ __forceinline__ void bdia_node(const double *a, const int *off, int n
                                           const double *x, double (&s)[3])
 {
     s[0] = s[1] = s[2] = 0.0;
-    // block d of node at, times x of node j; below: the block's transpose
-    auto block = [&](int d, int64_t at, int64_t j, bool below) {
-        double v[9], xv[3];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) v[k] = a[((int64_t)d * 9 + k) * nodes + at];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) xv[k] = x[3 * j + k];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-            s[r] += below ? v[r] * xv[0] + v[3 + r] * xv[1] + v[6 + r] * xv[2]
-                          : v[3 * r] * xv[0] + v[3 * r + 1] * xv[1] + v[3 * r + 2] * xv[2];
-    };
-    block(0, i, i, false);
+    bdia_block(a, nodes, 0, i, i, false, x, s);
 #pragma unroll 1
     for (int d = 1; d < nd; ++d) {
         const int64_t up = i + off[d], dn = i - off[d];
-        if (up < nodes) block(d, i, up, false);
-        if (dn >= 0) block(d, dn, dn, true);
+        if (up < nodes) bdia_block(a, nodes, d, i, up, false, x, s);
+        if (dn >= 0) bdia_block(a, nodes, d, dn, dn, true, x, s);
     }
 }
 
@@ -206,6 +224,21 @@ __device__ double product(const PcgArgs &g, const double *p, double *q)
             const double s = dia_row(g.a, g.off, g.nd, g.N, i, p);
             q[i] = s;
             dot += p[i] * s;
+        }
+    } else if constexpr (F == BDIA8) {  // four nodes to a warp
+        for (int64_t base = (t0 >> 5) * 4; base < g.nodes; base += (nt >> 5) * 4) {
+            const int64_t i = base + (lane & 3);
+            double s[3] = {0.0, 0.0, 0.0};
+            if (i < g.nodes) bdia_share(g.a, g.off, g.nd, g.nodes, i, lane >> 2, p, s);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+                if (lane < 4 && i < g.nodes) {
+                    q[3 * i + k] = s[k];
+                    dot += p[3 * i + k] * s[k];
+                }
+            }
         }
     } else if constexpr (F == BDIA) {
         for (int64_t i = t0; i < g.nodes; i += nt) {
