@@ -720,6 +720,9 @@ static bool coarse_aggregate(sfc_system *s, int size)
                     nbr[(size_t)a * kSlots + (x % 3) + 3 * (y % 3) + 9 * (z % 3)] = b;
                 }
     }
+    int64_t runs = 0;  // of nodes of one aggregate
+    for (int64_t i = 0; i < nodes; ++i) runs += i == 0 || node_agg[i] != node_agg[i - 1];
+    cs.scattered = 4 * runs > nodes;
     cs.nagg = nagg;
     cs.dof = dof;
     cs.nodes = nodes;

@@ -348,6 +348,7 @@ struct CoarseSpace {
     int64_t nagg = 0, nc = 0;           // aggregates, coarse dofs
     int nb[3] = {1, 1, 1};              // boxes per axis
     int dropped = 0;                    // dependent coarse dofs left out of the inverse
+    bool scattered = false;             // an aggregate's nodes are not runs of the numbering
     DBuf<int32_t> node_agg;             // nodes
     DBuf<int32_t> agg_free;             // scalar meshes: node_agg, -1 on constrained nodes (per operator)
     DBuf<int32_t> agg_ptr, agg_nodes;   // aggregate -> its nodes

@@ -65,6 +65,47 @@ __device__ void restrict_add(double *c, int agg, double (&v)[M])
         for (int m = 0; m < M; ++m) atomicAdd(c + (int64_t)M * agg + m, v[m]);
 }
 
+// The restriction by the aggregates' own lists, as many warps to one as the grid
+// has: where the nodes of an aggregate are scattered over the numbering, an
+// atomic per node and mode queues up on its addresses (6,859 nodes, 27 aggregates
+// of six modes: an iteration 35.1 us, 27.1 with the lists and their barrier)
+template <int PRE>
+__device__ void restrict_lists(const PcgArgs &g, double *c)
+{
+    constexpr int M = PRE == 1 ? 1 : 6;
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5), per = max((int64_t)1, min((int64_t)16, warps / g.nagg));
+    for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < per * g.nagg; w += warps) {
+        const int64_t a = w / per;
+        const int32_t end = g.agg_ptr[a + 1];
+        double v[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m) v[m] = 0.0;
+        for (int32_t t = g.agg_ptr[a] + (int32_t)(w % per) * 32 + lane; t < end; t += (int32_t)per * 32) {
+            const int64_t n = g.agg_nodes[t];
+            if constexpr (PRE == 1) {
+                if (g.agg[n] >= 0) v[0] += g.r[n];
+            } else {
+                const float4 m = g.mode[n];
+                const int bits = (int)m.w;
+                const double r0 = bits & 1 ? 0.0 : g.r[3 * n], r1 = bits & 2 ? 0.0 : g.r[3 * n + 1],
+                             r2 = bits & 4 ? 0.0 : g.r[3 * n + 2];
+                v[0] += r0;
+                v[1] += r1;
+                v[2] += r2;
+                v[3] += (double)m.y * r2 - (double)m.z * r1;
+                v[4] += (double)m.z * r0 - (double)m.x * r2;
+                v[5] += (double)m.x * r1 - (double)m.y * r0;
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            v[m] = warp_total(v[m]);
+            if (lane == 0) atomicAdd(c + M * a + m, v[m]);
+        }
+    }
+}
+
 __device__ __forceinline__ void block_jacobi(const float *D, const double (&r)[3], double (&z)[3])
 {
 #pragma unroll
@@ -76,7 +117,7 @@ __device__ __forceinline__ void block_jacobi(const float *D, const double (&r)[3
 // two-level with nodal blocks and six rigid-body modes.  r -= alpha q (INIT:
 // r = b) with r.z (the Jacobi share) and r.r, and the restriction of r into c.
 // x += alpha p waits for the p update, which reads p anyway.
-template <int PRE, bool INIT>
+template <int PRE, bool INIT, bool LIST>
 __device__ void update(const PcgArgs &g, double alpha, double *c, double &rz, double &rr)
 {
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
@@ -102,7 +143,7 @@ __device__ void update(const PcgArgs &g, double alpha, double *c, double &rz, do
                 a = g.agg[i];
                 v[0] = a >= 0 ? ri : 0.0;
             }
-            restrict_add<1>(c, a, v);
+            if (!LIST) restrict_add<1>(c, a, v);
         }
     } else {
         for (int64_t base = t0 - (threadIdx.x & 31); base < g.nodes; base += nt) {
@@ -136,7 +177,7 @@ __device__ void update(const PcgArgs &g, double alpha, double *c, double &rz, do
                 v[4] = (double)m.z * rv[0] - (double)m.x * rv[2];
                 v[5] = (double)m.x * rv[1] - (double)m.y * rv[0];
             }
-            restrict_add<6>(c, a, v);
+            if (!LIST) restrict_add<6>(c, a, v);
         }
     }
 }
@@ -222,20 +263,25 @@ __device__ void direction(const PcgArgs &g, double alpha, double beta)
     }
 }
 
-template <int F, int PRE, bool CL>
+// LIST: the restriction by the aggregates' lists, a phase of its own
+template <int F, int PRE, bool CL, bool LIST = false>
 __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_constant__ PcgArgs g)
 {
     __shared__ CommShared sh;
     Comm<CL> comm{g, sh};
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
     double rz, rr, none = 0.0;
-    update<PRE, true>(g, 0.0, g.c, rz, rr);
+    update<PRE, true, LIST>(g, 0.0, g.c, rz, rr);
     if (!comm.template sum<2>(rz, rr, sum_slot(RZ, 0), sum_slot(RR, 0))) return;
     if (rr == 0.0) {
         for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x) g.x[i] = 0.0;
         if (first) g.out[1] = 1;
     } else {
         if constexpr (PRE > 0) {
+            if constexpr (LIST) {
+                restrict_lists<PRE>(g, g.c);
+                if (!comm.barrier()) return;
+            }
             double ce = coarse_product(g, g.c, sh.rows);
             if (!comm.template sum<1>(ce, none, sum_slot(CE, 0), 0)) return;
             rz += ce;
@@ -256,7 +302,7 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
             double *c = g.c + ((it + 1) & 1) * g.nc;
             const double alpha = rz / pq;
             double rzn;
-            update<PRE, false>(g, alpha, c, rzn, rr);
+            update<PRE, false, LIST>(g, alpha, c, rzn, rr);
             if (!comm.template sum<2>(rzn, rr, sum_slot(RZ, it + 1), sum_slot(RR, it + 1))) return;
             if (rr <= thr) {
                 for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x)
@@ -268,6 +314,10 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
                 break;
             }
             if constexpr (PRE > 0) {
+                if constexpr (LIST) {
+                    restrict_lists<PRE>(g, c);
+                    if (!comm.barrier()) return;
+                }
                 double ce = coarse_product(g, c, sh.rows);
                 double *other = g.c + (it & 1) * g.nc;
                 for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < g.nc; k += (int64_t)gridDim.x * blockDim.x)
@@ -310,7 +360,7 @@ __device__ void add_sums(double a, double b, double *sa, double *sb)
     }
 }
 
-template <int PRE, bool INIT>
+template <int PRE, bool INIT, bool LIST>
 __global__ void __launch_bounds__(256) k_step_update(const __grid_constant__ PcgArgs g, int it)
 {
     if (g.out[1] | g.out[2]) return;
@@ -324,7 +374,7 @@ __global__ void __launch_bounds__(256) k_step_update(const __grid_constant__ Pcg
         alpha = (g.sums[sum_slot(RZ, it)] + g.sums[sum_slot(CE, it)]) / pq;
     }
     const int to = INIT ? 0 : it + 1;
-    update<PRE, INIT>(g, alpha, g.c + (to & 1) * g.nc, rz, rr);
+    update<PRE, INIT, LIST>(g, alpha, g.c + (to & 1) * g.nc, rz, rr);
     add_sums(rz, rr, g.sums + sum_slot(RZ, to), g.sums + sum_slot(RR, to));
 }
 
@@ -337,6 +387,12 @@ __global__ void __launch_bounds__(256) k_step_coarse(const __grid_constant__ Pcg
     double *other = g.c + ((to + 1) & 1) * g.nc;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < g.nc; k += (int64_t)gridDim.x * blockDim.x) other[k] = 0.0;
     add_sums(ce, 0.0, g.sums + sum_slot(CE, to), nullptr);
+}
+
+__global__ void __launch_bounds__(256) k_step_restrict(const __grid_constant__ PcgArgs g, int to)
+{
+    if (g.out[1] | g.out[2]) return;
+    restrict_lists<1>(g, g.c + (to & 1) * g.nc);
 }
 
 template <int PRE, bool INIT>
@@ -551,7 +607,7 @@ PcgArgs operator_args(sfc_system *s, bool dia)
 
 using PcgKernel = void (*)(PcgArgs);
 
-template <int PRE>
+template <int PRE, bool LIST>
 PcgStats pcg64_launches(sfc_system *s, const PcgArgs &g)
 {
     sfc_ctx *ctx = s->ctx;
@@ -560,11 +616,12 @@ PcgStats pcg64_launches(sfc_system *s, const PcgArgs &g)
     cudaStream_t st = ctx->stream;
     auto coarse = [&](int to) {
         if constexpr (PRE > 0) {
+            if (LIST) k_step_restrict<<<grid, 256, 0, st>>>(g, to);
             k_step_coarse<<<rows, 256, 0, st>>>(g, to);
-            count_launch(ctx);
+            count_launch(ctx, LIST ? 2 : 1);
         }
     };
-    k_step_update<PRE, true><<<grid, 256, 0, st>>>(g, 0);
+    k_step_update<PRE, true, LIST><<<grid, 256, 0, st>>>(g, 0);
     coarse(0);
     k_step_direction<PRE, true><<<grid, 256, 0, st>>>(g, 0, 0.0);
     count_launch(ctx, 2);
@@ -574,7 +631,7 @@ PcgStats pcg64_launches(sfc_system *s, const PcgArgs &g)
     const double thr = g.tol * g.tol * rr;
     for (int it = 0; it < g.max_iter; ++it) {
         spmv_op64_dot(s, g.p, g.q, g.sums + sum_slot(PQ, it), g.out + 1);
-        k_step_update<PRE, false><<<grid, 256, 0, st>>>(g, it);
+        k_step_update<PRE, false, LIST><<<grid, 256, 0, st>>>(g, it);
         coarse(it + 1);
         k_step_direction<PRE, false><<<grid, 256, 0, st>>>(g, it, thr);
         count_launch(ctx, 2);
@@ -651,6 +708,9 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
         g.mode = cs.mode.p;
         g.ac = cs.a64.p;
         g.nc = cs.nc;
+        g.agg_ptr = cs.agg_ptr.p;
+        g.agg_nodes = cs.agg_nodes.p;
+        g.nagg = cs.nagg;
         g.c = s->coarse.c64.p;
         g.e = s->coarse.e64.p;
         SFC_CK(cudaMemsetAsync(g.c, 0, 2 * cs.nc * sizeof(double), ctx->stream));
@@ -667,26 +727,28 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
         g.sums = s->scal.p;
         SFC_CK(cudaMemsetAsync(g.sums, 0, slots * sizeof(double), ctx->stream));
         ProfScope ps(ctx, "pcg64", 0.0);
-        return pre ? pcg64_launches<1>(s, g) : pcg64_launches<0>(s, g);
+        return !pre ? pcg64_launches<0, false>(s, g) : cs.scattered ? pcg64_launches<1, true>(s, g) : pcg64_launches<1, false>(s, g);
     }
     // One cluster of up to 16 blocks while a thread has few rows: a barrier
     // takes it 1.0 us and a sum 1.5, the grid 1.6 and 2.5.
-    static const PcgKernel table[2][5][3] = {
-        {{k_pcg64<CSR, 0, false>, k_pcg64<CSR, 1, false>, nullptr},
-         {k_pcg64<DIA, 0, false>, k_pcg64<DIA, 1, false>, nullptr},
-         {k_pcg64<BSR, 0, false>, nullptr, k_pcg64<BSR, 2, false>},
-         {k_pcg64<BDIA, 0, false>, nullptr, k_pcg64<BDIA, 2, false>},
-         {k_pcg64<BDIA8, 0, false>, nullptr, k_pcg64<BDIA8, 2, false>}},
-        {{k_pcg64<CSR, 0, true>, k_pcg64<CSR, 1, true>, nullptr},
-         {k_pcg64<DIA, 0, true>, k_pcg64<DIA, 1, true>, nullptr},
-         {k_pcg64<BSR, 0, true>, nullptr, k_pcg64<BSR, 2, true>},
-         {k_pcg64<BDIA, 0, true>, nullptr, k_pcg64<BDIA, 2, true>},
-         {k_pcg64<BDIA8, 0, true>, nullptr, k_pcg64<BDIA8, 2, true>}}};
+    static const PcgKernel table[2][5][5] = {
+        {{k_pcg64<CSR, 0, false>, k_pcg64<CSR, 1, false>, nullptr, k_pcg64<CSR, 1, false, true>, nullptr},
+         {k_pcg64<DIA, 0, false>, k_pcg64<DIA, 1, false>, nullptr, nullptr, nullptr},
+         {k_pcg64<BSR, 0, false>, nullptr, k_pcg64<BSR, 2, false>, nullptr, k_pcg64<BSR, 2, false, true>},
+         {k_pcg64<BDIA, 0, false>, nullptr, k_pcg64<BDIA, 2, false>, nullptr, nullptr},
+         {k_pcg64<BDIA8, 0, false>, nullptr, k_pcg64<BDIA8, 2, false>, nullptr, nullptr}},
+        {{k_pcg64<CSR, 0, true>, k_pcg64<CSR, 1, true>, nullptr, k_pcg64<CSR, 1, true, true>, nullptr},
+         {k_pcg64<DIA, 0, true>, k_pcg64<DIA, 1, true>, nullptr, nullptr, nullptr},
+         {k_pcg64<BSR, 0, true>, nullptr, k_pcg64<BSR, 2, true>, nullptr, k_pcg64<BSR, 2, true, true>},
+         {k_pcg64<BDIA, 0, true>, nullptr, k_pcg64<BDIA, 2, true>, nullptr, nullptr},
+         {k_pcg64<BDIA8, 0, true>, nullptr, k_pcg64<BDIA8, 2, true>, nullptr, nullptr}}};
     // Eight lanes per node while that leaves every warp with one piece of work: a
     // thread per node uses a tenth of the SMs at a few thousand nodes (an iteration
     // on 1,331, 6,859 and 17,576 nodes: 22.9, 23.3, 23.7 us; 8.5, 10.2, 13.2 so).
     if (f == BDIA && s->nodes * 8 <= 1024 * (int64_t)ctx->sm_count) f = BDIA8;
-    SFC_REQUIRE(table[0][f][pre], "no PCG kernel for this operator and preconditioner");
+    // the aggregates' lists where their nodes are scattered (and so no diagonals)
+    const int form = pre && cs.scattered && (f == CSR || f == BSR) ? pre + 2 : pre;
+    SFC_REQUIRE(table[0][f][form], "no PCG kernel for this operator and preconditioner");
     const int64_t threads = f == BSR ? s->nodes * 32 : f == BDIA8 ? s->nodes * 8 : f == BDIA ? s->nodes : f == CSR ? N * g.lanes : N;
     const double work = f == BSR || f == BDIA || f == BDIA8 ? (double)s->nblocks * 9 : (double)s->nnz;
     ProfScope ps(ctx, "pcg64", 0.0);
@@ -699,7 +761,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
     if (cluster) {
         unsigned blocks = 1;
         while (blocks < 16 && (int64_t)blocks * 512 < threads) blocks *= 2;
-        const PcgKernel kernel = table[1][f][pre];
+        const PcgKernel kernel = table[1][f][form];
         SFC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = blocks;
@@ -712,7 +774,7 @@ PcgStats pcg64(sfc_system *s, const double *b, double *x, double tol, int max_it
         else cudaGetLastError();
     }
     if (!cluster) {
-        const PcgKernel kernel = table[0][f][pre];
+        const PcgKernel kernel = table[0][f][form];
         int occ = 0;
         SFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 1024, 0));
         attr.id = cudaLaunchAttributeCooperative;

@@ -31,6 +31,9 @@ struct PcgArgs {
     const double *ac;          // nc x nc inverse
     int64_t nc;
     double *c, *e;             // [2][nc], [nc]
+    // nodes by aggregate, where the numbering scatters those of an aggregate
+    const int32_t *agg_ptr, *agg_nodes;
+    int64_t nagg;
     double *sums;              // [sum][kSumRing]: slots of the sums, zero at the start
     unsigned *bar;
     double tol;
