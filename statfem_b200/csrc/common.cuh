@@ -385,17 +385,6 @@ __device__ __forceinline__ void ldv(const float *p, float (&v)[V])
         v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
     }
 }
-// the same, zeros without `live`
-template <int V>
-__device__ __forceinline__ void ldv_if(bool live, const float *p, float (&v)[V])
-{
-    if (live) {
-        ldv<V>(p, v);
-    } else {
-#pragma unroll
-        for (int k = 0; k < V; ++k) v[k] = 0.f;
-    }
-}
 template <int V>
 __device__ __forceinline__ void stv(float *p, const float (&v)[V])
 {
