@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256) k_spmm32(const int32_t *__restrict__ rp, 
 // three P rows (3*K contiguous floats) once and updates all three output rows,
 // so every gathered row of P feeds three rows of Q.
 template <int V>
-__global__ void __launch_bounds__(256) k_bspmm32(const int32_t *__restrict__ bptr, const int32_t *__restrict__ bcol,
+__global__ void __launch_bounds__(256, V == 1 ? 8 : V == 2 ? 5 : 4) k_bspmm32(const int32_t *__restrict__ bptr, const int32_t *__restrict__ bcol,
                                                  const float *__restrict__ bval, const float *__restrict__ P,
                                                  float *__restrict__ Q, int64_t nodes, double *pq, const double *thr,
                                                  const int *stop)
@@ -649,7 +649,7 @@ __device__ void iteration_end(const IterEnd &e)
 
 // p = D^-1 r + beta p for active columns (rr' > thr)
 template <int V>
-__global__ void __launch_bounds__(256) k_bpupdate32(float *__restrict__ p, const float *__restrict__ r,
+__global__ void __launch_bounds__(256, V == 1 ? 8 : V == 2 ? 6 : 5) k_bpupdate32(float *__restrict__ p, const float *__restrict__ r,
                                                     const float *__restrict__ dinv, int64_t N, const double *rz,
                                                     const double *rz_next, const double *rr_next, const double *thr,
                                                     const int *stop, const int *brk, IterEnd end_of)
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(256) k_bpupdate32(float *__restrict__ p, const
 // scalar two-level p update: z = D^-1 r + e[agg(i)] (0 on constrained dofs),
 // p = z + beta p for the active columns (INIT: p = z for the restarted ones)
 template <int V, bool INIT>
-__global__ void __launch_bounds__(256) k_cbpupdate32(float *__restrict__ p, const float *__restrict__ r,
+__global__ void __launch_bounds__(256, V == 1 ? 8 : V == 2 ? 6 : 5) k_cbpupdate32(float *__restrict__ p, const float *__restrict__ r,
                                                      const float *__restrict__ dinv,
                                                      const int32_t *__restrict__ node_agg,
                                                      const float4 *__restrict__ mode, const float *__restrict__ e,
@@ -1040,7 +1040,7 @@ __global__ void __launch_bounds__(256) k_npupdate32(float *__restrict__ p, const
 // columns.  INIT: p = z for the restarted columns, others keep p.
 // (four 256-thread CTAs per SM: at most 64 registers)
 template <int V, bool INIT>
-__global__ void __launch_bounds__(256, 4) k_ncpupdate32(float *__restrict__ p, const float *__restrict__ r,
+__global__ void __launch_bounds__(256, V == 1 ? 5 : 4) k_ncpupdate32(float *__restrict__ p, const float *__restrict__ r,
                                                      const float *__restrict__ bdinv,
                                                      const int32_t *__restrict__ node_agg,
                                                      const float4 *__restrict__ mode, const float *__restrict__ e,
@@ -1370,17 +1370,24 @@ void block_mixed(sfc_system *s, const double *B, double *X, int nrhs, int ld, sf
     // block without a row
     const unsigned gw = (grid_for((bsr ? s->nodes : N) * 32, 256, ctx->sm_count * 8) + kColCluster - 1) / kColCluster *
                         kColCluster;
-    // The updates start, and add up their columns, once per CTA: r updates two
-    // to an SM, p updates (no sums) four, which is one wave.  52,728 dofs, 40
-    // columns, us with 8, 4, 2: r update 18.4, 16.4, 13.7, p update 16.8, 16.3,
-    // 20.8; 151,959 dofs, 128 columns, r update with 6, 4, 2: 49, 54, 46.
-    const unsigned gu = std::min<unsigned>(gw, (unsigned)ctx->sm_count / 4 * kColCluster),
-                   gp = std::min<unsigned>(gw, (unsigned)ctx->sm_count * 4);
     const bool two_any = use_two_level(s);
     const CoarseSpace &crs = s->coarse;
     const bool two = two_any && crs.dof == 3;   // block Jacobi + rigid-body modes
     const bool two1 = two_any && crs.dof == 1;  // point Jacobi + constant modes (scalar mesh)
     const bool bj = bsr && (o.precond == SFC_PRECOND_BLOCK_JACOBI || two) && s->bdinv32.p;
+    // CTAs of the updates.  The r updates add up their columns once per CTA, so
+    // a CTA wants work enough: three to an SM for node blocks; for rows of 32,
+    // 64 and 128 columns up to six, five and four, but eight rows of 128 columns
+    // (or as much) to a warp.  The p updates (no sums) take four, and eight
+    // where a row is only 128 bytes.  us per iteration with r updates of 2, 3,
+    // 4, 5, 6, 8: 491,401 rows, 64 columns 617, 429, 397, 383, 441, 405, 128
+    // columns -, 706, 683, 754, 722, 692; 22,801 rows, 128 columns 41, 51, 51, -,
+    // 58, 57; 117,649 nodes, 128 columns 472, 470, 489, -, 476, 488; p updates of
+    // 4 and 8 there with 32 columns 214, 194.
+    const int64_t sm = ctx->sm_count;
+    const int64_t r_ctas = bj ? 3 : std::max<int64_t>(2, std::min<int64_t>(K == 32 ? 6 : K == 64 ? 5 : 4, N / (sm * 8 * 8 * K / 128)));
+    const unsigned gu = std::min<unsigned>(gw, (unsigned)(sm * r_ctas / kColCluster * kColCluster)),
+                   gp = std::min<unsigned>(gw, (unsigned)(sm * (K == 32 ? 8 : 4)));
     // two-level with block Jacobi: the r update and the coarse restriction in
     // one pass over r (SFC_RESTRICT=separate keeps the two kernels)
     const char *fenv = std::getenv("SFC_RESTRICT");
