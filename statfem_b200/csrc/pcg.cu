@@ -289,11 +289,14 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
         direction<PRE, true>(g, 0.0, 0.0);
         if (!comm.barrier()) return;
         const double thr = g.tol * g.tol * rr;
-        int it = 0;
+        // `at` is it mod kSumRing, counted: with the slots by it & 3 the same loop
+        // took 15.3 us instead of 13.0 on 33,124 rows
+        int it = 0, at = 0;
         for (; it < g.max_iter; ++it) {
+            const int nx = at == kSumRing - 1 ? 0 : at + 1;
             double pq = product<F>(g, g.p, g.q);
-            if (!comm.template sum<1>(pq, none, sum_slot(PQ, it), 0)) return;
-            if (!CL && first) clear_slots<SUMS>(g.sums, it);
+            if (!comm.template sum<1>(pq, none, ring_slot(PQ, at), 0)) return;
+            if (!CL && first) clear_slots<SUMS>(g.sums, at);
             if (!(pq > 0.0)) {
                 if (first) g.out[2] = 1;
                 break;
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
             const double alpha = rz / pq;
             double rzn;
             update<PRE, false, LIST>(g, alpha, c, rzn, rr);
-            if (!comm.template sum<2>(rzn, rr, sum_slot(RZ, it + 1), sum_slot(RR, it + 1))) return;
+            if (!comm.template sum<2>(rzn, rr, ring_slot(RZ, nx), ring_slot(RR, nx))) return;
             if (rr <= thr) {
                 for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x)
                     g.x[i] += alpha * g.p[i];
@@ -322,11 +325,12 @@ __global__ void __launch_bounds__(CL ? 512 : 1024, 1) k_pcg64(const __grid_const
                 double *other = g.c + (it & 1) * g.nc;
                 for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < g.nc; k += (int64_t)gridDim.x * blockDim.x)
                     other[k] = 0.0;
-                if (!comm.template sum<1>(ce, none, sum_slot(CE, it + 1), 0)) return;
+                if (!comm.template sum<1>(ce, none, ring_slot(CE, nx), 0)) return;
                 rzn += ce;
             }
             direction<PRE, false>(g, alpha, rzn / rz);
             rz = rzn;
+            at = nx;
             if (!comm.barrier()) return;
         }
         if (first && it == g.max_iter) g.out[0] = it;

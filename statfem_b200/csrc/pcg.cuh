@@ -51,7 +51,8 @@ namespace {
 // slot of sum k in iteration it, and the clearing: by one thread of the grid,
 // behind the first barrier of iteration it (every block has then read what
 // iteration it - 1 and those before it added up)
-__host__ __device__ __forceinline__ int sum_slot(int k, int it) { return k * kSumRing + (it & (kSumRing - 1)); }
+__host__ __device__ __forceinline__ int ring_slot(int k, int at) { return k * kSumRing + at; }
+__host__ __device__ __forceinline__ int sum_slot(int k, int it) { return ring_slot(k, it & (kSumRing - 1)); }
 template <int SUMS>
 __device__ __forceinline__ void clear_slots(double *sums, int it)
 {
