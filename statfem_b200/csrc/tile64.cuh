@@ -13,8 +13,12 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// The range of recip: d positive, d and 1 / d normal numbers
-__device__ __forceinline__ bool recip_takes(double d) { return d >= 0x1p-1022 && d <= 0x1p1022; }
+// The range of recip: d positive and below 2^1022, d and 1 / d normal numbers,
+// by the exponent (as FP64 comparisons a block elimination took 4 % longer)
+__device__ __forceinline__ bool recip_takes(double d)
+{
+    return (unsigned)__double2hiint(d) - 0x00100000u < 0x7fc00000u;
+}
 
 // 1 / d by Newton's iteration on the hardware's approximation (about 20 bits;
 // two steps reach rounding), which flushes subnormal numbers, its own result
