@@ -4,14 +4,13 @@
 //     A[i,j] <- A[i,j] - A[i,k] D^-1 A[k,j]
 // for 32-wide panels k (D the panel's diagonal block), one launch per panel: a
 // tile's own values are read and written by one CTA, and the panel's rows and
-// columns, which the others read, were copied by the launch before.  Used for the coarse matrix of the two-level preconditioner (with
-// dependent pivots dropped: a generalised inverse on the independent modes)
-// and for the sensor-space matrices of the KOH likelihood and posterior
+// columns, which the others read, were copied by the launch before.  Used for
+// the coarse matrix of the two-level preconditioner (with dependent pivots
+// dropped: a generalised inverse on the independent modes) and for the
+// sensor-space matrices of the KOH likelihood and posterior
 // (LikelihoodKOH.ipp:75-120, 311-361), where a non-positive pivot is the
 // reference's failed LLT.  The Schur-complement pivots are the squared
 // diagonal of the Cholesky factor, so their logarithms sum to log det A.
-
-#include <algorithm>
 
 #include <algorithm>
 
@@ -25,31 +24,47 @@ namespace {
 constexpr int kGJ = 32;     // panel width
 constexpr int kGjTile = 64; // tile of A per CTA
 
-// Inverse of the kb x kb symmetric block in D (row stride LD) by the first
-// four warps (sweep_inverse), written to out (32 x 32, zero outside).  A pivot
-// not above rel x the dof's original diagonal (thr) is dropped: its row and
-// column are zeroed.  buf: 2 x 32.
-template <int LD>
-__device__ void gj_block_inverse(const double *D, int kb, const double *thr, double *buf, double *out, int *dropped,
-                                 double *pivots)
+// The sweep of gj_block_inverse, with 1 / d by recip or by division; returns
+// whether every pivot taken was in recip's range (the same in all threads)
+template <int LD, bool DIVIDE>
+__device__ __forceinline__ bool gj_sweep(const double *D, int kb, const double *thr, double *buf, double (&v)[8],
+                                         int &ndrop, double *pivots)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int r = 8 * warp + i;
         v[i] = r < kb && lane < kb ? D[r * LD + lane] : (r == lane ? 1.0 : 0.0);
     }
-    int ndrop = 0;
+    bool ok = true;
+    ndrop = 0;
     sweep_inverse(v, kGJ, buf, [&](int k, double d, double &inv) {
         const bool drop = k < kb && !(d > thr[k]);
         if (threadIdx.x == 0 && k < kb) {
             if (pivots) pivots[k] = d;
             ndrop += drop;
         }
-        if (!drop) inv = recip_takes(d) ? recip(d) : 1.0 / d;
+        ok = ok && (drop || recip_takes(d));
+        if (!drop) inv = DIVIDE ? 1.0 / d : recip(d);
         return !drop;
     });
+    return ok;
+}
+
+// Inverse of the kb x kb symmetric block in D (row stride LD) by the first
+// four warps (sweep_inverse), written to out (32 x 32, zero outside).  A pivot
+// not above rel x the dof's original diagonal (thr) is dropped: its row and
+// column are zeroed.  A block with a pivot outside recip's range is swept again,
+// with divisions (with the choice at each pivot a step of 1,000 x 1,000 took
+// 17.2 us, 16.2 so).  buf: 2 x 32.
+template <int LD>
+__device__ void gj_block_inverse(const double *D, int kb, const double *thr, double *buf, double *out, int *dropped,
+                                 double *pivots)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[8];
+    int ndrop;
+    if (!gj_sweep<LD, false>(D, kb, thr, buf, v, ndrop, pivots)) gj_sweep<LD, true>(D, kb, thr, buf, v, ndrop, pivots);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int r = 8 * warp + i;
@@ -94,9 +109,10 @@ __global__ void __launch_bounds__(256) k_gj_first(const double *__restrict__ A, 
 //   columns of the panel:  A[i][j] = -colp[i] r[:, j]
 //   elsewhere:             A[i][j] -= colp[i] r[:, j]
 // on FP64 matrix instructions, every CTA forming the r of its columns itself
-// and copying what it has of the next panel's rows and columns.  The first CTA takes the tile with the next panel's diagonal block
-// and inverts that too, while the others are at their products: the chain
-// from panel to panel is a launch, a tile and an inverse of 3 us.  1,000 x
+// and copying what it has of the next panel's rows and columns.  The first CTA
+// takes the tile with the next panel's diagonal block and inverts that too,
+// while the others are at their products: the chain from panel to panel is a
+// launch, a tile and an inverse of 3 us.  1,000 x
 // 1,000: 468 us; 1,202 as two launches per panel, the inverse (with a barrier
 // of the whole CTA and a division per pivot) before the panel's products.
 __global__ void __launch_bounds__(256) k_gj_step(double *__restrict__ A, int64_t n, int64_t k0, int kb,
