@@ -56,7 +56,7 @@ __device__ __forceinline__ bool gj_sweep(const double *D, int kb, const double *
 // not above rel x the dof's original diagonal (thr) is dropped: its row and
 // column are zeroed.  A block with a pivot outside recip's range is swept again,
 // with divisions (with the choice at each pivot a step of 1,000 x 1,000 took
-// 17.2 us, 16.2 so).  buf: 2 x 32.
+// 17.2 us, 16.3 so).  buf: 2 x 32.
 template <int LD>
 __device__ void gj_block_inverse(const double *D, int kb, const double *thr, double *buf, double *out, int *dropped,
                                  double *pivots)
