@@ -100,9 +100,10 @@ typedef struct sfc_solver_options {
 
 typedef struct sfc_solve_stats {
     int32_t iterations;       /* max over right-hand sides, inner iterations
-                                 (0: solved by block elimination, the solves
-                                 inside the statX objects on small-bandwidth
-                                 meshes)                                      */
+                                 (0: solved by block elimination, which the
+                                 statX objects' own solves take on meshes of
+                                 small bandwidth where it is estimated to be
+                                 faster)                                      */
     int32_t refinements;      /* FP64 refinement cycles (mixed solver)         */
     int32_t num_rhs;
     int32_t converged;        /* 1 when every RHS met tol (the FP64 methods: by
@@ -463,8 +464,8 @@ int32_t sfc_system_set_mpnn(sfc_system_t *sys, sfc_mpnn_t *net);
  * instance to the relative residual tol (FP64 block elimination along the
  * grid lines where the mesh couples neighbouring lines only and max_iter is
  * at least 32 per line; FP32 block PCG with FP64 residual refinement
- * otherwise, or where the elimination misses tol), forms mean and C_s at the
- * sensors (C_s with the Kronecker-factored forcing covariance) and evaluates
+ * otherwise, or where the elimination misses tol or meets a pivot that is not
+ * positive), forms mean and C_s at the sensors (C_s with the Kronecker-factored forcing covariance) and evaluates
  * the log-likelihood and the posterior mean / covariance at the sensors in
  * FP64.  Per-instance status: SFC_OK, SFC_ERR_NOT_CONVERGED or
  * SFC_ERR_NOT_SPD (breakdown, NaN, Cholesky failure); a failing instance
