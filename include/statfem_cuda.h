@@ -465,9 +465,9 @@ int32_t sfc_system_set_mpnn(sfc_system_t *sys, sfc_mpnn_t *net);
  * grid lines where the mesh couples neighbouring lines only and max_iter is
  * at least 32 per line; FP32 block PCG with FP64 residual refinement
  * otherwise, or where the elimination misses tol or meets a pivot that is not
- * positive), forms mean and C_s at the sensors (C_s with the Kronecker-factored forcing covariance) and evaluates
- * the log-likelihood and the posterior mean / covariance at the sensors in
- * FP64.  Per-instance status: SFC_OK, SFC_ERR_NOT_CONVERGED or
+ * positive), forms mean and C_s at the sensors (C_s with the
+ * Kronecker-factored forcing covariance) and evaluates the log-likelihood and
+ * the posterior mean / covariance at the sensors in FP64.  Per-instance status: SFC_OK, SFC_ERR_NOT_CONVERGED or
  * SFC_ERR_NOT_SPD (breakdown, NaN, Cholesky failure); a failing instance
  * does not stop the others. */
 typedef struct sfc_batch sfc_batch_t;
